@@ -9,8 +9,8 @@ files, unchanged and from where they lie in the read-only project checkout,
 for sm_100a, each together with a few lines of ``extern "C"`` glue from
 ``ref_glue/`` (ours), into ``oracle/_ref/*.so``.  Nothing is copied out of the
 project tree; only the built objects land in ``oracle/_ref/`` (git-ignored).
-It is a no-op when the checkout or nvcc is absent (e.g. on a GPU box, where the
-prebuilt objects are used).
+It is a no-op when the checkout (or a source file of it) or nvcc is absent (e.g. on a
+GPU box, where the prebuilt objects are used).
 """
 from __future__ import annotations
 
@@ -52,7 +52,8 @@ _REF_TARGETS = [
 
 def build_ref(force: bool = False) -> list[str]:
     """Compile the project's CUDA WKV kernels for sm_100a into oracle/_ref/."""
-    if not os.path.isdir(REF_ROOT) or shutil.which("nvcc") is None:
+    have = all(os.path.isfile(os.path.join(REF_ROOT, t[1])) for t in _REF_TARGETS)
+    if not have or shutil.which("nvcc") is None:
         return [os.path.join(REF_DIR, t[0]) for t in _REF_TARGETS
                 if os.path.exists(os.path.join(REF_DIR, t[0]))]
     import torch
