@@ -6,6 +6,7 @@ no PyTorch or CPU fallback behind any op of this package.
 from __future__ import annotations
 
 import ctypes
+import importlib.util
 import os
 
 import torch
@@ -52,6 +53,26 @@ EXPORTS = [
 ]
 
 _lib = None
+_native = None
+
+
+def native():
+    """The PyTorch binding (``_native.so``, csrc/native_*.cpp): argument checks, allocation and the
+    autograd nodes of the ops, on top of libwkv_b200.so."""
+    global _native
+    if _native is None:
+        load()
+        path = _build.NATIVE
+        if not _build.native_is_current():
+            if _build.have_nvcc():
+                path = _build.build_native()
+            elif not os.path.exists(path):
+                raise ImportError(f"{path} is missing and there is no compiler to build it")
+        spec = importlib.util.spec_from_file_location(_build.NATIVE_NAME, path)
+        mod = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(mod)
+        _native = mod
+    return _native
 
 
 def load() -> ctypes.CDLL:

@@ -1,0 +1,422 @@
+// PyTorch binding of the WKV ops: argument checks, output and workspace allocation, autograd nodes.
+// All of it is host work on the way to the C ABI; it is native because a call of the op is a handful of
+// microsecond kernels when heads, tokens or batch are few, and the same steps in Python take hundreds of
+// microseconds (v6, 5 heads, 4096-token segments: 284 us per call in Python, of which the GPU was busy 56).
+#include "native_common.h"
+
+namespace wkv_native {
+
+// ------------------------------------------------------------------------------ status words
+namespace {
+constexpr int MAX_DEVICES = 64;
+std::atomic<int *> g_status[MAX_DEVICES];
+std::mutex g_status_lock;
+
+void raise_if_set(int device, int *word) {
+    const int code = *reinterpret_cast<volatile int *>(word);
+    if (code == 0) return;
+    *reinterpret_cast<volatile int *>(word) = 0;      // reported once
+    TORCH_CHECK(false, "a v5/v6 call on cuda:", device, ": a device-side wait ran out (status ", code,
+                "); the outputs of that call are invalid");
+}
+}  // namespace
+
+int *status_word(int device) {
+    TORCH_CHECK(device >= 0 && device < MAX_DEVICES, "device index out of range");
+    int *p = g_status[device].load(std::memory_order_acquire);
+    if (p == nullptr) {
+        std::lock_guard<std::mutex> hold(g_status_lock);
+        p = g_status[device].load(std::memory_order_acquire);
+        if (p == nullptr) {
+            // a cache line per device, kept for the life of the process
+            C10_CUDA_CHECK(cudaHostAlloc((void **)&p, 128, cudaHostAllocPortable | cudaHostAllocMapped));
+            *p = 0;
+            g_status[device].store(p, std::memory_order_release);
+        }
+    }
+    return p;
+}
+
+void poll_status(int device, bool wait) {
+    for (int d = 0; d < MAX_DEVICES; d++) {
+        int *p = g_status[d].load(std::memory_order_acquire);
+        if ((device >= 0 && d != device) || p == nullptr) continue;
+        if (wait) {
+            c10::cuda::CUDAGuard guard(d);
+            C10_CUDA_CHECK(cudaDeviceSynchronize());
+        }
+        raise_if_set(d, p);
+    }
+}
+
+// ------------------------------------------------------------------------------ v5 / v6 calls
+namespace {
+
+wkv_args_t make_args(const Tensor &r, int w_kind, int layout, int path, int time_groups) {
+    wkv_args_t a = {};
+    a.B = (int)r.size(0); a.T = (int)r.size(1); a.H = (int)(r.size(2) / HEAD); a.N = (int)HEAD;
+    a.dtype = dtype_code(r.scalar_type());
+    a.w_kind = w_kind; a.state_layout = layout; a.path = path; a.time_groups = time_groups;
+    return a;
+}
+
+void check_btc(const Tensor &r, const Tensor &t, const char *name) {
+    TORCH_CHECK_VALUE(t.sizes() == r.sizes(), name, " must have shape ", r.sizes(), ", got ", t.sizes());
+    TORCH_CHECK_VALUE(t.is_contiguous(), name, " must be contiguous (a [:, t0:t1] view of a longer tensor is not)");
+}
+void check_contig(const Tensor &t, const char *name) {
+    TORCH_CHECK_VALUE(!t.defined() || t.is_contiguous(), name, " must be contiguous");
+}
+// the kernels take raw pointers: everything has to have the element type and size they assume
+void check_call(bool v6, const Tensor &r, const Tensor &k, const Tensor &v, const Tensor &w, const Tensor &u,
+                const Tensor &state, int w_kind) {
+    TORCH_CHECK_VALUE(r.dim() == 3 && r.size(2) % HEAD == 0, "r must be [B,T,H*64]");
+    check_btc(r, r, "r"); check_btc(r, k, "k"); check_btc(r, v, "v");
+    if (v6) check_btc(r, w, "w");
+    check_contig(u, "u"); check_contig(state, "state_in");
+}
+
+}  // namespace
+
+struct Fwd {
+    Tensor y, state_out, ckpt;
+};
+
+// saved_mode: WKV_GROUP_STATES_*; with it `saved` is the buffer (see wkv_args_t.group_states)
+Fwd wkv56_forward(bool v6, const Tensor &r, const Tensor &k, const Tensor &v, const Tensor &w, const Tensor &u,
+                  const Tensor &state_in, int w_kind, int layout, int path, const Tensor &state_out, bool save_ckpt,
+                  int time_groups, const Tensor &saved, int saved_mode, bool sync_check) {
+    require_cuda({&r, &k, &v, &w, &u, &state_in});
+    check_call(v6, r, k, v, w, u, state_in, w_kind);
+    check_contig(state_out, "state_out");
+    const int dev = r.device().index();
+    int *status = status_word(dev);
+    raise_if_set(dev, status);
+    c10::cuda::OptionalCUDAGuard guard(r.device());
+    Fwd out;
+    out.y = at::empty_like(r);
+    wkv_args_t a = make_args(r, w_kind, layout, path, time_groups);
+    out.state_out = state_out.defined() ? state_out : at::empty({a.B, a.H, HEAD, HEAD}, r.options().dtype(at::kFloat));
+    a.r = ptr(r); a.k = ptr(k); a.v = ptr(v); a.w = ptr(w); a.u = ptr(u);
+    a.state_in = (const float *)ptr(state_in);
+    a.y = ptr(out.y); a.state_out = (float *)ptr(out.state_out);
+    if (save_ckpt) {
+        a.state_ckpt_bytes = wkv56_state_ckpt_bytes(&a, v6);
+        out.ckpt = bytes_like(r, a.state_ckpt_bytes);
+        a.state_ckpt = ptr(out.ckpt);
+    }
+    if (saved_mode != WKV_GROUP_STATES_NONE) {
+        a.group_states = ptr(saved);
+        a.group_states_bytes = (size_t)saved.numel();
+        a.group_states_mode = saved_mode;
+    }
+    a.workspace_bytes = v6 ? wkv6_forward_workspace(&a) : wkv5_forward_workspace(&a);
+    Tensor ws = bytes_like(r, a.workspace_bytes);
+    a.workspace = ptr(ws);
+    check(wkv56x_forward(&a, v6, status, stream_of(r)), v6 ? "wkv6_forward" : "wkv5_forward");
+    if (sync_check) poll_status(dev, true);
+    return out;
+}
+
+struct Bwd {
+    Tensor gr, gk, gv, gw, gu, gstate_in;
+};
+
+// gw: v6 [B,T,C] in r's type.  gu [H,64] in u's type and v5's gw [H,64] in `w_type` are summed over the
+// batch; with per_batch they are the C ABI's fp32 [B,C] partials instead.
+Bwd wkv56_backward(bool v6, const Tensor &r, const Tensor &k, const Tensor &v, const Tensor &w, const Tensor &u,
+                   const Tensor &state_in, const Tensor &gy, const Tensor &gstate_out, int w_kind, int layout, int path,
+                   bool want_gstate, const Tensor &ckpt, int time_groups, bool per_batch, at::ScalarType u_type,
+                   at::ScalarType w_type, bool sync_check) {
+    require_cuda({&r, &k, &v, &w, &u, &state_in, &gy, &gstate_out});
+    check_call(v6, r, k, v, w, u, state_in, w_kind);
+    check_btc(r, gy, "gy");
+    check_contig(gstate_out, "gstate_out");
+    const int dev = r.device().index();
+    int *status = status_word(dev);
+    raise_if_set(dev, status);
+    c10::cuda::OptionalCUDAGuard guard(r.device());
+    wkv_args_t a = make_args(r, w_kind, layout, path, time_groups);
+    const auto f32 = r.options().dtype(at::kFloat);
+    const int64_t B = a.B, H = a.H;
+    Bwd g;
+    g.gr = at::empty_like(r); g.gk = at::empty_like(r); g.gv = at::empty_like(r);
+    const bool empty = B == 0 || H == 0;
+    if (per_batch) {
+        g.gu = at::empty({B, H * HEAD}, f32);
+        g.gw = v6 ? at::empty_like(r) : at::empty({B, H * HEAD}, f32);
+    } else {
+        g.gu = empty ? at::zeros({H, HEAD}, r.options().dtype(u_type)) : at::empty({H, HEAD}, r.options().dtype(u_type));
+        g.gw = v6 ? at::empty_like(r)
+                  : (empty ? at::zeros({H, HEAD}, r.options().dtype(w_type)) : at::empty({H, HEAD}, r.options().dtype(w_type)));
+    }
+    if (want_gstate) g.gstate_in = at::empty({B, H, HEAD, HEAD}, f32);
+    a.r = ptr(r); a.k = ptr(k); a.v = ptr(v); a.w = ptr(w); a.u = ptr(u);
+    a.state_in = (const float *)ptr(state_in);
+    a.gy = ptr(gy); a.gstate_out = (const float *)ptr(gstate_out);
+    a.gr = ptr(g.gr); a.gk = ptr(g.gk); a.gv = ptr(g.gv);
+    if (v6 || per_batch) a.gw = ptr(g.gw);
+    if (per_batch) a.gu = (float *)ptr(g.gu);
+    a.gstate_in = (float *)ptr(g.gstate_in);
+    if (ckpt.defined()) { a.state_ckpt = ptr(ckpt); a.state_ckpt_bytes = (size_t)ckpt.numel(); }
+    const char *what = v6 ? "wkv6_backward" : "wkv5_backward";
+    a.workspace_bytes = !per_batch ? wkv56x_backward_workspace(&a, v6)
+                                   : (v6 ? wkv6_backward_workspace(&a) : wkv5_backward_workspace(&a));
+    Tensor ws = bytes_like(r, a.workspace_bytes);
+    a.workspace = ptr(ws);
+    if (per_batch) {
+        // (the public entry point keeps its status word in the workspace: read it there when asked to)
+        check((v6 ? wkv6_backward : wkv5_backward)(&a, stream_of(r)), what);
+        if (sync_check && ws.defined() && wkv56_uses_chunked(&a, v6)) {
+            const int code = ws.slice(0, 0, 4).view(at::kInt).item<int>();
+            TORCH_CHECK(code == 0, what, ": a device-side wait ran out (status ", code, ")");
+        }
+    } else {
+        check(wkv56x_backward(&a, v6, status, ptr(g.gu), dtype_code(u_type), v6 ? nullptr : ptr(g.gw),
+                              v6 ? 0 : dtype_code(w_type), stream_of(r)),
+              what);
+        if (sync_check) poll_status(dev, true);
+    }
+    return g;
+}
+
+// ------------------------------------------------------------------------------ v5 / v6 autograd node
+namespace {
+
+struct Wkv56Function : torch::autograd::Function<Wkv56Function> {
+    // w: v6 in r's type, v5 fp32.  w_type / u_type: the element types the caller's parameters have.
+    static variable_list forward(AutogradContext *ctx, bool v6, const Tensor &r, const Tensor &k, const Tensor &v,
+                                 const Tensor &w, const Tensor &u, const Tensor &state, int64_t path, const Tensor *saved,
+                                 int64_t saved_mode, bool sync_check) {
+        const auto dt = r.scalar_type();
+        const Tensor rc = contig(r), kc = as_contig(k, dt), vc = as_contig(v, dt), uc = as_contig(u, dt),
+                     wc = as_contig(w, v6 ? dt : at::kFloat), sc = as_contig(state, at::kFloat);
+        Fwd o = wkv56_forward(v6, rc, kc, vc, wc, uc, sc, WKV_W_RAW, WKV_STATE_KV, (int)path, Tensor(), true, 0, *saved,
+                              (int)saved_mode, sync_check);
+        // (with a hand-over the backward pass does not need the initial state)
+        variable_list keep = {rc, kc, vc, wc, uc, sc};
+        if (o.ckpt.defined()) keep.push_back(o.ckpt);
+        ctx->save_for_backward(keep);
+        ctx->saved_data["v6"] = v6;
+        ctx->saved_data["path"] = path;
+        ctx->saved_data["sync"] = sync_check;
+        ctx->saved_data["types"] = std::vector<int64_t>{(int64_t)k.scalar_type(), (int64_t)v.scalar_type(), (int64_t)w.scalar_type(),
+                                                        (int64_t)u.scalar_type(), (int64_t)state.scalar_type()};
+        ctx->saved_data["w_shape"] = w.sizes().vec();
+        ctx->saved_data["u_shape"] = u.sizes().vec();
+        ctx->saved_data["s_shape"] = state.sizes().vec();
+        ctx->set_materialize_grads(false);
+        return {o.y, o.state_out};
+    }
+    static variable_list backward(AutogradContext *ctx, variable_list grads) {
+        const variable_list st = ctx->get_saved_variables();
+        const Tensor &r = st[0];
+        const bool v6 = ctx->saved_data["v6"].toBool();
+        const auto types = ctx->saved_data["types"].toIntVector();
+        const auto type = [&](int i) { return (at::ScalarType)types[i]; };
+        const Tensor gy = grads[0].defined() ? as_contig(grads[0], r.scalar_type()) : at::zeros_like(r);
+        const Tensor gs = grads[1].defined() ? as_contig(grads[1], at::kFloat) : Tensor();
+        Bwd g = wkv56_backward(v6, r, st[1], st[2], st[3], st[4], st[5], gy, gs, WKV_W_RAW, WKV_STATE_KV,
+                               (int)ctx->saved_data["path"].toInt(), ctx->needs_input_grad(5), st.size() > 6 ? st[6] : Tensor(), 0,
+                               false, type(3), v6 ? at::kFloat : type(2), ctx->saved_data["sync"].toBool());
+        Tensor gw = v6 ? g.gw.to(type(2)) : g.gw.view(ctx->saved_data["w_shape"].toIntVector());
+        Tensor gsi = g.gstate_in.defined() ? g.gstate_in.to(type(4)).view(ctx->saved_data["s_shape"].toIntVector()) : Tensor();
+        return {Tensor(), g.gr, g.gk.to(type(0)), g.gv.to(type(1)), gw, g.gu.view(ctx->saved_data["u_shape"].toIntVector()), gsi,
+                Tensor(), Tensor(), Tensor(), Tensor()};
+    }
+};
+
+void check_shapes56(bool v6, int64_t B, int64_t T, int64_t C, int64_t H, const Tensor &r, const Tensor &k, const Tensor &v,
+                    const Tensor &w, const Tensor &u, const Tensor &state) {
+    TORCH_CHECK_VALUE(C == H * HEAD, "C must equal H*64");
+    const auto is_btc = [&](const Tensor &t) { return t.dim() == 3 && t.size(0) == B && t.size(1) == T && t.size(2) == C; };
+    TORCH_CHECK_VALUE(is_btc(r), "r must be [B,T,C]");
+    TORCH_CHECK_VALUE(is_btc(k), "k must be [B,T,C]");
+    TORCH_CHECK_VALUE(is_btc(v), "v must be [B,T,C]");
+    TORCH_CHECK_VALUE(v6 ? is_btc(w) : w.numel() == C, v6 ? "w must be [B,T,C]" : "w must have H*64 elements");
+    TORCH_CHECK_VALUE(u.numel() == C, "u must have H*64 elements");
+    TORCH_CHECK_VALUE(state.numel() == B * H * HEAD * HEAD, "state must be [B,H,64,64]");
+}
+
+}  // namespace
+
+// WKV5.apply / WKV6.apply -> (y, state_out)
+std::tuple<Tensor, Tensor> wkv56_apply(bool v6, int64_t B, int64_t T, int64_t C, int64_t H, const Tensor &r, const Tensor &k,
+                                       const Tensor &v, const Tensor &w, const Tensor &u, const Tensor &state, int64_t path,
+                                       const OptTensor &saved, int64_t saved_mode, bool sync_check) {
+    check_shapes56(v6, B, T, C, H, r, k, v, w, u, state);
+    const Tensor buf = saved.has_value() ? *saved : Tensor();
+    if (wants_grad({&r, &k, &v, &w, &u, &state})) {
+        variable_list o = Wkv56Function::apply(v6, r, k, v, w, u, state, path, &buf, saved_mode, sync_check);
+        return {o[0], o[1]};
+    }
+    const auto dt = r.scalar_type();
+    Fwd o = wkv56_forward(v6, contig(r), as_contig(k, dt), as_contig(v, dt), as_contig(w, v6 ? dt : at::kFloat),
+                          as_contig(u, dt), as_contig(state, at::kFloat), WKV_W_RAW, WKV_STATE_KV, (int)path, Tensor(), false, 0,
+                          buf, (int)saved_mode, sync_check);
+    return {o.y, o.state_out};
+}
+
+// ------------------------------------------------------------------------------ drop-in wrappers
+// RWKV-v5/src/module/TimeMix.py:20-143 and RWKV-v6/src/module/TimeMix.py:19-109: the state is updated in
+// place in the [value,key] layout and the gradient of the state after the call is taken as zero.
+namespace {
+
+struct DropinFunction : torch::autograd::Function<DropinFunction> {
+    static Tensor forward(AutogradContext *ctx, bool v6, const Tensor &r, const Tensor &k, const Tensor &v, const Tensor &w,
+                          const Tensor &u, const Tensor &state, bool save, bool sync_check) {
+        const Tensor wc = as_contig(w, v6 ? r.scalar_type() : at::kFloat);
+        const Tensor s32 = as_contig(state, at::kFloat);
+        // the chunked kernels hand the states over; the token-serial ones start backward from the state itself
+        wkv_args_t a = make_args(r, WKV_W_RAW, WKV_STATE_VK, WKV_PATH_AUTO, 0);
+        const Tensor s_in = save && !wkv56_uses_chunked(&a, v6) ? s32.clone() : Tensor();
+        Fwd o = wkv56_forward(v6, r, k, v, wc, u, s32, WKV_W_RAW, WKV_STATE_VK, WKV_PATH_AUTO, s32, save, 0, Tensor(),
+                              WKV_GROUP_STATES_NONE, sync_check);
+        if (s32.data_ptr() != state.data_ptr()) {
+            Tensor dst = state.detach();
+            dst.copy_(s32.view_as(state));
+        }
+        if (save) {
+            ctx->save_for_backward({r, k, v, wc, u, s_in, o.ckpt});
+            ctx->saved_data["v6"] = v6;
+            ctx->saved_data["sync"] = sync_check;
+            ctx->saved_data["types"] = std::vector<int64_t>{(int64_t)w.scalar_type(), (int64_t)state.scalar_type()};
+            ctx->saved_data["w_shape"] = w.sizes().vec();
+            ctx->saved_data["u_shape"] = u.sizes().vec();
+            ctx->saved_data["s_shape"] = state.sizes().vec();
+        }
+        return o.y;
+    }
+    static variable_list backward(AutogradContext *ctx, variable_list grads) {
+        const variable_list st = ctx->get_saved_variables();
+        const Tensor &r = st[0];
+        const bool v6 = ctx->saved_data["v6"].toBool();
+        const auto types = ctx->saved_data["types"].toIntVector();
+        // (the v5 wrapper gives its state no gradient)
+        const bool want_gs = v6 && ctx->needs_input_grad(5);
+        Bwd g = wkv56_backward(v6, r, st[1], st[2], st[3], st[4], st[5], as_contig(grads[0], r.scalar_type()), Tensor(), WKV_W_RAW,
+                               WKV_STATE_VK, WKV_PATH_AUTO, want_gs, st[6], 0, false, r.scalar_type(), (at::ScalarType)types[0],
+                               ctx->saved_data["sync"].toBool());
+        Tensor gw = v6 ? g.gw.to((at::ScalarType)types[0]) : g.gw.view(ctx->saved_data["w_shape"].toIntVector());
+        Tensor gs = want_gs ? g.gstate_in.to((at::ScalarType)types[1]).view(ctx->saved_data["s_shape"].toIntVector()) : Tensor();
+        return {Tensor(), g.gr, g.gk, g.gv, gw, g.gu.view(ctx->saved_data["u_shape"].toIntVector()), gs, Tensor(), Tensor()};
+    }
+};
+
+}  // namespace
+
+Tensor wkv56_dropin(bool v6, int64_t B, int64_t T, int64_t C, int64_t H, const Tensor &r, const Tensor &k, const Tensor &v,
+                    const Tensor &w, const Tensor &u, const Tensor &state, bool sync_check) {
+    for (const Tensor *t : {&r, &k, &v, &w, &u, &state}) TORCH_CHECK_VALUE(t->is_contiguous(), "inputs must be contiguous");
+    const auto dt = r.scalar_type();
+    TORCH_CHECK_TYPE(dt == k.scalar_type() && dt == v.scalar_type() && dt == u.scalar_type(), "r,k,v,u must share one dtype");
+    if (!v6)
+        TORCH_CHECK_TYPE(state.scalar_type() == at::kFloat && w.scalar_type() == at::kFloat, "state and w must be float32");
+    dtype_code(dt);
+    check_shapes56(v6, B, T, C, H, r, k, v, w, u, state);
+    return DropinFunction::apply(v6, r, k, v, w, u, state, wants_grad({&r, &k, &v, &w, &u, &state}), sync_check);
+}
+
+// ------------------------------------------------------------------------------ v4
+namespace {
+
+// RWKV-v4neo/cuda/wkv_op_bf16.cpp:13-92
+struct Wkv4Function : torch::autograd::Function<Wkv4Function> {
+    static variable_list forward(AutogradContext *ctx, const Tensor &raw_w, const Tensor &raw_u, const Tensor &raw_k,
+                                 const Tensor &raw_v, const Tensor &raw_state, bool save) {
+        const int B = (int)raw_k.size(0), T = (int)raw_k.size(1), C = (int)raw_k.size(2);
+        const auto dt = raw_k.scalar_type();
+        c10::cuda::OptionalCUDAGuard guard(raw_k.device());
+        const Tensor w = as_contig(raw_w, at::kFloat).exp().neg_(), u = as_contig(raw_u, dt), k = contig(raw_k),
+                     v = as_contig(raw_v, dt), state = as_contig(raw_state, at::kFloat);
+        Tensor y = at::empty_like(k), new_state = at::empty_like(state);
+        const size_t nws = wkv4_forward_workspace(B, T, C), nck = save ? wkv4_state_ckpt_bytes(B, T, C) : 0;
+        Tensor ws = bytes_like(k, nws), ck = bytes_like(k, nck);
+        check(wkv4_forward_ckpt(B, T, C, dtype_code(dt), (const float *)ptr(w), ptr(u), ptr(k), ptr(v), (const float *)ptr(state),
+                                ptr(y), (float *)ptr(new_state), ptr(ws), nws, ptr(ck), nck, stream_of(k)),
+              "wkv4_forward");
+        if (save) {
+            ctx->save_for_backward({w, u, k, v, state, ck});
+            ctx->saved_data["types"] = std::vector<int64_t>{(int64_t)raw_w.scalar_type(), (int64_t)raw_u.scalar_type(),
+                                                            (int64_t)raw_v.scalar_type(), (int64_t)raw_state.scalar_type()};
+            ctx->set_materialize_grads(false);
+        }
+        return {y, new_state};
+    }
+    static variable_list backward(AutogradContext *ctx, variable_list grads) {
+        const variable_list st = ctx->get_saved_variables();
+        const Tensor &w = st[0], &u = st[1], &k = st[2], &v = st[3], &state = st[4], &ck = st[5];
+        const int B = (int)k.size(0), T = (int)k.size(1), C = (int)k.size(2);
+        const auto types = ctx->saved_data["types"].toIntVector();
+        c10::cuda::OptionalCUDAGuard guard(k.device());
+        const Tensor gy = grads[0].defined() ? as_contig(grads[0], k.scalar_type()) : at::zeros_like(k);
+        const Tensor gs = grads[1].defined() ? as_contig(grads[1], at::kFloat) : Tensor();
+        Tensor gw = at::empty({B, C}, w.options()), gu = at::empty({B, C}, w.options()), gk = at::empty_like(k),
+               gv = at::empty_like(k), glast = at::empty_like(state);
+        const size_t nws = wkv4_backward_workspace(B, T, C);
+        Tensor ws = bytes_like(k, nws);
+        check(wkv4_backward_ckpt(B, T, C, dtype_code(k.scalar_type()), (const float *)ptr(w), ptr(u), ptr(k), ptr(v),
+                                 (const float *)ptr(state), ptr(gy), (const float *)ptr(gs), (float *)ptr(gw), (float *)ptr(gu),
+                                 ptr(gk), ptr(gv), (float *)ptr(glast), ptr(ws), nws, ptr(ck), ck.defined() ? (size_t)ck.numel() : 0,
+                                 stream_of(k)),
+              "wkv4_backward");
+        return {gw.sum(0).to((at::ScalarType)types[0]), gu.sum(0).to((at::ScalarType)types[1]), gk, gv.to((at::ScalarType)types[2]),
+                glast.to((at::ScalarType)types[3]), Tensor()};
+    }
+};
+
+}  // namespace
+
+std::vector<Tensor> wkv4(const Tensor &w, const Tensor &u, const Tensor &k, const Tensor &v, const Tensor &state) {
+    TORCH_CHECK_VALUE(k.dim() == 3, "k must be [B,T,C]");
+    const int64_t C = k.size(2);
+    TORCH_CHECK_VALUE(w.dim() == 1 && w.size(0) == C && u.dim() == 1 && u.size(0) == C, "time_decay and time_first must be [C]");
+    TORCH_CHECK_VALUE(v.sizes() == k.sizes(), "v must match k");
+    TORCH_CHECK_VALUE(state.dim() == 3 && state.size(0) == k.size(0) && state.size(1) == C && state.size(2) == 3,
+                      "last_state must be [B,C,3]");
+    require_cuda({&w, &u, &k, &v, &state});
+    dtype_code(k.scalar_type());
+    return Wkv4Function::apply(w, u, k, v, state, wants_grad({&w, &u, &k, &v, &state}));
+}
+
+}  // namespace wkv_native
+
+TORCH_LIBRARY(rwkv, m) {
+    // RWKV-v4neo/cuda/wkv_op_bf16.cpp:98
+    m.def("wkv(Tensor w, Tensor u, Tensor k, Tensor v, Tensor last_state) -> Tensor[]");
+    m.impl("wkv", c10::DispatchKey::CompositeImplicitAutograd, TORCH_FN(wkv_native::wkv4));
+}
+
+namespace {
+using namespace wkv_native;
+Tensor opt(const OptTensor &t) { return t.has_value() ? *t : Tensor(); }
+py::object none_or(const Tensor &t) { return t.defined() ? py::cast(t) : py::none(); }
+}  // namespace
+
+void bind_timemix(py::module_ &m);
+
+PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
+    m.def("wkv56_apply", &wkv56_apply);
+    m.def("wkv56_dropin", &wkv56_dropin);
+    m.def("wkv4", &wkv4);
+    m.def("poll_status", &poll_status);
+    m.def("wkv56_forward",
+          [](bool v6, const Tensor &r, const Tensor &k, const Tensor &v, const Tensor &w, const Tensor &u, const OptTensor &s,
+             int w_kind, int layout, int path, const OptTensor &s_out, bool save_ckpt, int time_groups, const OptTensor &saved,
+             int saved_mode, bool sync_check) {
+              at::NoGradGuard no_grad;
+              Fwd o = wkv56_forward(v6, r, k, v, w, u, opt(s), w_kind, layout, path, opt(s_out), save_ckpt, time_groups, opt(saved),
+                                    saved_mode, sync_check);
+              return py::make_tuple(o.y, o.state_out, none_or(o.ckpt));
+          });
+    m.def("wkv56_backward",
+          [](bool v6, const Tensor &r, const Tensor &k, const Tensor &v, const Tensor &w, const Tensor &u, const OptTensor &s,
+             const Tensor &gy, const OptTensor &gs, int w_kind, int layout, int path, bool want_gstate, const OptTensor &ckpt,
+             int time_groups, bool sync_check) {
+              at::NoGradGuard no_grad;
+              Bwd g = wkv56_backward(v6, r, k, v, w, u, opt(s), gy, opt(gs), w_kind, layout, path, want_gstate, opt(ckpt), time_groups,
+                                     true, at::kFloat, at::kFloat, sync_check);
+              return py::make_tuple(g.gr, g.gk, g.gv, g.gw, g.gu, none_or(g.gstate_in));
+          });
+    bind_timemix(m);
+}

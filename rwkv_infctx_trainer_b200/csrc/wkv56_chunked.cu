@@ -796,7 +796,7 @@ size_t chunked_forward_workspace(const wkv_args_t *a, bool per_token_w) {
 }
 
 int chunked_forward_impl(const wkv_args_t *a, bool per_token_w, void *state_ckpt, void *group_ws,
-                         const ChunkedTest &tst, cudaStream_t stream) {
+                         const CallOpts &opt, cudaStream_t stream) {
     const int B = a->B, T = a->T, H = a->H, C = H * 64, BH = B * H;
     CUtensorMap mr, mk, mv, mw;
     if (!make_btc_map(&mr, a->r, B, T, C) || !make_btc_map(&mk, a->k, B, T, C) ||
@@ -817,10 +817,10 @@ int chunked_forward_impl(const wkv_args_t *a, bool per_token_w, void *state_ckpt
     p.Lsave = SAVE_EVERY;
     p.u = (const __nv_bfloat16 *)a->u;
     p.wvec = per_token_w ? nullptr : (const float *)a->w;
-    p.status = (int *)a->workspace;
+    p.status = opt.status ? opt.status : (int *)a->workspace;
     p.mildflag = nullptr;
-    p.wait_limit = tst.wait_limit;
-    p.skip_load = tst.kernel == 0 ? tst.skip_load : -1;
+    p.wait_limit = opt.wait_limit;
+    p.skip_load = opt.kernel == 0 ? opt.skip_load : -1;
     const size_t smem = sizeof(FwdSmem) + 1024;
     const int mode = a->y == nullptr ? FWD_STATES : FWD_FULL;
     using Kern = void (*)(const CUtensorMap, const CUtensorMap, const CUtensorMap, const CUtensorMap,
@@ -867,15 +867,15 @@ int chunked_forward_impl(const wkv_args_t *a, bool per_token_w, void *state_ckpt
     return launch_chained(kerns[pt][mode], dim3(gp.G, BH), dim3(FWD_THREADS), smem, stream, mr, mk, mv, mw, mrh, p);
 }
 
-int chunked_forward(const wkv_args_t *a0, bool per_token_w, const ChunkedTest &tst, cudaStream_t stream) {
+int chunked_forward(const wkv_args_t *a0, bool per_token_w, const CallOpts &opt, cudaStream_t stream) {
     wkv_args_t a = *a0;
-    if (cudaMemsetAsync(a.workspace, 0, 256, stream) != cudaSuccess) return WKV_ERR_LAUNCH;
+    if (!opt.status && cudaMemsetAsync(a.workspace, 0, 256, stream) != cudaSuccess) return WKV_ERR_LAUNCH;
     const size_t conv = chunked_wconv_bytes(&a, per_token_w);
     if (conv) {   // the converted decay tensor sits at the end of the workspace
         const int err = chunked_convert_w(&a, per_token_w, (char *)a.workspace + chunked_forward_workspace(a0, per_token_w) - conv, stream);
         if (err != WKV_OK) return err;
     }
-    return chunked_forward_impl(&a, per_token_w, a.state_ckpt, (char *)a.workspace + 256, tst, stream);
+    return chunked_forward_impl(&a, per_token_w, a.state_ckpt, (char *)a.workspace + 256, opt, stream);
 }
 
 }  // namespace wkv

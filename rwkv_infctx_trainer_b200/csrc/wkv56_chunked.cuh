@@ -251,14 +251,24 @@ int launch_group_scan(const void *group_ws, int BH, int G, const float *init, fl
 
 }  // namespace chunked
 
-// What only the wait-timeout self-test changes: how many polls a device-side wait makes before it
-// gives up, and one TMA load that is deliberately never issued (kernel: 0 forward, 1 dS scan,
-// 2 per-chunk backward; skip_load: local chunk / step index, -1 = none).
-struct ChunkedTest {
+// How a call differs from the public one.
+struct CallOpts {
+    // only the wait-timeout self-test changes these: how many polls a device-side wait makes before it
+    // gives up, and one TMA load that is deliberately never issued (kernel: 0 forward, 1 dS scan,
+    // 2 per-chunk backward; skip_load: local chunk / step index, -1 = none)
     uint32_t wait_limit = 4000000u;
     int kernel = -1;
     int skip_load = -1;
+    // status word (NULL: the first word of the workspace, cleared by the call)
+    int *status = nullptr;
+    // parameter gradients summed over the batch, in the parameter's element type (NULL: a->gu, a->gw)
+    void *gu_sum = nullptr, *gw_sum = nullptr;
+    int gu_dtype = 0, gw_dtype = 0;
 };
+
+// opt.gu_sum / gw_sum [H,64] = gu_part / gw_part [B*H, n, 64] summed over the batch and n (wkv_api.cu);
+// gw_part NULL: gu alone
+int fold_param_grads(const float *gu_part, const float *gw_part, int B, int H, int n, const CallOpts &opt, cudaStream_t s);
 
 int device_sm_count();
 size_t chunked_group_states_bytes(const wkv_args_t *a);
@@ -283,8 +293,8 @@ inline bool set_max_smem_once(K kern, int bytes, unsigned char (&done)[64]) {
 // reuse from the forward pass; y is not produced when `y` in `a` is NULL; `group_ws` is
 // chunked::group_layout() bytes of scratch, used when the chains are split into time groups
 int chunked_forward_impl(const wkv_args_t *a, bool per_token_w, void *state_ckpt, void *group_ws,
-                         const ChunkedTest &tst, cudaStream_t s);
-int chunked_forward(const wkv_args_t *a, bool per_token_w, const ChunkedTest &tst, cudaStream_t s);
-int chunked_backward(const wkv_args_t *a, bool per_token_w, const ChunkedTest &tst, cudaStream_t s);
+                         const CallOpts &opt, cudaStream_t s);
+int chunked_forward(const wkv_args_t *a, bool per_token_w, const CallOpts &opt, cudaStream_t s);
+int chunked_backward(const wkv_args_t *a, bool per_token_w, const CallOpts &opt, cudaStream_t s);
 
 }  // namespace wkv

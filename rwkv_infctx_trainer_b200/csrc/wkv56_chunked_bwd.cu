@@ -1130,13 +1130,14 @@ BwdLayout bwd_layout(const wkv_args_t *a, bool per_token_w) {
 
 size_t chunked_backward_workspace(const wkv_args_t *a, bool per_token_w) { return bwd_layout(a, per_token_w).total; }
 
-int chunked_backward(const wkv_args_t *a0, bool per_token_w, const ChunkedTest &tst, cudaStream_t stream) {
+int chunked_backward(const wkv_args_t *a0, bool per_token_w, const CallOpts &opt, cudaStream_t stream) {
     wkv_args_t args = *a0;
     wkv_args_t *a = &args;
     const int B = a->B, T = a->T, H = a->H, C = H * 64, n = (T + CH - 1) / CH, BH = B * H;
     const BwdLayout L = bwd_layout(a, per_token_w);
     char *ws = (char *)a->workspace;
-    if (cudaMemsetAsync(ws, 0, 256, stream) != cudaSuccess) return WKV_ERR_LAUNCH;
+    int *status = opt.status ? opt.status : (int *)ws;
+    if (!opt.status && cudaMemsetAsync(ws, 0, 256, stream) != cudaSuccess) return WKV_ERR_LAUNCH;
     if (chunked_convert_w(a, per_token_w, ws + L.wconv, stream) != WKV_OK) return WKV_ERR_LAUNCH;
     // what the forward kernel leaves for this call: chunk-start states, r e^{cp}, chunk decays
     char *fwd_ck = a->state_ckpt ? (char *)a->state_ckpt : ws + L.sck;
@@ -1151,7 +1152,7 @@ int chunked_backward(const wkv_args_t *a0, bool per_token_w, const ChunkedTest &
         f.state_out = nullptr;
         f.group_states = nullptr;
         f.group_states_mode = WKV_GROUP_STATES_NONE;
-        const int err = chunked_forward_impl(&f, per_token_w, fwd_ck, ws + L.groups, tst, stream);
+        const int err = chunked_forward_impl(&f, per_token_w, fwd_ck, ws + L.groups, opt, stream);
         if (err != WKV_OK) return err;
     }
     CUtensorMap mr, mk, mv, mw, mgy, ms, md, mgr, mgk, mgv, mgw, mrh;
@@ -1173,9 +1174,9 @@ int chunked_backward(const wkv_args_t *a0, bool per_token_w, const ChunkedTest &
         p.T = T; p.H = H; p.nchunk = n; p.layout = a->state_layout;
         p.G = gp.G; p.L = gp.L;
         p.dchunk = (const float *)(fwd_ck + CL.dchunk);
-        p.dck = (__nv_bfloat16 *)dck; p.e0 = e0; p.status = (int *)ws;
-        p.wait_limit = tst.wait_limit;
-        p.skip_load = tst.kernel == 1 ? tst.skip_load : -1;
+        p.dck = (__nv_bfloat16 *)dck; p.e0 = e0; p.status = status;
+        p.wait_limit = opt.wait_limit;
+        p.skip_load = opt.kernel == 1 ? opt.skip_load : -1;
         const size_t smem = sizeof(DscanSmem) + 1024;
         static unsigned char attr_done[64];
         if (!set_max_smem_once(k_chunk_dscan, (int)smem, attr_done)) return WKV_ERR_LAUNCH;
@@ -1203,9 +1204,9 @@ int chunked_backward(const wkv_args_t *a0, bool per_token_w, const ChunkedTest &
         p.prefetch_dist = 2 * device_sm_count();      // two CTAs of this kernel fit on an SM
         p.u = (const __nv_bfloat16 *)a->u;
         p.wvec = per_token_w ? nullptr : (const float *)a->w;
-        p.e0 = e0; p.gu_part = gu_part; p.gw_part = gw_part; p.status = (int *)ws;
-        p.wait_limit = tst.wait_limit;
-        p.skip_load = tst.kernel == 2 ? tst.skip_load : -1;
+        p.e0 = e0; p.gu_part = gu_part; p.gw_part = gw_part; p.status = status;
+        p.wait_limit = opt.wait_limit;
+        p.skip_load = opt.kernel == 2 ? opt.skip_load : -1;
         p.mildflag = (const unsigned char *)(fwd_ck + CL.mild);
         const size_t smem = sizeof(BwdSmem);
         auto kern = per_token_w ? k_chunk_bwd<true> : k_chunk_bwd<false>;
@@ -1225,8 +1226,10 @@ int chunked_backward(const wkv_args_t *a0, bool per_token_w, const ChunkedTest &
                            mgk, mgv, mgw, p, BH * n) != WKV_OK)
             return WKV_ERR_LAUNCH;
     }
-    // 4. fold the per-chunk partial sums
-    {
+    // 4. fold the per-chunk partial sums: over the chunks and the batch, or over the chunks alone
+    if (opt.gu_sum) {
+        if (fold_param_grads(gu_part, per_token_w ? nullptr : gw_part, B, H, n, opt, stream) != WKV_OK) return WKV_ERR_LAUNCH;
+    } else {
         const int total = BH * 64;
         if (launch_chained(k_reduce_partials, dim3((total + 255) / 256), dim3(256), 0, stream, (const float *)gu_part,
                            (float *)a->gu, n, total) != WKV_OK)

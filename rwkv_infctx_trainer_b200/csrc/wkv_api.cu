@@ -3,6 +3,53 @@
 #include "wkv56_chunked.cuh"
 #include "wkv_common.cuh"
 
+#include "wkv_internal.h"
+
+namespace wkv {
+namespace {
+
+__device__ __forceinline__ void store_as(void *p, int dtype, int i, float x) {
+    if (dtype == WKV_F32) ((float *)p)[i] = x;
+    else if (dtype == WKV_BF16) ((__nv_bfloat16 *)p)[i] = __float2bfloat16_rn(x);
+    else ((__half *)p)[i] = __float2half_rn(x);
+}
+
+// One CTA per (head, parameter): 16 groups of 64 threads (a channel each) take every 16th of the
+// B*n rows, the groups meet in shared memory in a fixed order.  Latency-bound (a few hundred KB from
+// L2): the width is there to have many loads in flight.
+__global__ void __launch_bounds__(1024)
+k_fold_heads(const float *__restrict__ gu_part, const float *__restrict__ gw_part, void *gu, int gu_dtype, void *gw,
+             int gw_dtype, int B, int H, int n) {
+    pdl_wait();
+    pdl_trigger();
+    __shared__ float red[16][64];
+    const int h = blockIdx.x, k = threadIdx.x & 63, g = threadIdx.x >> 6, rows = B * n;
+    const float *part = blockIdx.y ? gw_part : gu_part;
+    float acc = 0.f;
+#pragma unroll 8
+    for (int i = g; i < rows; i += 16) {
+        const int b = i / n, j = i - b * n;
+        acc += part[(((size_t)b * H + h) * n + j) * 64 + k];
+    }
+    red[g][k] = acc;
+    __syncthreads();
+    if (g == 0) {
+#pragma unroll
+        for (int q = 1; q < 16; q++) acc += red[q][k];
+        if (blockIdx.y) store_as(gw, gw_dtype, h * 64 + k, acc);
+        else store_as(gu, gu_dtype, h * 64 + k, acc);
+    }
+}
+
+}  // namespace
+
+int fold_param_grads(const float *gu_part, const float *gw_part, int B, int H, int n, const CallOpts &opt, cudaStream_t s) {
+    return launch_chained(k_fold_heads, dim3(H, gw_part ? 2 : 1), dim3(1024), 0, s, gu_part, gw_part, opt.gu_sum,
+                          opt.gu_dtype, opt.gw_sum, opt.gw_dtype, B, H, n);
+}
+
+}  // namespace wkv
+
 using namespace wkv;
 
 namespace {
@@ -59,7 +106,7 @@ size_t bwd_ws(const wkv_args_t *a, bool pt) {
     return use_chunked(a, pt, &err) ? chunked_backward_workspace(a, pt) : scalar_backward_workspace(a);
 }
 
-int forward(const wkv_args_t *a, bool pt, void *stream, const ChunkedTest &tst = ChunkedTest()) {
+int forward(const wkv_args_t *a, bool pt, void *stream, const CallOpts &opt = CallOpts()) {
     int err = check_common(a, false, pt);
     if (err != WKV_OK) return err;
     if (a->B == 0 || a->H == 0) return WKV_OK;
@@ -73,10 +120,10 @@ int forward(const wkv_args_t *a, bool pt, void *stream, const ChunkedTest &tst =
         if (!ch) return WKV_ERR_UNSUPPORTED;
         if (a->group_states_bytes < wkv56_group_states_bytes(a)) return WKV_ERR_WORKSPACE;
     }
-    return ch ? chunked_forward(a, pt, tst, s) : scalar_forward(a, pt, s);
+    return ch ? chunked_forward(a, pt, opt, s) : scalar_forward(a, pt, s);
 }
 
-int backward(const wkv_args_t *a, bool pt, void *stream, const ChunkedTest &tst = ChunkedTest()) {
+int backward(const wkv_args_t *a, bool pt, void *stream, const CallOpts &opt = CallOpts()) {
     int err = check_common(a, true, pt);
     if (err != WKV_OK) return err;
     if (a->B == 0 || a->H == 0) return WKV_OK;
@@ -86,7 +133,10 @@ int backward(const wkv_args_t *a, bool pt, void *stream, const ChunkedTest &tst 
     const size_t need = bwd_ws(a, pt);
     if (need && (!a->workspace || a->workspace_bytes < need)) return WKV_ERR_WORKSPACE;
     if (ch && a->state_ckpt && a->state_ckpt_bytes < wkv56_state_ckpt_bytes(a, pt)) return WKV_ERR_WORKSPACE;
-    return ch ? chunked_backward(a, pt, tst, s) : scalar_backward(a, pt, s);
+    if (ch) return chunked_backward(a, pt, opt, s);
+    err = scalar_backward(a, pt, s);
+    if (err != WKV_OK || !opt.gu_sum) return err;
+    return fold_param_grads(a->gu, pt ? nullptr : (const float *)a->gw, a->B, a->H, 1, opt, s);
 }
 
 }  // namespace
@@ -128,6 +178,35 @@ int wkv56_uses_chunked(const wkv_args_t *a, int per_token_w) {
     return use_chunked(a, per_token_w != 0, &err) ? 1 : 0;
 }
 
+int wkv56x_forward(const wkv_args_t *a, int per_token_w, int *status, void *stream) {
+    CallOpts opt;
+    opt.status = status;
+    return forward(a, per_token_w != 0, stream, opt);
+}
+
+// the per-batch partials of the public call go behind the workspace it asks for
+size_t wkv56x_backward_workspace(const wkv_args_t *a, int per_token_w) {
+    if (!a || a->B <= 0 || a->H <= 0 || a->N != HEAD) return 0;
+    return ((bwd_ws(a, per_token_w != 0) + 255) & ~(size_t)255) + 2 * (size_t)a->B * a->H * HEAD * sizeof(float);
+}
+
+int wkv56x_backward(const wkv_args_t *a0, int per_token_w, int *status, void *gu_sum, int gu_dtype, void *gw_sum,
+                    int gw_dtype, void *stream) {
+    if (!a0 || !gu_sum || (!per_token_w && !gw_sum)) return WKV_ERR_NULL;
+    const size_t need = wkv56x_backward_workspace(a0, per_token_w);
+    if (need && (!a0->workspace || a0->workspace_bytes < need)) return WKV_ERR_WORKSPACE;
+    if (need == 0) return WKV_OK;
+    wkv_args_t a = *a0;
+    float *partials = (float *)((char *)a.workspace + need) - 2 * (size_t)a.B * a.H * HEAD;
+    a.gu = partials;
+    if (!per_token_w) a.gw = partials + (size_t)a.B * a.H * HEAD;
+    CallOpts opt;
+    opt.status = status;
+    opt.gu_sum = gu_sum; opt.gu_dtype = gu_dtype;
+    opt.gw_sum = gw_sum; opt.gw_dtype = gw_dtype;
+    return backward(&a, per_token_w != 0, stream, opt);
+}
+
 int wkv_selftest_wait_timeout(int *status_word, unsigned limit, void *stream) {
     if (!status_word) return WKV_ERR_NULL;
     return selftest_wait(status_word, limit, (cudaStream_t)stream);
@@ -137,11 +216,11 @@ int wkv56_selftest_abort(const wkv_args_t *a, int per_token_w, int backward_call
                          unsigned limit, void *stream) {
     if (limit == 0 || limit > 100000u || kernel < 0 || kernel > 2 || skip_chunk < 0) return WKV_ERR_SHAPE;
     if (!wkv56_uses_chunked(a, per_token_w)) return WKV_ERR_UNSUPPORTED;
-    ChunkedTest tst;
-    tst.wait_limit = limit;
-    tst.kernel = kernel;
-    tst.skip_load = skip_chunk;
-    return backward_call ? backward(a, per_token_w != 0, stream, tst) : forward(a, per_token_w != 0, stream, tst);
+    CallOpts opt;
+    opt.wait_limit = limit;
+    opt.kernel = kernel;
+    opt.skip_load = skip_chunk;
+    return backward_call ? backward(a, per_token_w != 0, stream, opt) : forward(a, per_token_w != 0, stream, opt);
 }
 
 size_t wkv5_forward_workspace(const wkv_args_t *a) { return fwd_ws(a, false); }

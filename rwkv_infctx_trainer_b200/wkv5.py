@@ -25,46 +25,10 @@ from . import wkv56
 N = wkv56.HEAD_SIZE
 
 
-def _check_shapes(B, T, C, H, r, k, v, u, state):
-    if C != H * N:
-        raise ValueError(f"C must equal H*{N}")
-    for name, t in (("r", r), ("k", k), ("v", v)):
-        if tuple(t.shape) != (B, T, C):
-            raise ValueError(f"{name} must be [B,T,C]")
-    if u.numel() != C:
-        raise ValueError("u must have H*N elements")
-    if state is not None and state.numel() != B * H * N * N:
-        raise ValueError("state must be [B,H,N,N]")
-
-
-class WKV5(torch.autograd.Function):
+class WKV5:
     @staticmethod
-    def forward(ctx, B, T, C, H, r, k, v, w, u, state_in, path=L.WKV_PATH_AUTO, saved=None):
-        _check_shapes(B, T, C, H, r, k, v, u, state_in)
-        dt = r.dtype
-        r, k, v = r.contiguous(), k.to(dt).contiguous(), v.to(dt).contiguous()
-        wf = w.float().contiguous()
-        uf = u.to(dt).contiguous()
-        s_in = state_in.float().contiguous()
-        y, s_out, ckpt = wkv56.forward("wkv5", r, k, v, wf, uf, s_in, w_kind=L.WKV_W_RAW, path=path,
-                                       save_ckpt=any(ctx.needs_input_grad), saved=saved)
-        ctx.has_ckpt = ckpt is not None
-        ctx.save_for_backward(*((r, k, v, wf, uf, s_in) + ((ckpt,) if ckpt is not None else ())))
-        ctx.meta = (B, T, C, H, path, w.dtype, u.dtype, w.shape, u.shape, state_in.dtype)
-        return y, s_out.view(B, H, N, N)
-
-    @staticmethod
-    def backward(ctx, gy, gstate_out):
-        st = ctx.saved_tensors          # (one access: saved-tensor hooks unpack once)
-        r, k, v, wf, uf, s_in = st[:6]
-        ckpt = st[6] if ctx.has_ckpt else None
-        B, T, C, H, path, wdt, udt, wshape, ushape, sdt = ctx.meta
-        gy = gy.to(r.dtype).contiguous()
-        gso = None if gstate_out is None else gstate_out.float().contiguous()
-        gr, gk, gv, gw, gu, gsi = wkv56.backward("wkv5", r, k, v, wf, uf, s_in, gy, gso,
-                                                 w_kind=L.WKV_W_RAW, path=path, ckpt=ckpt)
-        return (None, None, None, None, gr, gk, gv, gw.sum(0).view(wshape).to(wdt),
-                gu.sum(0).view(ushape).to(udt), gsi.to(sdt), None, None)
+    def apply(B, T, C, H, r, k, v, w, u, state_in, path=L.WKV_PATH_AUTO, saved=None):
+        return wkv56.apply("wkv5", B, T, C, H, r, k, v, w, u, state_in, path, saved)
 
 
 def wkv5(r, k, v, w, u, state_in, path=L.WKV_PATH_AUTO):
@@ -113,46 +77,13 @@ class _Wkv5Kernel:
 wkv5_cuda_kernel = _Wkv5Kernel()
 
 
-class WKV5_CUDA(torch.autograd.Function):
+class WKV5_CUDA:
     """RWKV-v5/src/module/TimeMix.py:20-143: ``apply(B,T,C,H,state,r,k,v,w,u) -> y``;
     ``state`` (fp32, [B,H,value,key]) is updated in place; no gradient flows to it."""
 
     @staticmethod
-    def forward(ctx, B, T, C, H, state, r, k, v, w, u):
-        with torch.no_grad():
-            dtype = r.dtype
-            ctx.B, ctx.T, ctx.C, ctx.H, ctx.dtype = B, T, C, H, dtype
-            if state.dtype != torch.float32 or w.dtype != torch.float32:
-                raise TypeError("state and w must be float32")
-            for t in (state, w, r, k, v, u):
-                if not t.is_contiguous():
-                    raise ValueError("inputs must be contiguous")
-            if not (dtype == k.dtype == v.dtype == u.dtype):
-                raise TypeError("r,k,v,u must share one dtype")
-            if dtype not in L.DTYPE_CODE:
-                raise ValueError(f"Unsupported dtype {dtype} for WKV5_CUDA")
-            ew = (-torch.exp(w.float())).contiguous()
-            eew = torch.exp(ew).contiguous()
-            ctx.save_for_backward(r, k, v, eew, ew, u, state.clone())
-            y = torch.empty(B, T, C, device=r.device, dtype=dtype)
-            name = {torch.bfloat16: "bf16", torch.float16: "fp16", torch.float32: "fp32"}[dtype]
-            getattr(wkv5_cuda_kernel, "forward_" + name)(B, T, C, H, state, r, k, v, eew, u, y)
-            return y
-
-    @staticmethod
-    def backward(ctx, gy):
-        with torch.no_grad():
-            B, T, C, H, dtype = ctx.B, ctx.T, ctx.C, ctx.H, ctx.dtype
-            gy = gy.to(dtype).contiguous()
-            r, k, v, eew, ew, u, in_state = ctx.saved_tensors
-            mk = lambda *s: torch.empty(s, device=gy.device, dtype=dtype)
-            gr, gk, gv, gw, gu = mk(B, T, C), mk(B, T, C), mk(B, T, C), mk(B, C), mk(B, C)
-            name = {torch.bfloat16: "bf16", torch.float16: "fp16", torch.float32: "fp32"}[dtype]
-            getattr(wkv5_cuda_kernel, "backward_" + name)(B, T, C, H, in_state, r, k, v, eew, ew,
-                                                          u, gy, gr, gk, gv, gw, gu)
-            gw = torch.sum(gw, 0).view(H, C // H)
-            gu = torch.sum(gu, 0).view(H, C // H)
-            return (None, None, None, None, None, gr, gk, gv, gw, gu)
+    def apply(B, T, C, H, state, r, k, v, w, u):
+        return wkv56.apply_dropin("wkv5", B, T, C, H, r, k, v, w, u, state)
 
 
 def RUN_WKV5_CUDA(B, T, C, H, state, r, k, v, w, u):

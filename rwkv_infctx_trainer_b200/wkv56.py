@@ -9,24 +9,23 @@ from . import _lib as L
 
 HEAD_SIZE = 64
 
-# The chunked kernels keep a status word at the start of their workspace: non-zero means that a
-# bounded device-side wait ran out, the kernel gave up, and its outputs are invalid.  Every call
-# copies that word to pinned host memory (on a side stream, without synchronising); the copies
-# that have completed are looked at when the next v5/v6 call (forward or backward) on that device
-# starts, and ``poll_status()`` looks at them on demand.  A non-zero word raises there.
-# With CHECK_STATUS = True every call synchronises and checks its own word before returning
-# (tests do that).
+# A chunked kernel whose bounded device-side wait runs out gives up and says so in a status word: its
+# outputs are invalid.  The ops of this package keep one word per device in mapped host memory, look at
+# it when the next v5/v6 call (forward or backward) on that device starts, and raise there if it is not
+# zero; ``poll_status()`` looks on demand.  With CHECK_STATUS = True every call synchronises and checks
+# before returning (tests do that).
 CHECK_STATUS = False
 
-_pending = {}      # device index -> list of (event, pinned int32 tensor, description)
-_side_streams = {}  # device index -> stream the status words are copied on
+_pending = {}      # device index -> list of (event, pinned int32 tensor, description): words of a caller's
+                   # own C-ABI calls, looked at in the same places
 
 
 def poll_status(device=None, wait=False):
     """Raise if a chunked-kernel call on ``device`` (default: all devices) reported a device-side
     wait that ran out.  ``wait=True`` first waits for the calls issued so far."""
-    keys = list(_pending) if device is None else [torch.device(device).index or 0]
-    for key in keys:
+    index = None if device is None else (torch.device(device).index or 0)
+    L.native().poll_status(-1 if index is None else index, wait)
+    for key in list(_pending) if index is None else [index]:
         still = []
         for ev, word, what in _pending.get(key, []):
             if wait:
@@ -42,30 +41,24 @@ def poll_status(device=None, wait=False):
         _pending[key] = still
 
 
-def _watch_status(lib, a, variant, ws, what):
-    if ws is None or ws.numel() < 4 or not lib.wkv56_uses_chunked(ctypes.byref(a), int(variant == "wkv6")):
-        return
-    if CHECK_STATUS:
-        torch.cuda.synchronize(ws.device)
-        code = int(ws[:4].view(torch.int32).item())
-        if code != 0:
-            raise RuntimeError(f"{what}: a device-side wait ran out (status {code})")
-        return
-    key = ws.device.index or 0
-    side = _side_streams.get(key)
-    if side is None:
-        side = _side_streams[key] = torch.cuda.Stream(ws.device)
-    # the copy runs on a side stream so that it never sits between two kernels of the caller's stream
-    done = torch.cuda.Event()
-    done.record(torch.cuda.current_stream(ws.device))
-    word = torch.empty(1, dtype=torch.int32, pin_memory=True)
-    with torch.cuda.stream(side):
-        side.wait_event(done)
-        word.copy_(ws[:4].view(torch.int32), non_blocking=True)
-        ev = torch.cuda.Event()
-        ev.record(side)
-    ws.record_stream(side)
-    _pending.setdefault(key, []).append((ev, word, what))
+def apply(variant, B, T, C, H, r, k, v, w, u, state_in, path, saved):
+    """``WKV5.apply`` / ``WKV6.apply``"""
+    if _pending:
+        poll_status(r.device)
+    if saved is None:
+        return L.native().wkv56_apply(variant == "wkv6", B, T, C, H, r, k, v, w, u, state_in, path, None, 0,
+                                      CHECK_STATUS)
+    mode, buf = saved._attach(variant, r, path)
+    out = L.native().wkv56_apply(variant == "wkv6", B, T, C, H, r, k, v, w, u, state_in, path, buf, mode, CHECK_STATUS)
+    saved._done(mode)
+    return out
+
+
+def apply_dropin(variant, B, T, C, H, r, k, v, w, u, state):
+    """``WKV5_CUDA.apply`` / ``WKV6STATE_CUDA.apply``: ``state`` [B,H,value,key] updated in place"""
+    if _pending:
+        poll_status(r.device)
+    return L.native().wkv56_dropin(variant == "wkv6", B, T, C, H, r, k, v, w, u, state, CHECK_STATUS)
 
 
 def _check_layout(B, T, C, **tensors):
@@ -105,39 +98,14 @@ def forward(variant: str, r, k, v, w, u, state_in, *, w_kind, layout=L.WKV_STATE
     ``time_groups``: see ``wkv_args_t.time_groups`` (0 = the library decides).
     ``saved``: a ``SavedStates``; empty, the call fills it; filled (by a call with the same
     inputs), the call restarts from it instead of scanning over T."""
-    B, T, C = r.shape
-    H = C // HEAD_SIZE
-    dev = L.require_cuda(r, k, v, w, u, state_in)
-    _check_layout(B, T, C, r=r, k=k, v=v, w=w if variant == "wkv6" else None)
-    for name, t in (("u", u), ("state_in", state_in), ("state_out", state_out)):
-        if t is not None and not t.is_contiguous():
-            raise ValueError(f"{name} must be contiguous")
-    poll_status(dev)
-    y = torch.empty_like(r)
-    if state_out is None:
-        state_out = torch.empty((B, H, HEAD_SIZE, HEAD_SIZE), device=dev, dtype=torch.float32)
-    lib = L.load()
-    with torch.cuda.device(dev):
-        a = _args(variant, B, T, H, r.dtype, w_kind, layout, path, time_groups, r=r, k=k, v=v, w=w,
-                  u=u, state_in=state_in, y=y, state_out=state_out)
-        ckpt = None
-        if save_ckpt:
-            nck = lib.wkv56_state_ckpt_bytes(ctypes.byref(a), int(variant == "wkv6"))
-            if nck:
-                ckpt = torch.empty(nck, dtype=torch.uint8, device=dev)
-                a.state_ckpt, a.state_ckpt_bytes = L.ptr(ckpt), nck
-        if saved is not None and lib.wkv56_uses_chunked(ctypes.byref(a), int(variant == "wkv6")):
-            saved._attach(lib, a, (variant, B, T, H, r.dtype, w_kind, layout), dev)
-        ws = _with_workspace(lib, variant, "forward", a, dev)
-        L.check(getattr(lib, f"{variant}_forward")(ctypes.byref(a), L.stream_handle(dev)),
-                f"{variant}_forward")
-        if saved is not None:
-            saved._done(a, state_out)
-        _watch_status(lib, a, variant, ws, f"{variant}_forward")
-        del ws
-    if save_ckpt:
-        return y, state_out, ckpt
-    return y, state_out
+    if _pending:
+        poll_status(r.device)
+    mode, buf = (0, None) if saved is None else saved._attach(variant, r, path, w_kind, layout)
+    y, state_out, ckpt = L.native().wkv56_forward(variant == "wkv6", r, k, v, w, u, state_in, w_kind, layout, path,
+                                                  state_out, save_ckpt, time_groups, buf, mode, CHECK_STATUS)
+    if saved is not None:
+        saved._done(mode)
+    return (y, state_out, ckpt) if save_ckpt else (y, state_out)
 
 
 def backward(variant: str, r, k, v, w, u, state_in, gy, gstate_out, *, w_kind,
@@ -145,35 +113,10 @@ def backward(variant: str, r, k, v, w, u, state_in, gy, gstate_out, *, w_kind,
              time_groups=0):
     """Launch wkv5_backward / wkv6_backward.  Returns gr, gk, gv, gw, gu, gstate_in with
     gw = [B,T,C] (v6, activation dtype) or [B,C] fp32 per-batch partials (v5); gu [B,C] fp32."""
-    B, T, C = r.shape
-    H = C // HEAD_SIZE
-    dev = L.require_cuda(r, k, v, w, u, state_in, gy, gstate_out)
-    _check_layout(B, T, C, r=r, k=k, v=v, gy=gy, w=w if variant == "wkv6" else None)
-    for name, t in (("u", u), ("state_in", state_in), ("gstate_out", gstate_out)):
-        if t is not None and not t.is_contiguous():
-            raise ValueError(f"{name} must be contiguous")
-    poll_status(dev)
-    gr, gk, gv = torch.empty_like(r), torch.empty_like(r), torch.empty_like(r)
-    if variant == "wkv6":
-        gw = torch.empty_like(r)
-    else:
-        gw = torch.empty((B, C), device=dev, dtype=torch.float32)
-    gu = torch.empty((B, C), device=dev, dtype=torch.float32)
-    gsi = (torch.empty((B, H, HEAD_SIZE, HEAD_SIZE), device=dev, dtype=torch.float32)
-           if want_gstate else None)
-    lib = L.load()
-    with torch.cuda.device(dev):
-        a = _args(variant, B, T, H, r.dtype, w_kind, layout, path, time_groups, r=r, k=k, v=v, w=w,
-                  u=u, state_in=state_in, gy=gy, gstate_out=gstate_out, gr=gr, gk=gk, gv=gv, gw=gw,
-                  gu=gu, gstate_in=gsi)
-        if ckpt is not None:
-            a.state_ckpt, a.state_ckpt_bytes = L.ptr(ckpt), ckpt.numel()
-        ws = _with_workspace(lib, variant, "backward", a, dev)
-        L.check(getattr(lib, f"{variant}_backward")(ctypes.byref(a), L.stream_handle(dev)),
-                f"{variant}_backward")
-        _watch_status(lib, a, variant, ws, f"{variant}_backward")
-        del ws
-    return gr, gk, gv, gw, gu, gsi
+    if _pending:
+        poll_status(r.device)
+    return L.native().wkv56_backward(variant == "wkv6", r, k, v, w, u, state_in, gy, gstate_out, w_kind, layout, path,
+                                     want_gstate, ckpt, time_groups, CHECK_STATUS)
 
 
 class Prepared:
@@ -264,18 +207,23 @@ class SavedStates:
     def clear(self):
         self.buf, self.key, self.filled, self.restarts = None, None, False, 0
 
-    def _attach(self, lib, a, key, dev):
-        n = lib.wkv56_group_states_bytes(ctypes.byref(a))
+    def _attach(self, variant, r, path, w_kind=L.WKV_W_RAW, layout=L.WKV_STATE_KV):
+        """-> (group_states_mode, buffer) for a call on these tensors; (NONE, None) when it would not run on
+        the chunked kernels"""
+        B, T, C = r.shape
+        dev = L.require_cuda(r)
+        lib = L.load()
+        a = _args(variant, B, T, C // HEAD_SIZE, r.dtype, w_kind, layout, path)
+        if not lib.wkv56_uses_chunked(ctypes.byref(a), int(variant == "wkv6")):
+            return L.WKV_GROUP_STATES_NONE, None
+        key = (variant, B, T, C, r.dtype, w_kind, layout)
         if self.filled and self.key == key and self.buf is not None and self.buf.device == dev:
-            a.group_states, a.group_states_bytes = L.ptr(self.buf), n
-            a.group_states_mode = L.WKV_GROUP_STATES_USE
             self.restarts += 1
-        else:
-            self.buf = torch.empty(n, dtype=torch.uint8, device=dev)
-            self.key, self.filled = key, False
-            a.group_states, a.group_states_bytes = L.ptr(self.buf), n
-            a.group_states_mode = L.WKV_GROUP_STATES_SAVE
+            return L.WKV_GROUP_STATES_USE, self.buf
+        self.buf = torch.empty(lib.wkv56_group_states_bytes(ctypes.byref(a)), dtype=torch.uint8, device=dev)
+        self.key, self.filled = key, False
+        return L.WKV_GROUP_STATES_SAVE, self.buf
 
-    def _done(self, a, state_out):
-        if a.group_states_mode == L.WKV_GROUP_STATES_SAVE:
+    def _done(self, mode):
+        if mode == L.WKV_GROUP_STATES_SAVE:
             self.filled = True

@@ -25,42 +25,10 @@ from . import wkv56
 N = wkv56.HEAD_SIZE
 
 
-class WKV6(torch.autograd.Function):
+class WKV6:
     @staticmethod
-    def forward(ctx, B, T, C, H, r, k, v, w, u, state_in, path=L.WKV_PATH_AUTO, saved=None):
-        if C != H * N:
-            raise ValueError(f"C must equal H*{N}")
-        for name, t in (("r", r), ("k", k), ("v", v), ("w", w)):
-            if tuple(t.shape) != (B, T, C):
-                raise ValueError(f"{name} must be [B,T,C]")
-        if u.numel() != C or state_in.numel() != B * H * N * N:
-            raise ValueError("u must be [H,N] and state [B,H,N,N]")
-        dt = r.dtype
-        r, k, v = r.contiguous(), k.to(dt).contiguous(), v.to(dt).contiguous()
-        wx = w.to(dt).contiguous()
-        uf = u.to(dt).contiguous()
-        s_in = state_in.float().contiguous()
-        # the hand-over to backward is only built when something asks for a gradient (not in the
-        # first, autograd-free run of a checkpointed block)
-        y, s_out, ckpt = wkv56.forward("wkv6", r, k, v, wx, uf, s_in, w_kind=L.WKV_W_RAW, path=path,
-                                       save_ckpt=any(ctx.needs_input_grad), saved=saved)
-        ctx.has_ckpt = ckpt is not None
-        ctx.save_for_backward(*((r, k, v, wx, uf, s_in) + ((ckpt,) if ckpt is not None else ())))
-        ctx.meta = (B, T, C, H, path, w.dtype, u.dtype, u.shape, state_in.dtype)
-        return y, s_out.view(B, H, N, N)
-
-    @staticmethod
-    def backward(ctx, gy, gstate_out):
-        st = ctx.saved_tensors          # (one access: saved-tensor hooks unpack once)
-        r, k, v, wx, uf, s_in = st[:6]
-        ckpt = st[6] if ctx.has_ckpt else None
-        B, T, C, H, path, wdt, udt, ushape, sdt = ctx.meta
-        gy = gy.to(r.dtype).contiguous()
-        gso = None if gstate_out is None else gstate_out.float().contiguous()
-        gr, gk, gv, gw, gu, gsi = wkv56.backward("wkv6", r, k, v, wx, uf, s_in, gy, gso,
-                                                 w_kind=L.WKV_W_RAW, path=path, ckpt=ckpt)
-        return (None, None, None, None, gr, gk, gv, gw.to(wdt), gu.sum(0).view(ushape).to(udt),
-                gsi.to(sdt), None, None)
+    def apply(B, T, C, H, r, k, v, w, u, state_in, path=L.WKV_PATH_AUTO, saved=None):
+        return wkv56.apply("wkv6", B, T, C, H, r, k, v, w, u, state_in, path, saved)
 
 
 def wkv6(r, k, v, w, u, state_in, path=L.WKV_PATH_AUTO, saved=None):
@@ -141,7 +109,7 @@ class _Wkv6Kernel:
 wkv6_cuda_kernel = _Wkv6Kernel()
 
 
-class WKV6STATE_CUDA(torch.autograd.Function):
+class WKV6STATE_CUDA:
     """RWKV-v6/src/module/TimeMix.py:19-109: ``apply(B,T,C,H,r,k,v,w,u,s) -> y`` with
     ``s`` updated in place ([value,key] layout, any float dtype, indexed per batch row);
     backward returns (gr,gk,gv,gw,gu,gs).  The raw decay activation ``w`` goes to the
@@ -150,43 +118,8 @@ class WKV6STATE_CUDA(torch.autograd.Function):
     signature with the precomputed ``ew`` for callers that use it directly."""
 
     @staticmethod
-    def forward(ctx, B, T, C, H, r, k, v, w, u, s):
-        with torch.no_grad():
-            dtype = r.dtype
-            ctx.B, ctx.T, ctx.C, ctx.H, ctx.dtype = B, T, C, H, dtype
-            for t in (s, w, r, k, v, u):
-                if not t.is_contiguous():
-                    raise ValueError("inputs must be contiguous")
-            if not (dtype == k.dtype == v.dtype == u.dtype):
-                raise TypeError("r,k,v,u must share one dtype")
-            if dtype not in L.DTYPE_CODE:
-                raise ValueError(f"Unsupported dtype {dtype} for WKV6_CUDA")
-            wx = w.to(dtype).contiguous()
-            s32 = s.float().contiguous()
-            s_in = s32.clone()
-            y, _, ckpt = wkv56.forward("wkv6", r, k, v, wx, u, s32, w_kind=L.WKV_W_RAW,
-                                       layout=L.WKV_STATE_VK, state_out=s32, save_ckpt=True)
-            if s32.data_ptr() != s.data_ptr():
-                s.copy_(s32.view_as(s))
-            ctx.has_ckpt = ckpt is not None
-            ctx.save_for_backward(*((r, k, v, wx, u, s_in) + ((ckpt,) if ckpt is not None else ())))
-            ctx.s_dtype, ctx.w_dtype = s.dtype, w.dtype
-            return y
-
-    @staticmethod
-    def backward(ctx, gy):
-        with torch.no_grad():
-            B, T, C, H, dtype = ctx.B, ctx.T, ctx.C, ctx.H, ctx.dtype
-            gy = gy.to(dtype).contiguous()
-            st = ctx.saved_tensors          # (one access: saved-tensor hooks unpack once)
-            r, k, v, wx, u, s_in = st[:6]
-            ckpt = st[6] if ctx.has_ckpt else None
-            gr, gk, gv, gw, gu, gs = wkv56.backward("wkv6", r, k, v, wx, u, s_in, gy, None,
-                                                    w_kind=L.WKV_W_RAW, layout=L.WKV_STATE_VK,
-                                                    ckpt=ckpt)
-            gu = torch.sum(gu, 0).view(H, C // H).to(dtype)
-            return (None, None, None, None, gr, gk, gv, gw.to(ctx.w_dtype), gu,
-                    gs.view(B, H, C // H, C // H).to(ctx.s_dtype))
+    def apply(B, T, C, H, r, k, v, w, u, s):
+        return wkv56.apply_dropin("wkv6", B, T, C, H, r, k, v, w, u, s)
 
 
 def RUN_WKV6STATE_CUDA(B, T, C, H, r, k, v, w, u, s):
