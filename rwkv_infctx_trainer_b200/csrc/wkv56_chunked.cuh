@@ -270,7 +270,6 @@ struct CallOpts {
 // gw_part NULL: gu alone
 int fold_param_grads(const float *gu_part, const float *gw_part, int B, int H, int n, const CallOpts &opt, cudaStream_t s);
 
-int device_sm_count();
 size_t chunked_group_states_bytes(const wkv_args_t *a);
 // v6 with the fp32 ew = -exp(x) encoding: bytes of, and conversion into, a bf16 x tensor (a no-op otherwise)
 size_t chunked_wconv_bytes(const wkv_args_t *a, bool per_token_w);

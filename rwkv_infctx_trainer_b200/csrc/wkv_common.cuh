@@ -56,9 +56,12 @@ inline int launch_chained(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t 
     return cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...) == cudaSuccess ? WKV_OK : WKV_ERR_LAUNCH;
 }
 
+int device_sm_count();    // of the current device (wkv56_chunked.cu)
+
 // scalar (token-serial) v5/v6 kernels, wkv56_scalar.cu
 size_t scalar_backward_workspace(const wkv_args_t *a);
-int scalar_forward(const wkv_args_t *a, bool per_token_w, cudaStream_t s);
+// floor: decays floored at 0.005, as the chunked kernels do
+int scalar_forward(const wkv_args_t *a, bool per_token_w, bool floor, cudaStream_t s);
 int scalar_backward(const wkv_args_t *a, bool per_token_w, cudaStream_t s);
 
 // chunked tensor-core v5/v6 kernels, wkv56_chunked.cu
