@@ -87,9 +87,9 @@ const char *wkv_error_string(int code);
  *              multiplied by w (wkv_cuda_bf16.cu:156)
  *   gstate_*   fp32 [B,C,3] = (gp,gq,go) in the exponent-scaled convention of
  *              wkv_cuda_bf16.cu:116-152; gstate_out may be NULL (= none)
- * No compile-time limit on T (the project needs T <= Tmax).  Segments of 128 tokens or
- * more are cut into 64-token pieces that run in parallel (piece summaries are folded per
- * channel); that needs the scratch memory wkv4_*_workspace() sizes.
+ * No compile-time limit on T (the project needs T <= Tmax).  Segments of 16 tokens or more
+ * run in tiles of 8 tokens in parallel (tile summaries are folded per channel).  The workspace
+ * must be at least what wkv4_*_workspace() says.
  */
 size_t wkv4_forward_workspace(int B, int T, int C);
 
@@ -106,10 +106,9 @@ int wkv4_backward(int B, int T, int C, int dtype, const float *w, const void *u,
                   size_t workspace_bytes, void *stream);
 
 /* Optional hand-over from forward to backward of the same segment (no counterpart in the project,
- * whose backward recomputes everything): wkv4_state_ckpt_bytes() bytes (2.5 per token-channel) that
- * receive, for every 8th token, the state and its derivative w.r.t. the decay.  Backward given the
- * buffer skips rebuilding the states and the forward sweeps of its two passes (three passes over k
- * and v less).  0 bytes / NULL for segments under 128 tokens; NULL is always allowed and
+ * whose backward recomputes everything): wkv4_state_ckpt_bytes() bytes (1.5 per token-channel) that
+ * receive the state at every 8th token.  Backward given the buffer skips rebuilding the states (a pass
+ * over k and v).  0 bytes / NULL for segments under 128 tokens; NULL is always allowed and
  * makes the _ckpt entry points identical to the plain ones. */
 size_t wkv4_state_ckpt_bytes(int B, int T, int C);
 int wkv4_forward_ckpt(int B, int T, int C, int dtype, const float *w, const void *u, const void *k,

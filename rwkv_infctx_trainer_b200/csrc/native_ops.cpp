@@ -327,13 +327,13 @@ struct Wkv4Function : torch::autograd::Function<Wkv4Function> {
         const int B = (int)raw_k.size(0), T = (int)raw_k.size(1), C = (int)raw_k.size(2);
         const auto dt = raw_k.scalar_type();
         c10::cuda::OptionalCUDAGuard guard(raw_k.device());
-        const Tensor w = as_contig(raw_w, at::kFloat).exp().neg_(), u = as_contig(raw_u, dt), k = contig(raw_k),
-                     v = as_contig(raw_v, dt), state = as_contig(raw_state, at::kFloat);
+        const auto wt = raw_w.scalar_type() == at::kDouble ? at::kFloat : raw_w.scalar_type();
+        const Tensor w = as_contig(raw_w, wt), u = as_contig(raw_u, dt), k = contig(raw_k), v = as_contig(raw_v, dt),
+                     state = as_contig(raw_state, at::kFloat);
         Tensor y = at::empty_like(k), new_state = at::empty_like(state);
-        const size_t nws = wkv4_forward_workspace(B, T, C), nck = save ? wkv4_state_ckpt_bytes(B, T, C) : 0;
-        Tensor ws = bytes_like(k, nws), ck = bytes_like(k, nck);
-        check(wkv4_forward_ckpt(B, T, C, dtype_code(dt), (const float *)ptr(w), ptr(u), ptr(k), ptr(v), (const float *)ptr(state),
-                                ptr(y), (float *)ptr(new_state), ptr(ws), nws, ptr(ck), nck, stream_of(k)),
+        Tensor ck = bytes_like(k, save ? wkv4_state_ckpt_bytes(B, T, C) : 0);
+        check(wkv4x_forward(B, T, C, dtype_code(dt), ptr(w), dtype_code(wt), ptr(u), ptr(k), ptr(v), (const float *)ptr(state), ptr(y),
+                            (float *)ptr(new_state), ptr(ck), stream_of(k)),
               "wkv4_forward");
         if (save) {
             ctx->save_for_backward({w, u, k, v, state, ck});
@@ -351,16 +351,15 @@ struct Wkv4Function : torch::autograd::Function<Wkv4Function> {
         c10::cuda::OptionalCUDAGuard guard(k.device());
         const Tensor gy = grads[0].defined() ? as_contig(grads[0], k.scalar_type()) : at::zeros_like(k);
         const Tensor gs = grads[1].defined() ? as_contig(grads[1], at::kFloat) : Tensor();
-        Tensor gw = at::empty({B, C}, w.options()), gu = at::empty({B, C}, w.options()), gk = at::empty_like(k),
-               gv = at::empty_like(k), glast = at::empty_like(state);
-        const size_t nws = wkv4_backward_workspace(B, T, C);
-        Tensor ws = bytes_like(k, nws);
-        check(wkv4_backward_ckpt(B, T, C, dtype_code(k.scalar_type()), (const float *)ptr(w), ptr(u), ptr(k), ptr(v),
-                                 (const float *)ptr(state), ptr(gy), (const float *)ptr(gs), (float *)ptr(gw), (float *)ptr(gu),
-                                 ptr(gk), ptr(gv), (float *)ptr(glast), ptr(ws), nws, ptr(ck), ck.defined() ? (size_t)ck.numel() : 0,
-                                 stream_of(k)),
+        const auto u_type = (at::ScalarType)types[1] == at::kDouble ? at::kFloat : (at::ScalarType)types[1];
+        Tensor gw = B ? at::empty_like(w) : at::zeros_like(w), gk = at::empty_like(k), gv = at::empty_like(k), glast = at::empty_like(state),
+               gu = B ? at::empty({C}, u.options().dtype(u_type)) : at::zeros({C}, u.options().dtype(u_type));
+        Tensor ws = bytes_like(k, wkv4x_backward_workspace(B, T, C, ck.defined()));
+        check(wkv4x_backward(B, T, C, dtype_code(k.scalar_type()), ptr(w), dtype_code(w.scalar_type()), ptr(u), ptr(k), ptr(v),
+                             (const float *)ptr(state), ptr(gy), (const float *)ptr(gs), ptr(gw), ptr(gu), dtype_code(u_type), ptr(gk),
+                             ptr(gv), (float *)ptr(glast), ptr(ws), ptr(ck), stream_of(k)),
               "wkv4_backward");
-        return {gw.sum(0).to((at::ScalarType)types[0]), gu.sum(0).to((at::ScalarType)types[1]), gk, gv.to((at::ScalarType)types[2]),
+        return {gw.to((at::ScalarType)types[0]), gu.to((at::ScalarType)types[1]), gk, gv.to((at::ScalarType)types[2]),
                 glast.to((at::ScalarType)types[3]), Tensor()};
     }
 };

@@ -1,18 +1,22 @@
 // v4 WKV (aa/bb/pp state): log-space-stabilised scan over T, forward and backward
 // with the (p,q,o) state and its (gp,gq,go) gradient carried across segments.
 //
+// This file: the one-thread-per-chain kernels for segments of a few tokens (decode), and the C ABI.
+// Longer segments run on the time-parallel kernels of wkv4_par.cu.
+//
 // Math: RWKV-v4neo/cuda/wkv_cuda_bf16.cu:7-53 (forward), :55-158 (backward).
 // Differences in execution: one of the two exponentials of every max-shifted
 // pair is exp(0), so each pair costs one exp; the backward keeps no per-thread
 // T-sized arrays -- a forward sweep writes the state at the start of every
 // TILE tokens to the workspace and the reverse sweep recomputes one tile at a
 // time into registers; T is a run-time argument.
-#include "wkv_common.cuh"
+#include "wkv4_common.cuh"
+#include "wkv_internal.h"
 
 namespace wkv {
 namespace {
 
-constexpr float MIN_VALUE = -1e38f;
+constexpr float MIN_VALUE = V4_MIN_VALUE;
 constexpr int TILE = 16;
 constexpr int THREADS = 128;
 
@@ -28,13 +32,13 @@ __device__ __forceinline__ void exp_pair(float a, float b, float &A, float &Bv, 
 
 template <typename F>
 __global__ void __launch_bounds__(THREADS)
-k_v4_fwd(int B, int T, int C, const float *__restrict__ w_, const F *__restrict__ u_,
+k_v4_fwd(int B, int T, int C, const Decay4 w_, const F *__restrict__ u_,
          const F *__restrict__ k_, const F *__restrict__ v_, const float *__restrict__ state_in,
          F *__restrict__ y_, float *__restrict__ state_out) {
     const int idx = blockIdx.x * THREADS + threadIdx.x;
     if (idx >= B * C) return;
     const int b = idx / C, c = idx % C;
-    const float w = w_[c], u = Elem<F>::ld(u_ + c);
+    const float w = w_.at(c), u = Elem<F>::ld(u_ + c);
     const size_t off = (size_t)b * T * C + c, so = (size_t)idx * 3;
     float p = 0.f, q = 0.f, o = MIN_VALUE;
     if (state_in) { p = state_in[so]; q = state_in[so + 1]; o = state_in[so + 2]; }
@@ -52,7 +56,7 @@ k_v4_fwd(int B, int T, int C, const float *__restrict__ w_, const F *__restrict_
 
 template <typename F>
 __global__ void __launch_bounds__(THREADS)
-k_v4_bwd(int B, int T, int C, const float *__restrict__ w_, const F *__restrict__ u_,
+k_v4_bwd(int B, int T, int C, const Decay4 w_, const F *__restrict__ u_,
          const F *__restrict__ k_, const F *__restrict__ v_, const float *__restrict__ state_in,
          const F *__restrict__ gy_, const float *__restrict__ gstate_out, float *__restrict__ gw_,
          float *__restrict__ gu_, F *__restrict__ gk_, F *__restrict__ gv_,
@@ -60,7 +64,7 @@ k_v4_bwd(int B, int T, int C, const float *__restrict__ w_, const F *__restrict_
     const int idx = blockIdx.x * THREADS + threadIdx.x;
     if (idx >= B * C) return;
     const int b = idx / C, c = idx % C;
-    const float w = w_[c], u = Elem<F>::ld(u_ + c);
+    const float w = w_.at(c), u = Elem<F>::ld(u_ + c);
     const size_t off = (size_t)b * T * C + c, so = (size_t)idx * 3;
     const int ntile = (T + TILE - 1) / TILE;
     // workspace [B][ntile][3][C]
@@ -134,7 +138,7 @@ k_v4_bwd(int B, int T, int C, const float *__restrict__ w_, const F *__restrict_
 }
 
 template <typename F>
-int fwd(int B, int T, int C, const float *w, const void *u, const void *k, const void *v,
+int fwd(int B, int T, int C, const Decay4 &w, const void *u, const void *k, const void *v,
         const float *si, void *y, float *so, cudaStream_t s) {
     const int n = B * C;
     k_v4_fwd<F><<<(n + THREADS - 1) / THREADS, THREADS, 0, s>>>(
@@ -143,7 +147,7 @@ int fwd(int B, int T, int C, const float *w, const void *u, const void *k, const
 }
 
 template <typename F>
-int bwd(int B, int T, int C, const float *w, const void *u, const void *k, const void *v,
+int bwd(int B, int T, int C, const Decay4 &w, const void *u, const void *k, const void *v,
         const float *si, const void *gy, const float *gso, float *gw, float *gu, void *gk,
         void *gv, float *gsi, float *ws, cudaStream_t s) {
     const int n = B * C;
@@ -153,8 +157,33 @@ int bwd(int B, int T, int C, const float *w, const void *u, const void *k, const
     return launch_status();
 }
 
-// segments shorter than this run on the one-thread-per-chain kernels above
-constexpr int PAR_MIN_T = 128;
+// Segments shorter than this run on the kernels above: with two tiles of 8 tokens there is little to
+// parallelise, and the time-parallel kernels' barriers cost more than the chain.
+constexpr int PAR_MIN_T = 16;
+// Segments of at least this many tokens hand tile states from forward to backward (part of the ABI, as are the
+// workspace sizes below, which the kernels use only a part of).
+constexpr int CKPT_MIN_T = 128;
+constexpr int PIECE = 64;
+
+// gw_sum, gu_sum [C]: the per-batch partials [B,C] summed over the batch, in the parameters' element types
+__device__ __forceinline__ void store_as(void *p, int dtype, int i, float x) {
+    if (dtype == WKV_F32) ((float *)p)[i] = x;
+    else if (dtype == WKV_BF16) ((__nv_bfloat16 *)p)[i] = __float2bfloat16_rn(x);
+    else ((__half *)p)[i] = __float2half_rn(x);
+}
+__global__ void __launch_bounds__(THREADS)
+k_v4_fold(const float *__restrict__ gw, const float *__restrict__ gu, void *gw_sum, int gw_dtype, void *gu_sum, int gu_dtype,
+          int B, int C) {
+    pdl_wait();
+    pdl_trigger();
+    const int c = blockIdx.x * THREADS + threadIdx.x;
+    if (c >= C) return;
+    const float *src = blockIdx.y ? gu : gw;
+    float a = 0.f;
+#pragma unroll 8
+    for (int b = 0; b < B; b++) a += src[(size_t)b * C + c];
+    store_as(blockIdx.y ? gu_sum : gw_sum, blockIdx.y ? gu_dtype : gw_dtype, c, a);
+}
 
 size_t serial_backward_workspace(int B, int T, int C) {
     if (B <= 0 || T <= 0 || C <= 0) return 0;
@@ -165,25 +194,48 @@ size_t serial_backward_workspace(int B, int T, int C) {
 }  // namespace
 
 // time-parallel kernels, wkv4_par.cu
-size_t v4_par_forward_workspace(int B, int T, int C);
-size_t v4_par_backward_workspace(int B, int T, int C);
 size_t v4_par_ckpt_bytes(int B, int T, int C);
-int v4_par_forward(int B, int T, int C, int dtype, const float *w, const void *u, const void *k, const void *v,
-                   const float *si, void *y, float *so, float *ws, float *ckpt, cudaStream_t s);
-int v4_par_backward(int B, int T, int C, int dtype, const float *w, const void *u, const void *k, const void *v,
+int v4_par_forward(int B, int T, int C, int dtype, const Decay4 &w, const void *u, const void *k, const void *v,
+                   const float *si, void *y, float *so, float *ckpt, cudaStream_t s);
+int v4_par_backward(int B, int T, int C, int dtype, const Decay4 &w, const void *u, const void *k, const void *v,
                     const float *si, const void *gy, const float *gso, float *gw, float *gu, void *gk, void *gv,
                     float *gsi, float *ws, const float *ckpt, cudaStream_t s);
+
+namespace {
+
+int run_forward(int B, int T, int C, int dtype, const Decay4 &w, const void *u, const void *k, const void *v,
+                const float *si, void *y, float *so, float *ckpt, cudaStream_t s) {
+    if (T >= PAR_MIN_T) return v4_par_forward(B, T, C, dtype, w, u, k, v, si, y, so, ckpt, s);
+    switch (dtype) {
+        case WKV_F32: return fwd<float>(B, T, C, w, u, k, v, si, y, so, s);
+        case WKV_BF16: return fwd<__nv_bfloat16>(B, T, C, w, u, k, v, si, y, so, s);
+        default: return fwd<__half>(B, T, C, w, u, k, v, si, y, so, s);
+    }
+}
+int run_backward(int B, int T, int C, int dtype, const Decay4 &w, const void *u, const void *k, const void *v,
+                 const float *si, const void *gy, const float *gso, float *gw, float *gu, void *gk, void *gv, float *gsi,
+                 float *ws, const float *ckpt, cudaStream_t s) {
+    if (T >= PAR_MIN_T) return v4_par_backward(B, T, C, dtype, w, u, k, v, si, gy, gso, gw, gu, gk, gv, gsi, ws, ckpt, s);
+    switch (dtype) {
+        case WKV_F32: return bwd<float>(B, T, C, w, u, k, v, si, gy, gso, gw, gu, gk, gv, gsi, ws, s);
+        case WKV_BF16: return bwd<__nv_bfloat16>(B, T, C, w, u, k, v, si, gy, gso, gw, gu, gk, gv, gsi, ws, s);
+        default: return bwd<__half>(B, T, C, w, u, k, v, si, gy, gso, gw, gu, gk, gv, gsi, ws, s);
+    }
+}
+bool known_dtype(int dtype) { return dtype == WKV_F32 || dtype == WKV_BF16 || dtype == WKV_F16; }
+
+}  // namespace
 }  // namespace wkv
 
 using namespace wkv;
 
 extern "C" size_t wkv4_forward_workspace(int B, int T, int C) {
-    if (B <= 0 || C <= 0 || T < PAR_MIN_T) return 0;
-    return v4_par_forward_workspace(B, T, C);
+    if (B <= 0 || C <= 0 || T < CKPT_MIN_T) return 0;
+    return 2 * (size_t)B * ((T + PIECE - 1) / PIECE) * 3 * C * sizeof(float);
 }
 
 extern "C" size_t wkv4_state_ckpt_bytes(int B, int T, int C) {
-    if (B <= 0 || C <= 0 || T < PAR_MIN_T) return 0;
+    if (B <= 0 || C <= 0 || T < CKPT_MIN_T) return 0;
     return v4_par_ckpt_bytes(B, T, C);
 }
 
@@ -203,25 +255,19 @@ extern "C" int wkv4_forward_ckpt(int B, int T, int C, int dtype, const float *w,
     if (!w || !u) return WKV_ERR_NULL;
     if (T > 0 && (!k || !v || !y)) return WKV_ERR_NULL;
     if (dtype != WKV_F32 && dtype != WKV_BF16 && dtype != WKV_F16) return WKV_ERR_DTYPE;
-    cudaStream_t s = (cudaStream_t)stream;
-    if (T >= PAR_MIN_T) {
+    if (T >= CKPT_MIN_T) {
         if (!workspace || workspace_bytes < wkv4_forward_workspace(B, T, C)) return WKV_ERR_WORKSPACE;
         if (state_ckpt && state_ckpt_bytes < wkv4_state_ckpt_bytes(B, T, C)) return WKV_ERR_WORKSPACE;
-        return v4_par_forward(B, T, C, dtype, w, u, k, v, state_in, y, state_out, (float *)workspace,
-                              (float *)state_ckpt, s);
+    } else {
+        state_ckpt = nullptr;
     }
-    switch (dtype) {
-        case WKV_F32: return fwd<float>(B, T, C, w, u, k, v, state_in, y, state_out, s);
-        case WKV_BF16: return fwd<__nv_bfloat16>(B, T, C, w, u, k, v, state_in, y, state_out, s);
-        case WKV_F16: return fwd<__half>(B, T, C, w, u, k, v, state_in, y, state_out, s);
-    }
-    return WKV_ERR_DTYPE;
+    return run_forward(B, T, C, dtype, Decay4{w, -1}, u, k, v, state_in, y, state_out, (float *)state_ckpt, (cudaStream_t)stream);
 }
 
 extern "C" size_t wkv4_backward_workspace(int B, int T, int C) {
     if (B <= 0 || T <= 0 || C <= 0) return 0;
     const size_t a = serial_backward_workspace(B, T, C);
-    const size_t b = T >= PAR_MIN_T ? v4_par_backward_workspace(B, T, C) : 0;
+    const size_t b = T >= CKPT_MIN_T ? (4 * 3 + 2) * (size_t)B * ((T + PIECE - 1) / PIECE) * C * sizeof(float) : 0;
     return a > b ? a : b;
 }
 
@@ -246,22 +292,48 @@ extern "C" int wkv4_backward_ckpt(int B, int T, int C, int dtype, const float *w
     const size_t need = wkv4_backward_workspace(B, T, C);
     if (need && (!workspace || workspace_bytes < need)) return WKV_ERR_WORKSPACE;
     if (dtype != WKV_F32 && dtype != WKV_BF16 && dtype != WKV_F16) return WKV_ERR_DTYPE;
+    if (T < CKPT_MIN_T) state_ckpt = nullptr;
+    else if (state_ckpt && state_ckpt_bytes < wkv4_state_ckpt_bytes(B, T, C)) return WKV_ERR_WORKSPACE;
+    return run_backward(B, T, C, dtype, Decay4{w, -1}, u, k, v, state_in, gy, gstate_out, gw, gu, gk, gv, gstate_in,
+                        (float *)workspace, (const float *)state_ckpt, (cudaStream_t)stream);
+}
+
+extern "C" int wkv4x_forward(int B, int T, int C, int dtype, const void *time_decay, int decay_dtype, const void *u,
+                             const void *k, const void *v, const float *state_in, void *y, float *state_out,
+                             void *state_ckpt, void *stream) {
+    if (B < 0 || T < 0 || C < 0) return WKV_ERR_SHAPE;
+    if (B == 0 || C == 0) return WKV_OK;
+    if (!time_decay || !u || (T > 0 && (!k || !v || !y))) return WKV_ERR_NULL;
+    if (!known_dtype(dtype) || !known_dtype(decay_dtype)) return WKV_ERR_DTYPE;
+    return run_forward(B, T, C, dtype, Decay4{time_decay, decay_dtype}, u, k, v, state_in, y, state_out,
+                       T < CKPT_MIN_T ? nullptr : (float *)state_ckpt, (cudaStream_t)stream);
+}
+
+// workspace: the states a call without a hand-over rebuilds, then the per-batch partials of gw and gu
+extern "C" size_t wkv4x_backward_workspace(int B, int T, int C, int has_ckpt) {
+    if (B <= 0 || C <= 0) return 0;
+    const size_t states = has_ckpt || T <= 0 ? 0 : T < PAR_MIN_T ? serial_backward_workspace(B, T, C)
+                                                 : (size_t)B * ((T + PIECE - 1) / PIECE) * 3 * C * sizeof(float);
+    return ((states + 255) & ~(size_t)255) + 2 * (size_t)B * C * sizeof(float);
+}
+
+extern "C" int wkv4x_backward(int B, int T, int C, int dtype, const void *time_decay, int decay_dtype, const void *u,
+                              const void *k, const void *v, const float *state_in, const void *gy, const float *gstate_out,
+                              void *gw_sum, void *gu_sum, int gu_dtype, void *gk, void *gv, float *gstate_in, void *workspace,
+                              const void *state_ckpt, void *stream) {
+    if (B < 0 || T < 0 || C < 0) return WKV_ERR_SHAPE;
+    if (B == 0 || C == 0) return WKV_OK;
+    if (!time_decay || !u || !gw_sum || !gu_sum || !workspace || (T > 0 && (!k || !v || !gy || !gk || !gv))) return WKV_ERR_NULL;
+    if (!known_dtype(dtype) || !known_dtype(decay_dtype) || !known_dtype(gu_dtype)) return WKV_ERR_DTYPE;
+    if (T < CKPT_MIN_T) state_ckpt = nullptr;
+    const size_t n = wkv4x_backward_workspace(B, T, C, state_ckpt != nullptr);
+    float *gw = (float *)((char *)workspace + n) - 2 * (size_t)B * C, *gu = gw + (size_t)B * C;
     cudaStream_t s = (cudaStream_t)stream;
-    float *ws = (float *)workspace;
-    if (T >= PAR_MIN_T) {
-        if (state_ckpt && state_ckpt_bytes < wkv4_state_ckpt_bytes(B, T, C)) return WKV_ERR_WORKSPACE;
-        return v4_par_backward(B, T, C, dtype, w, u, k, v, state_in, gy, gstate_out, gw, gu, gk, gv, gstate_in, ws,
-                               (const float *)state_ckpt, s);
-    }
-    switch (dtype) {
-        case WKV_F32:
-            return bwd<float>(B, T, C, w, u, k, v, state_in, gy, gstate_out, gw, gu, gk, gv, gstate_in, ws, s);
-        case WKV_BF16:
-            return bwd<__nv_bfloat16>(B, T, C, w, u, k, v, state_in, gy, gstate_out, gw, gu, gk, gv, gstate_in, ws, s);
-        case WKV_F16:
-            return bwd<__half>(B, T, C, w, u, k, v, state_in, gy, gstate_out, gw, gu, gk, gv, gstate_in, ws, s);
-    }
-    return WKV_ERR_DTYPE;
+    const int err = run_backward(B, T, C, dtype, Decay4{time_decay, decay_dtype}, u, k, v, state_in, gy, gstate_out, gw, gu, gk, gv,
+                                 gstate_in, (float *)workspace, (const float *)state_ckpt, s);
+    if (err != WKV_OK) return err;
+    return launch_chained(k_v4_fold, dim3((C + THREADS - 1) / THREADS, 2), dim3(THREADS), 0, s, (const float *)gw, (const float *)gu,
+                          gw_sum, decay_dtype, gu_sum, gu_dtype, B, C);
 }
 
 // ---------------------------------------------------------------------------
@@ -325,17 +397,6 @@ extern "C" int wkv4_backward_static(int B, int T, int C, int dtype, const float 
     if (err != WKV_OK) return err;
     cudaStream_t s = (cudaStream_t)stream;
     float *ws = (float *)scratch;
-    // Nothing in the scratch has to start at zero: both kernel families write every word of it
-    // that they later read (tile-start states; piece summaries, scanned states and partial sums).
-    if (T >= PAR_MIN_T)   // the same time-parallel kernels wkv4_backward runs, on the built-in array
-        return v4_par_backward(B, T, C, dtype, w, u, k, v, state_in, gy, gstate_out, gw, gu, gk, gv, gstate_in, ws,
-                               nullptr, s);
-    switch (dtype) {
-        case WKV_F32:
-            return bwd<float>(B, T, C, w, u, k, v, state_in, gy, gstate_out, gw, gu, gk, gv, gstate_in, ws, s);
-        case WKV_BF16:
-            return bwd<__nv_bfloat16>(B, T, C, w, u, k, v, state_in, gy, gstate_out, gw, gu, gk, gv, gstate_in, ws, s);
-        default:
-            return bwd<__half>(B, T, C, w, u, k, v, state_in, gy, gstate_out, gw, gu, gk, gv, gstate_in, ws, s);
-    }
+    // Nothing in the scratch has to start at zero: the kernels write every word of it that they later read.
+    return run_backward(B, T, C, dtype, Decay4{w, -1}, u, k, v, state_in, gy, gstate_out, gw, gu, gk, gv, gstate_in, ws, nullptr, s);
 }

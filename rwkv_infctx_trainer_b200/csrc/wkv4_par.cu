@@ -1,783 +1,444 @@
-// v4 WKV, parallel over time.
+// v4 WKV, parallel over time: one kernel forward, one backward, every tensor read once.
 //
-// One thread per (batch, channel) chain leaves a B200 mostly idle (B*C chains, each a
-// dependent chain over T).  The state recurrence is linear in (p, q) with a constant decay
-// per step, so T is cut into segments of SEG tokens that are processed independently:
+// One thread per (batch, channel) chain leaves a B200 mostly idle and waits for every token.  The state
+// recurrence is linear in (p, q) with a constant decay per token, so pieces of the token axis can be
+// summarised independently and folded:  a (earlier) then b of n tokens:
+//   o' = o_a + n w;  m = max(o', o_b);  (p,q) = e^{o'-m}(p_a,q_a) + e^{o_b-m}(p_b,q_b);  o = m
+// -- the max-shift the serial kernel makes token by token.  The state gradient (gp,gq,go) folds the same
+// way in reverse.
 //
-//   forward   1. k_seg_summary   each segment's (p,q,o) from an empty state
-//             2. k_seg_scan      per chain, fold the summaries: state at every segment start
-//             3. k_seg_forward   each segment from its true start state -> y
-//   backward  1-2 as above (segment-start states)
-//             3. k_seg_rsummary  each segment's reverse accumulation (gp,gq,go) from an empty
-//                                incoming gradient (needs the forward quantities of the segment)
-//             4. k_seg_rscan     per chain, fold them in reverse: (gp,gq,go) at every segment end
-//             5. k_seg_backward  each segment with its start state and end gradient -> gk, gv and
-//                                per-segment partial gw, gu
-//             6. k_seg_reduce    sum the partials over the segments in a fixed order
+// A CTA owns 16 channels of one batch row and walks the tokens in slabs of 8*NT; thread = one channel, one
+// tile of 8 tokens.  Per slab:
+//   forward   every thread summarises its tile from an empty state; the NT summaries meet in shared memory;
+//             every thread folds those before it onto the carried state and runs its tile from there -> y.
+//   backward  slabs in reverse.  Every thread recomputes y, 1/denominator and the exponent of its 8 tokens from the
+//             state at its tile's start, runs the reverse recurrence over them from an empty gradient, folds the
+//             summaries of the tiles after it onto the carried gradient and runs them again -> gk, gv.
+// The tile's tokens stay on chip between the two sweeps (in shared memory, filled by cp.async a slab ahead), so
+// k, v, gy cross HBM once: 12 + 20 bytes per token and channel in fp32, plus what forward leaves for backward:
+// the state at the start of every tile (3 floats per 8 tokens).  gw needs no running derivative across
+// tiles: with the true gradient at its own tile's end a tile's contribution is complete.
 //
-// Per-segment arithmetic is the math of RWKV-v4neo/cuda/wkv_cuda_bf16.cu:7-158; folding two
-// pieces a (earlier, n tokens after it) and b:  o' = o_a + n*w;  m = max(o', o_b);
-// (p,q) = e^{o'-m}(p_a,q_a) + e^{o_b-m}(p_b,q_b);  o = m  -- the same max-shift the kernel uses
-// token by token.  Threads of a warp hold consecutive channels: every access is coalesced.
-#include "wkv_common.cuh"
+// The CTAs (B * C/16 of them) are all resident at once at the sizes that matter (8 CTAs of 128 threads and
+// 64 registers per SM), so nothing waits for a second wave; with few of them the slab is made longer (NT 16, 32)
+// and the walk shorter.  What bounds it: instruction issue (about 45 instructions per token-channel forward, 90
+// backward) and HBM in the same range; bf16 by issue alone.
+//
+// Exponents are carried in base 2 inside the kernels (ex2 needs no multiply then) and converted at the
+// boundaries.  Per-tile arithmetic is the math of RWKV-v4neo/cuda/wkv_cuda_bf16.cu:7-158.
+#include "wkv4_common.cuh"
 
 namespace wkv {
 namespace {
 
-constexpr float MIN_VALUE = -1e38f;
-constexpr int SEG = 64;     // tokens per segment
-constexpr int TILE = 4;     // tokens recomputed at a time inside a segment (register stash).  Small on purpose:
-                            // the backward kernels are bound by latency at low occupancy, and 4-token tiles need 72-96
-                            // registers where 16-token tiles needed 128-168 (measured: 1.21 -> 1.09 ms on the v4 workload)
-constexpr int THREADS = 128;
+constexpr int CT = 16;      // channels per CTA
+constexpr int TK = 8;       // tokens per tile (one thread)
+constexpr int COARSE = 64;  // tokens between the states kept when forward left nothing
 
-__device__ __forceinline__ void exp_pair(float a, float b, float &A, float &Bv, float &m) {
-    const float d = a - b;
-    const float e = __expf(-fabsf(d));
+struct St {
+    float p, q, o;
+};
+__device__ __forceinline__ float ex2(float x) {
+    float y;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+// (A,E) = (2^{a-m}, 2^{b-m}), m = max(a,b): one ex2
+__device__ __forceinline__ void exp2_pair(float a, float b, float &A, float &E, float &m) {
+    const float d = a - b, e = ex2(-fabsf(d));
     const bool ge = d >= 0.f;
     A = ge ? 1.f : e;
-    Bv = ge ? e : 1.f;
-    m = ge ? a : b;
+    E = ge ? e : 1.f;
+    m = fmaxf(a, b);
+}
+// `a`, then `nw` of decay, then `b`
+__device__ __forceinline__ St fold(const St &a, float nw, const St &b) {
+    float A, E, m;
+    exp2_pair(a.o + nw, b.o, A, E, m);
+    return St{fmaf(A, a.p, E * b.p), fmaf(A, a.q, E * b.q), m};
 }
 
-struct Dims {
-    int B, T, C, nseg;
+struct Par {
+    int B, T, C, nslab;
+    Decay4 w;
+    const void *u, *k, *v, *gy;
+    const float *state_in, *gstate_out;
+    void *y, *gk, *gv;
+    float *state_out, *gstate_in, *gw, *gu;
+    float *fine;        // [B][T/8][3][C]: state at the start of every tile (exponent in base 2), or NULL
+    float *coarse;      // [B][T/64][3][C]: at the start of every 64 tokens, or NULL
 };
 
-// thread -> (b, seg, c); c fastest so that a warp reads consecutive channels
-__device__ __forceinline__ bool locate(const Dims &d, int &b, int &seg, int &c, int &t0, int &len) {
-    const long long idx = (long long)blockIdx.x * THREADS + threadIdx.x;
-    if (idx >= (long long)d.B * d.nseg * d.C) return false;
-    c = (int)(idx % d.C);
-    seg = (int)((idx / d.C) % d.nseg);
-    b = (int)(idx / ((long long)d.C * d.nseg));
-    t0 = seg * SEG;
-    len = min(SEG, d.T - t0);
-    return true;
+// Shared memory: the slab's k, v (and gy) as [stage][tensor][tile][8 tokens + 1 of padding][16 channels] -- the
+// padding keeps the two tiles a warp reads in different banks -- then the tile summaries.
+template <typename F, int NT, int NTENS, bool ASYNC> struct Smem {
+    static constexpr int TILE = (TK + 1) * CT;                  // elements
+    F slab[ASYNC ? 2 : 1][NTENS][ASYNC ? NT * TILE : 1];
+    St sum[NT][CT];
+    St gsum[NT / 8][CT];
+    St carry[2][CT];
+};
+
+// Copy slab `s` of the tensors to shared memory, 16 bytes at a time.  Rows past the end and channels past the last
+// are zero-filled.
+template <typename F, int NT, int NTENS, class S>
+__device__ __forceinline__ void fetch_slab(S &sm, int stage, const F *const (&src)[NTENS], int T, int C, int c0, int t0, int tid) {
+    constexpr int PER = 16 / sizeof(F), CPR = CT / PER;         // elements per chunk, chunks per row
+#pragma unroll
+    for (int n = 0; n < NTENS; n++)
+#pragma unroll
+        for (int i = 0; i < (NT * TK * CPR) / (NT * CT); i++) {
+            const int x = tid + i * NT * CT, row = x / CPR, ch = (x % CPR) * PER, t = t0 + row;
+            const bool in = t < T && c0 + ch < C;
+            const F *g = in ? src[n] + (size_t)t * C + c0 + ch : src[n];
+            const uint32_t d = (uint32_t)__cvta_generic_to_shared(
+                &sm.slab[stage][n][(row / TK) * S::TILE + (row % TK) * CT + ch]);
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(g), "r"(in ? 16 : 0) : "memory");
+        }
 }
-// summaries / segment states: [B][nseg][3][C]
-__device__ __forceinline__ size_t sidx(const Dims &d, int b, int seg, int c) {
-    return ((size_t)(b * d.nseg + seg) * 3) * d.C + c;
+__device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+__device__ __forceinline__ void cp_wait0() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
+
+// What thread (tile i, channel c) starts from: `carry` folded with everything between the slab's edge and tile i --
+// the tiles before i, or (REV) the tiles after it.  `mine` is this tile's summary, len(j) the tokens of tile j.
+// The tile at the far edge leaves the next slab's carry in `next`.  Contains the barriers.
+template <int NT, bool REV, class S, class Len>
+__device__ __forceinline__ St fold_tiles(S &sm, const St &mine, const St &carry, int i, int c, float w, Len len, St *next) {
+    sm.sum[i][c] = mine;
+    __syncthreads();
+    const int g = i >> 3, k = REV ? 7 - (i & 7) : (i & 7);      // group of eight tiles; how many of it are in between
+    auto at = [&](int j) { return REV ? 8 * g + 7 - j : 8 * g + j; };
+    St s = NT == 8 ? carry : St{0.f, 0.f, V4_MIN_VALUE};
+    int n = 0;
+    for (int j = 0; j < k; j++) {
+        const int l = len(at(j));
+        s = fold(s, (float)l * w, sm.sum[at(j)][c]);
+        n += l;
+    }
+    if constexpr (NT > 8) {
+        if (k == 7) sm.gsum[g][c] = fold(s, (float)len(i) * w, mine);
+        __syncthreads();
+        St t = carry;
+        for (int j = REV ? NT / 8 - 1 : 0; REV ? j > g : j < g; j += REV ? -1 : 1) {
+            int l = 0;
+#pragma unroll
+            for (int e = 0; e < 8; e++) l += len(8 * j + e);
+            t = fold(t, (float)l * w, sm.gsum[j][c]);
+        }
+        s = fold(t, (float)n * w, s);
+    }
+    if (i == (REV ? 0 : NT - 1)) *next = fold(s, (float)len(i) * w, mine);
+    return s;
 }
 
-template <typename F>
-__global__ void __launch_bounds__(THREADS)
-k_seg_summary(Dims d, const float *__restrict__ w_, const F *__restrict__ k_, const F *__restrict__ v_,
-              float *__restrict__ loc) {
+// ---------------------------------------------------------------------------------------------- forward
+// STATES: only the coarse states are wanted (backward without a hand-over)
+template <typename F, int NT, bool ASYNC, bool STATES>
+__global__ void __launch_bounds__(NT * CT, NT == 8 ? 8 : NT == 16 ? 4 : 2) k_v4_par_fwd(const Par P) {
     pdl_wait();
     pdl_trigger();
-    int b, seg, c, t0, len;
-    if (!locate(d, b, seg, c, t0, len)) return;
-    const float w = w_[c];
-    const size_t off = ((size_t)b * d.T + t0) * d.C + c;
-    float p = 0.f, q = 0.f, o = MIN_VALUE;
-    // loads of 8 tokens go out together, then the dependent chain runs over them
-    for (int t8 = 0; t8 < len; t8 += 8) {
-        float kk[8], vv[8];
+    typedef Smem<F, NT, 2, ASYNC> S;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    S &sm = *reinterpret_cast<S *>(smem_raw);
+    const int ncb = (P.C + CT - 1) / CT, b = blockIdx.x / ncb, c0 = (blockIdx.x - b * ncb) * CT;
+    const int tid = threadIdx.x, c = tid & (CT - 1), i = tid / CT, ch = min(c0 + c, P.C - 1), T = P.T, C = P.C;
+    const bool live = c0 + c < C;
+    const float w = P.w.at(ch) * V4_LOG2E, u = Elem<F>::ld((const F *)P.u + ch) * V4_LOG2E;
+    const size_t row = (size_t)b * T * C, so = ((size_t)b * C + ch) * 3;
+    const F *const src[2] = {(const F *)P.k + row, (const F *)P.v + row};
+    if (i == 0)
+        sm.carry[0][c] = P.state_in ? St{P.state_in[so], P.state_in[so + 1], to_base2(P.state_in[so + 2])} : St{0.f, 0.f, V4_MIN_VALUE};
+    if (ASYNC) { fetch_slab<F, NT, 2>(sm, 0, src, T, C, c0, 0, tid); cp_commit(); }
+    const int n8 = (T + TK - 1) / TK, n64 = (T + COARSE - 1) / COARSE;
+
+    for (int s = 0; s < P.nslab; s++) {
+        const int t0 = s * NT * TK, mine0 = t0 + i * TK;      // first token of the slab, of this tile
+        if (ASYNC) cp_wait0();
+        __syncthreads();
+        if (ASYNC && s + 1 < P.nslab) { fetch_slab<F, NT, 2>(sm, (s + 1) & 1, src, T, C, c0, t0 + NT * TK, tid); cp_commit(); }
+        auto len = [&](int j) { return min(TK, max(0, T - t0 - j * TK)); };
+        const int n = len(i);
+        float kk[TK], vv[TK];
 #pragma unroll
-        for (int j = 0; j < 8; j++) {
-            const bool in = t8 + j < len;
-            kk[j] = in ? Elem<F>::ld(k_ + off + (size_t)(t8 + j) * d.C) : 0.f;
-            vv[j] = in ? Elem<F>::ld(v_ + off + (size_t)(t8 + j) * d.C) : 0.f;
+        for (int j = 0; j < TK; j++) {
+            if (ASYNC) {
+                kk[j] = Elem<F>::ld(&sm.slab[s & 1][0][i * S::TILE + j * CT + c]) * V4_LOG2E;
+                vv[j] = Elem<F>::ld(&sm.slab[s & 1][1][i * S::TILE + j * CT + c]);
+            } else {
+                const size_t o = (size_t)min(mine0 + j, T - 1) * C + ch;
+                kk[j] = Elem<F>::ld(src[0] + o) * V4_LOG2E;
+                vv[j] = Elem<F>::ld(src[1] + o);
+            }
         }
+        St a{0.f, 0.f, V4_MIN_VALUE};
 #pragma unroll
-        for (int j = 0; j < 8; j++) {
-            if (t8 + j < len) {
+        for (int j = 0; j < TK; j++)
+            if (j < n) {
                 float A, E, m;
-                exp_pair(w + o, kk[j], A, E, m);
-                p = A * p + E * vv[j]; q = A * q + E; o = m;
+                exp2_pair(w + a.o, kk[j], A, E, m);
+                a.p = fmaf(A, a.p, E * vv[j]); a.q = fmaf(A, a.q, E); a.o = m;
+            }
+        St x = fold_tiles<NT, false>(sm, a, sm.carry[s & 1][c], i, c, w, len, &sm.carry[(s + 1) & 1][c]);
+        if (live && n > 0) {
+            if (!STATES && P.fine) {
+                float *f = P.fine + ((size_t)b * n8 + mine0 / TK) * 3 * C + ch;
+                f[0] = x.p; f[C] = x.q; f[2 * (size_t)C] = x.o;
+            }
+            if (P.coarse && (i & 7) == 0) {
+                float *f = P.coarse + ((size_t)b * n64 + mine0 / COARSE) * 3 * C + ch;
+                f[0] = x.p; f[C] = x.q; f[2 * (size_t)C] = x.o;
             }
         }
-    }
-    const size_t s = sidx(d, b, seg, c);
-    loc[s] = p; loc[s + d.C] = q; loc[s + 2 * (size_t)d.C] = o;
-}
-
-// per chain: state at the start of every segment, and the final state
-__global__ void __launch_bounds__(THREADS)
-k_seg_scan(Dims d, const float *__restrict__ w_, const float *__restrict__ state_in,
-           const float *__restrict__ loc, float *__restrict__ st, float *__restrict__ state_out) {
-    pdl_wait();
-    pdl_trigger();
-    const int idx = blockIdx.x * THREADS + threadIdx.x;
-    if (idx >= d.B * d.C) return;
-    const int b = idx / d.C, c = idx % d.C;
-    const float w = w_[c];
-    float p = 0.f, q = 0.f, o = MIN_VALUE;
-    if (state_in) { p = state_in[(size_t)idx * 3]; q = state_in[(size_t)idx * 3 + 1]; o = state_in[(size_t)idx * 3 + 2]; }
-    // (the summaries of 8 pieces are fetched together: the chain is short, the loads are what takes time)
-    for (int s8 = 0; s8 < d.nseg; s8 += 8) {
-        float lp[8], lq[8], lo[8];
+        if (!STATES) {
+            F *y = (F *)P.y + row + ch;
 #pragma unroll
-        for (int j = 0; j < 8; j++) {
-            const bool in = s8 + j < d.nseg;
-            const size_t s = sidx(d, b, in ? s8 + j : s8, c);
-            lp[j] = in ? loc[s] : 0.f; lq[j] = in ? loc[s + d.C] : 0.f; lo[j] = in ? loc[s + 2 * (size_t)d.C] : 0.f;
-        }
-#pragma unroll
-        for (int j = 0; j < 8; j++) {
-            const int seg = s8 + j;
-            if (seg < d.nseg) {
-                const size_t s = sidx(d, b, seg, c);
-                st[s] = p; st[s + d.C] = q; st[s + 2 * (size_t)d.C] = o;
-                const int len = min(SEG, d.T - seg * SEG);
-                float A, E, m;
-                exp_pair(o + len * w, lo[j], A, E, m);
-                p = A * p + E * lp[j]; q = A * q + E * lq[j]; o = m;
-            }
-        }
-    }
-    if (state_out) { state_out[(size_t)idx * 3] = p; state_out[(size_t)idx * 3 + 1] = q; state_out[(size_t)idx * 3 + 2] = o; }
-}
-
-// What forward leaves for backward (optional): at the start of every CK-token tile of every piece the
-// state (p,q,o) and its derivative w.r.t. the decay accumulated since the piece start (dpdw,dqdw) --
-// [B][nseg][SEG/CK][5][C] floats, 2.5 bytes per token-channel.  With it neither backward pass needs its
-// forward sweep over the piece (which is there only to find the tile-start values).
-constexpr int CK = 8;
-constexpr int NCK = SEG / CK;
-__device__ __forceinline__ size_t cidx(const Dims &d, int b, int seg, int tile, int c) {
-    return (((size_t)(b * d.nseg + seg) * NCK + tile) * 5) * d.C + c;
-}
-
-template <typename F>
-__global__ void __launch_bounds__(THREADS)
-k_seg_forward(Dims d, const float *__restrict__ w_, const F *__restrict__ u_, const F *__restrict__ k_,
-              const F *__restrict__ v_, const float *__restrict__ st, F *__restrict__ y_, float *__restrict__ ck) {
-    pdl_wait();
-    pdl_trigger();
-    int b, seg, c, t0, len;
-    if (!locate(d, b, seg, c, t0, len)) return;
-    const float w = w_[c], u = Elem<F>::ld(u_ + c);
-    const size_t off = ((size_t)b * d.T + t0) * d.C + c;
-    const size_t s = sidx(d, b, seg, c);
-    float p = st[s], q = st[s + d.C], o = st[s + 2 * (size_t)d.C];
-    float dpdw = 0.f, dqdw = 0.f;
-    for (int t8 = 0; t8 < len; t8 += 8) {
-        if (ck) {      // (8 = CK: every load batch starts a tile)
-            const size_t i = cidx(d, b, seg, t8 / CK, c);
-            ck[i] = p; ck[i + d.C] = q; ck[i + 2 * (size_t)d.C] = o;
-            ck[i + 3 * (size_t)d.C] = dpdw; ck[i + 4 * (size_t)d.C] = dqdw;
-        }
-        float kk[8], vv[8];
-#pragma unroll
-        for (int j = 0; j < 8; j++) {
-            const bool in = t8 + j < len;
-            kk[j] = in ? Elem<F>::ld(k_ + off + (size_t)(t8 + j) * d.C) : 0.f;
-            vv[j] = in ? Elem<F>::ld(v_ + off + (size_t)(t8 + j) * d.C) : 0.f;
-        }
-#pragma unroll
-        for (int j = 0; j < 8; j++) {
-            if (t8 + j < len) {
-                float A, E, m;
-                exp_pair(o, u + kk[j], A, E, m);
-                Elem<F>::st(y_ + off + (size_t)(t8 + j) * d.C, __fdividef(A * p + E * vv[j], A * q + E));
-                exp_pair(w + o, kk[j], A, E, m);
-                if (ck) { dpdw = A * (p + dpdw); dqdw = A * (q + dqdw); }
-                p = A * p + E * vv[j]; q = A * q + E; o = m;
-            }
-        }
-    }
-}
-
-// One segment backward.  FINAL = false: only the reverse accumulation from an empty incoming
-// gradient (the segment's reverse summary).  FINAL = true: with the true incoming gradient,
-// writing gk, gv and the segment's gw, gu.
-template <typename F, bool FINAL>
-__global__ void __launch_bounds__(THREADS)
-k_seg_backward(Dims d, const float *__restrict__ w_, const F *__restrict__ u_, const F *__restrict__ k_,
-               const F *__restrict__ v_, const F *__restrict__ gy_, const float *__restrict__ st,
-               const float *__restrict__ gend, float *__restrict__ rloc, F *__restrict__ gk_,
-               F *__restrict__ gv_, float *__restrict__ gw_part, float *__restrict__ gu_part) {
-    pdl_wait();
-    pdl_trigger();
-    int b, seg, c, t0, len;
-    if (!locate(d, b, seg, c, t0, len)) return;
-    const float w = w_[c], u = Elem<F>::ld(u_ + c);
-    const size_t off = ((size_t)b * d.T + t0) * d.C + c;
-    const size_t s = sidx(d, b, seg, c);
-    constexpr int NT = SEG / TILE;
-    float cp[NT], cq[NT], co[NT];   // state at the start of every tile of the segment
-    float p = st[s], q = st[s + d.C], o = st[s + 2 * (size_t)d.C];
-    float gw = 0.f, gu = 0.f, dpdw = 0.f, dqdw = 0.f;
-    // every tile: its loads go out together (independent of the recurrence), then the chain runs.
-    // The tile loops stay rolled: unrolled, the compiler hoists the loads of all four tiles and
-    // runs out of registers; the 12 tile-start values then live in (L1-resident) local memory.
-#pragma unroll 1
-    for (int tile = 0; tile < NT; tile++) {
-        cp[tile] = p; cq[tile] = q; co[tile] = o;
-        if (tile * TILE < len) {
-            float kk[TILE], vv[TILE], gg[TILE];
-#pragma unroll
-            for (int j = 0; j < TILE; j++) {
-                const int t = tile * TILE + j;
-                const bool in = t < len;
-                kk[j] = in ? Elem<F>::ld(k_ + off + (size_t)t * d.C) : 0.f;
-                vv[j] = in ? Elem<F>::ld(v_ + off + (size_t)t * d.C) : 0.f;
-                gg[j] = (FINAL && in) ? Elem<F>::ld(gy_ + off + (size_t)t * d.C) : 0.f;
-            }
-#pragma unroll
-            for (int j = 0; j < TILE; j++) {
-                if (tile * TILE + j < len) {
+            for (int j = 0; j < TK; j++)
+                if (j < n) {
                     float A, E, m;
-                    if (FINAL) {
-                        exp_pair(o, u + kk[j], A, E, m);
-                        const float iden = __fdividef(1.f, A * q + E);
-                        const float y = (A * p + E * vv[j]) * iden;
-                        gw += gg[j] * (dpdw - dqdw * y) * iden * A;
-                        gu += gg[j] * (vv[j] - y) * E * iden;
-                    }
-                    exp_pair(w + o, kk[j], A, E, m);
-                    if (FINAL) { dpdw = A * (p + dpdw); dqdw = A * (q + dqdw); }
-                    p = A * p + E * vv[j]; q = A * q + E; o = m;
+                    exp2_pair(x.o, u + kk[j], A, E, m);
+                    const float out = __fdividef(fmaf(A, x.p, E * vv[j]), fmaf(A, x.q, E));
+                    if (live) Elem<F>::st(y + (size_t)(mine0 + j) * C, out);
+                    exp2_pair(w + x.o, kk[j], A, E, m);
+                    x.p = fmaf(A, x.p, E * vv[j]); x.q = fmaf(A, x.q, E); x.o = m;
                 }
-            }
         }
     }
-    float gp = 0.f, gq = 0.f, go = MIN_VALUE;
-    if (FINAL) {
-        gp = gend[s]; gq = gend[s + d.C]; go = gend[s + 2 * (size_t)d.C];
-        gw += (gp * dpdw + gq * dqdw) * __expf(o + go);
-    }
-#pragma unroll 1
-    for (int tile = NT - 1; tile >= 0; tile--) {
-        if (tile * TILE < len) {
-            p = cp[tile]; q = cq[tile]; o = co[tile];
-            float kk[TILE], vv[TILE], gg[TILE];
-#pragma unroll
-            for (int j = 0; j < TILE; j++) {
-                const int t = tile * TILE + j;
-                const bool in = t < len;
-                kk[j] = in ? Elem<F>::ld(k_ + off + (size_t)t * d.C) : 0.f;
-                vv[j] = in ? Elem<F>::ld(v_ + off + (size_t)t * d.C) : 0.f;
-                gg[j] = in ? Elem<F>::ld(gy_ + off + (size_t)t * d.C) : 0.f;
-            }
-            float ys[TILE], zs[TILE], ze[TILE];
-#pragma unroll
-            for (int j = 0; j < TILE; j++) {
-                if (tile * TILE + j < len) {
-                    float A, E, m;
-                    exp_pair(o, u + kk[j], A, E, m);
-                    const float iden = __fdividef(1.f, A * q + E);
-                    ys[j] = (A * p + E * vv[j]) * iden; zs[j] = iden; ze[j] = kk[j] + u - m;
-                    exp_pair(w + o, kk[j], A, E, m);
-                    p = A * p + E * vv[j]; q = A * q + E; o = m;
-                }
-            }
-#pragma unroll
-            for (int j = TILE - 1; j >= 0; j--) {
-                const int t = tile * TILE + j;
-                if (t < len) {
-                    const size_t ii = off + (size_t)t * d.C;
-                    const float gz = gg[j] * zs[j];
-                    float A, E, m;
-                    if (FINAL) {
-                        A = gz * __expf(ze[j]);
-                        E = __expf(kk[j] + go);
-                        Elem<F>::st(gk_ + ii, A * (vv[j] - ys[j]) + E * (gp * vv[j] + gq));
-                        Elem<F>::st(gv_ + ii, A + E * gp);
-                    }
-                    exp_pair(w + go, ze[j] - kk[j] - u, A, E, m);
-                    E *= gz;
-                    gp = A * gp + E; gq = A * gq - E * ys[j]; go = m;
-                }
-            }
+    if (!STATES && P.state_out) {
+        __syncthreads();
+        if (i == 0 && live) {
+            const St f = sm.carry[P.nslab & 1][c];
+            P.state_out[so] = f.p; P.state_out[so + 1] = f.q; P.state_out[so + 2] = from_base2(f.o);
         }
-    }
-    if (FINAL) {
-        gw_part[(size_t)(b * d.nseg + seg) * d.C + c] = gw * w;
-        gu_part[(size_t)(b * d.nseg + seg) * d.C + c] = gu;
-    } else {
-        rloc[s] = gp; rloc[s + d.C] = gq; rloc[s + 2 * (size_t)d.C] = go;
     }
 }
 
-// The same two passes when the forward call left its tile checkpoints: no forward sweep.  Tiles of CK
-// tokens are taken in reverse; each starts from its checkpoint, recomputes y, 1/denominator and the
-// exponent for its tokens (FINAL: and adds the tile's share of gw, gu, whose running derivatives
-// dpdw, dqdw come from the checkpoint too), then runs the reverse recurrence over them.
-template <typename F, bool FINAL>
-__global__ void __launch_bounds__(THREADS)
-k_seg_backward_ck(Dims d, const float *__restrict__ w_, const F *__restrict__ u_, const F *__restrict__ k_,
-                  const F *__restrict__ v_, const F *__restrict__ gy_, const float *__restrict__ ck,
-                  const float *__restrict__ gend, float *__restrict__ rloc, F *__restrict__ gk_,
-                  F *__restrict__ gv_, float *__restrict__ gw_part, float *__restrict__ gu_part) {
+// ---------------------------------------------------------------------------------------------- backward
+// FINE: forward left the state at the start of every tile; else the slab's states are rebuilt from the coarse ones
+// (or, one slab only, from state_in) by one more summary and fold.
+template <typename F, int NT, bool ASYNC, bool FINE>
+__global__ void __launch_bounds__(NT * CT, NT == 8 ? 7 : NT == 16 ? 3 : 1) k_v4_par_bwd(const Par P) {
     pdl_wait();
     pdl_trigger();
-    int b, seg, c, t0, len;
-    if (!locate(d, b, seg, c, t0, len)) return;
-    const float w = w_[c], u = Elem<F>::ld(u_ + c);
-    const size_t off = ((size_t)b * d.T + t0) * d.C + c;
-    const size_t s = sidx(d, b, seg, c);
+    typedef Smem<F, NT, 3, ASYNC> S;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    S &sm = *reinterpret_cast<S *>(smem_raw);
+    const int ncb = (P.C + CT - 1) / CT, b = blockIdx.x / ncb, c0 = (blockIdx.x - b * ncb) * CT;
+    const int tid = threadIdx.x, c = tid & (CT - 1), i = tid / CT, ch = min(c0 + c, P.C - 1), T = P.T, C = P.C;
+    const bool live = c0 + c < C;
+    const float wn = P.w.at(ch), w = wn * V4_LOG2E, u = Elem<F>::ld((const F *)P.u + ch) * V4_LOG2E;
+    const size_t row = (size_t)b * T * C, so = ((size_t)b * C + ch) * 3;
+    const F *const src[3] = {(const F *)P.k + row, (const F *)P.v + row, (const F *)P.gy + row};
+    const int n8 = (T + TK - 1) / TK, n64 = (T + COARSE - 1) / COARSE, last = P.nslab - 1;
+    if (i == 0) {
+        St g{0.f, 0.f, V4_MIN_VALUE};
+        if (P.gstate_out) {
+            g.p = P.gstate_out[so]; g.q = P.gstate_out[so + 1];
+            if (g.p != 0.f || g.q != 0.f) g.o = to_base2(P.gstate_out[so + 2]);
+        }
+        sm.carry[last & 1][c] = g;
+    }
+    // the state at the start of this thread's tile (FINE) or of the 64 tokens around it, for slab s
+    auto start_state = [&](int s) {
+        const int t = s * NT * TK + i * TK;
+        if (!FINE && !P.coarse) return P.state_in ? St{P.state_in[so], P.state_in[so + 1], to_base2(P.state_in[so + 2])} : St{0.f, 0.f, V4_MIN_VALUE};
+        const float *f = FINE ? P.fine + ((size_t)b * n8 + min(t / TK, n8 - 1)) * 3 * C + ch
+                              : P.coarse + ((size_t)b * n64 + min(t / COARSE, n64 - 1)) * 3 * C + ch;
+        return St{f[0], f[C], f[2 * (size_t)C]};
+    };
+    St x = start_state(last);
+    if (ASYNC) { fetch_slab<F, NT, 3>(sm, last & 1, src, T, C, c0, last * NT * TK, tid); cp_commit(); }
     float gw = 0.f, gu = 0.f;
-    float gp = 0.f, gq = 0.f, go = MIN_VALUE;
-    if (FINAL) { gp = gend[s]; gq = gend[s + d.C]; go = gend[s + 2 * (size_t)d.C]; }
-    const int last = (len - 1) / CK;
-#pragma unroll 1
-    for (int tile = last; tile >= 0; tile--) {
-        const size_t ci = cidx(d, b, seg, tile, c);
-        float p = ck[ci], q = ck[ci + d.C], o = ck[ci + 2 * (size_t)d.C];
-        float dpdw = 0.f, dqdw = 0.f;
-        if (FINAL) { dpdw = ck[ci + 3 * (size_t)d.C]; dqdw = ck[ci + 4 * (size_t)d.C]; }
-        float kk[CK], vv[CK], gg[CK];
-#pragma unroll
-        for (int j = 0; j < CK; j++) {
-            const int t = tile * CK + j;
-            const bool in = t < len;
-            kk[j] = in ? Elem<F>::ld(k_ + off + (size_t)t * d.C) : 0.f;
-            vv[j] = in ? Elem<F>::ld(v_ + off + (size_t)t * d.C) : 0.f;
-            gg[j] = in ? Elem<F>::ld(gy_ + off + (size_t)t * d.C) : 0.f;
+
+    for (int s = last; s >= 0; s--) {
+        const int t0 = s * NT * TK, mine0 = t0 + i * TK;
+        if (ASYNC) cp_wait0();
+        __syncthreads();
+        St x_next;
+        if (s > 0) {
+            if (ASYNC) { fetch_slab<F, NT, 3>(sm, (s - 1) & 1, src, T, C, c0, t0 - NT * TK, tid); cp_commit(); }
+            x_next = start_state(s - 1);
         }
-        float ys[CK], zs[CK], ze[CK];
+        auto len = [&](int j) { return min(TK, max(0, T - t0 - j * TK)); };
+        const int n = len(i);
+        auto ld = [&](int tens, int j) {
+            return Elem<F>::ld(ASYNC ? &sm.slab[s & 1][tens][i * S::TILE + j * CT + c] : src[tens] + (size_t)min(mine0 + j, T - 1) * C + ch);
+        };
+        if constexpr (!FINE) {
+            // the state at the tile's start: fold the summaries of the tiles between the kept state and it.
+            // Without `coarse` there is one slab and the kept state is the initial one.
+            St a{0.f, 0.f, V4_MIN_VALUE};
 #pragma unroll
-        for (int j = 0; j < CK; j++) {
-            if (tile * CK + j < len) {
+            for (int j = 0; j < TK; j++)
+                if (j < n) {
+                    float A, E, m;
+                    const float k = ld(0, j) * V4_LOG2E, v = ld(1, j);
+                    exp2_pair(w + a.o, k, A, E, m);
+                    a.p = fmaf(A, a.p, E * v); a.q = fmaf(A, a.q, E); a.o = m;
+                }
+            sm.sum[i][c] = a;
+            __syncthreads();
+            for (int j = P.coarse ? (i & ~7) : 0; j < i; j++) x = fold(x, (float)len(j) * w, sm.sum[j][c]);
+            __syncthreads();
+        }
+        float ys[TK], zs[TK], ze[TK];      // y, gy / denominator, exponent of the token's own term in it
+        float dpdw = 0.f, dqdw = 0.f;      // d(p,q)/dw since the tile's start
+#pragma unroll
+        for (int j = 0; j < TK; j++)
+            if (j < n) {
                 float A, E, m;
-                exp_pair(o, u + kk[j], A, E, m);
-                const float iden = __fdividef(1.f, A * q + E);
-                ys[j] = (A * p + E * vv[j]) * iden; zs[j] = iden; ze[j] = kk[j] + u - m;
-                if (FINAL) {
-                    gw += gg[j] * (dpdw - dqdw * ys[j]) * iden * A;
-                    gu += gg[j] * (vv[j] - ys[j]) * E * iden;
-                }
-                exp_pair(w + o, kk[j], A, E, m);
-                if (FINAL) { dpdw = A * (p + dpdw); dqdw = A * (q + dqdw); }
-                p = A * p + E * vv[j]; q = A * q + E; o = m;
+                const float k = ld(0, j) * V4_LOG2E, v = ld(1, j), g = ld(2, j);
+                exp2_pair(x.o, u + k, A, E, m);
+                const float iden = __fdividef(1.f, fmaf(A, x.q, E));
+                ys[j] = fmaf(A, x.p, E * v) * iden;
+                zs[j] = g * iden;
+                ze[j] = k + u - m;
+                gw = fmaf(zs[j] * A, fmaf(-dqdw, ys[j], dpdw), gw);
+                gu = fmaf(zs[j] * E, v - ys[j], gu);
+                exp2_pair(w + x.o, k, A, E, m);
+                dpdw = A * (x.p + dpdw); dqdw = A * (x.q + dqdw);
+                x.p = fmaf(A, x.p, E * v); x.q = fmaf(A, x.q, E); x.o = m;
             }
-        }
-        // the piece's end: what the incoming gradient sees of the decay through the whole piece
-        if (FINAL && tile == last) gw += (gp * dpdw + gq * dqdw) * __expf(o + go);
+        // reverse over the tile from an empty gradient
+        St a{0.f, 0.f, V4_MIN_VALUE};
 #pragma unroll
-        for (int j = CK - 1; j >= 0; j--) {
-            const int t = tile * CK + j;
-            if (t < len) {
-                const size_t ii = off + (size_t)t * d.C;
-                const float gz = gg[j] * zs[j];
+        for (int j = TK - 1; j >= 0; j--)
+            if (j < n) {
                 float A, E, m;
-                if (FINAL) {
-                    A = gz * __expf(ze[j]);
-                    E = __expf(kk[j] + go);
-                    Elem<F>::st(gk_ + ii, A * (vv[j] - ys[j]) + E * (gp * vv[j] + gq));
-                    Elem<F>::st(gv_ + ii, A + E * gp);
-                }
-                exp_pair(w + go, ze[j] - kk[j] - u, A, E, m);
-                E *= gz;
-                gp = A * gp + E; gq = A * gq - E * ys[j]; go = m;
+                exp2_pair(w + a.o, ze[j] - ld(0, j) * V4_LOG2E - u, A, E, m);
+                E *= zs[j];
+                a.p = fmaf(A, a.p, E); a.q = fmaf(A, a.q, -E * ys[j]); a.o = m;
             }
-        }
-    }
-    if (FINAL) {
-        gw_part[(size_t)(b * d.nseg + seg) * d.C + c] = gw * w;
-        gu_part[(size_t)(b * d.nseg + seg) * d.C + c] = gu;
-    } else {
-        rloc[s] = gp; rloc[s + d.C] = gq; rloc[s + 2 * (size_t)d.C] = go;
-    }
-}
-
-// ---------------------------------------------------------------------------
-// The same three hot kernels with TWO adjacent channels per thread (used whenever C is even).  These
-// kernels are bound by latency, so what counts is the bytes each access in flight carries: with a
-// channel pair per thread every k, v, gy, y, gk, gv access is 4 bytes per lane for 16-bit types
-// (128 bytes per warp instead of 64) and 8 bytes for fp32, half as many threads run the same number
-// of chains, and every thread has two independent chains to interleave.  Measured on the v4
-// workload: bf16 1.07 -> 0.93 ms, fp32 1.00 -> 0.86 ms.
-template <typename F> struct Pair;
-template <> struct Pair<__nv_bfloat16> {
-    static __device__ __forceinline__ float2 ld(const __nv_bfloat16 *p) {
-        return __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162 *>(p));
-    }
-    static __device__ __forceinline__ void st(__nv_bfloat16 *p, float a, float b) {
-        *reinterpret_cast<__nv_bfloat162 *>(p) = __floats2bfloat162_rn(a, b);
-    }
-};
-template <> struct Pair<float> {
-    static __device__ __forceinline__ float2 ld(const float *p) { return *reinterpret_cast<const float2 *>(p); }
-    static __device__ __forceinline__ void st(float *p, float a, float b) { *reinterpret_cast<float2 *>(p) = make_float2(a, b); }
-};
-template <> struct Pair<__half> {
-    static __device__ __forceinline__ float2 ld(const __half *p) {
-        return __half22float2(*reinterpret_cast<const __half2 *>(p));
-    }
-    static __device__ __forceinline__ void st(__half *p, float a, float b) {
-        *reinterpret_cast<__half2 *>(p) = __floats2half2_rn(a, b);
-    }
-};
-
-// thread -> (b, seg, channel pair c, c+1)
-__device__ __forceinline__ bool locate2(const Dims &d, int &b, int &seg, int &c, int &t0, int &len) {
-    const long long idx = (long long)blockIdx.x * THREADS + threadIdx.x;
-    const int half = d.C / 2;
-    if (idx >= (long long)d.B * d.nseg * half) return false;
-    c = 2 * (int)(idx % half);
-    seg = (int)((idx / half) % d.nseg);
-    b = (int)(idx / ((long long)half * d.nseg));
-    t0 = seg * SEG;
-    len = min(SEG, d.T - t0);
-    return true;
-}
-
-template <typename F>
-__global__ void __launch_bounds__(THREADS)
-k_seg_summary2(Dims d, const float *__restrict__ w_, const F *__restrict__ k_, const F *__restrict__ v_,
-               float *__restrict__ loc) {
-    pdl_wait();
-    pdl_trigger();
-    int b, seg, c, t0, len;
-    if (!locate2(d, b, seg, c, t0, len)) return;
-    const float w[2] = {w_[c], w_[c + 1]};
-    const size_t off = ((size_t)b * d.T + t0) * d.C + c;
-    float p[2] = {0.f, 0.f}, q[2] = {0.f, 0.f}, o[2] = {MIN_VALUE, MIN_VALUE};
-    for (int t8 = 0; t8 < len; t8 += 8) {
-        float2 kk[8], vv[8];
+        St g = fold_tiles<NT, true>(sm, a, sm.carry[s & 1][c], i, c, w, len, &sm.carry[(s + 1) & 1][c]);
+        // what the gradient at the tile's end sees of the decay inside the tile
+        if (n > 0) gw = fmaf(fmaf(g.p, dpdw, g.q * dqdw), ex2(x.o + g.o), gw);
+        F *gk = (F *)P.gk + row + ch, *gv = (F *)P.gv + row + ch;
 #pragma unroll
-        for (int j = 0; j < 8; j++) {
-            const bool in = t8 + j < len;
-            kk[j] = in ? Pair<F>::ld(k_ + off + (size_t)(t8 + j) * d.C) : make_float2(0.f, 0.f);
-            vv[j] = in ? Pair<F>::ld(v_ + off + (size_t)(t8 + j) * d.C) : make_float2(0.f, 0.f);
-        }
-#pragma unroll
-        for (int j = 0; j < 8; j++) {
-            if (t8 + j < len) {
-                const float kj[2] = {kk[j].x, kk[j].y}, vj[2] = {vv[j].x, vv[j].y};
-#pragma unroll
-                for (int n = 0; n < 2; n++) {
-                    float A, E, m;
-                    exp_pair(w[n] + o[n], kj[n], A, E, m);
-                    p[n] = A * p[n] + E * vj[n]; q[n] = A * q[n] + E; o[n] = m;
+        for (int j = TK - 1; j >= 0; j--)
+            if (j < n) {
+                const float k = ld(0, j) * V4_LOG2E, v = ld(1, j);
+                float A = zs[j] * ex2(ze[j]), E = ex2(k + g.o), m;
+                if (live) {
+                    Elem<F>::st(gk + (size_t)(mine0 + j) * C, fmaf(A, v - ys[j], E * fmaf(g.p, v, g.q)));
+                    Elem<F>::st(gv + (size_t)(mine0 + j) * C, fmaf(E, g.p, A));
                 }
+                exp2_pair(w + g.o, ze[j] - k - u, A, E, m);
+                E *= zs[j];
+                g.p = fmaf(A, g.p, E); g.q = fmaf(A, g.q, -E * ys[j]); g.o = m;
             }
-        }
+        x = x_next;
     }
-    const size_t s = sidx(d, b, seg, c);
-    *reinterpret_cast<float2 *>(loc + s) = make_float2(p[0], p[1]);
-    *reinterpret_cast<float2 *>(loc + s + d.C) = make_float2(q[0], q[1]);
-    *reinterpret_cast<float2 *>(loc + s + 2 * (size_t)d.C) = make_float2(o[0], o[1]);
-}
-
-template <typename F>
-__global__ void __launch_bounds__(THREADS)
-k_seg_forward2(Dims d, const float *__restrict__ w_, const F *__restrict__ u_, const F *__restrict__ k_,
-               const F *__restrict__ v_, const float *__restrict__ st, F *__restrict__ y_, float *__restrict__ ck) {
-    pdl_wait();
-    pdl_trigger();
-    int b, seg, c, t0, len;
-    if (!locate2(d, b, seg, c, t0, len)) return;
-    const float w[2] = {w_[c], w_[c + 1]};
-    const float2 u2 = Pair<F>::ld(u_ + c);
-    const float u[2] = {u2.x, u2.y};
-    const size_t off = ((size_t)b * d.T + t0) * d.C + c;
-    const size_t s = sidx(d, b, seg, c);
-    float p[2], q[2], o[2], dpdw[2] = {0.f, 0.f}, dqdw[2] = {0.f, 0.f};
-    {
-        const float2 a = *reinterpret_cast<const float2 *>(st + s), e = *reinterpret_cast<const float2 *>(st + s + d.C),
-                     f = *reinterpret_cast<const float2 *>(st + s + 2 * (size_t)d.C);
-        p[0] = a.x; p[1] = a.y; q[0] = e.x; q[1] = e.y; o[0] = f.x; o[1] = f.y;
-    }
-    for (int t8 = 0; t8 < len; t8 += 8) {
-        if (ck) {
-            const size_t i = cidx(d, b, seg, t8 / CK, c);
-            *reinterpret_cast<float2 *>(ck + i) = make_float2(p[0], p[1]);
-            *reinterpret_cast<float2 *>(ck + i + d.C) = make_float2(q[0], q[1]);
-            *reinterpret_cast<float2 *>(ck + i + 2 * (size_t)d.C) = make_float2(o[0], o[1]);
-            *reinterpret_cast<float2 *>(ck + i + 3 * (size_t)d.C) = make_float2(dpdw[0], dpdw[1]);
-            *reinterpret_cast<float2 *>(ck + i + 4 * (size_t)d.C) = make_float2(dqdw[0], dqdw[1]);
-        }
-        float2 kk[8], vv[8];
-#pragma unroll
-        for (int j = 0; j < 8; j++) {
-            const bool in = t8 + j < len;
-            kk[j] = in ? Pair<F>::ld(k_ + off + (size_t)(t8 + j) * d.C) : make_float2(0.f, 0.f);
-            vv[j] = in ? Pair<F>::ld(v_ + off + (size_t)(t8 + j) * d.C) : make_float2(0.f, 0.f);
-        }
-#pragma unroll
-        for (int j = 0; j < 8; j++) {
-            if (t8 + j < len) {
-                const float kj[2] = {kk[j].x, kk[j].y}, vj[2] = {vv[j].x, vv[j].y};
-                float yo[2];
-#pragma unroll
-                for (int n = 0; n < 2; n++) {
-                    float A, E, m;
-                    exp_pair(o[n], u[n] + kj[n], A, E, m);
-                    yo[n] = __fdividef(A * p[n] + E * vj[n], A * q[n] + E);
-                    exp_pair(w[n] + o[n], kj[n], A, E, m);
-                    if (ck) { dpdw[n] = A * (p[n] + dpdw[n]); dqdw[n] = A * (q[n] + dqdw[n]); }
-                    p[n] = A * p[n] + E * vj[n]; q[n] = A * q[n] + E; o[n] = m;
-                }
-                Pair<F>::st(y_ + off + (size_t)(t8 + j) * d.C, yo[0], yo[1]);
-            }
-        }
-    }
-}
-
-template <typename F, bool FINAL>
-__global__ void __launch_bounds__(THREADS)
-k_seg_backward_ck2(Dims d, const float *__restrict__ w_, const F *__restrict__ u_, const F *__restrict__ k_,
-                   const F *__restrict__ v_, const F *__restrict__ gy_, const float *__restrict__ ck,
-                   const float *__restrict__ gend, float *__restrict__ rloc, F *__restrict__ gk_,
-                   F *__restrict__ gv_, float *__restrict__ gw_part, float *__restrict__ gu_part) {
-    pdl_wait();
-    pdl_trigger();
-    int b, seg, c, t0, len;
-    if (!locate2(d, b, seg, c, t0, len)) return;
-    const float w[2] = {w_[c], w_[c + 1]};
-    const float2 u2 = Pair<F>::ld(u_ + c);
-    const float u[2] = {u2.x, u2.y};
-    const size_t off = ((size_t)b * d.T + t0) * d.C + c;
-    const size_t s = sidx(d, b, seg, c);
-    auto ld2 = [](const float *p, float (&x)[2]) { const float2 a = *reinterpret_cast<const float2 *>(p); x[0] = a.x; x[1] = a.y; };
-    float gw[2] = {0.f, 0.f}, gu[2] = {0.f, 0.f};
-    float gp[2] = {0.f, 0.f}, gq[2] = {0.f, 0.f}, go[2] = {MIN_VALUE, MIN_VALUE};
-    if (FINAL) { ld2(gend + s, gp); ld2(gend + s + d.C, gq); ld2(gend + s + 2 * (size_t)d.C, go); }
-    const int last = (len - 1) / CK;
-#pragma unroll 1
-    for (int tile = last; tile >= 0; tile--) {
-        const size_t ci = cidx(d, b, seg, tile, c);
-        float p[2], q[2], o[2], dpdw[2] = {0.f, 0.f}, dqdw[2] = {0.f, 0.f};
-        ld2(ck + ci, p); ld2(ck + ci + d.C, q); ld2(ck + ci + 2 * (size_t)d.C, o);
-        if (FINAL) { ld2(ck + ci + 3 * (size_t)d.C, dpdw); ld2(ck + ci + 4 * (size_t)d.C, dqdw); }
-        float2 kk[CK], vv[CK], gg[CK];
-#pragma unroll
-        for (int j = 0; j < CK; j++) {
-            const int t = tile * CK + j;
-            const bool in = t < len;
-            kk[j] = in ? Pair<F>::ld(k_ + off + (size_t)t * d.C) : make_float2(0.f, 0.f);
-            vv[j] = in ? Pair<F>::ld(v_ + off + (size_t)t * d.C) : make_float2(0.f, 0.f);
-            gg[j] = in ? Pair<F>::ld(gy_ + off + (size_t)t * d.C) : make_float2(0.f, 0.f);
-        }
-        float ys[CK][2], zs[CK][2], ze[CK][2];
-#pragma unroll
-        for (int j = 0; j < CK; j++) {
-            if (tile * CK + j < len) {
-                const float kj[2] = {kk[j].x, kk[j].y}, vj[2] = {vv[j].x, vv[j].y}, gj[2] = {gg[j].x, gg[j].y};
-#pragma unroll
-                for (int n = 0; n < 2; n++) {
-                    float A, E, m;
-                    exp_pair(o[n], u[n] + kj[n], A, E, m);
-                    const float iden = __fdividef(1.f, A * q[n] + E);
-                    ys[j][n] = (A * p[n] + E * vj[n]) * iden; zs[j][n] = iden; ze[j][n] = kj[n] + u[n] - m;
-                    if (FINAL) {
-                        gw[n] += gj[n] * (dpdw[n] - dqdw[n] * ys[j][n]) * iden * A;
-                        gu[n] += gj[n] * (vj[n] - ys[j][n]) * E * iden;
-                    }
-                    exp_pair(w[n] + o[n], kj[n], A, E, m);
-                    if (FINAL) { dpdw[n] = A * (p[n] + dpdw[n]); dqdw[n] = A * (q[n] + dqdw[n]); }
-                    p[n] = A * p[n] + E * vj[n]; q[n] = A * q[n] + E; o[n] = m;
-                }
-            }
-        }
-        if (FINAL && tile == last) {
-#pragma unroll
-            for (int n = 0; n < 2; n++) gw[n] += (gp[n] * dpdw[n] + gq[n] * dqdw[n]) * __expf(o[n] + go[n]);
-        }
-#pragma unroll
-        for (int j = CK - 1; j >= 0; j--) {
-            const int t = tile * CK + j;
-            if (t < len) {
-                const size_t ii = off + (size_t)t * d.C;
-                const float kj[2] = {kk[j].x, kk[j].y}, vj[2] = {vv[j].x, vv[j].y}, gj[2] = {gg[j].x, gg[j].y};
-                float ok[2], ov[2];
-#pragma unroll
-                for (int n = 0; n < 2; n++) {
-                    const float gz = gj[n] * zs[j][n];
-                    float A, E, m;
-                    if (FINAL) {
-                        A = gz * __expf(ze[j][n]);
-                        E = __expf(kj[n] + go[n]);
-                        ok[n] = A * (vj[n] - ys[j][n]) + E * (gp[n] * vj[n] + gq[n]);
-                        ov[n] = A + E * gp[n];
-                    }
-                    exp_pair(w[n] + go[n], ze[j][n] - kj[n] - u[n], A, E, m);
-                    E *= gz;
-                    gp[n] = A * gp[n] + E; gq[n] = A * gq[n] - E * ys[j][n]; go[n] = m;
-                }
-                if (FINAL) {
-                    Pair<F>::st(gk_ + ii, ok[0], ok[1]);
-                    Pair<F>::st(gv_ + ii, ov[0], ov[1]);
-                }
-            }
-        }
-    }
-    if (FINAL) {
-        const size_t gi = (size_t)(b * d.nseg + seg) * d.C + c;
-        *reinterpret_cast<float2 *>(gw_part + gi) = make_float2(gw[0] * w[0], gw[1] * w[1]);
-        *reinterpret_cast<float2 *>(gu_part + gi) = make_float2(gu[0], gu[1]);
-    } else {
-        *reinterpret_cast<float2 *>(rloc + s) = make_float2(gp[0], gp[1]);
-        *reinterpret_cast<float2 *>(rloc + s + d.C) = make_float2(gq[0], gq[1]);
-        *reinterpret_cast<float2 *>(rloc + s + 2 * (size_t)d.C) = make_float2(go[0], go[1]);
-    }
-}
-
-// per chain, in reverse: incoming gradient at the end of every segment, and the chain's glast_state
-__global__ void __launch_bounds__(THREADS)
-k_seg_rscan(Dims d, const float *__restrict__ w_, const float *__restrict__ gstate_out,
-            const float *__restrict__ rloc, float *__restrict__ gend, float *__restrict__ gstate_in) {
-    pdl_wait();
-    pdl_trigger();
-    const int idx = blockIdx.x * THREADS + threadIdx.x;
-    if (idx >= d.B * d.C) return;
-    const int b = idx / d.C, c = idx % d.C;
-    const float w = w_[c];
-    float gp = 0.f, gq = 0.f, go = MIN_VALUE;
-    if (gstate_out) {
-        gp = gstate_out[(size_t)idx * 3]; gq = gstate_out[(size_t)idx * 3 + 1]; go = gstate_out[(size_t)idx * 3 + 2];
-        if (gp == 0.f && gq == 0.f) go = MIN_VALUE;
-    }
-    for (int s8 = d.nseg - 1; s8 >= 0; s8 -= 8) {
-        float lp[8], lq[8], lo[8];
-#pragma unroll
-        for (int j = 0; j < 8; j++) {
-            const bool in = s8 - j >= 0;
-            const size_t s = sidx(d, b, in ? s8 - j : 0, c);
-            lp[j] = in ? rloc[s] : 0.f; lq[j] = in ? rloc[s + d.C] : 0.f; lo[j] = in ? rloc[s + 2 * (size_t)d.C] : 0.f;
-        }
-#pragma unroll
-        for (int j = 0; j < 8; j++) {
-            const int seg = s8 - j;
-            if (seg >= 0) {
-                const size_t s = sidx(d, b, seg, c);
-                gend[s] = gp; gend[s + d.C] = gq; gend[s + 2 * (size_t)d.C] = go;
-                const int len = min(SEG, d.T - seg * SEG);
-                float A, E, m;
-                exp_pair(go + len * w, lo[j], A, E, m);
-                gp = A * gp + E * lp[j]; gq = A * gq + E * lq[j]; go = m;
-            }
-        }
-    }
-    if (gstate_in) { gstate_in[(size_t)idx * 3] = gp; gstate_in[(size_t)idx * 3 + 1] = gq; gstate_in[(size_t)idx * 3 + 2] = go; }
-}
-
-__global__ void __launch_bounds__(THREADS)
-k_seg_reduce(Dims d, const float *__restrict__ gw_part, const float *__restrict__ gu_part,
-             float *__restrict__ gw, float *__restrict__ gu) {
-    pdl_wait();
-    pdl_trigger();
-    const int idx = blockIdx.x * THREADS + threadIdx.x;
-    if (idx >= d.B * d.C) return;
-    const int b = idx / d.C, c = idx % d.C;
-    float a = 0.f, e = 0.f;
+    // the tiles' shares of gw and gu, summed in a fixed order
+    __syncthreads();
+    sm.sum[i][c] = St{gw, gu, 0.f};
+    __syncthreads();
+    if (i == 0 && live) {
+        float a = 0.f, e = 0.f;
 #pragma unroll 8
-    for (int seg = 0; seg < d.nseg; seg++) {
-        a += gw_part[(size_t)(b * d.nseg + seg) * d.C + c];
-        e += gu_part[(size_t)(b * d.nseg + seg) * d.C + c];
-    }
-    gw[idx] = a;
-    gu[idx] = e;
-}
-
-inline unsigned blocks(long long n) { return (unsigned)((n + THREADS - 1) / THREADS); }
-
-// `ckpt` (or NULL): where the piece-start states go instead of the workspace, for the backward call to reuse
-template <typename F>
-int par_fwd(Dims d, const float *w, const void *u, const void *k, const void *v, const float *si, void *y,
-            float *so, float *ws, float *ckpt, cudaStream_t s) {
-    const size_t n3 = (size_t)d.B * d.nseg * 3 * d.C;
-    float *loc = ws, *st = ws + n3;
-    const long long nthr = (long long)d.B * d.nseg * d.C;
-    int err = WKV_OK;
-    if constexpr (sizeof(F) >= 2) {
-        if (d.C % 2 == 0) {      // a channel pair per thread (every dtype)
-            err |= launch_chained(k_seg_summary2<F>, dim3(blocks(nthr / 2)), dim3(THREADS), 0, s, d, w,
-                                  (const F *)k, (const F *)v, loc);
-            err |= launch_chained(k_seg_scan, dim3(blocks((long long)d.B * d.C)), dim3(THREADS), 0, s, d, w, si,
-                                  loc, st, so);
-            err |= launch_chained(k_seg_forward2<F>, dim3(blocks(nthr / 2)), dim3(THREADS), 0, s, d, w,
-                                  (const F *)u, (const F *)k, (const F *)v, st, (F *)y, ckpt);
-            return err ? WKV_ERR_LAUNCH : WKV_OK;
+        for (int j = 0; j < NT; j++) { a += sm.sum[j][c].p; e += sm.sum[j][c].q; }
+        P.gw[(size_t)b * C + ch] = a * wn;
+        P.gu[(size_t)b * C + ch] = e;
+        if (P.gstate_in) {
+            const St f = sm.carry[1][c];      // (slab 0 leaves its carry there)
+            P.gstate_in[so] = f.p; P.gstate_in[so + 1] = f.q; P.gstate_in[so + 2] = from_base2(f.o);
         }
     }
-    err |= launch_chained(k_seg_summary<F>, dim3(blocks(nthr)), dim3(THREADS), 0, s, d, w, (const F *)k,
-                          (const F *)v, loc);
-    err |= launch_chained(k_seg_scan, dim3(blocks((long long)d.B * d.C)), dim3(THREADS), 0, s, d, w, si, loc, st,
-                          so);
-    err |= launch_chained(k_seg_forward<F>, dim3(blocks(nthr)), dim3(THREADS), 0, s, d, w, (const F *)u,
-                          (const F *)k, (const F *)v, st, (F *)y, ckpt);
-    return err ? WKV_ERR_LAUNCH : WKV_OK;
+}
+
+// Tiles per slab: 8 (8 CTAs of 128 threads per SM) once the CTAs alone fill the SMs; else longer slabs, and never
+// much longer than the segment.
+int pick_tiles(int B, int T, int C) {
+    const long long ctas = (long long)B * ((C + CT - 1) / CT), sms = device_sm_count();
+    if (ctas >= 4 * sms || T <= 64) return 8;
+    return ctas >= 2 * sms || T <= 128 ? 16 : 32;
+}
+
+template <class K>
+int launch(K kern, size_t smem, unsigned char (&attr_done)[64], const Par &P, int nt, cudaStream_t s) {
+    if (!set_max_smem_once(kern, (int)smem, attr_done)) return WKV_ERR_LAUNCH;
+    return launch_chained(kern, dim3(P.B * ((P.C + CT - 1) / CT)), dim3(nt * CT), smem, s, P);
+}
+template <typename F, int NT, bool ASYNC>
+int launch_fwd(Par P, bool states, cudaStream_t s) {
+    static unsigned char done[2][64];
+    P.nslab = (P.T + NT * TK - 1) / (NT * TK);
+    const size_t smem = sizeof(Smem<F, NT, 2, ASYNC>);
+    return states ? launch(k_v4_par_fwd<F, NT, ASYNC, true>, smem, done[0], P, NT, s)
+                  : launch(k_v4_par_fwd<F, NT, ASYNC, false>, smem, done[1], P, NT, s);
+}
+template <typename F, int NT, bool ASYNC>
+int launch_bwd(Par P, cudaStream_t s) {
+    static unsigned char done[2][64];
+    P.nslab = (P.T + NT * TK - 1) / (NT * TK);
+    const size_t smem = sizeof(Smem<F, NT, 3, ASYNC>);
+    return P.fine ? launch(k_v4_par_bwd<F, NT, ASYNC, true>, smem, done[0], P, NT, s)
+                  : launch(k_v4_par_bwd<F, NT, ASYNC, false>, smem, done[1], P, NT, s);
+}
+
+// 16-byte copies need rows that start on 16 bytes; other widths load element by element
+template <typename F>
+bool rows_aligned(const Par &P) {
+    return (size_t)P.C * sizeof(F) % 16 == 0 && aligned16(P.k) && aligned16(P.v) && (!P.gy || aligned16(P.gy));
 }
 
 template <typename F>
-int par_bwd(Dims d, const float *w, const void *u, const void *k, const void *v, const float *si,
-            const void *gy, const float *gso, float *gw, float *gu, void *gk, void *gv, float *gsi, float *ws,
-            const float *ckpt, cudaStream_t s) {
-    const size_t n3 = (size_t)d.B * d.nseg * 3 * d.C, n1 = (size_t)d.B * d.nseg * d.C;
-    float *loc = ws, *stw = loc + n3, *rloc = stw + n3, *gend = rloc + n3, *gwp = gend + n3, *gup = gwp + n1;
-    const long long nthr = (long long)d.B * d.nseg * d.C;
-    const unsigned nb = blocks(nthr), nc = blocks((long long)d.B * d.C);
-    int err = WKV_OK;
-    if constexpr (sizeof(F) >= 2) {
-        if (ckpt && d.C % 2 == 0) {      // tile checkpoints and a channel pair per thread
-            const unsigned nb2 = blocks(nthr / 2);
-            err |= launch_chained(k_seg_backward_ck2<F, false>, dim3(nb2), dim3(THREADS), 0, s, d, w, (const F *)u,
-                                  (const F *)k, (const F *)v, (const F *)gy, ckpt, nullptr, rloc, nullptr, nullptr,
-                                  nullptr, nullptr);
-            err |= launch_chained(k_seg_rscan, dim3(nc), dim3(THREADS), 0, s, d, w, gso, rloc, gend, gsi);
-            err |= launch_chained(k_seg_backward_ck2<F, true>, dim3(nb2), dim3(THREADS), 0, s, d, w, (const F *)u,
-                                  (const F *)k, (const F *)v, (const F *)gy, ckpt, gend, nullptr, (F *)gk, (F *)gv,
-                                  gwp, gup);
-            err |= launch_chained(k_seg_reduce, dim3(nc), dim3(THREADS), 0, s, d, gwp, gup, gw, gu);
-            return err ? WKV_ERR_LAUNCH : WKV_OK;
-        }
+int forward_as(const Par &P, bool states, cudaStream_t s) {
+    if (!rows_aligned<F>(P)) return launch_fwd<F, 16, false>(P, states, s);
+    switch (pick_tiles(P.B, P.T, P.C)) {
+        case 8: return launch_fwd<F, 8, true>(P, states, s);
+        case 16: return launch_fwd<F, 16, true>(P, states, s);
+        default: return launch_fwd<F, 32, true>(P, states, s);
     }
-    if (ckpt) {
-        // the forward call left its tile checkpoints: neither pass needs a forward sweep
-        err |= launch_chained(k_seg_backward_ck<F, false>, dim3(nb), dim3(THREADS), 0, s, d, w, (const F *)u,
-                              (const F *)k, (const F *)v, (const F *)gy, ckpt, nullptr, rloc, nullptr, nullptr,
-                              nullptr, nullptr);
-        err |= launch_chained(k_seg_rscan, dim3(nc), dim3(THREADS), 0, s, d, w, gso, rloc, gend, gsi);
-        err |= launch_chained(k_seg_backward_ck<F, true>, dim3(nb), dim3(THREADS), 0, s, d, w, (const F *)u,
-                              (const F *)k, (const F *)v, (const F *)gy, ckpt, gend, nullptr, (F *)gk, (F *)gv, gwp,
-                              gup);
-    } else {
-        // rebuild the piece-start states, then the two passes with their own forward sweeps
-        err |= launch_chained(k_seg_summary<F>, dim3(nb), dim3(THREADS), 0, s, d, w, (const F *)k, (const F *)v,
-                              loc);
-        err |= launch_chained(k_seg_scan, dim3(nc), dim3(THREADS), 0, s, d, w, si, loc, stw, nullptr);
-        err |= launch_chained(k_seg_backward<F, false>, dim3(nb), dim3(THREADS), 0, s, d, w, (const F *)u,
-                              (const F *)k, (const F *)v, (const F *)gy, stw, nullptr, rloc, nullptr, nullptr,
-                              nullptr, nullptr);
-        err |= launch_chained(k_seg_rscan, dim3(nc), dim3(THREADS), 0, s, d, w, gso, rloc, gend, gsi);
-        err |= launch_chained(k_seg_backward<F, true>, dim3(nb), dim3(THREADS), 0, s, d, w, (const F *)u,
-                              (const F *)k, (const F *)v, (const F *)gy, stw, gend, nullptr, (F *)gk, (F *)gv, gwp,
-                              gup);
+}
+template <typename F>
+int backward_as(Par P, float *scratch, cudaStream_t s) {
+    const bool aligned = rows_aligned<F>(P);
+    const int nt = aligned ? pick_tiles(P.B, P.T, P.C) : 16;
+    if (!P.fine && P.T > nt * TK) {
+        // nothing was handed over and there is more than one slab: the states every 64 tokens first
+        P.coarse = scratch;
+        const int err = forward_as<F>(P, true, s);
+        if (err != WKV_OK) return err;
     }
-    err |= launch_chained(k_seg_reduce, dim3(nc), dim3(THREADS), 0, s, d, gwp, gup, gw, gu);
-    return err ? WKV_ERR_LAUNCH : WKV_OK;
+    if (!aligned) return launch_bwd<F, 16, false>(P, s);
+    switch (nt) {
+        case 8: return launch_bwd<F, 8, true>(P, s);
+        case 16: return launch_bwd<F, 16, true>(P, s);
+        default: return launch_bwd<F, 32, true>(P, s);
+    }
+}
+
+Par make_par(int B, int T, int C, const Decay4 &w, const void *u, const void *k, const void *v, const float *si) {
+    Par P = {};
+    P.B = B; P.T = T; P.C = C; P.w = w; P.u = u; P.k = k; P.v = v; P.state_in = si;
+    return P;
 }
 
 }  // namespace
 
-size_t v4_par_forward_workspace(int B, int T, int C) {
-    const size_t nseg = (size_t)(T + SEG - 1) / SEG;
-    return 2 * (size_t)B * nseg * 3 * C * sizeof(float);
-}
-size_t v4_par_backward_workspace(int B, int T, int C) {
-    const size_t nseg = (size_t)(T + SEG - 1) / SEG;
-    return (4 * 3 + 2) * (size_t)B * nseg * C * sizeof(float);
-}
+size_t v4_par_ckpt_bytes(int B, int T, int C) { return (size_t)B * ((T + TK - 1) / TK) * 3 * C * sizeof(float); }
 
-size_t v4_par_ckpt_bytes(int B, int T, int C) {
-    return (size_t)B * ((T + SEG - 1) / SEG) * NCK * 5 * C * sizeof(float);
-}
-
-int v4_par_forward(int B, int T, int C, int dtype, const float *w, const void *u, const void *k, const void *v,
-                   const float *si, void *y, float *so, float *ws, float *ckpt, cudaStream_t s) {
-    const Dims d{B, T, C, (T + SEG - 1) / SEG};
+int v4_par_forward(int B, int T, int C, int dtype, const Decay4 &w, const void *u, const void *k, const void *v,
+                   const float *si, void *y, float *so, float *ckpt, cudaStream_t s) {
+    Par P = make_par(B, T, C, w, u, k, v, si);
+    P.y = y; P.state_out = so; P.fine = ckpt;
     switch (dtype) {
-        case WKV_F32: return par_fwd<float>(d, w, u, k, v, si, y, so, ws, ckpt, s);
-        case WKV_BF16: return par_fwd<__nv_bfloat16>(d, w, u, k, v, si, y, so, ws, ckpt, s);
-        case WKV_F16: return par_fwd<__half>(d, w, u, k, v, si, y, so, ws, ckpt, s);
+        case WKV_F32: return forward_as<float>(P, false, s);
+        case WKV_BF16: return forward_as<__nv_bfloat16>(P, false, s);
+        case WKV_F16: return forward_as<__half>(P, false, s);
     }
     return WKV_ERR_DTYPE;
 }
 
-int v4_par_backward(int B, int T, int C, int dtype, const float *w, const void *u, const void *k, const void *v,
+int v4_par_backward(int B, int T, int C, int dtype, const Decay4 &w, const void *u, const void *k, const void *v,
                     const float *si, const void *gy, const float *gso, float *gw, float *gu, void *gk, void *gv,
                     float *gsi, float *ws, const float *ckpt, cudaStream_t s) {
-    const Dims d{B, T, C, (T + SEG - 1) / SEG};
+    Par P = make_par(B, T, C, w, u, k, v, si);
+    P.gy = gy; P.gstate_out = gso; P.gw = gw; P.gu = gu; P.gk = gk; P.gv = gv; P.gstate_in = gsi;
+    P.fine = const_cast<float *>(ckpt);
     switch (dtype) {
-        case WKV_F32: return par_bwd<float>(d, w, u, k, v, si, gy, gso, gw, gu, gk, gv, gsi, ws, ckpt, s);
-        case WKV_BF16: return par_bwd<__nv_bfloat16>(d, w, u, k, v, si, gy, gso, gw, gu, gk, gv, gsi, ws, ckpt, s);
-        case WKV_F16: return par_bwd<__half>(d, w, u, k, v, si, gy, gso, gw, gu, gk, gv, gsi, ws, ckpt, s);
+        case WKV_F32: return backward_as<float>(P, ws, s);
+        case WKV_BF16: return backward_as<__nv_bfloat16>(P, ws, s);
+        case WKV_F16: return backward_as<__half>(P, ws, s);
     }
     return WKV_ERR_DTYPE;
 }

@@ -276,18 +276,6 @@ size_t chunked_wconv_bytes(const wkv_args_t *a, bool per_token_w);
 int chunked_convert_w(wkv_args_t *a, bool per_token_w, void *scratch, cudaStream_t s);
 int selftest_wait(int *status, uint32_t limit, cudaStream_t s);
 
-// cudaFuncAttributeMaxDynamicSharedMemorySize is a per-device property of a kernel: set it on
-// the first launch on each device only (`done` is the call site's own per-device record)
-template <class K>
-inline bool set_max_smem_once(K kern, int bytes, unsigned char (&done)[64]) {
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess) return false;
-    if (dev >= 0 && dev < 64 && __atomic_load_n(&done[dev], __ATOMIC_ACQUIRE)) return true;
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess) return false;
-    if (dev >= 0 && dev < 64) __atomic_store_n(&done[dev], (unsigned char)1, __ATOMIC_RELEASE);
-    return true;
-}
-
 // `state_ckpt` (laid out as chunked::CkptLayout, or NULL) receives what the backward kernels
 // reuse from the forward pass; y is not produced when `y` in `a` is NULL; `group_ws` is
 // chunked::group_layout() bytes of scratch, used when the chains are split into time groups

@@ -56,6 +56,18 @@ inline int launch_chained(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t 
     return cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...) == cudaSuccess ? WKV_OK : WKV_ERR_LAUNCH;
 }
 
+// cudaFuncAttributeMaxDynamicSharedMemorySize is a per-device property of a kernel: set it on
+// the first launch on each device only (`done` is the call site's own per-device record)
+template <class K>
+inline bool set_max_smem_once(K kern, int bytes, unsigned char (&done)[64]) {
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return false;
+    if (dev >= 0 && dev < 64 && __atomic_load_n(&done[dev], __ATOMIC_ACQUIRE)) return true;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess) return false;
+    if (dev >= 0 && dev < 64) __atomic_store_n(&done[dev], (unsigned char)1, __ATOMIC_RELEASE);
+    return true;
+}
+
 int device_sm_count();    // of the current device (wkv56_chunked.cu)
 
 // scalar (token-serial) v5/v6 kernels, wkv56_scalar.cu

@@ -22,6 +22,16 @@ size_t wkv56x_backward_workspace(const wkv_args_t *a, int per_token_w);
 int wkv56x_backward(const wkv_args_t *a, int per_token_w, int *status, void *gu_sum, int gu_dtype,
                     void *gw_sum, int gw_dtype, void *stream);
 
+/* wkv4_forward_ckpt / wkv4_backward_ckpt from the time_decay parameter itself (any element type), without a
+ * forward workspace, and with the parameter gradients summed over the batch in the parameters' types
+ * (gw_sum [C] in decay_dtype, gu_sum [C] in gu_dtype).  state_ckpt: wkv4_state_ckpt_bytes() bytes or NULL. */
+int wkv4x_forward(int B, int T, int C, int dtype, const void *time_decay, int decay_dtype, const void *u, const void *k,
+                  const void *v, const float *state_in, void *y, float *state_out, void *state_ckpt, void *stream);
+size_t wkv4x_backward_workspace(int B, int T, int C, int has_ckpt);
+int wkv4x_backward(int B, int T, int C, int dtype, const void *time_decay, int decay_dtype, const void *u, const void *k,
+                   const void *v, const float *state_in, const void *gy, const float *gstate_out, void *gw_sum, void *gu_sum,
+                   int gu_dtype, void *gk, void *gv, float *gstate_in, void *workspace, const void *state_ckpt, void *stream);
+
 #ifdef __cplusplus
 }
 #endif

@@ -1,0 +1,58 @@
+"""The time-parallel v4 kernels at the edges of what they cut the tokens and channels into: tiles of 8 tokens,
+slabs of 64, 128 and 256, channel blocks of 16, rows that are and are not 16-byte aligned, with and without
+the hand-over from forward to backward."""
+import numpy as np
+import pytest
+import torch
+
+import inputs
+import wkv_testlib as TL
+from oracle import wkv_oracle as O
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("B,T,C,dtype", [
+    (1, 16, 16, torch.float32), (2, 17, 24, torch.bfloat16), (1, 63, 40, torch.float32), (2, 64, 20, torch.bfloat16),
+    (1, 65, 7, torch.float32), (1, 129, 9, torch.float32), (1, 127, 16, torch.float32), (1, 128, 32, torch.bfloat16), (3, 257, 48, torch.float32),
+    (1, 511, 16, torch.float16), (2, 300, 1, torch.float32), (4, 200, 1264, torch.float32), (8, 136, 1200, torch.bfloat16)])
+def test_v4_matches_oracle(B, T, C, dtype):
+    import rwkv_infctx_trainer_b200 as W
+    from rwkv_infctx_trainer_b200 import _lib as L
+    c = inputs.wkv4_case(B, T, C, seed=800 + T)
+    d = {n: TL.to_dev(c[n], dtype) for n in ("u", "k", "v", "gy")}
+    td = TL.to_dev(c["td"], torch.float32)
+    f64 = lambda t: t.detach().float().cpu().double().numpy()
+    w64 = -np.exp(f64(td))
+    s0 = np.stack([inputs.normal((B, C), 1, stream=40), inputs.uniform((B, C), 1, 0.5, 2.0, stream=41),
+                   inputs.normal((B, C), 1, stream=42)], -1)
+    gs = np.stack([inputs.normal((B, C), 1, stream=43), inputs.normal((B, C), 1, stream=44),
+                   inputs.uniform((B, C), 1, -1.0, 0.0, stream=45)], -1)
+    s0, gs = TL.to_dev(s0, torch.float32), TL.to_dev(gs, torch.float32)
+    yo, so = O.wkv4_fwd(w64, f64(d["u"]), f64(d["k"]), f64(d["v"]), f64(s0))
+    g = O.wkv4_bwd(w64, f64(d["u"]), f64(d["k"]), f64(d["v"]), f64(s0), f64(d["gy"]), f64(gs))
+    tol = TL.TOL[dtype]
+    state = lambda t: (f64(t)[..., :2] * np.exp(f64(t)[..., 2:])) if torch.is_tensor(t) else t[..., :2] * np.exp(t[..., 2:])
+
+    leaves = [t.clone().requires_grad_(True) for t in (td, d["u"], d["k"], d["v"], s0)]
+    y, s1 = W.wkv_op(*leaves)
+    got = torch.autograd.grad((y, s1), leaves, (d["gy"], gs))
+    TL.assert_close("y", y, yo, tol)
+    TL.assert_close("state", state(s1), state(so), tol)
+    for n, a, b in (("gw", got[0], g["gw"].sum(0)), ("gu", got[1], g["gu"].sum(0)), ("gk", got[2], g["gk"]), ("gv", got[3], g["gv"]),
+                    ("gstate", state(got[4]), state(g["gstate_in"]))):
+        TL.assert_close(n, a, b, tol)
+
+    # without a hand-over, through the C ABI
+    lib, st = L.load(), torch.cuda.current_stream().cuda_stream
+    w = -torch.exp(td)
+    o = {n: torch.empty_like(d["k"]) for n in ("gk", "gv")}
+    gw, gu, gsi = torch.empty((B, C), device="cuda"), torch.empty((B, C), device="cuda"), torch.empty_like(s0)
+    n = lib.wkv4_backward_workspace(B, T, C)
+    ws = torch.empty(n, dtype=torch.uint8, device="cuda")
+    L.check(lib.wkv4_backward(B, T, C, L.DTYPE_CODE[dtype], w.data_ptr(), d["u"].data_ptr(), d["k"].data_ptr(), d["v"].data_ptr(),
+                              s0.data_ptr(), d["gy"].data_ptr(), gs.data_ptr(), gw.data_ptr(), gu.data_ptr(), o["gk"].data_ptr(),
+                              o["gv"].data_ptr(), gsi.data_ptr(), ws.data_ptr(), n, st), "wkv4_backward")
+    for n, a, b in (("gw", gw, g["gw"]), ("gu", gu, g["gu"]), ("gk", o["gk"], g["gk"]), ("gv", o["gv"], g["gv"]),
+                    ("gstate", state(gsi), state(g["gstate_in"]))):
+        TL.assert_close("no hand-over " + n, a, b, tol)
