@@ -7,8 +7,8 @@
 // -- the max-shift the serial kernel makes token by token.  The state gradient (gp,gq,go) folds the same
 // way in reverse.
 //
-// A CTA owns 16 channels of one batch row and walks the tokens in slabs of 8*NT; thread = one channel, one
-// tile of 8 tokens.  Per slab:
+// A CTA owns 16 channels of one batch row and walks the tokens in slabs of 8*NT; thread = two adjacent
+// channels, one tile of 8 tokens.  Per slab:
 //   forward   every thread summarises its tile from an empty state; the NT summaries meet in shared memory;
 //             every thread folds those before it onto the carried state and runs its tile from there -> y.
 //   backward  slabs in reverse.  Every thread recomputes y, 1/denominator and the exponent of its 8 tokens from the
@@ -19,31 +19,89 @@
 // the state at the start of every tile (3 floats per 8 tokens).  gw needs no running derivative across
 // tiles: with the true gradient at its own tile's end a tile's contribution is complete.
 //
-// The CTAs (B * C/16 of them) are all resident at once at the sizes that matter (8 CTAs of 128 threads and
-// 64 registers per SM), so nothing waits for a second wave; with few of them the slab is made longer (NT 16, 32)
-// and the walk shorter.  What bounds it: instruction issue (about 45 instructions per token-channel forward, 90
-// backward) and HBM in the same range; bf16 by issue alone.
+// The CTAs (B * C/16 of them) are all resident at once at the sizes that matter (7 CTAs of 64 threads per SM), so
+// nothing waits for a second wave; with few of them the slab is made longer (NT 16, 32) and the walk shorter.
+// Issue slots and HBM time are of the same size here, so the inner loops work on channel pairs: the packed fp32
+// instructions (fma.f32x2) take two channels each, and so does every address, load and store.
 //
 // Exponents are carried in base 2 inside the kernels (ex2 needs no multiply then) and converted at the
-// boundaries.  Per-tile arithmetic is the math of RWKV-v4neo/cuda/wkv_cuda_bf16.cu:7-158.
+// boundaries.
+//
+// Inside a tile the max-shift is done once.  With one reference exponent M for the tile's 8 tokens, p~ = p 2^{o-M}
+// and e_t = 2^{k_t-M}, a token is  y = (p~ + U e v) / (q~ + U e),  p~ <- W p~ + e v,  q~ <- W q~ + e  with W = e^w and U = e^u
+// constant: one ex2 and one reciprocal instead of two max-shifted pairs, and the reverse recurrence needs no exponential at
+// all (gp <- W gp + z, gq <- W gq - z y with z = gy / denominator).  That is sound while nothing leaves the fp32
+// range: |u| plus the distance of any k from M at most 60, the incoming state at most 2^60 above M, the incoming
+// gradient at most 2^90.  A tile that is not (`tame` false) takes the token-by-token max-shift of
+// RWKV-v4neo/cuda/wkv_cuda_bf16.cu:7-158; both give the same state representation (o = the running maximum) at
+// tile boundaries.
+#include <type_traits>
+
 #include "wkv4_common.cuh"
 
 namespace wkv {
 namespace {
 
 constexpr int CT = 16;      // channels per CTA
+constexpr int CP = CT / 2;  // threads (channel pairs) per tile
 constexpr int TK = 8;       // tokens per tile (one thread)
 constexpr int COARSE = 64;  // tokens between the states kept when forward left nothing
+constexpr float RANGE = 60.f;        // how far (log2) a tame tile's exponents may lie from its reference
+constexpr float GRAD_RANGE = 90.f;
 
-struct St {
-    float p, q, o;
-};
 __device__ __forceinline__ float ex2(float x) {
     float y;
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
-// (A,E) = (2^{a-m}, 2^{b-m}), m = max(a,b): one ex2
+__device__ __forceinline__ float rcp(float x) {
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+
+// ---- two channels at a time
+typedef float2 f2;
+__device__ __forceinline__ unsigned long long bits(const f2 &a) { return *reinterpret_cast<const unsigned long long *>(&a); }
+__device__ __forceinline__ f2 from_bits(unsigned long long v) { return *reinterpret_cast<f2 *>(&v); }
+__device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c) {
+    unsigned long long r;
+    asm("fma.rn.ftz.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(bits(a)), "l"(bits(b)), "l"(bits(c)));
+    return from_bits(r);
+}
+__device__ __forceinline__ f2 mul2(f2 a, f2 b) {
+    unsigned long long r;
+    asm("mul.rn.ftz.f32x2 %0, %1, %2;" : "=l"(r) : "l"(bits(a)), "l"(bits(b)));
+    return from_bits(r);
+}
+__device__ __forceinline__ f2 add2(f2 a, f2 b) {
+    unsigned long long r;
+    asm("add.rn.ftz.f32x2 %0, %1, %2;" : "=l"(r) : "l"(bits(a)), "l"(bits(b)));
+    return from_bits(r);
+}
+__device__ __forceinline__ f2 both(float x) { return make_float2(x, x); }
+__device__ __forceinline__ f2 sub2(f2 a, f2 b) { return fma2(b, both(-1.f), a); }
+__device__ __forceinline__ f2 neg2(f2 a) { return make_float2(-a.x, -a.y); }
+__device__ __forceinline__ f2 max2(f2 a, f2 b) { return make_float2(fmaxf(a.x, b.x), fmaxf(a.y, b.y)); }
+__device__ __forceinline__ f2 min2(f2 a, f2 b) { return make_float2(fminf(a.x, b.x), fminf(a.y, b.y)); }
+__device__ __forceinline__ f2 ex2_2(f2 a) { return make_float2(ex2(a.x), ex2(a.y)); }
+__device__ __forceinline__ f2 rcp2(f2 a) { return make_float2(rcp(a.x), rcp(a.y)); }
+template <int H> __device__ __forceinline__ float &part(f2 &a) { return H ? a.y : a.x; }
+template <int H> __device__ __forceinline__ float part(const f2 &a) { return H ? a.y : a.x; }
+typedef std::integral_constant<int, 0> FirstChannel;
+typedef std::integral_constant<int, 1> SecondChannel;
+
+struct St {
+    f2 p, q, o;
+};
+__device__ __forceinline__ St empty_state() { return St{both(0.f), both(0.f), both(V4_MIN_VALUE)}; }
+// `a`, then `nw` of decay, then `b`
+__device__ __forceinline__ St fold(const St &a, f2 nw, const St &b) {
+    const f2 d = add2(a.o, nw), m = max2(d, b.o), A = ex2_2(sub2(d, m)), E = ex2_2(sub2(b.o, m));
+    return St{fma2(A, a.p, mul2(E, b.p)), fma2(A, a.q, mul2(E, b.q)), m};
+}
+
+// ---- one channel: the token-by-token max-shift.  (A,E) = (2^{a-m}, 2^{b-m}), m = max(a,b): one ex2
 __device__ __forceinline__ void exp2_pair(float a, float b, float &A, float &E, float &m) {
     const float d = a - b, e = ex2(-fabsf(d));
     const bool ge = d >= 0.f;
@@ -51,12 +109,23 @@ __device__ __forceinline__ void exp2_pair(float a, float b, float &A, float &E, 
     E = ge ? e : 1.f;
     m = fmaxf(a, b);
 }
-// `a`, then `nw` of decay, then `b`
-__device__ __forceinline__ St fold(const St &a, float nw, const St &b) {
-    float A, E, m;
-    exp2_pair(a.o + nw, b.o, A, E, m);
-    return St{fmaf(A, a.p, E * b.p), fmaf(A, a.q, E * b.q), m};
-}
+
+// ---- two adjacent elements
+template <typename F> struct Pair;
+template <> struct Pair<float> {
+    static __device__ __forceinline__ f2 ld(const float *p) { return *reinterpret_cast<const f2 *>(p); }
+    static __device__ __forceinline__ void st(float *p, f2 v) { *reinterpret_cast<f2 *>(p) = v; }
+};
+template <> struct Pair<__nv_bfloat16> {
+    static __device__ __forceinline__ f2 ld(const __nv_bfloat16 *p) {
+        return __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162 *>(p));
+    }
+    static __device__ __forceinline__ void st(__nv_bfloat16 *p, f2 v) { *reinterpret_cast<__nv_bfloat162 *>(p) = __floats2bfloat162_rn(v.x, v.y); }
+};
+template <> struct Pair<__half> {
+    static __device__ __forceinline__ f2 ld(const __half *p) { return __half22float2(*reinterpret_cast<const __half2 *>(p)); }
+    static __device__ __forceinline__ void st(__half *p, f2 v) { *reinterpret_cast<__half2 *>(p) = __floats2half2_rn(v.x, v.y); }
+};
 
 struct Par {
     int B, T, C, nslab;
@@ -70,145 +139,256 @@ struct Par {
 };
 
 // Shared memory: the slab's k, v (and gy) as [stage][tensor][tile][8 tokens + 1 of padding][16 channels] -- the
-// padding keeps the two tiles a warp reads in different banks -- then the tile summaries.
+// padding keeps the tiles a warp reads in different banks -- then the tile summaries.
 template <typename F, int NT, int NTENS, bool ASYNC> struct Smem {
     static constexpr int TILE = (TK + 1) * CT;                  // elements
-    F slab[ASYNC ? 2 : 1][NTENS][ASYNC ? NT * TILE : 1];
-    St sum[NT][CT];
-    St gsum[NT / 8][CT];
-    St carry[2][CT];
+    F slab[ASYNC ? 2 : 1][NTENS][ASYNC ? NT * TILE : 8];
+    St sum[NT][CP];
+    St gsum[NT / 8][CP];
+    St carry[2][CP];
 };
 
-// Copy slab `s` of the tensors to shared memory, 16 bytes at a time.  Rows past the end and channels past the last
-// are zero-filled.
+// The copies of a slab this thread makes, 16 bytes each: row r0 + i * ROWS of the slab, channels ch0 .. .
+template <typename F, int NT> struct Copy {
+    static constexpr int PER = 16 / sizeof(F), CPR = CT / PER;          // elements per copy, copies per row
+    static constexpr int ROWS = NT * CP / CPR, N = NT * TK / ROWS;      // rows the CTA covers at once, copies per thread
+    int r0, ch0;
+    uint32_t dst;       // byte offset of row r0 inside a tensor's slab
+    bool in;            // its channels exist
+    __device__ __forceinline__ Copy(int tid, int c0, int C) {
+        r0 = tid / CPR;
+        ch0 = c0 + (tid % CPR) * PER;
+        in = ch0 < C;
+        dst = (((r0 / TK) * (TK + 1) + r0 % TK) * CT + (tid % CPR) * PER) * sizeof(F);
+    }
+    static_assert(ROWS % TK == 0, "");
+    static constexpr uint32_t STEP = (ROWS / TK) * (TK + 1) * CT * sizeof(F);
+};
+// rows past the end and channels past the last are zero-filled
 template <typename F, int NT, int NTENS, class S>
-__device__ __forceinline__ void fetch_slab(S &sm, int stage, const F *const (&src)[NTENS], int T, int C, int c0, int t0, int tid) {
-    constexpr int PER = 16 / sizeof(F), CPR = CT / PER;         // elements per chunk, chunks per row
+__device__ __forceinline__ void fetch_slab(S &sm, const Copy<F, NT> &cp, int stage, const F *const (&src)[NTENS], int T, int C, int t0) {
+    typedef Copy<F, NT> K;
+    const bool full = t0 + NT * TK <= T;
+    const size_t off = (size_t)(t0 + cp.r0) * C + cp.ch0;
 #pragma unroll
-    for (int n = 0; n < NTENS; n++)
+    for (int n = 0; n < NTENS; n++) {
+        const uint32_t d = (uint32_t)__cvta_generic_to_shared(&sm.slab[stage][n][0]) + cp.dst;
 #pragma unroll
-        for (int i = 0; i < (NT * TK * CPR) / (NT * CT); i++) {
-            const int x = tid + i * NT * CT, row = x / CPR, ch = (x % CPR) * PER, t = t0 + row;
-            const bool in = t < T && c0 + ch < C;
-            const F *g = in ? src[n] + (size_t)t * C + c0 + ch : src[n];
-            const uint32_t d = (uint32_t)__cvta_generic_to_shared(
-                &sm.slab[stage][n][(row / TK) * S::TILE + (row % TK) * CT + ch]);
-            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(g), "r"(in ? 16 : 0) : "memory");
+        for (int i = 0; i < K::N; i++) {
+            const bool in = cp.in && (full || t0 + cp.r0 + i * K::ROWS < T);
+            const F *g = in ? src[n] + off + (size_t)i * K::ROWS * C : src[n];
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d + i * K::STEP), "l"(g), "r"(in ? 16 : 0) : "memory");
         }
+    }
 }
 __device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 __device__ __forceinline__ void cp_wait0() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
 
-// What thread (tile i, channel c) starts from: `carry` folded with everything between the slab's edge and tile i --
+// What thread (tile i, pair c) starts from: `carry` folded with everything between the slab's edge and tile i --
 // the tiles before i, or (REV) the tiles after it.  `mine` is this tile's summary, len(j) the tokens of tile j.
 // The tile at the far edge leaves the next slab's carry in `next`.  Contains the barriers.
-template <int NT, bool REV, class S, class Len>
-__device__ __forceinline__ St fold_tiles(S &sm, const St &mine, const St &carry, int i, int c, float w, Len len, St *next) {
+template <int NT, bool REV, bool FULL, class S, class Len>
+__device__ __forceinline__ St fold_tiles(S &sm, const St &mine, const St &carry, int i, int c, f2 w, Len len, St *next) {
     sm.sum[i][c] = mine;
     __syncthreads();
     const int g = i >> 3, k = REV ? 7 - (i & 7) : (i & 7);      // group of eight tiles; how many of it are in between
     auto at = [&](int j) { return REV ? 8 * g + 7 - j : 8 * g + j; };
-    St s = NT == 8 ? carry : St{0.f, 0.f, V4_MIN_VALUE};
+    const f2 w8 = mul2(w, both((float)TK));
+    auto decay = [&](int n) { return mul2(w, both((float)n)); };
+    St s = NT == 8 ? carry : empty_state();
     int n = 0;
+#pragma unroll 1
     for (int j = 0; j < k; j++) {
-        const int l = len(at(j));
-        s = fold(s, (float)l * w, sm.sum[at(j)][c]);
+        const int l = FULL ? TK : len(at(j));
+        s = fold(s, FULL ? w8 : decay(l), sm.sum[at(j)][c]);
         n += l;
     }
     if constexpr (NT > 8) {
-        if (k == 7) sm.gsum[g][c] = fold(s, (float)len(i) * w, mine);
+        if (k == 7) sm.gsum[g][c] = fold(s, FULL ? w8 : decay(len(i)), mine);
         __syncthreads();
         St t = carry;
         for (int j = REV ? NT / 8 - 1 : 0; REV ? j > g : j < g; j += REV ? -1 : 1) {
-            int l = 0;
+            int l = 8 * TK;
+            if (!FULL) {
+                l = 0;
 #pragma unroll
-            for (int e = 0; e < 8; e++) l += len(8 * j + e);
-            t = fold(t, (float)l * w, sm.gsum[j][c]);
+                for (int e = 0; e < 8; e++) l += len(8 * j + e);
+            }
+            t = fold(t, decay(l), sm.gsum[j][c]);
         }
-        s = fold(t, (float)n * w, s);
+        s = fold(t, decay(n), s);
     }
-    if (i == (REV ? 0 : NT - 1)) *next = fold(s, (float)len(i) * w, mine);
+    if (i == (REV ? 0 : NT - 1)) *next = fold(s, FULL ? w8 : decay(len(i)), mine);
     return s;
 }
+
+// What both kernels know of their place: batch row, first channel, the pair and tile of the thread.
+template <bool ASYNC> struct Place {
+    int b, c0, c, i, ch, ch1, C, T;
+    bool live, live1;
+    size_t row;
+    __device__ __forceinline__ Place(const Par &P) {
+        C = P.C; T = P.T;
+        const int ncb = (C + CT - 1) / CT, tid = threadIdx.x;
+        b = blockIdx.x / ncb; c0 = (blockIdx.x - b * ncb) * CT;
+        c = tid & (CP - 1); i = tid / CP;
+        live = c0 + 2 * c < C; live1 = ASYNC ? live : c0 + 2 * c + 1 < C;
+        ch = ASYNC ? (live ? c0 + 2 * c : C - 2) : min(c0 + 2 * c, C - 1);
+        ch1 = ASYNC ? ch + 1 : min(ch + 1, C - 1);
+        row = (size_t)b * T * C;
+    }
+    template <typename F> __device__ __forceinline__ f2 ld(const F *p, size_t o) const {
+        if (ASYNC) return Pair<F>::ld(p + o + ch);
+        return make_float2(Elem<F>::ld(p + o + ch), Elem<F>::ld(p + o + ch1));
+    }
+    // `p` points at channel ch
+    template <typename F> __device__ __forceinline__ void st(F *p, f2 v) const {
+        if (ASYNC) {
+            if (live) Pair<F>::st(p, v);
+        } else {
+            if (live) Elem<F>::st(p, v.x);
+            if (live1) Elem<F>::st(p + 1, v.y);
+        }
+    }
+    __device__ __forceinline__ St ext_state(const float *s) const {
+        if (!s) return empty_state();
+        const float *x = s + ((size_t)b * C + ch) * 3, *y = s + ((size_t)b * C + ch1) * 3;
+        return St{make_float2(x[0], y[0]), make_float2(x[1], y[1]), make_float2(to_base2(x[2]), to_base2(y[2]))};
+    }
+    __device__ __forceinline__ void put_state(float *s, const St &f) const {
+        float *x = s + ((size_t)b * C + ch) * 3;
+        if (live) { x[0] = f.p.x; x[1] = f.q.x; x[2] = from_base2(f.o.x); }
+        if (live1) { x[3] = f.p.y; x[4] = f.q.y; x[5] = from_base2(f.o.y); }
+    }
+    // the three rows of a kept state ([..][3][C]); f points at its first row
+    __device__ __forceinline__ St kept(const float *f) const { return St{ld(f, 0), ld(f, C), ld(f, 2 * (size_t)C)}; }
+    __device__ __forceinline__ void keep(float *f, const St &x) const {
+        st(f + ch, x.p); st(f + C + ch, x.q); st(f + 2 * (size_t)C + ch, x.o);
+    }
+};
 
 // ---------------------------------------------------------------------------------------------- forward
 // STATES: only the coarse states are wanted (backward without a hand-over)
 template <typename F, int NT, bool ASYNC, bool STATES>
-__global__ void __launch_bounds__(NT * CT, NT == 8 ? 8 : NT == 16 ? 4 : 2) k_v4_par_fwd(const Par P) {
+__global__ void __launch_bounds__(NT * CP, NT == 8 ? 8 : NT == 16 ? 4 : 2) k_v4_par_fwd(const Par P) {
     pdl_wait();
     pdl_trigger();
     typedef Smem<F, NT, 2, ASYNC> S;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     S &sm = *reinterpret_cast<S *>(smem_raw);
-    const int ncb = (P.C + CT - 1) / CT, b = blockIdx.x / ncb, c0 = (blockIdx.x - b * ncb) * CT;
-    const int tid = threadIdx.x, c = tid & (CT - 1), i = tid / CT, ch = min(c0 + c, P.C - 1), T = P.T, C = P.C;
-    const bool live = c0 + c < C;
-    const float w = P.w.at(ch) * V4_LOG2E, u = Elem<F>::ld((const F *)P.u + ch) * V4_LOG2E;
-    const size_t row = (size_t)b * T * C, so = ((size_t)b * C + ch) * 3;
-    const F *const src[2] = {(const F *)P.k + row, (const F *)P.v + row};
-    if (i == 0)
-        sm.carry[0][c] = P.state_in ? St{P.state_in[so], P.state_in[so + 1], to_base2(P.state_in[so + 2])} : St{0.f, 0.f, V4_MIN_VALUE};
-    if (ASYNC) { fetch_slab<F, NT, 2>(sm, 0, src, T, C, c0, 0, tid); cp_commit(); }
+    const Place<ASYNC> L(P);
+    const int c = L.c, i = L.i, T = L.T, C = L.C;
+    const Copy<F, NT> cp(threadIdx.x, L.c0, C);
+    const f2 w = make_float2(P.w.at(L.ch) * V4_LOG2E, P.w.at(L.ch1) * V4_LOG2E), u = mul2(L.ld((const F *)P.u, 0), both(V4_LOG2E));
+    const F *const src[2] = {(const F *)P.k + L.row, (const F *)P.v + L.row};
+    if (i == 0) sm.carry[0][c] = L.ext_state(P.state_in);
+    if (ASYNC) { fetch_slab<F, NT, 2>(sm, cp, 0, src, T, C, 0); cp_commit(); }
     const int n8 = (T + TK - 1) / TK, n64 = (T + COARSE - 1) / COARSE;
-
-    for (int s = 0; s < P.nslab; s++) {
+    const f2 W = ex2_2(w), U = ex2_2(u);
+    const float range = RANGE - fmaxf(fabsf(u.x), fabsf(u.y));
+    // FULL: every tile of the slab has its 8 tokens
+    auto slab = [&](auto full_tag, int s) {
+        constexpr bool FULL = decltype(full_tag)::value;
         const int t0 = s * NT * TK, mine0 = t0 + i * TK;      // first token of the slab, of this tile
-        if (ASYNC) cp_wait0();
-        __syncthreads();
-        if (ASYNC && s + 1 < P.nslab) { fetch_slab<F, NT, 2>(sm, (s + 1) & 1, src, T, C, c0, t0 + NT * TK, tid); cp_commit(); }
         auto len = [&](int j) { return min(TK, max(0, T - t0 - j * TK)); };
-        const int n = len(i);
-        float kk[TK], vv[TK];
-#pragma unroll
-        for (int j = 0; j < TK; j++) {
-            if (ASYNC) {
-                kk[j] = Elem<F>::ld(&sm.slab[s & 1][0][i * S::TILE + j * CT + c]) * V4_LOG2E;
-                vv[j] = Elem<F>::ld(&sm.slab[s & 1][1][i * S::TILE + j * CT + c]);
-            } else {
-                const size_t o = (size_t)min(mine0 + j, T - 1) * C + ch;
-                kk[j] = Elem<F>::ld(src[0] + o) * V4_LOG2E;
-                vv[j] = Elem<F>::ld(src[1] + o);
-            }
-        }
-        St a{0.f, 0.f, V4_MIN_VALUE};
+        const int n = FULL ? TK : len(i);
+        auto ld = [&](int tens, int j) {
+            if (ASYNC) return Pair<F>::ld(&sm.slab[s & 1][tens][i * S::TILE + j * CT + 2 * c]);
+            return L.ld(src[tens], (size_t)min(mine0 + j, T - 1) * C);
+        };
+        // the tile's own exponent (what the token-by-token maximum ends at) is its reference
+        f2 e[TK];       // k, then 2^{k - reference}
+        St a = empty_state();
+        e[0] = mul2(ld(0, 0), both(V4_LOG2E));
+        f2 kmin = e[0], kmax = e[0];
 #pragma unroll
         for (int j = 0; j < TK; j++)
-            if (j < n) {
-                float A, E, m;
-                exp2_pair(w + a.o, kk[j], A, E, m);
-                a.p = fmaf(A, a.p, E * vv[j]); a.q = fmaf(A, a.q, E); a.o = m;
+            if (FULL || j < n) {
+                if (j > 0) e[j] = mul2(ld(0, j), both(V4_LOG2E));
+                a.o = max2(add2(a.o, w), e[j]);
+                kmin = min2(kmin, e[j]);
+                kmax = max2(kmax, e[j]);
             }
-        St x = fold_tiles<NT, false>(sm, a, sm.carry[s & 1][c], i, c, w, len, &sm.carry[(s + 1) & 1][c]);
-        if (live && n > 0) {
-            if (!STATES && P.fine) {
-                float *f = P.fine + ((size_t)b * n8 + mine0 / TK) * 3 * C + ch;
-                f[0] = x.p; f[C] = x.q; f[2 * (size_t)C] = x.o;
-            }
-            if (P.coarse && (i & 7) == 0) {
-                float *f = P.coarse + ((size_t)b * n64 + mine0 / COARSE) * 3 * C + ch;
-                f[0] = x.p; f[C] = x.q; f[2 * (size_t)C] = x.o;
-            }
-        }
-        if (!STATES) {
-            F *y = (F *)P.y + row + ch;
+        const f2 up = sub2(kmax, a.o), down = sub2(a.o, kmin);
+        const bool tame = n > 0 && fmaxf(up.x, up.y) <= range && fmaxf(down.x, down.y) <= range;
+        if (tame) {
+            const f2 ref = neg2(a.o);
 #pragma unroll
             for (int j = 0; j < TK; j++)
-                if (j < n) {
-                    float A, E, m;
-                    exp2_pair(x.o, u + kk[j], A, E, m);
-                    const float out = __fdividef(fmaf(A, x.p, E * vv[j]), fmaf(A, x.q, E));
-                    if (live) Elem<F>::st(y + (size_t)(mine0 + j) * C, out);
-                    exp2_pair(w + x.o, kk[j], A, E, m);
-                    x.p = fmaf(A, x.p, E * vv[j]); x.q = fmaf(A, x.q, E); x.o = m;
+                if (FULL || j < n) {
+                    e[j] = ex2_2(add2(e[j], ref));
+                    a.p = fma2(W, a.p, mul2(e[j], ld(1, j)));
+                    a.q = fma2(W, a.q, e[j]);
                 }
+        } else {
+            auto one = [&](auto half) {
+                constexpr int H = decltype(half)::value;
+                float p = 0.f, q = 0.f, o = V4_MIN_VALUE;
+#pragma unroll
+                for (int j = 0; j < TK; j++)
+                    if (FULL || j < n) {
+                        float A, E, m;
+                        exp2_pair(part<H>(w) + o, part<H>(e[j]), A, E, m);
+                        p = fmaf(A, p, E * part<H>(ld(1, j))); q = fmaf(A, q, E); o = m;
+                    }
+                part<H>(a.p) = p; part<H>(a.q) = q; part<H>(a.o) = o;
+            };
+            one(FirstChannel{});
+            one(SecondChannel{});
         }
+        St x = fold_tiles<NT, false, FULL>(sm, a, sm.carry[s & 1][c], i, c, w, len, &sm.carry[(s + 1) & 1][c]);
+        if (n > 0) {
+            if (!STATES && P.fine) L.keep(P.fine + ((size_t)L.b * n8 + mine0 / TK) * 3 * C, x);
+            if (STATES && (i & 7) == 0) L.keep(P.coarse + ((size_t)L.b * n64 + mine0 / COARSE) * 3 * C, x);
+        }
+        if (!STATES) {
+            F *y = (F *)P.y + L.row + (size_t)mine0 * C + L.ch;
+            const f2 above = sub2(x.o, a.o);
+            if (tame && fmaxf(above.x, above.y) <= RANGE) {
+                const f2 sc = ex2_2(above);
+                f2 p = mul2(x.p, sc), q = mul2(x.q, sc);
+#pragma unroll
+                for (int j = 0; j < TK; j++)
+                    if (FULL || j < n) {
+                        const f2 v = ld(1, j), eu = mul2(U, e[j]);
+                        L.st(y, mul2(fma2(eu, v, p), rcp2(add2(q, eu))));
+                        y += C;
+                        p = fma2(W, p, mul2(e[j], v));
+                        q = fma2(W, q, e[j]);
+                    }
+            } else {
+                auto one = [&](auto half) {
+                    constexpr int H = decltype(half)::value;
+                    float p = part<H>(x.p), q = part<H>(x.q), o = part<H>(x.o);
+                    F *yo = y + H;
+#pragma unroll
+                    for (int j = 0; j < TK; j++)
+                        if (FULL || j < n) {
+                            float A, E, m;
+                            const float k = part<H>(ld(0, j)) * V4_LOG2E, v = part<H>(ld(1, j));
+                            exp2_pair(o, part<H>(u) + k, A, E, m);
+                            const float out = __fdividef(fmaf(A, p, E * v), fmaf(A, q, E));
+                            if (H ? L.live1 : L.live) Elem<F>::st(yo, out);
+                            yo += C;
+                            exp2_pair(part<H>(w) + o, k, A, E, m);
+                            p = fmaf(A, p, E * v); q = fmaf(A, q, E); o = m;
+                        }
+                };
+                one(FirstChannel{});
+                one(SecondChannel{});
+            }
+        }
+    };
+    for (int s = 0; s < P.nslab; s++) {
+        if (ASYNC) cp_wait0();
+        __syncthreads();
+        if (ASYNC && s + 1 < P.nslab) { fetch_slab<F, NT, 2>(sm, cp, (s + 1) & 1, src, T, C, (s + 1) * NT * TK); cp_commit(); }
+        if ((s + 1) * NT * TK <= T) slab(std::true_type{}, s);
+        else slab(std::false_type{}, s);
     }
     if (!STATES && P.state_out) {
         __syncthreads();
-        if (i == 0 && live) {
-            const St f = sm.carry[P.nslab & 1][c];
-            P.state_out[so] = f.p; P.state_out[so + 1] = f.q; P.state_out[so + 2] = from_base2(f.o);
-        }
+        if (i == 0) L.put_state(P.state_out, sm.carry[P.nslab & 1][c]);
     }
 }
 
@@ -216,135 +396,241 @@ __global__ void __launch_bounds__(NT * CT, NT == 8 ? 8 : NT == 16 ? 4 : 2) k_v4_
 // FINE: forward left the state at the start of every tile; else the slab's states are rebuilt from the coarse ones
 // (or, one slab only, from state_in) by one more summary and fold.
 template <typename F, int NT, bool ASYNC, bool FINE>
-__global__ void __launch_bounds__(NT * CT, NT == 8 ? 7 : NT == 16 ? 3 : 1) k_v4_par_bwd(const Par P) {
+__global__ void __launch_bounds__(NT * CP, NT == 8 ? 7 : NT == 16 ? 3 : 1) k_v4_par_bwd(const Par P) {
     pdl_wait();
     pdl_trigger();
     typedef Smem<F, NT, 3, ASYNC> S;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     S &sm = *reinterpret_cast<S *>(smem_raw);
-    const int ncb = (P.C + CT - 1) / CT, b = blockIdx.x / ncb, c0 = (blockIdx.x - b * ncb) * CT;
-    const int tid = threadIdx.x, c = tid & (CT - 1), i = tid / CT, ch = min(c0 + c, P.C - 1), T = P.T, C = P.C;
-    const bool live = c0 + c < C;
-    const float wn = P.w.at(ch), w = wn * V4_LOG2E, u = Elem<F>::ld((const F *)P.u + ch) * V4_LOG2E;
-    const size_t row = (size_t)b * T * C, so = ((size_t)b * C + ch) * 3;
-    const F *const src[3] = {(const F *)P.k + row, (const F *)P.v + row, (const F *)P.gy + row};
+    const Place<ASYNC> L(P);
+    const int c = L.c, i = L.i, T = L.T, C = L.C;
+    const Copy<F, NT> cp(threadIdx.x, L.c0, C);
+    const f2 w = make_float2(P.w.at(L.ch) * V4_LOG2E, P.w.at(L.ch1) * V4_LOG2E), u = mul2(L.ld((const F *)P.u, 0), both(V4_LOG2E));
+    const F *const src[3] = {(const F *)P.k + L.row, (const F *)P.v + L.row, (const F *)P.gy + L.row};
     const int n8 = (T + TK - 1) / TK, n64 = (T + COARSE - 1) / COARSE, last = P.nslab - 1;
     if (i == 0) {
-        St g{0.f, 0.f, V4_MIN_VALUE};
-        if (P.gstate_out) {
-            g.p = P.gstate_out[so]; g.q = P.gstate_out[so + 1];
-            if (g.p != 0.f || g.q != 0.f) g.o = to_base2(P.gstate_out[so + 2]);
-        }
+        St g = L.ext_state(P.gstate_out);
+        if (g.p.x == 0.f && g.q.x == 0.f) g.o.x = V4_MIN_VALUE;
+        if (g.p.y == 0.f && g.q.y == 0.f) g.o.y = V4_MIN_VALUE;
         sm.carry[last & 1][c] = g;
     }
     // the state at the start of this thread's tile (FINE) or of the 64 tokens around it, for slab s
     auto start_state = [&](int s) {
         const int t = s * NT * TK + i * TK;
-        if (!FINE && !P.coarse) return P.state_in ? St{P.state_in[so], P.state_in[so + 1], to_base2(P.state_in[so + 2])} : St{0.f, 0.f, V4_MIN_VALUE};
-        const float *f = FINE ? P.fine + ((size_t)b * n8 + min(t / TK, n8 - 1)) * 3 * C + ch
-                              : P.coarse + ((size_t)b * n64 + min(t / COARSE, n64 - 1)) * 3 * C + ch;
-        return St{f[0], f[C], f[2 * (size_t)C]};
+        if (FINE) return L.kept(P.fine + ((size_t)L.b * n8 + min(t / TK, n8 - 1)) * 3 * C);
+        if (P.coarse) return L.kept(P.coarse + ((size_t)L.b * n64 + min(t / COARSE, n64 - 1)) * 3 * C);
+        return L.ext_state(P.state_in);
     };
-    St x = start_state(last);
-    if (ASYNC) { fetch_slab<F, NT, 3>(sm, last & 1, src, T, C, c0, last * NT * TK, tid); cp_commit(); }
-    float gw = 0.f, gu = 0.f;
-
-    for (int s = last; s >= 0; s--) {
+    St x0 = start_state(last);
+    if (ASYNC) { fetch_slab<F, NT, 3>(sm, cp, last & 1, src, T, C, last * NT * TK); cp_commit(); }
+    f2 gw = both(0.f), gu = both(0.f);
+    const f2 W = ex2_2(w), U = ex2_2(u);
+    const float range = RANGE - fmaxf(fabsf(u.x), fabsf(u.y));
+    // x: the state at the start of this thread's tile; FULL as in forward
+    auto slab = [&](auto full_tag, int s, St x) {
+        constexpr bool FULL = decltype(full_tag)::value;
         const int t0 = s * NT * TK, mine0 = t0 + i * TK;
-        if (ASYNC) cp_wait0();
-        __syncthreads();
-        St x_next;
-        if (s > 0) {
-            if (ASYNC) { fetch_slab<F, NT, 3>(sm, (s - 1) & 1, src, T, C, c0, t0 - NT * TK, tid); cp_commit(); }
-            x_next = start_state(s - 1);
-        }
         auto len = [&](int j) { return min(TK, max(0, T - t0 - j * TK)); };
-        const int n = len(i);
+        const int n = FULL ? TK : len(i);
         auto ld = [&](int tens, int j) {
-            return Elem<F>::ld(ASYNC ? &sm.slab[s & 1][tens][i * S::TILE + j * CT + c] : src[tens] + (size_t)min(mine0 + j, T - 1) * C + ch);
+            if (ASYNC) return Pair<F>::ld(&sm.slab[s & 1][tens][i * S::TILE + j * CT + 2 * c]);
+            return L.ld(src[tens], (size_t)min(mine0 + j, T - 1) * C);
         };
         if constexpr (!FINE) {
             // the state at the tile's start: fold the summaries of the tiles between the kept state and it.
             // Without `coarse` there is one slab and the kept state is the initial one.
-            St a{0.f, 0.f, V4_MIN_VALUE};
+            St a = empty_state();
+            auto one = [&](auto half) {
+                constexpr int H = decltype(half)::value;
+                float p = 0.f, q = 0.f, o = V4_MIN_VALUE;
 #pragma unroll
-            for (int j = 0; j < TK; j++)
-                if (j < n) {
-                    float A, E, m;
-                    const float k = ld(0, j) * V4_LOG2E, v = ld(1, j);
-                    exp2_pair(w + a.o, k, A, E, m);
-                    a.p = fmaf(A, a.p, E * v); a.q = fmaf(A, a.q, E); a.o = m;
-                }
+                for (int j = 0; j < TK; j++)
+                    if (j < n) {
+                        float A, E, m;
+                        exp2_pair(part<H>(w) + o, part<H>(ld(0, j)) * V4_LOG2E, A, E, m);
+                        p = fmaf(A, p, E * part<H>(ld(1, j))); q = fmaf(A, q, E); o = m;
+                    }
+                part<H>(a.p) = p; part<H>(a.q) = q; part<H>(a.o) = o;
+            };
+            one(FirstChannel{});
+            one(SecondChannel{});
             sm.sum[i][c] = a;
             __syncthreads();
-            for (int j = P.coarse ? (i & ~7) : 0; j < i; j++) x = fold(x, (float)len(j) * w, sm.sum[j][c]);
+            for (int j = P.coarse ? (i & ~7) : 0; j < i; j++) x = fold(x, mul2(w, both((float)len(j))), sm.sum[j][c]);
             __syncthreads();
         }
-        float ys[TK], zs[TK], ze[TK];      // y, gy / denominator, exponent of the token's own term in it
-        float dpdw = 0.f, dqdw = 0.f;      // d(p,q)/dw since the tile's start
+        // e: k;  then, tame, 2^{k-M}, M = max k;  else the exponent of the token's own term in its denominator
+        f2 ys[TK], zs[TK], e[TK];
+        e[0] = mul2(ld(0, 0), both(V4_LOG2E));
+        f2 kmin = e[0], M = e[0];
 #pragma unroll
-        for (int j = 0; j < TK; j++)
-            if (j < n) {
-                float A, E, m;
-                const float k = ld(0, j) * V4_LOG2E, v = ld(1, j), g = ld(2, j);
-                exp2_pair(x.o, u + k, A, E, m);
-                const float iden = __fdividef(1.f, fmaf(A, x.q, E));
-                ys[j] = fmaf(A, x.p, E * v) * iden;
-                zs[j] = g * iden;
-                ze[j] = k + u - m;
-                gw = fmaf(zs[j] * A, fmaf(-dqdw, ys[j], dpdw), gw);
-                gu = fmaf(zs[j] * E, v - ys[j], gu);
-                exp2_pair(w + x.o, k, A, E, m);
-                dpdw = A * (x.p + dpdw); dqdw = A * (x.q + dqdw);
-                x.p = fmaf(A, x.p, E * v); x.q = fmaf(A, x.q, E); x.o = m;
+        for (int j = 1; j < TK; j++)
+            if (FULL || j < n) {
+                e[j] = mul2(ld(0, j), both(V4_LOG2E));
+                kmin = min2(kmin, e[j]);
+                M = max2(M, e[j]);
             }
-        // reverse over the tile from an empty gradient
-        St a{0.f, 0.f, V4_MIN_VALUE};
+        const f2 wide = sub2(M, kmin), above = sub2(x.o, M);
+        const bool tame = fmaxf(wide.x, wide.y) <= range && fmaxf(above.x, above.y) <= RANGE;
+        f2 dpdw = both(0.f), dqdw = both(0.f);      // d(p,q)/dw since the tile's start ...
+        f2 dscale;                                  // ... and the exponent that scales them at the tile's end
+        St a = empty_state();
+        if (tame) {
+            // the exponent of the gradient that leaves the tile at its start: the maximum over the tokens of j w minus
+            // the exponent of the token's denominator, as the token-by-token recurrence keeps it.  Only gstate_in
+            // shows which representation was used.
+            if (P.gstate_in) {
+                f2 o = x.o, back = both(0.f);
 #pragma unroll
-        for (int j = TK - 1; j >= 0; j--)
-            if (j < n) {
-                float A, E, m;
-                exp2_pair(w + a.o, ze[j] - ld(0, j) * V4_LOG2E - u, A, E, m);
-                E *= zs[j];
-                a.p = fmaf(A, a.p, E); a.q = fmaf(A, a.q, -E * ys[j]); a.o = m;
+                for (int j = 0; j < TK; j++)
+                    if (FULL || j < n) {
+                        a.o = max2(a.o, sub2(back, max2(o, add2(u, e[j]))));
+                        back = add2(back, w);
+                        o = max2(add2(o, w), e[j]);
+                    }
             }
-        St g = fold_tiles<NT, true>(sm, a, sm.carry[s & 1][c], i, c, w, len, &sm.carry[(s + 1) & 1][c]);
-        // what the gradient at the tile's end sees of the decay inside the tile
-        if (n > 0) gw = fmaf(fmaf(g.p, dpdw, g.q * dqdw), ex2(x.o + g.o), gw);
-        F *gk = (F *)P.gk + row + ch, *gv = (F *)P.gv + row + ch;
+            const f2 sc = ex2_2(above), ref = neg2(M);
+            f2 p = mul2(x.p, sc), q = mul2(x.q, sc);
 #pragma unroll
-        for (int j = TK - 1; j >= 0; j--)
-            if (j < n) {
-                const float k = ld(0, j) * V4_LOG2E, v = ld(1, j);
-                float A = zs[j] * ex2(ze[j]), E = ex2(k + g.o), m;
-                if (live) {
-                    Elem<F>::st(gk + (size_t)(mine0 + j) * C, fmaf(A, v - ys[j], E * fmaf(g.p, v, g.q)));
-                    Elem<F>::st(gv + (size_t)(mine0 + j) * C, fmaf(E, g.p, A));
+            for (int j = 0; j < TK; j++)
+                if (FULL || j < n) {
+                    const f2 v = ld(1, j);
+                    e[j] = ex2_2(add2(e[j], ref));
+                    const f2 eu = mul2(U, e[j]), iden = rcp2(add2(q, eu));
+                    ys[j] = mul2(fma2(eu, v, p), iden);
+                    zs[j] = mul2(ld(2, j), iden);
+                    gw = fma2(zs[j], fma2(neg2(dqdw), ys[j], dpdw), gw);
+                    gu = fma2(mul2(zs[j], eu), sub2(v, ys[j]), gu);
+                    const f2 wp = mul2(W, p), wq = mul2(W, q);
+                    dpdw = fma2(W, dpdw, wp); dqdw = fma2(W, dqdw, wq);
+                    p = fma2(e[j], v, wp); q = add2(wq, e[j]);
                 }
-                exp2_pair(w + g.o, ze[j] - k - u, A, E, m);
-                E *= zs[j];
-                g.p = fmaf(A, g.p, E); g.q = fmaf(A, g.q, -E * ys[j]); g.o = m;
+            dscale = M;
+            // the reverse recurrence from an empty gradient: exponent -M throughout
+#pragma unroll
+            for (int j = TK - 1; j >= 0; j--)
+                if (FULL || j < n) {
+                    a.p = fma2(W, a.p, zs[j]);
+                    a.q = fma2(W, a.q, neg2(mul2(zs[j], ys[j])));
+                }
+            if (P.gstate_in) {
+                const f2 r = ex2_2(sub2(ref, a.o));
+                a.p = mul2(a.p, r); a.q = mul2(a.q, r);
+            } else {
+                a.o = ref;
             }
-        x = x_next;
+        } else {
+            auto one = [&](auto half) {
+                constexpr int H = decltype(half)::value;
+                float p = part<H>(x.p), q = part<H>(x.q), o = part<H>(x.o), dp = 0.f, dq = 0.f;
+#pragma unroll
+                for (int j = 0; j < TK; j++)
+                    if (FULL || j < n) {
+                        float A, E, m;
+                        const float k = part<H>(e[j]), v = part<H>(ld(1, j)), g = part<H>(ld(2, j));
+                        exp2_pair(o, part<H>(u) + k, A, E, m);
+                        const float iden = __fdividef(1.f, fmaf(A, q, E)), y = fmaf(A, p, E * v) * iden, z = g * iden;
+                        part<H>(ys[j]) = y;
+                        part<H>(zs[j]) = z;
+                        part<H>(e[j]) = k + part<H>(u) - m;
+                        part<H>(gw) = fmaf(z * A, fmaf(-dq, y, dp), part<H>(gw));
+                        part<H>(gu) = fmaf(z * E, v - y, part<H>(gu));
+                        exp2_pair(part<H>(w) + o, k, A, E, m);
+                        dp = A * (p + dp); dq = A * (q + dq);
+                        p = fmaf(A, p, E * v); q = fmaf(A, q, E); o = m;
+                    }
+                part<H>(dpdw) = dp; part<H>(dqdw) = dq; part<H>(dscale) = o;
+                float gp = 0.f, gq = 0.f, go = V4_MIN_VALUE;
+#pragma unroll
+                for (int j = TK - 1; j >= 0; j--)
+                    if (FULL || j < n) {
+                        float A, E, m;
+                        exp2_pair(part<H>(w) + go, part<H>(e[j]) - part<H>(ld(0, j)) * V4_LOG2E - part<H>(u), A, E, m);
+                        E *= part<H>(zs[j]);
+                        gp = fmaf(A, gp, E); gq = fmaf(A, gq, -E * part<H>(ys[j])); go = m;
+                    }
+                part<H>(a.p) = gp; part<H>(a.q) = gq; part<H>(a.o) = go;
+            };
+            one(FirstChannel{});
+            one(SecondChannel{});
+        }
+        if (!FULL && n == 0) a = empty_state();
+        St g = fold_tiles<NT, true, FULL>(sm, a, sm.carry[s & 1][c], i, c, w, len, &sm.carry[(s + 1) & 1][c]);
+        // what the gradient at the tile's end sees of the decay inside the tile
+        if (FULL || n > 0) gw = fma2(fma2(g.p, dpdw, mul2(g.q, dqdw)), ex2_2(add2(dscale, g.o)), gw);
+        const size_t out0 = L.row + (size_t)(mine0 + TK - 1) * C + L.ch;
+        F *gk = (F *)P.gk + out0, *gv = (F *)P.gv + out0;
+        const f2 gs = add2(g.o, M);
+        if (tame && fmaxf(gs.x, gs.y) <= GRAD_RANGE) {
+            const f2 sc = ex2_2(gs);
+            f2 gp = mul2(g.p, sc), gq = mul2(g.q, sc);
+#pragma unroll
+            for (int j = TK - 1; j >= 0; j--) {
+                if (FULL || j < n) {
+                    const f2 v = ld(1, j), t = mul2(zs[j], mul2(U, e[j]));
+                    L.st(gk, fma2(t, sub2(v, ys[j]), mul2(e[j], fma2(gp, v, gq))));
+                    L.st(gv, fma2(e[j], gp, t));
+                    gp = fma2(W, gp, zs[j]);
+                    gq = fma2(W, gq, neg2(mul2(zs[j], ys[j])));
+                }
+                gk -= C; gv -= C;
+            }
+        } else {
+            auto one = [&](auto half) {
+                constexpr int H = decltype(half)::value;
+                float gp = part<H>(g.p), gq = part<H>(g.q), go = part<H>(g.o);
+                F *ok = gk + H, *ov = gv + H;
+#pragma unroll
+                for (int j = TK - 1; j >= 0; j--) {
+                    if (FULL || j < n) {
+                        const float k = part<H>(ld(0, j)) * V4_LOG2E, v = part<H>(ld(1, j)), y = part<H>(ys[j]), z = part<H>(zs[j]);
+                        // (tame: z is scaled by 2^{-M}; its own term is z U e)
+                        const float t = tame ? z * (part<H>(U) * part<H>(e[j])) : z * ex2(part<H>(e[j]));
+                        float A, E = ex2(k + go), m;
+                        if (H ? L.live1 : L.live) {
+                            Elem<F>::st(ok, fmaf(t, v - y, E * fmaf(gp, v, gq)));
+                            Elem<F>::st(ov, fmaf(E, gp, t));
+                        }
+                        exp2_pair(part<H>(w) + go, tame ? -part<H>(M) : part<H>(e[j]) - k - part<H>(u), A, E, m);
+                        E *= z;
+                        gp = fmaf(A, gp, E); gq = fmaf(A, gq, -E * y); go = m;
+                    }
+                    ok -= C; ov -= C;
+                }
+            };
+            one(FirstChannel{});
+            one(SecondChannel{});
+        }
+    };
+    for (int s = last; s >= 0; s--) {
+        if (ASYNC) cp_wait0();
+        __syncthreads();
+        St next = x0;
+        if (s > 0) {
+            if (ASYNC) { fetch_slab<F, NT, 3>(sm, cp, (s - 1) & 1, src, T, C, (s - 1) * NT * TK); cp_commit(); }
+            next = start_state(s - 1);
+        }
+        if ((s + 1) * NT * TK <= T) slab(std::true_type{}, s, x0);
+        else slab(std::false_type{}, s, x0);
+        x0 = next;
     }
     // the tiles' shares of gw and gu, summed in a fixed order
     __syncthreads();
-    sm.sum[i][c] = St{gw, gu, 0.f};
+    sm.sum[i][c].p = gw;
+    sm.sum[i][c].q = gu;
     __syncthreads();
-    if (i == 0 && live) {
-        float a = 0.f, e = 0.f;
+    if (i == 0) {
+        f2 a = both(0.f), e = both(0.f);
 #pragma unroll 8
-        for (int j = 0; j < NT; j++) { a += sm.sum[j][c].p; e += sm.sum[j][c].q; }
-        P.gw[(size_t)b * C + ch] = a * wn;
-        P.gu[(size_t)b * C + ch] = e;
-        if (P.gstate_in) {
-            const St f = sm.carry[1][c];      // (slab 0 leaves its carry there)
-            P.gstate_in[so] = f.p; P.gstate_in[so + 1] = f.q; P.gstate_in[so + 2] = from_base2(f.o);
-        }
+        for (int j = 0; j < NT; j++) { a = add2(a, sm.sum[j][c].p); e = add2(e, sm.sum[j][c].q); }
+        const size_t o = (size_t)L.b * C + L.ch;
+        L.st(P.gw + o, mul2(a, mul2(w, both(V4_LN2))));
+        L.st(P.gu + o, e);
+        if (P.gstate_in) L.put_state(P.gstate_in, sm.carry[1][c]);      // (slab 0 leaves its carry there)
     }
 }
 
-// Tiles per slab: 8 (8 CTAs of 128 threads per SM) once the CTAs alone fill the SMs; else longer slabs, and never
+// Tiles per slab: 8 (7 CTAs of 64 threads per SM) once the CTAs alone fill the SMs; else longer slabs, and never
 // much longer than the segment.
 int pick_tiles(int B, int T, int C) {
     const long long ctas = (long long)B * ((C + CT - 1) / CT), sms = device_sm_count();
@@ -355,7 +641,7 @@ int pick_tiles(int B, int T, int C) {
 template <class K>
 int launch(K kern, size_t smem, unsigned char (&attr_done)[64], const Par &P, int nt, cudaStream_t s) {
     if (!set_max_smem_once(kern, (int)smem, attr_done)) return WKV_ERR_LAUNCH;
-    return launch_chained(kern, dim3(P.B * ((P.C + CT - 1) / CT)), dim3(nt * CT), smem, s, P);
+    return launch_chained(kern, dim3(P.B * ((P.C + CT - 1) / CT)), dim3(nt * CP), smem, s, P);
 }
 template <typename F, int NT, bool ASYNC>
 int launch_fwd(Par P, bool states, cudaStream_t s) {

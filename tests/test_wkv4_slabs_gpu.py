@@ -12,14 +12,25 @@ from oracle import wkv_oracle as O
 pytestmark = pytest.mark.gpu
 
 
+def spread(c, how):
+    """keys, bonus and decay that leave the range one reference exponent per tile can hold, for some channels and tokens"""
+    if how == "wild":
+        c["k"][:, ::5, ::3] += 70.0
+        c["k"][:, 3::7, 1::3] -= 90.0
+        c["u"][2::4] *= 50.0
+        c["td"][1::5] = 3.0
+    return c
+
+
+@pytest.mark.parametrize("how", ["plain", "wild"])
 @pytest.mark.parametrize("B,T,C,dtype", [
     (1, 16, 16, torch.float32), (2, 17, 24, torch.bfloat16), (1, 63, 40, torch.float32), (2, 64, 20, torch.bfloat16),
     (1, 65, 7, torch.float32), (1, 129, 9, torch.float32), (1, 127, 16, torch.float32), (1, 128, 32, torch.bfloat16), (3, 257, 48, torch.float32),
-    (1, 511, 16, torch.float16), (2, 300, 1, torch.float32), (4, 200, 1264, torch.float32), (8, 136, 1200, torch.bfloat16)])
-def test_v4_matches_oracle(B, T, C, dtype):
+    (1, 511, 16, torch.bfloat16), (2, 300, 1, torch.float32), (4, 200, 1264, torch.float32), (8, 136, 1200, torch.bfloat16)])
+def test_v4_matches_oracle(B, T, C, dtype, how):
     import rwkv_infctx_trainer_b200 as W
     from rwkv_infctx_trainer_b200 import _lib as L
-    c = inputs.wkv4_case(B, T, C, seed=800 + T)
+    c = spread(inputs.wkv4_case(B, T, C, seed=800 + T), how)
     d = {n: TL.to_dev(c[n], dtype) for n in ("u", "k", "v", "gy")}
     td = TL.to_dev(c["td"], torch.float32)
     f64 = lambda t: t.detach().float().cpu().double().numpy()
