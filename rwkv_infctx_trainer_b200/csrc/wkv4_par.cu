@@ -32,9 +32,9 @@
 // constant: one ex2 and one reciprocal instead of two max-shifted pairs, and the reverse recurrence needs no exponential at
 // all (gp <- W gp + z, gq <- W gq - z y with z = gy / denominator).  That is sound while nothing leaves the fp32
 // range: |u| plus the distance of any k from M at most 60, the incoming state at most 2^60 above M, the incoming
-// gradient at most 2^90.  A tile that is not (`tame` false) takes the token-by-token max-shift of
-// RWKV-v4neo/cuda/wkv_cuda_bf16.cu:7-158; both give the same state representation (o = the running maximum) at
-// tile boundaries.
+// gradient at most 2^90.  A CTA that meets a tile that is not tame in this sense starts its walk over by the
+// token-by-token max-shift of RWKV-v4neo/cuda/wkv_cuda_bf16.cu:7-158; both keep the same state representation (o =
+// the running maximum) at tile boundaries.
 #include <type_traits>
 
 #include "wkv4_common.cuh"
@@ -62,6 +62,8 @@ __device__ __forceinline__ float rcp(float x) {
 
 // ---- two channels at a time
 typedef float2 f2;
+// keeps loads of later tokens from being hoisted above this point: all eight at once do not fit the registers
+__device__ __forceinline__ void no_hoist() { asm volatile("" ::: "memory"); }
 __device__ __forceinline__ unsigned long long bits(const f2 &a) { return *reinterpret_cast<const unsigned long long *>(&a); }
 __device__ __forceinline__ f2 from_bits(unsigned long long v) { return *reinterpret_cast<f2 *>(&v); }
 __device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c) {
@@ -86,11 +88,6 @@ __device__ __forceinline__ f2 max2(f2 a, f2 b) { return make_float2(fmaxf(a.x, b
 __device__ __forceinline__ f2 min2(f2 a, f2 b) { return make_float2(fminf(a.x, b.x), fminf(a.y, b.y)); }
 __device__ __forceinline__ f2 ex2_2(f2 a) { return make_float2(ex2(a.x), ex2(a.y)); }
 __device__ __forceinline__ f2 rcp2(f2 a) { return make_float2(rcp(a.x), rcp(a.y)); }
-template <int H> __device__ __forceinline__ float &part(f2 &a) { return H ? a.y : a.x; }
-template <int H> __device__ __forceinline__ float part(const f2 &a) { return H ? a.y : a.x; }
-typedef std::integral_constant<int, 0> FirstChannel;
-typedef std::integral_constant<int, 1> SecondChannel;
-
 struct St {
     f2 p, q, o;
 };
@@ -99,15 +96,6 @@ __device__ __forceinline__ St empty_state() { return St{both(0.f), both(0.f), bo
 __device__ __forceinline__ St fold(const St &a, f2 nw, const St &b) {
     const f2 d = add2(a.o, nw), m = max2(d, b.o), A = ex2_2(sub2(d, m)), E = ex2_2(sub2(b.o, m));
     return St{fma2(A, a.p, mul2(E, b.p)), fma2(A, a.q, mul2(E, b.q)), m};
-}
-
-// ---- one channel: the token-by-token max-shift.  (A,E) = (2^{a-m}, 2^{b-m}), m = max(a,b): one ex2
-__device__ __forceinline__ void exp2_pair(float a, float b, float &A, float &E, float &m) {
-    const float d = a - b, e = ex2(-fabsf(d));
-    const bool ge = d >= 0.f;
-    A = ge ? 1.f : e;
-    E = ge ? e : 1.f;
-    m = fmaxf(a, b);
 }
 
 // ---- two adjacent elements
@@ -127,6 +115,81 @@ template <> struct Pair<__half> {
     static __device__ __forceinline__ void st(__half *p, f2 v) { *reinterpret_cast<__half2 *>(p) = __floats2half2_rn(v.x, v.y); }
 };
 
+// ---- One tile, one channel, by the token-by-token max-shift: what a CTA falls back to.
+// (A,E) = (2^{a-m}, 2^{b-m}), m = max(a,b): one ex2
+__device__ __forceinline__ void exp2_pair(float a, float b, float &A, float &E, float &m) {
+    const float d = a - b, e = ex2(-fabsf(d));
+    const bool ge = d >= 0.f;
+    A = ge ? 1.f : e;
+    E = ge ? e : 1.f;
+    m = fmaxf(a, b);
+}
+struct Slow {
+    float p, q, o;
+};
+// token j of the tile: element j * stride of k, v, gy
+template <typename F>
+__device__ __noinline__ Slow slow_summary(const F *k, const F *v, size_t stride, int n, float w) {
+    Slow a{0.f, 0.f, V4_MIN_VALUE};
+    for (int j = 0; j < n; j++) {
+        float A, E, m;
+        exp2_pair(w + a.o, Elem<F>::ld(k + j * stride) * V4_LOG2E, A, E, m);
+        a.p = fmaf(A, a.p, E * Elem<F>::ld(v + j * stride)); a.q = fmaf(A, a.q, E); a.o = m;
+    }
+    return a;
+}
+template <typename F>
+__device__ __noinline__ void slow_apply(const F *k, const F *v, size_t stride, int n, float w, float u, Slow x, F *y, size_t C) {
+    for (int j = 0; j < n; j++) {
+        float A, E, m;
+        const float kj = Elem<F>::ld(k + j * stride) * V4_LOG2E, vj = Elem<F>::ld(v + j * stride);
+        exp2_pair(x.o, u + kj, A, E, m);
+        Elem<F>::st(y + j * C, __fdividef(fmaf(A, x.p, E * vj), fmaf(A, x.q, E)));
+        exp2_pair(w + x.o, kj, A, E, m);
+        x.p = fmaf(A, x.p, E * vj); x.q = fmaf(A, x.q, E); x.o = m;
+    }
+}
+struct SlowGrads {
+    Slow a;                             // the reverse summary from an empty gradient
+    float gw, gu, dpdw, dqdw, o_end;
+};
+// x: the state at the tile's start.  With gk given, also the outputs, from the gradient g at the tile's end.
+template <typename F>
+__device__ __noinline__ SlowGrads slow_backward(const F *k, const F *v, const F *gy, size_t stride, int n, float w, float u, Slow x,
+                                                Slow g, F *gk, F *gv, size_t C) {
+    float ys[TK], zs[TK], ze[TK];
+    SlowGrads r{};
+    for (int j = 0; j < n; j++) {
+        float A, E, m;
+        const float kj = Elem<F>::ld(k + j * stride) * V4_LOG2E, vj = Elem<F>::ld(v + j * stride);
+        exp2_pair(x.o, u + kj, A, E, m);
+        const float iden = __fdividef(1.f, fmaf(A, x.q, E));
+        ys[j] = fmaf(A, x.p, E * vj) * iden;
+        zs[j] = Elem<F>::ld(gy + j * stride) * iden;
+        ze[j] = kj + u - m;
+        r.gw = fmaf(zs[j] * A, fmaf(-r.dqdw, ys[j], r.dpdw), r.gw);
+        r.gu = fmaf(zs[j] * E, vj - ys[j], r.gu);
+        exp2_pair(w + x.o, kj, A, E, m);
+        r.dpdw = A * (x.p + r.dpdw); r.dqdw = A * (x.q + r.dqdw);
+        x.p = fmaf(A, x.p, E * vj); x.q = fmaf(A, x.q, E); x.o = m;
+    }
+    r.o_end = x.o;
+    for (int j = n - 1; j >= 0; j--) {
+        float A, E, m;
+        const float kj = Elem<F>::ld(k + j * stride) * V4_LOG2E, vj = Elem<F>::ld(v + j * stride);
+        if (gk) {
+            const float t = zs[j] * ex2(ze[j]), e = ex2(kj + g.o);
+            Elem<F>::st(gk + j * C, fmaf(t, vj - ys[j], e * fmaf(g.p, vj, g.q)));
+            Elem<F>::st(gv + j * C, fmaf(e, g.p, t));
+        }
+        exp2_pair(w + g.o, ze[j] - kj - u, A, E, m);
+        E *= zs[j];
+        g.p = fmaf(A, g.p, E); g.q = fmaf(A, g.q, -E * ys[j]); g.o = m;
+    }
+    r.a = g;
+    return r;
+}
+
 struct Par {
     int B, T, C, nslab;
     Decay4 w;
@@ -138,10 +201,14 @@ struct Par {
     float *coarse;      // [B][T/64][3][C]: at the start of every 64 tokens, or NULL
 };
 
-// Shared memory: the slab's k, v (and gy) as [stage][tensor][tile][8 tokens + 1 of padding][16 channels] -- the
-// padding keeps the tiles a warp reads in different banks -- then the tile summaries.
+// Shared memory: the slab's k, v (and gy) as [stage][tensor][tile][8 tokens + padding][16 channels] -- the
+// padding keeps the tiles a warp reads in different banks, and in backward holds the tile's start state: 16 floats of
+// p, q, o behind its k, v, gy -- then the tile summaries.
+template <typename F> struct Tile {
+    static constexpr int SIZE = (TK + (sizeof(F) == 4 ? 1 : 3)) * CT;   // elements
+};
 template <typename F, int NT, int NTENS, bool ASYNC> struct Smem {
-    static constexpr int TILE = (TK + 1) * CT;                  // elements
+    static constexpr int TILE = Tile<F>::SIZE;
     F slab[ASYNC ? 2 : 1][NTENS][ASYNC ? NT * TILE : 8];
     St sum[NT][CP];
     St gsum[NT / 8][CP];
@@ -159,10 +226,10 @@ template <typename F, int NT> struct Copy {
         r0 = tid / CPR;
         ch0 = c0 + (tid % CPR) * PER;
         in = ch0 < C;
-        dst = (((r0 / TK) * (TK + 1) + r0 % TK) * CT + (tid % CPR) * PER) * sizeof(F);
+        dst = ((r0 / TK) * Tile<F>::SIZE + (r0 % TK) * CT + (tid % CPR) * PER) * sizeof(F);
     }
     static_assert(ROWS % TK == 0, "");
-    static constexpr uint32_t STEP = (ROWS / TK) * (TK + 1) * CT * sizeof(F);
+    static constexpr uint32_t STEP = (ROWS / TK) * Tile<F>::SIZE * sizeof(F);
 };
 // rows past the end and channels past the last are zero-filled
 template <typename F, int NT, int NTENS, class S>
@@ -181,16 +248,32 @@ __device__ __forceinline__ void fetch_slab(S &sm, const Copy<F, NT> &cp, int sta
         }
     }
 }
+// The start states of the slab's tiles (rows `first` .. of [..][3][C]) to the padding of the tiles.
+template <typename F, int NT, class S>
+__device__ __forceinline__ void fetch_states(S &sm, int stage, const float *fine, int first, int n8, int C, int c0, int tid) {
+#pragma unroll
+    for (int x = tid; x < NT * 12; x += NT * CP) {
+        const int tile = x / 12, r = x % 12 / 4, ch = x % 4 * 4;
+        const bool in = first + tile < n8 && c0 + ch < C;
+        const float *g = in ? fine + ((size_t)(first + tile) * 3 + r) * C + c0 + ch : fine;
+        const uint32_t d = (uint32_t)__cvta_generic_to_shared(&sm.slab[stage][r][tile * S::TILE + TK * CT]) + ch * 4;
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(g), "r"(in ? 16 : 0) : "memory");
+    }
+}
 __device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 __device__ __forceinline__ void cp_wait0() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
 
 // What thread (tile i, pair c) starts from: `carry` folded with everything between the slab's edge and tile i --
 // the tiles before i, or (REV) the tiles after it.  `mine` is this tile's summary, len(j) the tokens of tile j.
-// The tile at the far edge leaves the next slab's carry in `next`.  Contains the barriers.
+// The tile at the far edge leaves the next slab's carry in `next`.  Contains the barriers; the first also ORs
+// `bad` over the CTA, and when that is set nothing is folded and `stop` is.
 template <int NT, bool REV, bool FULL, class S, class Len>
-__device__ __forceinline__ St fold_tiles(S &sm, const St &mine, const St &carry, int i, int c, f2 w, Len len, St *next) {
+__device__ __forceinline__ St fold_tiles(S &sm, const St &mine, const St &carry, int i, int c, f2 w, Len len, St *next, bool bad, bool &stop) {
     sm.sum[i][c] = mine;
-    __syncthreads();
+    if (__syncthreads_or(bad)) {
+        stop = true;
+        return carry;
+    }
     const int g = i >> 3, k = REV ? 7 - (i & 7) : (i & 7);      // group of eight tiles; how many of it are in between
     auto at = [&](int j) { return REV ? 8 * g + 7 - j : 8 * g + j; };
     const f2 w8 = mul2(w, both((float)TK));
@@ -255,6 +338,13 @@ template <bool ASYNC> struct Place {
         const float *x = s + ((size_t)b * C + ch) * 3, *y = s + ((size_t)b * C + ch1) * 3;
         return St{make_float2(x[0], y[0]), make_float2(x[1], y[1]), make_float2(to_base2(x[2]), to_base2(y[2]))};
     }
+    // (an all-zero gradient carries no exponent)
+    __device__ __forceinline__ St ext_gradient(const float *s) const {
+        St g = ext_state(s);
+        if (g.p.x == 0.f && g.q.x == 0.f) g.o.x = V4_MIN_VALUE;
+        if (g.p.y == 0.f && g.q.y == 0.f) g.o.y = V4_MIN_VALUE;
+        return g;
+    }
     __device__ __forceinline__ void put_state(float *s, const St &f) const {
         float *x = s + ((size_t)b * C + ch) * 3;
         if (live) { x[0] = f.p.x; x[1] = f.q.x; x[2] = from_base2(f.o.x); }
@@ -268,6 +358,37 @@ template <bool ASYNC> struct Place {
 };
 
 // ---------------------------------------------------------------------------------------------- forward
+// The whole walk by the token-by-token max-shift: a CTA that meets a tile that is not tame starts over here.
+// Out of line and reached with nothing live, so that the usual path does not pay for it in registers.
+template <typename F, int NT, bool ASYNC, bool STATES, class S>
+__device__ __noinline__ void slow_forward(const Par &P, S &sm) {
+    const Place<ASYNC> L(P);
+    const int c = L.c, i = L.i, T = L.T, C = L.C, n8 = (T + TK - 1) / TK, n64 = (T + COARSE - 1) / COARSE;
+    const f2 w = make_float2(P.w.at(L.ch) * V4_LOG2E, P.w.at(L.ch1) * V4_LOG2E), u = mul2(L.ld((const F *)P.u, 0), both(V4_LOG2E));
+    const F *const k = (const F *)P.k + L.row, *const v = (const F *)P.v + L.row;
+    if (i == 0) sm.carry[0][c] = L.ext_state(P.state_in);
+    for (int s = 0; s < P.nslab; s++) {
+        __syncthreads();
+        const int t0 = s * NT * TK, mine0 = t0 + i * TK;
+        auto len = [&](int j) { return min(TK, max(0, T - t0 - j * TK)); };
+        const int n = len(i);
+        const size_t o0 = (size_t)min(mine0, T - 1) * C + L.ch, o1 = o0 - L.ch + L.ch1;
+        const Slow f = slow_summary<F>(k + o0, v + o0, C, n, w.x), g = slow_summary<F>(k + o1, v + o1, C, n, w.y);
+        bool stop = false;
+        const St x = fold_tiles<NT, false, false>(sm, St{make_float2(f.p, g.p), make_float2(f.q, g.q), make_float2(f.o, g.o)}, sm.carry[s & 1][c], i, c, w,
+                                                  len, &sm.carry[(s + 1) & 1][c], false, stop);
+        if (n > 0) {
+            if (!STATES && P.fine) L.keep(P.fine + ((size_t)L.b * n8 + mine0 / TK) * 3 * C, x);
+            if (STATES && (i & 7) == 0) L.keep(P.coarse + ((size_t)L.b * n64 + mine0 / COARSE) * 3 * C, x);
+        }
+        if (!STATES) {
+            F *y = (F *)P.y + L.row;
+            if (L.live) slow_apply<F>(k + o0, v + o0, C, n, w.x, u.x, Slow{x.p.x, x.q.x, x.o.x}, y + o0, C);
+            if (L.live1) slow_apply<F>(k + o1, v + o1, C, n, w.y, u.y, Slow{x.p.y, x.q.y, x.o.y}, y + o1, C);
+        }
+    }
+}
+
 // STATES: only the coarse states are wanted (backward without a hand-over)
 template <typename F, int NT, bool ASYNC, bool STATES>
 __global__ void __launch_bounds__(NT * CP, NT == 8 ? 8 : NT == 16 ? 4 : 2) k_v4_par_fwd(const Par P) {
@@ -286,7 +407,8 @@ __global__ void __launch_bounds__(NT * CP, NT == 8 ? 8 : NT == 16 ? 4 : 2) k_v4_
     const int n8 = (T + TK - 1) / TK, n64 = (T + COARSE - 1) / COARSE;
     const f2 W = ex2_2(w), U = ex2_2(u);
     const float range = RANGE - fmaxf(fabsf(u.x), fabsf(u.y));
-    // FULL: every tile of the slab has its 8 tokens
+    bool bad = false;       // a tile of this thread was not tame
+    // FULL: every tile of the slab has its 8 tokens.  Returns false when the CTA has to start over.
     auto slab = [&](auto full_tag, int s) {
         constexpr bool FULL = decltype(full_tag)::value;
         const int t0 = s * NT * TK, mine0 = t0 + i * TK;      // first token of the slab, of this tile
@@ -310,33 +432,18 @@ __global__ void __launch_bounds__(NT * CP, NT == 8 ? 8 : NT == 16 ? 4 : 2) k_v4_
                 kmax = max2(kmax, e[j]);
             }
         const f2 up = sub2(kmax, a.o), down = sub2(a.o, kmin);
-        const bool tame = n > 0 && fmaxf(up.x, up.y) <= range && fmaxf(down.x, down.y) <= range;
-        if (tame) {
-            const f2 ref = neg2(a.o);
+        if (n > 0 && !(fmaxf(up.x, up.y) <= range && fmaxf(down.x, down.y) <= range)) bad = true;
+        const f2 ref = neg2(a.o);
 #pragma unroll
-            for (int j = 0; j < TK; j++)
-                if (FULL || j < n) {
-                    e[j] = ex2_2(add2(e[j], ref));
-                    a.p = fma2(W, a.p, mul2(e[j], ld(1, j)));
-                    a.q = fma2(W, a.q, e[j]);
-                }
-        } else {
-            auto one = [&](auto half) {
-                constexpr int H = decltype(half)::value;
-                float p = 0.f, q = 0.f, o = V4_MIN_VALUE;
-#pragma unroll
-                for (int j = 0; j < TK; j++)
-                    if (FULL || j < n) {
-                        float A, E, m;
-                        exp2_pair(part<H>(w) + o, part<H>(e[j]), A, E, m);
-                        p = fmaf(A, p, E * part<H>(ld(1, j))); q = fmaf(A, q, E); o = m;
-                    }
-                part<H>(a.p) = p; part<H>(a.q) = q; part<H>(a.o) = o;
-            };
-            one(FirstChannel{});
-            one(SecondChannel{});
-        }
-        St x = fold_tiles<NT, false, FULL>(sm, a, sm.carry[s & 1][c], i, c, w, len, &sm.carry[(s + 1) & 1][c]);
+        for (int j = 0; j < TK; j++)
+            if (FULL || j < n) {
+                e[j] = ex2_2(add2(e[j], ref));
+                a.p = fma2(W, a.p, mul2(e[j], ld(1, j)));
+                a.q = fma2(W, a.q, e[j]);
+            }
+        bool stop = false;
+        St x = fold_tiles<NT, false, FULL>(sm, a, sm.carry[s & 1][c], i, c, w, len, &sm.carry[(s + 1) & 1][c], bad, stop);
+        if (stop) return false;
         if (n > 0) {
             if (!STATES && P.fine) L.keep(P.fine + ((size_t)L.b * n8 + mine0 / TK) * 3 * C, x);
             if (STATES && (i & 7) == 0) L.keep(P.coarse + ((size_t)L.b * n64 + mine0 / COARSE) * 3 * C, x);
@@ -344,55 +451,91 @@ __global__ void __launch_bounds__(NT * CP, NT == 8 ? 8 : NT == 16 ? 4 : 2) k_v4_
         if (!STATES) {
             F *y = (F *)P.y + L.row + (size_t)mine0 * C + L.ch;
             const f2 above = sub2(x.o, a.o);
-            if (tame && fmaxf(above.x, above.y) <= RANGE) {
-                const f2 sc = ex2_2(above);
-                f2 p = mul2(x.p, sc), q = mul2(x.q, sc);
+            if (n > 0 && !(fmaxf(above.x, above.y) <= RANGE)) bad = true;
+            const f2 sc = ex2_2(above);
+            f2 p = mul2(x.p, sc), q = mul2(x.q, sc);
 #pragma unroll
-                for (int j = 0; j < TK; j++)
-                    if (FULL || j < n) {
-                        const f2 v = ld(1, j), eu = mul2(U, e[j]);
-                        L.st(y, mul2(fma2(eu, v, p), rcp2(add2(q, eu))));
-                        y += C;
-                        p = fma2(W, p, mul2(e[j], v));
-                        q = fma2(W, q, e[j]);
-                    }
-            } else {
-                auto one = [&](auto half) {
-                    constexpr int H = decltype(half)::value;
-                    float p = part<H>(x.p), q = part<H>(x.q), o = part<H>(x.o);
-                    F *yo = y + H;
-#pragma unroll
-                    for (int j = 0; j < TK; j++)
-                        if (FULL || j < n) {
-                            float A, E, m;
-                            const float k = part<H>(ld(0, j)) * V4_LOG2E, v = part<H>(ld(1, j));
-                            exp2_pair(o, part<H>(u) + k, A, E, m);
-                            const float out = __fdividef(fmaf(A, p, E * v), fmaf(A, q, E));
-                            if (H ? L.live1 : L.live) Elem<F>::st(yo, out);
-                            yo += C;
-                            exp2_pair(part<H>(w) + o, k, A, E, m);
-                            p = fmaf(A, p, E * v); q = fmaf(A, q, E); o = m;
-                        }
-                };
-                one(FirstChannel{});
-                one(SecondChannel{});
-            }
+            for (int j = 0; j < TK; j++)
+                if (FULL || j < n) {
+                    const f2 v = ld(1, j), eu = mul2(U, e[j]);
+                    L.st(y, mul2(fma2(eu, v, p), rcp2(add2(q, eu))));
+                    y += C;
+                    p = fma2(W, p, mul2(e[j], v));
+                    q = fma2(W, q, e[j]);
+                }
         }
+        return true;
     };
     for (int s = 0; s < P.nslab; s++) {
         if (ASYNC) cp_wait0();
         __syncthreads();
         if (ASYNC && s + 1 < P.nslab) { fetch_slab<F, NT, 2>(sm, cp, (s + 1) & 1, src, T, C, (s + 1) * NT * TK); cp_commit(); }
-        if ((s + 1) * NT * TK <= T) slab(std::true_type{}, s);
-        else slab(std::false_type{}, s);
+        if (!((s + 1) * NT * TK <= T ? slab(std::true_type{}, s) : slab(std::false_type{}, s))) break;
+    }
+    if (__syncthreads_or(bad)) {
+        if (ASYNC) cp_wait0();
+        slow_forward<F, NT, ASYNC, STATES>(P, sm);
+        __syncthreads();
     }
     if (!STATES && P.state_out) {
-        __syncthreads();
         if (i == 0) L.put_state(P.state_out, sm.carry[P.nslab & 1][c]);
     }
 }
 
 // ---------------------------------------------------------------------------------------------- backward
+// The states at the start of a slab's tiles, when only coarser ones were kept: fold the summaries of the tiles between the
+// kept state and the tile.  Without `coarse` there is one slab and the kept state is the initial one.
+template <typename F, bool ASYNC, class S, class Len>
+__device__ __noinline__ St rebuild_state(const Par &P, S &sm, const Place<ASYNC> &L, int mine0, St x, f2 w, Len len) {
+    const int i = L.i, c = L.c;
+    const size_t o0 = L.row + (size_t)min(mine0, L.T - 1) * L.C + L.ch, o1 = o0 - L.ch + L.ch1;
+    const F *const k = (const F *)P.k, *const v = (const F *)P.v;
+    const int n = len(i);
+    const Slow f = slow_summary<F>(k + o0, v + o0, L.C, n, w.x), g = slow_summary<F>(k + o1, v + o1, L.C, n, w.y);
+    __syncthreads();
+    sm.sum[i][c] = St{make_float2(f.p, g.p), make_float2(f.q, g.q), make_float2(f.o, g.o)};
+    __syncthreads();
+    for (int j = P.coarse ? (i & ~7) : 0; j < i; j++) x = fold(x, mul2(w, both((float)len(j))), sm.sum[j][c]);
+    __syncthreads();
+    return x;
+}
+
+// As slow_forward.  gw, gu: this thread's sums.
+template <typename F, int NT, bool ASYNC, bool FINE, class S>
+__device__ __noinline__ void slow_walk_back(const Par &P, S &sm, f2 &gw, f2 &gu) {
+    const Place<ASYNC> L(P);
+    const int c = L.c, i = L.i, T = L.T, C = L.C, n8 = (T + TK - 1) / TK, n64 = (T + COARSE - 1) / COARSE, last = P.nslab - 1;
+    const f2 w = make_float2(P.w.at(L.ch) * V4_LOG2E, P.w.at(L.ch1) * V4_LOG2E), u = mul2(L.ld((const F *)P.u, 0), both(V4_LOG2E));
+    const F *const k = (const F *)P.k + L.row, *const v = (const F *)P.v + L.row, *const gy = (const F *)P.gy + L.row;
+    F *const gk = (F *)P.gk + L.row, *const gv = (F *)P.gv + L.row;
+    if (i == 0) sm.carry[last & 1][c] = L.ext_gradient(P.gstate_out);
+    gw = gu = both(0.f);
+    for (int s = last; s >= 0; s--) {
+        __syncthreads();
+        const int t0 = s * NT * TK, mine0 = t0 + i * TK;
+        auto len = [&](int j) { return min(TK, max(0, T - t0 - j * TK)); };
+        const int n = len(i);
+        St x;
+        if (FINE) x = L.kept(P.fine + ((size_t)L.b * n8 + min(mine0 / TK, n8 - 1)) * 3 * C);
+        else
+            x = rebuild_state<F, ASYNC>(P, sm, L, mine0,
+                                        P.coarse ? L.kept(P.coarse + ((size_t)L.b * n64 + min(mine0 / COARSE, n64 - 1)) * 3 * C) : L.ext_state(P.state_in), w, len);
+        const size_t o0 = (size_t)min(mine0, T - 1) * C + L.ch, o1 = o0 - L.ch + L.ch1;
+        const Slow x0{x.p.x, x.q.x, x.o.x}, x1{x.p.y, x.q.y, x.o.y}, none{0.f, 0.f, V4_MIN_VALUE};
+        const SlowGrads f = slow_backward<F>(k + o0, v + o0, gy + o0, C, n, w.x, u.x, x0, none, nullptr, nullptr, 0),
+                        g = slow_backward<F>(k + o1, v + o1, gy + o1, C, n, w.y, u.y, x1, none, nullptr, nullptr, 0);
+        bool stop = false;
+        const St e = fold_tiles<NT, true, false>(sm, St{make_float2(f.a.p, g.a.p), make_float2(f.a.q, g.a.q), make_float2(f.a.o, g.a.o)},
+                                                 sm.carry[s & 1][c], i, c, w, len, &sm.carry[(s + 1) & 1][c], false, stop);
+        if (n == 0) continue;
+        gu = add2(gu, make_float2(f.gu, g.gu));
+        gw = add2(gw, make_float2(f.gw + (e.p.x * f.dpdw + e.q.x * f.dqdw) * ex2(f.o_end + e.o.x),
+                                  g.gw + (e.p.y * g.dpdw + e.q.y * g.dqdw) * ex2(g.o_end + e.o.y)));
+        if (L.live) slow_backward<F>(k + o0, v + o0, gy + o0, C, n, w.x, u.x, x0, Slow{e.p.x, e.q.x, e.o.x}, gk + o0, gv + o0, C);
+        if (L.live1) slow_backward<F>(k + o1, v + o1, gy + o1, C, n, w.y, u.y, x1, Slow{e.p.y, e.q.y, e.o.y}, gk + o1, gv + o1, C);
+    }
+}
+
 // FINE: forward left the state at the start of every tile; else the slab's states are rebuilt from the coarse ones
 // (or, one slab only, from state_in) by one more summary and fold.
 template <typename F, int NT, bool ASYNC, bool FINE>
@@ -408,26 +551,32 @@ __global__ void __launch_bounds__(NT * CP, NT == 8 ? 7 : NT == 16 ? 3 : 1) k_v4_
     const f2 w = make_float2(P.w.at(L.ch) * V4_LOG2E, P.w.at(L.ch1) * V4_LOG2E), u = mul2(L.ld((const F *)P.u, 0), both(V4_LOG2E));
     const F *const src[3] = {(const F *)P.k + L.row, (const F *)P.v + L.row, (const F *)P.gy + L.row};
     const int n8 = (T + TK - 1) / TK, n64 = (T + COARSE - 1) / COARSE, last = P.nslab - 1;
-    if (i == 0) {
-        St g = L.ext_state(P.gstate_out);
-        if (g.p.x == 0.f && g.q.x == 0.f) g.o.x = V4_MIN_VALUE;
-        if (g.p.y == 0.f && g.q.y == 0.f) g.o.y = V4_MIN_VALUE;
-        sm.carry[last & 1][c] = g;
-    }
+    if (i == 0) sm.carry[last & 1][c] = L.ext_gradient(P.gstate_out);
+    const float *const fine = FINE ? P.fine + (size_t)L.b * n8 * 3 * C : nullptr;
+    // slab s on its way to shared memory
+    auto fetch = [&](int s) {
+        fetch_slab<F, NT, 3>(sm, cp, s & 1, src, T, C, s * NT * TK);
+        if (FINE) fetch_states<F, NT>(sm, s & 1, fine, s * NT, n8, C, L.c0, threadIdx.x);
+        cp_commit();
+    };
     // the state at the start of this thread's tile (FINE) or of the 64 tokens around it, for slab s
     auto start_state = [&](int s) {
         const int t = s * NT * TK + i * TK;
-        if (FINE) return L.kept(P.fine + ((size_t)L.b * n8 + min(t / TK, n8 - 1)) * 3 * C);
+        if (FINE && ASYNC) {
+            auto at = [&](int r) { return *reinterpret_cast<const f2 *>(reinterpret_cast<const float *>(&sm.slab[s & 1][r][i * S::TILE + TK * CT]) + 2 * c); };
+            return St{at(0), at(1), at(2)};
+        }
+        if (FINE) return L.kept(fine + (size_t)min(t / TK, n8 - 1) * 3 * C);
         if (P.coarse) return L.kept(P.coarse + ((size_t)L.b * n64 + min(t / COARSE, n64 - 1)) * 3 * C);
         return L.ext_state(P.state_in);
     };
-    St x0 = start_state(last);
-    if (ASYNC) { fetch_slab<F, NT, 3>(sm, cp, last & 1, src, T, C, last * NT * TK); cp_commit(); }
+    if (ASYNC) fetch(last);
     f2 gw = both(0.f), gu = both(0.f);
     const f2 W = ex2_2(w), U = ex2_2(u);
     const float range = RANGE - fmaxf(fabsf(u.x), fabsf(u.y));
-    // x: the state at the start of this thread's tile; FULL as in forward
-    auto slab = [&](auto full_tag, int s, St x) {
+    bool bad = false;
+    // FULL, the result and `bad` as in forward
+    auto slab = [&](auto full_tag, int s) {
         constexpr bool FULL = decltype(full_tag)::value;
         const int t0 = s * NT * TK, mine0 = t0 + i * TK;
         auto len = [&](int j) { return min(TK, max(0, T - t0 - j * TK)); };
@@ -436,46 +585,25 @@ __global__ void __launch_bounds__(NT * CP, NT == 8 ? 7 : NT == 16 ? 3 : 1) k_v4_
             if (ASYNC) return Pair<F>::ld(&sm.slab[s & 1][tens][i * S::TILE + j * CT + 2 * c]);
             return L.ld(src[tens], (size_t)min(mine0 + j, T - 1) * C);
         };
-        if constexpr (!FINE) {
-            // the state at the tile's start: fold the summaries of the tiles between the kept state and it.
-            // Without `coarse` there is one slab and the kept state is the initial one.
-            St a = empty_state();
-            auto one = [&](auto half) {
-                constexpr int H = decltype(half)::value;
-                float p = 0.f, q = 0.f, o = V4_MIN_VALUE;
-#pragma unroll
-                for (int j = 0; j < TK; j++)
-                    if (j < n) {
-                        float A, E, m;
-                        exp2_pair(part<H>(w) + o, part<H>(ld(0, j)) * V4_LOG2E, A, E, m);
-                        p = fmaf(A, p, E * part<H>(ld(1, j))); q = fmaf(A, q, E); o = m;
-                    }
-                part<H>(a.p) = p; part<H>(a.q) = q; part<H>(a.o) = o;
-            };
-            one(FirstChannel{});
-            one(SecondChannel{});
-            sm.sum[i][c] = a;
-            __syncthreads();
-            for (int j = P.coarse ? (i & ~7) : 0; j < i; j++) x = fold(x, mul2(w, both((float)len(j))), sm.sum[j][c]);
-            __syncthreads();
-        }
-        // e: k;  then, tame, 2^{k-M}, M = max k;  else the exponent of the token's own term in its denominator
-        f2 ys[TK], zs[TK], e[TK];
-        e[0] = mul2(ld(0, 0), both(V4_LOG2E));
-        f2 kmin = e[0], M = e[0];
+        St x = start_state(s);
+        if (!FINE) x = rebuild_state<F, ASYNC>(P, sm, L, mine0, x, w, len);
+        // y and gy / denominator stay in registers until the gradient at the tile's end is known; k and e = 2^{k-M},
+        // M = max k, are read and formed again (registers are what limits this kernel)
+        f2 ys[TK], zs[TK];
+        auto key = [&](int j) { return mul2(ld(0, j), both(V4_LOG2E)); };
+        f2 kmin = key(0), M = kmin;
 #pragma unroll
         for (int j = 1; j < TK; j++)
             if (FULL || j < n) {
-                e[j] = mul2(ld(0, j), both(V4_LOG2E));
-                kmin = min2(kmin, e[j]);
-                M = max2(M, e[j]);
+                const f2 k = key(j);
+                kmin = min2(kmin, k);
+                M = max2(M, k);
             }
         const f2 wide = sub2(M, kmin), above = sub2(x.o, M);
-        const bool tame = fmaxf(wide.x, wide.y) <= range && fmaxf(above.x, above.y) <= RANGE;
-        f2 dpdw = both(0.f), dqdw = both(0.f);      // d(p,q)/dw since the tile's start ...
-        f2 dscale;                                  // ... and the exponent that scales them at the tile's end
+        if (n > 0 && !(fmaxf(wide.x, wide.y) <= range && fmaxf(above.x, above.y) <= RANGE)) bad = true;
+        f2 dpdw = both(0.f), dqdw = both(0.f);      // d(p,q)/dw since the tile's start, scaled by 2^{-M}
         St a = empty_state();
-        if (tame) {
+        {
             // the exponent of the gradient that leaves the tile at its start: the maximum over the tokens of j w minus
             // the exponent of the token's denominator, as the token-by-token recurrence keeps it.  Only gstate_in
             // shows which representation was used.
@@ -484,9 +612,10 @@ __global__ void __launch_bounds__(NT * CP, NT == 8 ? 7 : NT == 16 ? 3 : 1) k_v4_
 #pragma unroll
                 for (int j = 0; j < TK; j++)
                     if (FULL || j < n) {
-                        a.o = max2(a.o, sub2(back, max2(o, add2(u, e[j]))));
+                        const f2 k = key(j);
+                        a.o = max2(a.o, sub2(back, max2(o, add2(u, k))));
                         back = add2(back, w);
-                        o = max2(add2(o, w), e[j]);
+                        o = max2(add2(o, w), k);
                     }
             }
             const f2 sc = ex2_2(above), ref = neg2(M);
@@ -494,18 +623,16 @@ __global__ void __launch_bounds__(NT * CP, NT == 8 ? 7 : NT == 16 ? 3 : 1) k_v4_
 #pragma unroll
             for (int j = 0; j < TK; j++)
                 if (FULL || j < n) {
-                    const f2 v = ld(1, j);
-                    e[j] = ex2_2(add2(e[j], ref));
-                    const f2 eu = mul2(U, e[j]), iden = rcp2(add2(q, eu));
+                    const f2 v = ld(1, j), e = ex2_2(add2(key(j), ref)), eu = mul2(U, e), iden = rcp2(add2(q, eu));
                     ys[j] = mul2(fma2(eu, v, p), iden);
                     zs[j] = mul2(ld(2, j), iden);
                     gw = fma2(zs[j], fma2(neg2(dqdw), ys[j], dpdw), gw);
                     gu = fma2(mul2(zs[j], eu), sub2(v, ys[j]), gu);
                     const f2 wp = mul2(W, p), wq = mul2(W, q);
                     dpdw = fma2(W, dpdw, wp); dqdw = fma2(W, dqdw, wq);
-                    p = fma2(e[j], v, wp); q = add2(wq, e[j]);
+                    p = fma2(e, v, wp); q = add2(wq, e);
+                    if (j & 1) no_hoist();
                 }
-            dscale = M;
             // the reverse recurrence from an empty gradient: exponent -M throughout
 #pragma unroll
             for (int j = TK - 1; j >= 0; j--)
@@ -519,100 +646,46 @@ __global__ void __launch_bounds__(NT * CP, NT == 8 ? 7 : NT == 16 ? 3 : 1) k_v4_
             } else {
                 a.o = ref;
             }
-        } else {
-            auto one = [&](auto half) {
-                constexpr int H = decltype(half)::value;
-                float p = part<H>(x.p), q = part<H>(x.q), o = part<H>(x.o), dp = 0.f, dq = 0.f;
-#pragma unroll
-                for (int j = 0; j < TK; j++)
-                    if (FULL || j < n) {
-                        float A, E, m;
-                        const float k = part<H>(e[j]), v = part<H>(ld(1, j)), g = part<H>(ld(2, j));
-                        exp2_pair(o, part<H>(u) + k, A, E, m);
-                        const float iden = __fdividef(1.f, fmaf(A, q, E)), y = fmaf(A, p, E * v) * iden, z = g * iden;
-                        part<H>(ys[j]) = y;
-                        part<H>(zs[j]) = z;
-                        part<H>(e[j]) = k + part<H>(u) - m;
-                        part<H>(gw) = fmaf(z * A, fmaf(-dq, y, dp), part<H>(gw));
-                        part<H>(gu) = fmaf(z * E, v - y, part<H>(gu));
-                        exp2_pair(part<H>(w) + o, k, A, E, m);
-                        dp = A * (p + dp); dq = A * (q + dq);
-                        p = fmaf(A, p, E * v); q = fmaf(A, q, E); o = m;
-                    }
-                part<H>(dpdw) = dp; part<H>(dqdw) = dq; part<H>(dscale) = o;
-                float gp = 0.f, gq = 0.f, go = V4_MIN_VALUE;
-#pragma unroll
-                for (int j = TK - 1; j >= 0; j--)
-                    if (FULL || j < n) {
-                        float A, E, m;
-                        exp2_pair(part<H>(w) + go, part<H>(e[j]) - part<H>(ld(0, j)) * V4_LOG2E - part<H>(u), A, E, m);
-                        E *= part<H>(zs[j]);
-                        gp = fmaf(A, gp, E); gq = fmaf(A, gq, -E * part<H>(ys[j])); go = m;
-                    }
-                part<H>(a.p) = gp; part<H>(a.q) = gq; part<H>(a.o) = go;
-            };
-            one(FirstChannel{});
-            one(SecondChannel{});
         }
         if (!FULL && n == 0) a = empty_state();
-        St g = fold_tiles<NT, true, FULL>(sm, a, sm.carry[s & 1][c], i, c, w, len, &sm.carry[(s + 1) & 1][c]);
+        bool stop = false;
+        const St g = fold_tiles<NT, true, FULL>(sm, a, sm.carry[s & 1][c], i, c, w, len, &sm.carry[(s + 1) & 1][c], bad, stop);
+        if (stop) return false;
         // what the gradient at the tile's end sees of the decay inside the tile
-        if (FULL || n > 0) gw = fma2(fma2(g.p, dpdw, mul2(g.q, dqdw)), ex2_2(add2(dscale, g.o)), gw);
+        if (FULL || n > 0) gw = fma2(fma2(g.p, dpdw, mul2(g.q, dqdw)), ex2_2(add2(M, g.o)), gw);
         const size_t out0 = L.row + (size_t)(mine0 + TK - 1) * C + L.ch;
         F *gk = (F *)P.gk + out0, *gv = (F *)P.gv + out0;
         const f2 gs = add2(g.o, M);
-        if (tame && fmaxf(gs.x, gs.y) <= GRAD_RANGE) {
-            const f2 sc = ex2_2(gs);
+        if (n > 0 && !(fmaxf(gs.x, gs.y) <= GRAD_RANGE)) bad = true;
+        {
+            const f2 sc = ex2_2(gs), ref = neg2(M);
             f2 gp = mul2(g.p, sc), gq = mul2(g.q, sc);
 #pragma unroll
             for (int j = TK - 1; j >= 0; j--) {
                 if (FULL || j < n) {
-                    const f2 v = ld(1, j), t = mul2(zs[j], mul2(U, e[j]));
-                    L.st(gk, fma2(t, sub2(v, ys[j]), mul2(e[j], fma2(gp, v, gq))));
-                    L.st(gv, fma2(e[j], gp, t));
+                    const f2 v = ld(1, j), e = ex2_2(add2(key(j), ref)), t = mul2(zs[j], mul2(U, e));
+                    L.st(gk, fma2(t, sub2(v, ys[j]), mul2(e, fma2(gp, v, gq))));
+                    L.st(gv, fma2(e, gp, t));
                     gp = fma2(W, gp, zs[j]);
                     gq = fma2(W, gq, neg2(mul2(zs[j], ys[j])));
+                    if (!(j & 1)) no_hoist();
                 }
                 gk -= C; gv -= C;
             }
-        } else {
-            auto one = [&](auto half) {
-                constexpr int H = decltype(half)::value;
-                float gp = part<H>(g.p), gq = part<H>(g.q), go = part<H>(g.o);
-                F *ok = gk + H, *ov = gv + H;
-#pragma unroll
-                for (int j = TK - 1; j >= 0; j--) {
-                    if (FULL || j < n) {
-                        const float k = part<H>(ld(0, j)) * V4_LOG2E, v = part<H>(ld(1, j)), y = part<H>(ys[j]), z = part<H>(zs[j]);
-                        // (tame: z is scaled by 2^{-M}; its own term is z U e)
-                        const float t = tame ? z * (part<H>(U) * part<H>(e[j])) : z * ex2(part<H>(e[j]));
-                        float A, E = ex2(k + go), m;
-                        if (H ? L.live1 : L.live) {
-                            Elem<F>::st(ok, fmaf(t, v - y, E * fmaf(gp, v, gq)));
-                            Elem<F>::st(ov, fmaf(E, gp, t));
-                        }
-                        exp2_pair(part<H>(w) + go, tame ? -part<H>(M) : part<H>(e[j]) - k - part<H>(u), A, E, m);
-                        E *= z;
-                        gp = fmaf(A, gp, E); gq = fmaf(A, gq, -E * y); go = m;
-                    }
-                    ok -= C; ov -= C;
-                }
-            };
-            one(FirstChannel{});
-            one(SecondChannel{});
         }
+        return true;
     };
     for (int s = last; s >= 0; s--) {
         if (ASYNC) cp_wait0();
         __syncthreads();
-        St next = x0;
-        if (s > 0) {
-            if (ASYNC) { fetch_slab<F, NT, 3>(sm, cp, (s - 1) & 1, src, T, C, (s - 1) * NT * TK); cp_commit(); }
-            next = start_state(s - 1);
-        }
-        if ((s + 1) * NT * TK <= T) slab(std::true_type{}, s, x0);
-        else slab(std::false_type{}, s, x0);
-        x0 = next;
+        if (ASYNC && s > 0) fetch(s - 1);
+        if (!((s + 1) * NT * TK <= T ? slab(std::true_type{}, s) : slab(std::false_type{}, s))) break;
+    }
+    if (__syncthreads_or(bad)) {
+        if (ASYNC) cp_wait0();
+        f2 a, e;
+        slow_walk_back<F, NT, ASYNC, FINE>(P, sm, a, e);
+        gw = a; gu = e;
     }
     // the tiles' shares of gw and gu, summed in a fixed order
     __syncthreads();
