@@ -20,7 +20,7 @@ SOURCES = ["wkv_api.cu", "wkv4.cu", "wkv4_par.cu", "wkv56_scalar.cu", "wkv56_chu
            "timemix_fused.cu"]
 NATIVE_NAME = "_wkv_native"
 NATIVE = os.path.join(PKG, NATIVE_NAME + ".so")
-NATIVE_SOURCES = ["native_ops.cpp", "native_timemix.cpp"]
+NATIVE_SOURCES = ["native_ops.cpp", "native_timemix.cpp", "native_blocks.cpp"]
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
               "--use_fast_math", "-Xcompiler", "-fPIC"]
 

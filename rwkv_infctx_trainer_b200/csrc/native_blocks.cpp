@@ -1,0 +1,400 @@
+// The time-mix blocks as one autograd node each: the projections are library GEMMs, everything between them is a
+// kernel of libwkv_b200.so, and the whole block is one call from Python.  (As Python modules over separate
+// autograd functions a block cost 1.5 ms of host time per forward and backward, six times what the GPU needed for a
+// small one; and its stacked mixes and states went through cat, slice and add kernels of their own.)
+//
+// Numerics are those of the separate functions: bf16 tensors, fp32 inside every kernel.
+#include "native_ops.h"
+
+namespace wkv_native {
+namespace {
+
+constexpr auto BF16 = at::kBFloat16;
+
+// a parameter as the GEMMs take it
+Tensor as_bf16(const Tensor &p) { return as_contig(p, BF16); }
+// x @ W^T into `out`
+void linear_into(Tensor out, const Tensor &x, const Tensor &W) { at::mm_out(out, x, W.t()); }
+
+// the parameters of a group of mixes: pointers for the kernels, in one element type
+struct Mixes {
+    std::vector<Tensor> t;
+    at::ScalarType type;
+    bool one_minus;
+    Mixes(std::initializer_list<Tensor> ps, bool one_minus_) : one_minus(one_minus_) {
+        type = param_type(*ps.begin());
+        for (const Tensor &p : ps)
+            if (param_type(p) != type) type = at::kFloat;
+        for (const Tensor &p : ps) t.push_back(as_contig(p, type));
+    }
+    int n() const { return (int)t.size(); }
+    std::array<const void *, 5> ptrs() const {
+        std::array<const void *, 5> p{};
+        for (int i = 0; i < n(); i++) p[i] = ptr(t[i]);
+        return p;
+    }
+};
+
+Tensor mix_forward(const Tensor &x, const Tensor &shift, const Mixes &mx, const Tensor &m) {
+    const int B = (int)x.size(0), T = (int)x.size(1), C = (int)x.size(2);
+    Tensor out = at::empty({mx.n(), B * (int64_t)T, C}, x.options());
+    const auto p = mx.ptrs();
+    check(wkvx_ddlerp_forward(B, T, C, mx.n(), ptr(x), ptr(shift), p.data(), dtype_code(mx.type), mx.one_minus, ptr(m), ptr(out), stream_of(x)),
+          "wkv_ddlerp_forward");
+    return out;
+}
+
+struct MixGrads {
+    Tensor gx, gm, gshift;
+    std::vector<Tensor> gmaa;       // in the kernel's parameter type
+};
+// gshift_in: gradient of the row's last token (the block's new shift state); *_add: gradients to accumulate
+MixGrads mix_backward(const Tensor &x, const Tensor &shift, const Mixes &mx, const Tensor &m, const Tensor &gout,
+                      const Tensor &gshift_in, const Tensor &gx_add, const Tensor &gshift_add) {
+    const int B = (int)x.size(0), T = (int)x.size(1), C = (int)x.size(2);
+    MixGrads g;
+    g.gx = at::empty_like(x);
+    if (m.defined()) g.gm = at::empty_like(m);
+    g.gshift = at::empty_like(shift);
+    std::array<void *, 5> gp{};
+    for (int i = 0; i < mx.n(); i++) {
+        g.gmaa.push_back(at::empty_like(mx.t[i]));
+        gp[i] = ptr(g.gmaa[i]);
+    }
+    const size_t n = wkv_ddlerp_backward_workspace(B, T, C, mx.n());
+    Tensor ws = bytes_like(x, n);
+    const auto p = mx.ptrs();
+    check(wkvx_ddlerp_backward(B, T, C, mx.n(), ptr(x), ptr(shift), p.data(), dtype_code(mx.type), mx.one_minus, ptr(m), ptr(gout),
+                               ptr(gshift_in), ptr(gx_add), ptr(gshift_add), ptr(g.gx), ptr(g.gm), ptr(g.gshift), gp.data(), ptr(ws), n,
+                               stream_of(x)),
+          "wkv_ddlerp_backward");
+    return g;
+}
+
+// GroupNorm(y) * silu(g)
+Tensor norm_gate_forward(const Tensor &y, const Tensor &g, const Tensor &lw, const Tensor &lb, double eps, int64_t H) {
+    Tensor out = at::empty_like(y);
+    check(wkvx_lnx_gate_forward((int)y.size(0), (int)H, ptr(y), ptr(g), ptr(lw), ptr(lb), dtype_code(lw.scalar_type()), (float)eps, 1, ptr(out),
+                                stream_of(y)),
+          "wkv_lnx_gate_forward");
+    return out;
+}
+struct NormGrads {
+    Tensor gy, gg, glw, glb;
+};
+NormGrads norm_gate_backward(const Tensor &y, const Tensor &g, const Tensor &lw, const Tensor &lb, double eps, int64_t H, const Tensor &gout) {
+    NormGrads r{at::empty_like(y), at::empty_like(g), at::empty_like(lw), at::empty_like(lb)};
+    const int tokens = (int)y.size(0);
+    const size_t n = wkv_lnx_gate_backward_workspace(tokens, (int)H);
+    Tensor ws = bytes_like(y, n);
+    check(wkvx_lnx_gate_backward(tokens, (int)H, ptr(y), ptr(g), ptr(lw), ptr(lb), dtype_code(lw.scalar_type()), (float)eps, 1, ptr(gout),
+                                 ptr(r.gy), ptr(r.gg), ptr(r.glw), ptr(r.glb), ptr(ws), n, stream_of(y)),
+          "wkv_lnx_gate_backward");
+    return r;
+}
+
+// what every block's Function is given and keeps besides its tensors
+struct Meta {
+    int64_t H = 0;
+    double eps = 0;
+    bool sync = false;
+};
+
+Tensor last_token(const Tensor &x) { return x.select(1, x.size(1) - 1).contiguous(); }
+
+// gradients in the parameters' own types and shapes
+void finish(variable_list &grads, size_t first, const variable_list &params) {
+    for (size_t i = 0; i < params.size(); i++) {
+        Tensor &g = grads[first + i];
+        if (!g.defined()) continue;
+        if (g.scalar_type() != params[i].scalar_type()) g = g.to(params[i].scalar_type());
+        if (g.sizes() != params[i].sizes()) g = g.view(params[i].sizes());
+    }
+}
+
+// A forward pass of a block: with `keep` it also appends what the backward pass reads.
+struct Out {
+    Tensor out, shift, state;
+};
+
+// ------------------------------------------------------------------------------ v6
+// params: time_maa_x, _w, _k, _v, _r, _g, time_maa_w1, w2, time_decay, time_decay_w1, w2, time_faaaa, receptance, key, value,
+// output, gate, ln_x.weight, ln_x.bias
+enum { P6_X, P6_MW, P6_MK, P6_MV, P6_MR, P6_MG, P6_W1, P6_W2, P6_DECAY, P6_D1, P6_D2, P6_U, P6_R, P6_K, P6_V, P6_O, P6_G, P6_LW, P6_LB, P6_N };
+
+Mixes first6(const variable_list &p) { return Mixes({p[P6_X]}, false); }
+Mixes five6(const variable_list &p) { return Mixes({p[P6_MW], p[P6_MK], p[P6_MV], p[P6_MR], p[P6_MG]}, false); }
+
+Out forward6(const Tensor &x, const Tensor &shift, const Tensor &state, const variable_list &p, const Meta &me, variable_list *keep) {
+    const int64_t B = x.size(0), T = x.size(1), C = x.size(2), M = B * T, H = me.H;
+    // the five mixes: a first lerp feeds the low-rank map that makes them data-dependent
+    const Tensor xxx = mix_forward(x, shift, first6(p), Tensor()).view({M, C});
+    const Tensor w1 = as_bf16(p[P6_W1]), w2 = as_bf16(p[P6_W2]);
+    const int64_t R = w2.size(1);
+    Tensor t1 = at::mm(xxx, w1).tanh_();
+    const Tensor m = at::bmm(t1.view({M, 5, R}).transpose(0, 1), w2);
+    const Tensor xs = mix_forward(x, shift, five6(p), m);
+    Tensor rkvg = at::empty({4, M, C}, x.options());
+    linear_into(rkvg[0], xs[3], as_bf16(p[P6_R]));
+    linear_into(rkvg[1], xs[1], as_bf16(p[P6_K]));
+    linear_into(rkvg[2], xs[2], as_bf16(p[P6_V]));
+    linear_into(rkvg[3], xs[4], as_bf16(p[P6_G]));
+    Tensor dd = at::mm(xs[0], as_bf16(p[P6_D1])).tanh_();
+    const Tensor w = at::addmm(as_bf16(p[P6_DECAY]).view({C}), dd, as_bf16(p[P6_D2]));
+    const auto btc = [&](const Tensor &t) { return t.view({B, T, C}); };
+    const Tensor u = as_bf16(p[P6_U]);
+    Fwd o = wkv56_forward(true, btc(rkvg[0]), btc(rkvg[1]), btc(rkvg[2]), btc(w), u, state, WKV_W_RAW, WKV_STATE_KV, WKV_PATH_AUTO, Tensor(),
+                          keep != nullptr, 0, Tensor(), WKV_GROUP_STATES_NONE, me.sync);
+    const auto lt = param_type(p[P6_LW]);
+    const Tensor y = o.y.view({M, C}), n = norm_gate_forward(y, rkvg[3], as_contig(p[P6_LW], lt), as_contig(p[P6_LB], lt), me.eps, H);
+    const Tensor out = at::mm(n, as_bf16(p[P6_O]).t());
+    if (keep) *keep = {xxx, t1, m, xs, rkvg, dd, w, u, y, n, o.ckpt};
+    return {out.view({B, T, C}), last_token(x), o.state_out};
+}
+
+variable_list backward6(const Tensor &x, const Tensor &shift, const Tensor &state, const variable_list &p, const Meta &me,
+                        const variable_list &kept, const Tensor &gout_, const Tensor &gshift_new, const Tensor &gstate, bool want_gs) {
+    const int64_t B = x.size(0), T = x.size(1), C = x.size(2), M = B * T, H = me.H;
+    const Tensor &xxx = kept[0], &t1 = kept[1], &m = kept[2], &xs = kept[3], &rkvg = kept[4], &dd = kept[5], &w = kept[6], &u = kept[7],
+                 &y = kept[8], &n = kept[9], &ckpt = kept[10];
+    const auto btc = [&](const Tensor &t) { return t.view({B, T, C}); };
+    variable_list g(3 + P6_N);
+    variable_list gp(P6_N);
+    const Tensor gout = gout_.view({M, C});
+    gp[P6_O] = at::mm(gout.t(), n);
+    const Tensor gn = at::mm(gout, as_bf16(p[P6_O]));
+    const auto lt = param_type(p[P6_LW]);
+    NormGrads ng = norm_gate_backward(y, rkvg[3], as_contig(p[P6_LW], lt), as_contig(p[P6_LB], lt), me.eps, H, gn);
+    gp[P6_LW] = ng.glw;
+    gp[P6_LB] = ng.glb;
+    Bwd o = wkv56_backward(true, btc(rkvg[0]), btc(rkvg[1]), btc(rkvg[2]), btc(w), u, state, btc(ng.gy), gstate, WKV_W_RAW, WKV_STATE_KV,
+                           WKV_PATH_AUTO, want_gs, ckpt, 0, false, param_type(p[P6_U]), at::kFloat, me.sync);
+    gp[P6_U] = o.gu;
+    const Tensor gr = o.gr.view({M, C}), gk = o.gk.view({M, C}), gv = o.gv.view({M, C}), gw = o.gw.view({M, C});
+    gp[P6_R] = at::mm(gr.t(), xs[3]);
+    gp[P6_K] = at::mm(gk.t(), xs[1]);
+    gp[P6_V] = at::mm(gv.t(), xs[2]);
+    gp[P6_G] = at::mm(ng.gg.t(), xs[4]);
+    Tensor gxs = at::empty_like(xs);
+    const auto into = [&](int i, const Tensor &a, const Tensor &b) { Tensor d = gxs[i]; at::mm_out(d, a, b); };
+    into(3, gr, as_bf16(p[P6_R]));
+    into(1, gk, as_bf16(p[P6_K]));
+    into(2, gv, as_bf16(p[P6_V]));
+    into(4, ng.gg, as_bf16(p[P6_G]));
+    // the decay's low-rank map
+    const Tensor d1 = as_bf16(p[P6_D1]), d2 = as_bf16(p[P6_D2]);
+    gp[P6_DECAY] = gw.sum(0);
+    gp[P6_D2] = at::mm(dd.t(), gw);
+    const Tensor gdd = at::tanh_backward(at::mm(gw, d2.t()), dd);
+    gp[P6_D1] = at::mm(xs[0].t(), gdd);
+    into(0, gdd, d1.t());
+    MixGrads mg = mix_backward(x, shift, five6(p), m, gxs, gshift_new, Tensor(), Tensor());
+    for (int i = 0; i < 5; i++) gp[P6_MW + i] = mg.gmaa[i];
+    // the mixes' low-rank map
+    const Tensor w1 = as_bf16(p[P6_W1]), w2 = as_bf16(p[P6_W2]);
+    const int64_t R = w2.size(1);
+    const Tensor t5 = t1.view({M, 5, R});
+    gp[P6_W2] = at::bmm(t5.permute({1, 2, 0}), mg.gm);
+    Tensor gt1 = at::empty_like(t1), gt5 = gt1.view({M, 5, R});
+    at::tanh_backward_out(gt5, at::bmm(mg.gm, w2.transpose(1, 2)).transpose(0, 1), t5);
+    gp[P6_W1] = at::mm(xxx.t(), gt1);
+    MixGrads m1 = mix_backward(x, shift, first6(p), Tensor(), at::mm(gt1, w1.t()), Tensor(), mg.gx, mg.gshift);
+    gp[P6_X] = m1.gmaa[0];
+    g[0] = m1.gx;
+    g[1] = m1.gshift;
+    g[2] = o.gstate_in;
+    for (int i = 0; i < P6_N; i++) g[3 + i] = gp[i];
+    return g;
+}
+
+// ------------------------------------------------------------------------------ v5
+// params: time_mix_k, _v, _r, _g, time_decay, time_faaaa, receptance, key, value, output, gate, ln_x.weight, ln_x.bias
+enum { P5_MK, P5_MV, P5_MR, P5_MG, P5_DECAY, P5_U, P5_R, P5_K, P5_V, P5_O, P5_G, P5_LW, P5_LB, P5_N };
+
+// x*mix + x_prev*(1-mix)  =  x + (x_prev - x)*(1-mix)
+Mixes four5(const variable_list &p) { return Mixes({p[P5_MK], p[P5_MV], p[P5_MR], p[P5_MG]}, true); }
+
+Out forward5(const Tensor &x, const Tensor &shift, const Tensor &state, const variable_list &p, const Meta &me, variable_list *keep) {
+    const int64_t B = x.size(0), T = x.size(1), C = x.size(2), M = B * T, H = me.H;
+    const Tensor xs = mix_forward(x, shift, four5(p), Tensor());
+    Tensor rkvg = at::empty({4, M, C}, x.options());
+    linear_into(rkvg[0], xs[2], as_bf16(p[P5_R]));
+    linear_into(rkvg[1], xs[0], as_bf16(p[P5_K]));
+    linear_into(rkvg[2], xs[1], as_bf16(p[P5_V]));
+    linear_into(rkvg[3], xs[3], as_bf16(p[P5_G]));
+    const auto btc = [&](const Tensor &t) { return t.view({B, T, C}); };
+    const Tensor u = as_bf16(p[P5_U]), w = as_contig(p[P5_DECAY], at::kFloat);
+    Fwd o = wkv56_forward(false, btc(rkvg[0]), btc(rkvg[1]), btc(rkvg[2]), w, u, state, WKV_W_RAW, WKV_STATE_KV, WKV_PATH_AUTO, Tensor(),
+                          keep != nullptr, 0, Tensor(), WKV_GROUP_STATES_NONE, me.sync);
+    const auto lt = param_type(p[P5_LW]);
+    const Tensor y = o.y.view({M, C}), n = norm_gate_forward(y, rkvg[3], as_contig(p[P5_LW], lt), as_contig(p[P5_LB], lt), me.eps, H);
+    const Tensor out = at::mm(n, as_bf16(p[P5_O]).t());
+    if (keep) *keep = {xs, rkvg, w, u, y, n, o.ckpt};
+    return {out.view({B, T, C}), last_token(x), o.state_out};
+}
+
+variable_list backward5(const Tensor &x, const Tensor &shift, const Tensor &state, const variable_list &p, const Meta &me,
+                        const variable_list &kept, const Tensor &gout_, const Tensor &gshift_new, const Tensor &gstate, bool want_gs) {
+    const int64_t B = x.size(0), T = x.size(1), C = x.size(2), M = B * T, H = me.H;
+    const Tensor &xs = kept[0], &rkvg = kept[1], &w = kept[2], &u = kept[3], &y = kept[4], &n = kept[5], &ckpt = kept[6];
+    const auto btc = [&](const Tensor &t) { return t.view({B, T, C}); };
+    variable_list gp(P5_N);
+    const Tensor gout = gout_.view({M, C});
+    gp[P5_O] = at::mm(gout.t(), n);
+    const Tensor gn = at::mm(gout, as_bf16(p[P5_O]));
+    const auto lt = param_type(p[P5_LW]);
+    NormGrads ng = norm_gate_backward(y, rkvg[3], as_contig(p[P5_LW], lt), as_contig(p[P5_LB], lt), me.eps, H, gn);
+    gp[P5_LW] = ng.glw;
+    gp[P5_LB] = ng.glb;
+    Bwd o = wkv56_backward(false, btc(rkvg[0]), btc(rkvg[1]), btc(rkvg[2]), w, u, state, btc(ng.gy), gstate, WKV_W_RAW, WKV_STATE_KV,
+                           WKV_PATH_AUTO, want_gs, ckpt, 0, false, param_type(p[P5_U]), param_type(p[P5_DECAY]), me.sync);
+    gp[P5_U] = o.gu;
+    gp[P5_DECAY] = o.gw;
+    const Tensor gr = o.gr.view({M, C}), gk = o.gk.view({M, C}), gv = o.gv.view({M, C});
+    gp[P5_R] = at::mm(gr.t(), xs[2]);
+    gp[P5_K] = at::mm(gk.t(), xs[0]);
+    gp[P5_V] = at::mm(gv.t(), xs[1]);
+    gp[P5_G] = at::mm(ng.gg.t(), xs[3]);
+    Tensor gxs = at::empty_like(xs);
+    const auto into = [&](int i, const Tensor &a, const Tensor &b) { Tensor d = gxs[i]; at::mm_out(d, a, b); };
+    into(2, gr, as_bf16(p[P5_R]));
+    into(0, gk, as_bf16(p[P5_K]));
+    into(1, gv, as_bf16(p[P5_V]));
+    into(3, ng.gg, as_bf16(p[P5_G]));
+    MixGrads mg = mix_backward(x, shift, four5(p), Tensor(), gxs, gshift_new, Tensor(), Tensor());
+    for (int i = 0; i < 4; i++) gp[P5_MK + i] = mg.gmaa[i];
+    variable_list g = {mg.gx, mg.gshift, o.gstate_in};
+    g.insert(g.end(), gp.begin(), gp.end());
+    return g;
+}
+
+// ------------------------------------------------------------------------------ v4
+// params: time_mix_k, _v, _r, time_decay, time_first, key, value, receptance, output
+enum { P4_MK, P4_MV, P4_MR, P4_DECAY, P4_U, P4_K, P4_V, P4_R, P4_O, P4_N };
+
+Mixes three4(const variable_list &p) { return Mixes({p[P4_MK], p[P4_MV], p[P4_MR]}, true); }
+
+Out forward4(const Tensor &x, const Tensor &shift, const Tensor &state, const variable_list &p, const Meta &, variable_list *keep) {
+    const int64_t B = x.size(0), T = x.size(1), C = x.size(2), M = B * T;
+    const Tensor xs = mix_forward(x, shift, three4(p), Tensor());
+    const int64_t A = p[P4_K].size(0);       // dim_att
+    Tensor kv = at::empty({2, M, A}, x.options());
+    linear_into(kv[0], xs[0], as_bf16(p[P4_K]));
+    linear_into(kv[1], xs[1], as_bf16(p[P4_V]));
+    Tensor sr = at::mm(xs[2], as_bf16(p[P4_R]).t()).sigmoid_();
+    const Tensor w = as_contig(p[P4_DECAY], param_type(p[P4_DECAY])), u = as_bf16(p[P4_U]);
+    Fwd4 o = wkv4_forward(w, u, kv[0].view({B, T, A}), kv[1].view({B, T, A}), state, keep != nullptr);
+    const Tensor y = o.y.view({M, A}), sy = at::mul(sr, y), out = at::mm(sy, as_bf16(p[P4_O]).t());
+    if (keep) *keep = {xs, kv, sr, w, u, y, sy, o.ckpt};
+    return {out.view({B, T, C}), last_token(x), o.state_out};
+}
+
+variable_list backward4(const Tensor &x, const Tensor &shift, const Tensor &state, const variable_list &p, const Meta &,
+                        const variable_list &kept, const Tensor &gout_, const Tensor &gshift_new, const Tensor &gstate, bool want_gs) {
+    const int64_t B = x.size(0), T = x.size(1), C = x.size(2), M = B * T;
+    const Tensor &xs = kept[0], &kv = kept[1], &sr = kept[2], &w = kept[3], &u = kept[4], &y = kept[5], &sy = kept[6], &ckpt = kept[7];
+    const int64_t A = kv.size(2);
+    variable_list gp(P4_N);
+    const Tensor gout = gout_.view({M, C});
+    gp[P4_O] = at::mm(gout.t(), sy);
+    const Tensor gsy = at::mm(gout, as_bf16(p[P4_O]));
+    const Tensor gr = at::sigmoid_backward(at::mul(gsy, y), sr), gy = at::mul(gsy, sr);
+    Bwd4 o = wkv4_backward(w, u, kv[0].view({B, T, A}), kv[1].view({B, T, A}), state, ckpt, gy.view({B, T, A}), gstate, param_type(p[P4_U]), want_gs);
+    gp[P4_DECAY] = o.gw;
+    gp[P4_U] = o.gu;
+    const Tensor gk = o.gk.view({M, A}), gv = o.gv.view({M, A});
+    gp[P4_K] = at::mm(gk.t(), xs[0]);
+    gp[P4_V] = at::mm(gv.t(), xs[1]);
+    gp[P4_R] = at::mm(gr.t(), xs[2]);
+    Tensor gxs = at::empty_like(xs);
+    const auto into = [&](int i, const Tensor &a, const Tensor &b) { Tensor d = gxs[i]; at::mm_out(d, a, b); };
+    into(0, gk, as_bf16(p[P4_K]));
+    into(1, gv, as_bf16(p[P4_V]));
+    into(2, gr, as_bf16(p[P4_R]));
+    MixGrads mg = mix_backward(x, shift, three4(p), Tensor(), gxs, gshift_new, Tensor(), Tensor());
+    for (int i = 0; i < 3; i++) gp[P4_MK + i] = mg.gmaa[i];
+    variable_list g = {mg.gx, mg.gshift, o.gstate};
+    g.insert(g.end(), gp.begin(), gp.end());
+    return g;
+}
+
+// ------------------------------------------------------------------------------ the node
+typedef Out (*ForwardFn)(const Tensor &, const Tensor &, const Tensor &, const variable_list &, const Meta &, variable_list *);
+typedef variable_list (*BackwardFn)(const Tensor &, const Tensor &, const Tensor &, const variable_list &, const Meta &,
+                                    const variable_list &, const Tensor &, const Tensor &, const Tensor &, bool);
+struct Kind {
+    ForwardFn forward;
+    BackwardFn backward;
+    size_t params;
+};
+const Kind &kind_of(int64_t version) {
+    static const Kind k4{forward4, backward4, P4_N}, k5{forward5, backward5, P5_N}, k6{forward6, backward6, P6_N};
+    TORCH_CHECK_VALUE(version >= 4 && version <= 6, "unknown block version");
+    return version == 4 ? k4 : version == 5 ? k5 : k6;
+}
+
+struct BlockFunction : torch::autograd::Function<BlockFunction> {
+    static variable_list forward(AutogradContext *ctx, int64_t version, const Tensor &x, const Tensor &shift, const Tensor &state,
+                                 at::TensorList params, int64_t H, double eps, bool sync) {
+        at::AutoDispatchBelowADInplaceOrView below;
+        c10::cuda::OptionalCUDAGuard guard(x.device());
+        const variable_list p(params.begin(), params.end());
+        variable_list kept;
+        const Out o = kind_of(version).forward(x, shift, state, p, Meta{H, eps, sync}, &kept);
+        variable_list save = {x, shift, state};
+        save.insert(save.end(), p.begin(), p.end());
+        save.insert(save.end(), kept.begin(), kept.end());
+        ctx->save_for_backward(save);
+        ctx->saved_data["i"] = std::vector<int64_t>{version, H, (int64_t)sync};
+        ctx->saved_data["eps"] = eps;
+        ctx->set_materialize_grads(false);
+        return {o.out, o.shift, o.state};
+    }
+    static variable_list backward(AutogradContext *ctx, variable_list grads) {
+        at::AutoDispatchBelowADInplaceOrView below;
+        const variable_list st = ctx->get_saved_variables();
+        const auto i = ctx->saved_data["i"].toIntVector();
+        const Kind &k = kind_of(i[0]);
+        const Tensor &x = st[0], &shift = st[1], &state = st[2];
+        c10::cuda::OptionalCUDAGuard guard(x.device());
+        const variable_list p(st.begin() + 3, st.begin() + 3 + k.params), kept(st.begin() + 3 + k.params, st.end());
+        const Tensor gout = grads[0].defined() ? as_contig(grads[0], BF16) : at::zeros_like(x);
+        const Tensor gshift = grads[1].defined() ? as_contig(grads[1], BF16) : Tensor();
+        const Tensor gstate = grads[2].defined() ? as_contig(grads[2], at::kFloat) : Tensor();
+        variable_list g = k.backward(x, shift, state, p, Meta{i[1], ctx->saved_data["eps"].toDouble(), i[2] != 0}, kept, gout, gshift, gstate,
+                                     ctx->needs_input_grad(2));
+        finish(g, 3, p);
+        variable_list r = {Tensor()};
+        r.insert(r.end(), g.begin(), g.end());
+        r.insert(r.end(), 3, Tensor());
+        return r;
+    }
+};
+
+}  // namespace
+
+std::tuple<Tensor, Tensor, Tensor> block(int64_t version, const Tensor &x_, const Tensor &shift_, const Tensor &state_,
+                                         const std::vector<Tensor> &params, int64_t H, double eps, bool sync) {
+    const Kind &k = kind_of(version);
+    TORCH_CHECK_VALUE(params.size() == k.params, "wrong number of parameters");
+    TORCH_CHECK_VALUE(x_.dim() == 3 && x_.size(1) > 0, "x must be [B,T,C] with T > 0");
+    require_cuda({&x_, &shift_, &state_, &params[0]});
+    const int64_t B = x_.size(0), C = x_.size(2);
+    TORCH_CHECK_VALUE(shift_.dim() == 2 && shift_.size(0) == B && shift_.size(1) == C, "the shift state must be [B,C]");
+    const Tensor x = x_.to(BF16).contiguous(), shift = shift_.to(BF16).contiguous(), state = state_.to(at::kFloat).contiguous();
+    bool grad = wants_grad({&x, &shift, &state});
+    if (!grad && at::GradMode::is_enabled())
+        for (const Tensor &p : params) grad |= p.requires_grad();
+    if (grad) {
+        variable_list o = BlockFunction::apply(version, x, shift, state, at::TensorList(params), H, eps, sync);
+        return {o[0], o[1], o[2]};
+    }
+    at::AutoDispatchBelowADInplaceOrView below;
+    c10::cuda::OptionalCUDAGuard guard(x.device());
+    const Out o = k.forward(x, shift, state, params, Meta{H, eps, sync}, nullptr);
+    return {o.out, o.shift, o.state};
+}
+
+}  // namespace wkv_native
+
+void bind_blocks(py::module_ &m) { m.def("block", &wkv_native::block); }

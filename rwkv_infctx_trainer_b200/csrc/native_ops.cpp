@@ -2,7 +2,7 @@
 // All of it is host work on the way to the C ABI; it is native because a call of the op is a handful of
 // microsecond kernels when heads, tokens or batch are few, and the same steps in Python take hundreds of
 // microseconds (v6, 5 heads, 4096-token segments: 284 us per call in Python, of which the GPU was busy 56).
-#include "native_common.h"
+#include "native_ops.h"
 
 namespace wkv_native {
 
@@ -78,11 +78,6 @@ void check_call(bool v6, const Tensor &r, const Tensor &k, const Tensor &v, cons
 
 }  // namespace
 
-struct Fwd {
-    Tensor y, state_out, ckpt;
-};
-
-// saved_mode: WKV_GROUP_STATES_*; with it `saved` is the buffer (see wkv_args_t.group_states)
 Fwd wkv56_forward(bool v6, const Tensor &r, const Tensor &k, const Tensor &v, const Tensor &w, const Tensor &u,
                   const Tensor &state_in, int w_kind, int layout, int path, const Tensor &state_out, bool save_ckpt,
                   int time_groups, const Tensor &saved, int saved_mode, bool sync_check) {
@@ -118,12 +113,6 @@ Fwd wkv56_forward(bool v6, const Tensor &r, const Tensor &k, const Tensor &v, co
     return out;
 }
 
-struct Bwd {
-    Tensor gr, gk, gv, gw, gu, gstate_in;
-};
-
-// gw: v6 [B,T,C] in r's type.  gu [H,64] in u's type and v5's gw [H,64] in `w_type` are summed over the
-// batch; with per_batch they are the C ABI's fp32 [B,C] partials instead.
 Bwd wkv56_backward(bool v6, const Tensor &r, const Tensor &k, const Tensor &v, const Tensor &w, const Tensor &u,
                    const Tensor &state_in, const Tensor &gy, const Tensor &gstate_out, int w_kind, int layout, int path,
                    bool want_gstate, const Tensor &ckpt, int time_groups, bool per_batch, at::ScalarType u_type,
@@ -318,49 +307,65 @@ Tensor wkv56_dropin(bool v6, int64_t B, int64_t T, int64_t C, int64_t H, const T
 }
 
 // ------------------------------------------------------------------------------ v4
+Fwd4 wkv4_forward(const Tensor &w, const Tensor &u, const Tensor &k, const Tensor &v, const Tensor &state, bool save) {
+    const int B = (int)k.size(0), T = (int)k.size(1), C = (int)k.size(2);
+    c10::cuda::OptionalCUDAGuard guard(k.device());
+    Fwd4 o;
+    o.y = at::empty_like(k);
+    o.state_out = at::empty_like(state);
+    o.ckpt = bytes_like(k, save ? wkv4_state_ckpt_bytes(B, T, C) : 0);
+    check(wkv4x_forward(B, T, C, dtype_code(k.scalar_type()), ptr(w), dtype_code(w.scalar_type()), ptr(u), ptr(k), ptr(v),
+                        (const float *)ptr(state), ptr(o.y), (float *)ptr(o.state_out), ptr(o.ckpt), stream_of(k)),
+          "wkv4_forward");
+    return o;
+}
+
+Bwd4 wkv4_backward(const Tensor &w, const Tensor &u, const Tensor &k, const Tensor &v, const Tensor &state, const Tensor &ckpt,
+                   const Tensor &gy, const Tensor &gstate_out, at::ScalarType u_type, bool want_gstate) {
+    const int B = (int)k.size(0), T = (int)k.size(1), C = (int)k.size(2);
+    c10::cuda::OptionalCUDAGuard guard(k.device());
+    Bwd4 g;
+    g.gw = B ? at::empty_like(w) : at::zeros_like(w);
+    g.gu = B ? at::empty({C}, u.options().dtype(u_type)) : at::zeros({C}, u.options().dtype(u_type));
+    g.gk = at::empty_like(k);
+    g.gv = at::empty_like(v);
+    if (want_gstate) g.gstate = at::empty_like(state);
+    Tensor ws = bytes_like(k, wkv4x_backward_workspace(B, T, C, ckpt.defined()));
+    check(wkv4x_backward(B, T, C, dtype_code(k.scalar_type()), ptr(w), dtype_code(w.scalar_type()), ptr(u), ptr(k), ptr(v),
+                         (const float *)ptr(state), ptr(gy), (const float *)ptr(gstate_out), ptr(g.gw), ptr(g.gu), dtype_code(u_type),
+                         ptr(g.gk), ptr(g.gv), (float *)ptr(g.gstate), ptr(ws), ptr(ckpt), stream_of(k)),
+          "wkv4_backward");
+    return g;
+}
+
 namespace {
 
 // RWKV-v4neo/cuda/wkv_op_bf16.cpp:13-92
 struct Wkv4Function : torch::autograd::Function<Wkv4Function> {
     static variable_list forward(AutogradContext *ctx, const Tensor &raw_w, const Tensor &raw_u, const Tensor &raw_k,
                                  const Tensor &raw_v, const Tensor &raw_state, bool save) {
-        const int B = (int)raw_k.size(0), T = (int)raw_k.size(1), C = (int)raw_k.size(2);
         const auto dt = raw_k.scalar_type();
-        c10::cuda::OptionalCUDAGuard guard(raw_k.device());
-        const auto wt = raw_w.scalar_type() == at::kDouble ? at::kFloat : raw_w.scalar_type();
-        const Tensor w = as_contig(raw_w, wt), u = as_contig(raw_u, dt), k = contig(raw_k), v = as_contig(raw_v, dt),
+        const Tensor w = as_contig(raw_w, param_type(raw_w)), u = as_contig(raw_u, dt), k = contig(raw_k), v = as_contig(raw_v, dt),
                      state = as_contig(raw_state, at::kFloat);
-        Tensor y = at::empty_like(k), new_state = at::empty_like(state);
-        Tensor ck = bytes_like(k, save ? wkv4_state_ckpt_bytes(B, T, C) : 0);
-        check(wkv4x_forward(B, T, C, dtype_code(dt), ptr(w), dtype_code(wt), ptr(u), ptr(k), ptr(v), (const float *)ptr(state), ptr(y),
-                            (float *)ptr(new_state), ptr(ck), stream_of(k)),
-              "wkv4_forward");
+        Fwd4 o = wkv4_forward(w, u, k, v, state, save);
         if (save) {
-            ctx->save_for_backward({w, u, k, v, state, ck});
+            ctx->save_for_backward({w, u, k, v, state, o.ckpt});
             ctx->saved_data["types"] = std::vector<int64_t>{(int64_t)raw_w.scalar_type(), (int64_t)raw_u.scalar_type(),
-                                                            (int64_t)raw_v.scalar_type(), (int64_t)raw_state.scalar_type()};
+                                                            (int64_t)raw_v.scalar_type(), (int64_t)raw_state.scalar_type(),
+                                                            (int64_t)param_type(raw_u)};
             ctx->set_materialize_grads(false);
         }
-        return {y, new_state};
+        return {o.y, o.state_out};
     }
     static variable_list backward(AutogradContext *ctx, variable_list grads) {
         const variable_list st = ctx->get_saved_variables();
-        const Tensor &w = st[0], &u = st[1], &k = st[2], &v = st[3], &state = st[4], &ck = st[5];
-        const int B = (int)k.size(0), T = (int)k.size(1), C = (int)k.size(2);
+        const Tensor &k = st[2];
         const auto types = ctx->saved_data["types"].toIntVector();
-        c10::cuda::OptionalCUDAGuard guard(k.device());
+        const auto type = [&](int i) { return (at::ScalarType)types[i]; };
         const Tensor gy = grads[0].defined() ? as_contig(grads[0], k.scalar_type()) : at::zeros_like(k);
         const Tensor gs = grads[1].defined() ? as_contig(grads[1], at::kFloat) : Tensor();
-        const auto u_type = (at::ScalarType)types[1] == at::kDouble ? at::kFloat : (at::ScalarType)types[1];
-        Tensor gw = B ? at::empty_like(w) : at::zeros_like(w), gk = at::empty_like(k), gv = at::empty_like(k), glast = at::empty_like(state),
-               gu = B ? at::empty({C}, u.options().dtype(u_type)) : at::zeros({C}, u.options().dtype(u_type));
-        Tensor ws = bytes_like(k, wkv4x_backward_workspace(B, T, C, ck.defined()));
-        check(wkv4x_backward(B, T, C, dtype_code(k.scalar_type()), ptr(w), dtype_code(w.scalar_type()), ptr(u), ptr(k), ptr(v),
-                             (const float *)ptr(state), ptr(gy), (const float *)ptr(gs), ptr(gw), ptr(gu), dtype_code(u_type), ptr(gk),
-                             ptr(gv), (float *)ptr(glast), ptr(ws), ptr(ck), stream_of(k)),
-              "wkv4_backward");
-        return {gw.to((at::ScalarType)types[0]), gu.to((at::ScalarType)types[1]), gk, gv.to((at::ScalarType)types[2]),
-                glast.to((at::ScalarType)types[3]), Tensor()};
+        Bwd4 g = wkv4_backward(st[0], st[1], k, st[3], st[4], st[5], gy, gs, type(4), ctx->needs_input_grad(4));
+        return {g.gw.to(type(0)), g.gu.to(type(1)), g.gk, g.gv.to(type(2)), g.gstate.defined() ? g.gstate.to(type(3)) : Tensor(), Tensor()};
     }
 };
 
@@ -393,6 +398,7 @@ py::object none_or(const Tensor &t) { return t.defined() ? py::cast(t) : py::non
 }  // namespace
 
 void bind_timemix(py::module_ &m);
+void bind_blocks(py::module_ &m);
 
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     m.def("wkv56_apply", &wkv56_apply);
@@ -418,4 +424,5 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
               return py::make_tuple(g.gr, g.gk, g.gv, g.gw, g.gu, none_or(g.gstate_in));
           });
     bind_timemix(m);
+    bind_blocks(m);
 }

@@ -1,5 +1,5 @@
 // PyTorch binding of the op's elementwise neighbours (see timemix_fused.cu) as autograd nodes.
-#include "native_common.h"
+#include "native_ops.h"
 
 namespace wkv_native {
 namespace {
@@ -9,15 +9,22 @@ const Tensor &bf16(const Tensor &t, const char *name) {
     return t;
 }
 
+// the rows of a [n, C] parameter matrix
+std::array<void *, 5> rows_of(const Tensor &t) {
+    std::array<void *, 5> p{};
+    for (int64_t i = 0; i < t.size(0) && i < 5; i++) p[i] = (char *)t.data_ptr() + i * t.size(1) * t.element_size();
+    return p;
+}
+
 struct LnxGate : torch::autograd::Function<LnxGate> {
     static Tensor forward(AutogradContext *ctx, const Tensor &y_, const Tensor &g_, const Tensor &weight, const Tensor &bias,
                           double eps, int64_t H) {
         c10::cuda::OptionalCUDAGuard guard(y_.device());
-        const Tensor y = contig(y_), g = contig(g_), ga = as_contig(weight, at::kFloat), be = as_contig(bias, at::kFloat);
+        const auto pt = weight.scalar_type() == bias.scalar_type() ? param_type(weight) : at::kFloat;
+        const Tensor y = contig(y_), g = contig(g_), ga = as_contig(weight, pt), be = as_contig(bias, pt);
         Tensor out = at::empty_like(y);
         const int tokens = (int)(y.numel() / (H * HEAD));
-        check(wkv_lnx_gate_forward(tokens, (int)H, ptr(y), ptr(g), (const float *)ptr(ga), (const float *)ptr(be), (float)eps, ptr(out),
-                                   stream_of(y)),
+        check(wkvx_lnx_gate_forward(tokens, (int)H, ptr(y), ptr(g), ptr(ga), ptr(be), dtype_code(pt), (float)eps, 0, ptr(out), stream_of(y)),
               "wkv_lnx_gate_forward");
         ctx->save_for_backward({y, g, ga, be});
         ctx->saved_data["eps"] = eps;
@@ -36,9 +43,9 @@ struct LnxGate : torch::autograd::Function<LnxGate> {
         Tensor gy = at::empty_like(y), gg = at::empty_like(g), gga = at::empty({C}, ga.options()), gbe = at::empty({C}, be.options());
         const size_t n = wkv_lnx_gate_backward_workspace(tokens, H);
         Tensor ws = bytes_like(y, n);
-        check(wkv_lnx_gate_backward(tokens, H, ptr(y), ptr(g), (const float *)ptr(ga), (const float *)ptr(be),
-                                    (float)ctx->saved_data["eps"].toDouble(), ptr(gout), ptr(gy), ptr(gg), (float *)ptr(gga),
-                                    (float *)ptr(gbe), ptr(ws), n, stream_of(y)),
+        check(wkvx_lnx_gate_backward(tokens, H, ptr(y), ptr(g), ptr(ga), ptr(be), dtype_code(ga.scalar_type()),
+                                     (float)ctx->saved_data["eps"].toDouble(), 0, ptr(gout), ptr(gy), ptr(gg), ptr(gga), ptr(gbe), ptr(ws), n,
+                                     stream_of(y)),
               "wkv_lnx_gate_backward");
         const auto types = ctx->saved_data["types"].toIntVector();
         return {gy, gg, gga.view(ctx->saved_data["w_shape"].toIntVector()).to((at::ScalarType)types[0]),
@@ -49,10 +56,12 @@ struct LnxGate : torch::autograd::Function<LnxGate> {
 struct DDLerp : torch::autograd::Function<DDLerp> {
     static Tensor forward(AutogradContext *ctx, const Tensor &x_, const Tensor &shift_, const Tensor &maa, const OptTensor &m_) {
         c10::cuda::OptionalCUDAGuard guard(x_.device());
-        const Tensor x = contig(x_), sh = contig(shift_), m = m_.has_value() ? contig(*m_) : Tensor(), ma = as_contig(maa, at::kFloat);
+        const Tensor x = contig(x_), sh = contig(shift_), m = m_.has_value() ? contig(*m_) : Tensor(), ma = as_contig(maa, param_type(maa));
         const int B = (int)x.size(0), T = (int)x.size(1), C = (int)x.size(2), n = (int)ma.size(0);
         Tensor out = at::empty({n, B, T, C}, x.options());
-        check(wkv_ddlerp_forward(B, T, C, n, ptr(x), ptr(sh), (const float *)ptr(ma), ptr(m), ptr(out), stream_of(x)), "wkv_ddlerp_forward");
+        const auto p = rows_of(ma);
+        check(wkvx_ddlerp_forward(B, T, C, n, ptr(x), ptr(sh), p.data(), dtype_code(ma.scalar_type()), 0, ptr(m), ptr(out), stream_of(x)),
+              "wkv_ddlerp_forward");
         ctx->save_for_backward({x, sh, ma, m});
         ctx->saved_data["type"] = (int64_t)maa.scalar_type();
         return out;
@@ -67,8 +76,9 @@ struct DDLerp : torch::autograd::Function<DDLerp> {
                gma = at::empty({n, C}, ma.options());
         const size_t nb = wkv_ddlerp_backward_workspace(B, T, C, n);
         Tensor ws = bytes_like(x, nb);
-        check(wkv_ddlerp_backward(B, T, C, n, ptr(x), ptr(sh), (const float *)ptr(ma), ptr(m), ptr(gout), nullptr, ptr(gx), ptr(gm),
-                                  ptr(gsh), (float *)ptr(gma), ptr(ws), nb, stream_of(x)),
+        const auto p = rows_of(ma), gp = rows_of(gma);
+        check(wkvx_ddlerp_backward(B, T, C, n, ptr(x), ptr(sh), p.data(), dtype_code(ma.scalar_type()), 0, ptr(m), ptr(gout), nullptr, nullptr,
+                                   nullptr, ptr(gx), ptr(gm), ptr(gsh), gp.data(), ptr(ws), nb, stream_of(x)),
               "wkv_ddlerp_backward");
         return {gx, gsh, gma.to((at::ScalarType)ctx->saved_data["type"].toInt()), gm};
     }

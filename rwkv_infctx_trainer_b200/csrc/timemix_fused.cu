@@ -11,7 +11,12 @@
 // All are HBM-bound: a thread owns 8 consecutive channels (one 16-byte access per tensor), the 8
 // lanes that share a head exchange their sums by shuffles, accumulation is fp32, parameter
 // gradients are reduced in a fixed order (per-CTA partials, then one fold): no atomics.
+// Parameters come in their own element type and from their own tensors (a block's mixes are
+// separate parameters), and their gradients go back the same way.
+#include <initializer_list>
+
 #include "wkv_common.cuh"
+#include "wkv_internal.h"
 
 namespace wkv {
 namespace {
@@ -40,10 +45,27 @@ __device__ __forceinline__ float head_sum(float v) {
     v += __shfl_xor_sync(0xffffffffu, v, 4);
     return v;
 }
-__device__ __forceinline__ void load8f(const float *p, float *f) {
-    const float4 a = __ldg(reinterpret_cast<const float4 *>(p)), b = __ldg(reinterpret_cast<const float4 *>(p) + 1);
-    f[0] = a.x; f[1] = a.y; f[2] = a.z; f[3] = a.w; f[4] = b.x; f[5] = b.y; f[6] = b.z; f[7] = b.w;
+// 8 channels of a parameter of element type `dtype`
+__device__ __forceinline__ void load8(const void *p, int dtype, size_t at, float *f) {
+    if (dtype == WKV_BF16) {
+        unpack8(__ldg(reinterpret_cast<const uint4 *>((const __nv_bfloat16 *)p + at)), f);
+    } else if (dtype == WKV_F32) {
+        const float4 *q = reinterpret_cast<const float4 *>((const float *)p + at);
+        const float4 a = __ldg(q), b = __ldg(q + 1);
+        f[0] = a.x; f[1] = a.y; f[2] = a.z; f[3] = a.w; f[4] = b.x; f[5] = b.y; f[6] = b.z; f[7] = b.w;
+    } else {
+        const __half2 *q = reinterpret_cast<const __half2 *>((const __half *)p + at);
+#pragma unroll
+        for (int i = 0; i < 4; i++) { const float2 v = __half22float2(q[i]); f[2 * i] = v.x; f[2 * i + 1] = v.y; }
+    }
 }
+__device__ __forceinline__ void store_as(void *p, int dtype, size_t i, float x) {
+    if (dtype == WKV_F32) ((float *)p)[i] = x;
+    else if (dtype == WKV_BF16) ((__nv_bfloat16 *)p)[i] = __float2bfloat16_rn(x);
+    else ((__half *)p)[i] = __float2half_rn(x);
+}
+__device__ __forceinline__ float sigmoidf(float x) { return __fdividef(1.f, 1.f + __expf(-x)); }
+__device__ __forceinline__ float bf16_round(float x) { return __bfloat162float(__float2bfloat16_rn(x)); }
 
 // Work split shared by the kernels: the C channels are cut into column blocks of 256 (a warp's
 // 32 lanes x 8 channels = 4 heads); blockIdx.x = column block + ncb * token slot; the 8 warps of
@@ -53,9 +75,13 @@ struct Split {
     int ncb, nslot;
 };
 
+// SILU: the gate is silu(g), rounded to bf16 as the tensor it stands for would be
+template <bool SILU>
 __global__ void __launch_bounds__(TPB)
 k_lnx_gate_fwd(int tokens, int C, Split sp, const uint4 *__restrict__ y, const uint4 *__restrict__ g,
-               const float *__restrict__ gamma, const float *__restrict__ beta, float eps, uint4 *__restrict__ out) {
+               const void *__restrict__ gamma, const void *__restrict__ beta, int pdtype, float eps, uint4 *__restrict__ out) {
+    pdl_wait();
+    pdl_trigger();
     const int cb = blockIdx.x % sp.ncb, slot = blockIdx.x / sp.ncb, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int c0 = cb * 256 + lane * 8;
     // (lanes past the last channel stay in the loop with zeros: the shuffles below name all 32 lanes)
@@ -64,8 +90,8 @@ k_lnx_gate_fwd(int tokens, int C, Split sp, const uint4 *__restrict__ y, const u
 #pragma unroll
     for (int q = 0; q < 8; q++) { ga[q] = 0.f; be[q] = 0.f; }
     if (live) {
-        load8f(gamma + c0, ga);
-        load8f(beta + c0, be);
+        load8(gamma, pdtype, c0, ga);
+        load8(beta, pdtype, c0, be);
     }
     const int stride = sp.nslot * 8, row16 = C / 8;
     for (int t = slot * 8 + warp; t < tokens; t += stride) {
@@ -74,6 +100,10 @@ k_lnx_gate_fwd(int tokens, int C, Split sp, const uint4 *__restrict__ y, const u
         const uint4 zero4 = make_uint4(0u, 0u, 0u, 0u);
         unpack8(live ? y[i] : zero4, yv);
         unpack8(live ? g[i] : zero4, gv);
+        if (SILU) {
+#pragma unroll
+            for (int q = 0; q < 8; q++) gv[q] = bf16_round(gv[q] * sigmoidf(gv[q]));
+        }
         float s = 0.f;
 #pragma unroll
         for (int q = 0; q < 8; q++) s += yv[q];
@@ -90,11 +120,14 @@ k_lnx_gate_fwd(int tokens, int C, Split sp, const uint4 *__restrict__ y, const u
 }
 
 // gy, gg and per-CTA partial sums of the gradients of gamma and beta ([nslot, 2, C])
+template <bool SILU>
 __global__ void __launch_bounds__(TPB)
 k_lnx_gate_bwd(int tokens, int C, Split sp, const uint4 *__restrict__ y, const uint4 *__restrict__ g,
-               const float *__restrict__ gamma, const float *__restrict__ beta, float eps,
+               const void *__restrict__ gamma, const void *__restrict__ beta, int pdtype, float eps,
                const uint4 *__restrict__ gout, uint4 *__restrict__ gy, uint4 *__restrict__ gg,
                float *__restrict__ part) {
+    pdl_wait();
+    pdl_trigger();
     __shared__ float red[8][2][256];
     const int cb = blockIdx.x % sp.ncb, slot = blockIdx.x / sp.ncb, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int c0 = cb * 256 + lane * 8;
@@ -105,8 +138,8 @@ k_lnx_gate_bwd(int tokens, int C, Split sp, const uint4 *__restrict__ y, const u
     {
         // (every lane runs the loop, lanes past the last channel on zeros: the shuffles name all 32 lanes)
         if (live) {
-            load8f(gamma + c0, ga);
-            load8f(beta + c0, be);
+            load8(gamma, pdtype, c0, ga);
+            load8(beta, pdtype, c0, be);
         }
         const int stride = sp.nslot * 8, row16 = C / 8;
         for (int t = slot * 8 + warp; t < tokens; t += stride) {
@@ -116,6 +149,15 @@ k_lnx_gate_bwd(int tokens, int C, Split sp, const uint4 *__restrict__ y, const u
             unpack8(live ? y[i] : zero4, yv);
             unpack8(live ? g[i] : zero4, gv);
             unpack8(live ? gout[i] : zero4, go);
+            float dsilu[8];
+            if (SILU) {
+#pragma unroll
+                for (int q = 0; q < 8; q++) {
+                    const float sg = sigmoidf(gv[q]);
+                    dsilu[q] = sg * (1.f + gv[q] * (1.f - sg));
+                    gv[q] = bf16_round(gv[q] * sg);
+                }
+            }
             float s = 0.f;
 #pragma unroll
             for (int q = 0; q < 8; q++) s += yv[q];
@@ -130,6 +172,7 @@ k_lnx_gate_bwd(int tokens, int C, Split sp, const uint4 *__restrict__ y, const u
                 const float xh = yv[q] * rstd;               // normalised value
                 const float dln = go[q] * gv[q];             // gradient at the GroupNorm output
                 dg[q] = go[q] * (xh * ga[q] + be[q]);
+                if (SILU) dg[q] *= dsilu[q];
                 dga[q] += dln * xh;
                 dbe[q] += dln;
                 dy[q] = dln * ga[q];                         // gradient at the normalised value
@@ -160,22 +203,51 @@ k_lnx_gate_bwd(int tokens, int C, Split sp, const uint4 *__restrict__ y, const u
     }
 }
 
+// Column sums of the per-CTA partials [rows, n*C] into n parameter gradients of C elements: 32 columns by 8 row groups
+// per CTA, many loads in flight; `sign` -1 for parameters that enter as 1 - p.
+struct GradPtrs {
+    void *p[5];
+};
 __global__ void __launch_bounds__(TPB)
-k_fold_params(const float *__restrict__ part, int nslot, int C, float *__restrict__ ggamma, float *__restrict__ gbeta) {
-    const int c = blockIdx.x * TPB + threadIdx.x;
-    if (c >= C) return;
-    float a = 0.f, b = 0.f;
-    for (int s = 0; s < nslot; s++) { a += part[((size_t)s * 2) * C + c]; b += part[((size_t)s * 2 + 1) * C + c]; }
-    ggamma[c] = a;
-    gbeta[c] = b;
+k_fold_cols(const float *__restrict__ part, int rows, int n, int C, GradPtrs out, int dtype, float sign) {
+    pdl_wait();
+    pdl_trigger();
+    __shared__ float red[8][32];
+    const int lane = threadIdx.x & 31, g = threadIdx.x >> 5, col = blockIdx.x * 32 + lane, cols = n * C;
+    float a = 0.f;
+    if (col < cols) {
+#pragma unroll 8
+        for (int r = g; r < rows; r += 8) a += part[(size_t)r * cols + col];
+    }
+    red[g][lane] = a;
+    __syncthreads();
+    if (g == 0 && col < cols) {
+#pragma unroll
+        for (int q = 1; q < 8; q++) a += red[q][lane];
+        store_as(out.p[col / C], dtype, col % C, sign * a);
+    }
 }
 
 // x_i = x + (x_prev - x) * (maa_i + m_i) for n mixes; x_prev of a row's first token is `shift` (the
 // last token of the previous segment).  m: [n, tokens, C] (NULL: no data-dependent part).
+struct MixPtrs {
+    const void *p[5];       // maa_i, [C] each
+    int dtype;
+    int one_minus;          // the parameters are 1 - maa_i
+    __device__ __forceinline__ void load(int n, int c, float *f) const {
+        load8(p[n], dtype, c, f);
+        if (one_minus) {
+#pragma unroll
+            for (int q = 0; q < 8; q++) f[q] = 1.f - f[q];
+        }
+    }
+};
 template <int NMIX>
 __global__ void __launch_bounds__(TPB)
-k_ddlerp_fwd(int B, int T, int C, const uint4 *__restrict__ x, const uint4 *__restrict__ shift,
-             const float *__restrict__ maa, const uint4 *__restrict__ m, uint4 *__restrict__ out) {
+k_ddlerp_fwd(int B, int T, int C, const uint4 *__restrict__ x, const uint4 *__restrict__ shift, const MixPtrs maa,
+             const uint4 *__restrict__ m, uint4 *__restrict__ out) {
+    pdl_wait();
+    pdl_trigger();
     const int row16 = C / 8;
     const size_t total = (size_t)B * T * row16, tokens = (size_t)B * T;
     for (size_t i = (size_t)blockIdx.x * TPB + threadIdx.x; i < total; i += (size_t)gridDim.x * TPB) {
@@ -189,7 +261,7 @@ k_ddlerp_fwd(int B, int T, int C, const uint4 *__restrict__ x, const uint4 *__re
 #pragma unroll
         for (int n = 0; n < NMIX; n++) {
             float a[8], mv[8], o[8];
-            load8f(maa + (size_t)n * C + c8 * 8, a);
+            maa.load(n, c8 * 8, a);
             if (m) {
                 unpack8(m[(size_t)n * tokens * row16 + i], mv);
 #pragma unroll
@@ -207,112 +279,184 @@ k_ddlerp_fwd(int B, int T, int C, const uint4 *__restrict__ x, const uint4 *__re
 //   gx_t = sum_i gout_i,t (1 - a_i,t)  +  sum_i gout_i,t+1 a_i,t+1     (the second term: token t is
 //   the predecessor of t+1; for a row's last token it comes from the next segment, `gshift_in`),
 //   gshift_out = sum_i gout_i,0 a_i,0   (gradient w.r.t. `shift`).
-// A thread walks the tokens of one (batch row, 8-channel column) so that the t+1 term is carried in
-// registers; rows x columns give B*C/8 threads... too few for small B, so T is also cut into pieces
-// and the carry of a piece is recomputed from the first token of the next piece.
-template <int NMIX>
-__global__ void __launch_bounds__(TPB)
-k_ddlerp_bwd(int B, int T, int C, int piece, const uint4 *__restrict__ x, const uint4 *__restrict__ shift,
-             const float *__restrict__ maa, const uint4 *__restrict__ m, const uint4 *__restrict__ gout,
-             const uint4 *__restrict__ gshift_in, uint4 *__restrict__ gx, uint4 *__restrict__ gm,
-             uint4 *__restrict__ gshift_out, float *__restrict__ part) {
-    const int row16 = C / 8, npiece = (T + piece - 1) / piece;
-    const size_t tokens = (size_t)B * T;
-    const size_t id = (size_t)blockIdx.x * TPB + threadIdx.x;
-    const size_t nthr = (size_t)B * npiece * row16;
+// A warp walks SUB consecutive tokens of 256 channels backward, so that the t+1 term is carried in registers and
+// recomputed once per SUB tokens; the 8 warps of a CTA take 8*SUB consecutive tokens of the same channels and pool
+// their sums of gm for gmaa.  (One thread per 64 tokens, as before, left half the SMs without a CTA: 191 us for
+// 4096 x 2560 tokens and 5 mixes, 17 tensors of 21 MB.)
+// gx_add, gshift_add: gradients of x and shift from elsewhere, added.
+template <int NMIX, int SUB>
+__global__ void __launch_bounds__(TPB, 2)
+k_ddlerp_bwd(int B, int T, int C, const uint4 *__restrict__ x, const uint4 *__restrict__ shift, const MixPtrs maa,
+             const uint4 *__restrict__ m, const uint4 *__restrict__ gout, const uint4 *__restrict__ gshift_in,
+             const uint4 *__restrict__ gx_add, const uint4 *__restrict__ gshift_add, uint4 *__restrict__ gx,
+             uint4 *__restrict__ gm, uint4 *__restrict__ gshift_out, float *__restrict__ part) {
+    pdl_wait();
+    pdl_trigger();
+    __shared__ float red[8][256];
+    const int row16 = C / 8, ncb = (C + 255) / 256, npiece = (T + 8 * SUB - 1) / (8 * SUB);
+    const int cb = blockIdx.x % ncb, rowp = blockIdx.x / ncb, b = rowp / npiece, pc = rowp - b * npiece;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, c8 = cb * 32 + lane;
+    const size_t tokens16 = (size_t)B * T * row16;
+    const int t0 = pc * 8 * SUB + warp * SUB, t1 = min(T, t0 + SUB);
     float acc[NMIX][8];
 #pragma unroll
     for (int n = 0; n < NMIX; n++)
 #pragma unroll
         for (int q = 0; q < 8; q++) acc[n][q] = 0.f;
-    const int c8 = (int)(id % row16);
-    if (id < nthr) {
-        const int pc = (int)((id / row16) % npiece), b = (int)(id / ((size_t)row16 * npiece));
-        const int t0 = pc * piece, t1 = min(T, t0 + piece);
-        float mz[NMIX][8];
-#pragma unroll
-        for (int n = 0; n < NMIX; n++) load8f(maa + (size_t)n * C + c8 * 8, mz[n]);
-        // carry: what token t1 (the first token after the piece) sends back to token t1-1
+    if (c8 < row16 && t0 < T) {
+        const size_t base = (size_t)b * T * row16 + c8;
+        // carry: what token t1 (the first after this warp's) sends back to token t1-1
         float carry[8];
-        if (t1 < T) {
-            const size_t j = ((size_t)b * T + t1) * row16 + c8;
 #pragma unroll
-            for (int q = 0; q < 8; q++) carry[q] = 0.f;
+        for (int q = 0; q < 8; q++) carry[q] = 0.f;
+        if (t1 < T) {
+            const size_t j = base + (size_t)t1 * row16;
 #pragma unroll
             for (int n = 0; n < NMIX; n++) {
-                float go[8], mv[8];
-                unpack8(gout[(size_t)n * tokens * row16 + j], go);
-                if (m) unpack8(m[(size_t)n * tokens * row16 + j], mv);
+                float go[8], a[8];
+                unpack8(gout[n * tokens16 + j], go);
+                maa.load(n, c8 * 8, a);
+                if (m) {
+                    float mv[8];
+                    unpack8(m[n * tokens16 + j], mv);
 #pragma unroll
-                for (int q = 0; q < 8; q++) carry[q] += go[q] * (mz[n][q] + (m ? mv[q] : 0.f));
+                    for (int q = 0; q < 8; q++) a[q] += mv[q];
+                }
+#pragma unroll
+                for (int q = 0; q < 8; q++) carry[q] += go[q] * a[q];
             }
         } else if (gshift_in) {
             unpack8(gshift_in[(size_t)b * row16 + c8], carry);
-        } else {
-#pragma unroll
-            for (int q = 0; q < 8; q++) carry[q] = 0.f;
         }
+        float xv[8];
+        unpack8(x[base + (size_t)(t1 - 1) * row16], xv);
+#pragma unroll 1
         for (int t = t1 - 1; t >= t0; t--) {
-            const size_t i = ((size_t)b * T + t) * row16 + c8;
-            float xv[8], pv[8], gxv[8], nxt[8];
-            unpack8(x[i], xv);
+            const size_t i = base + (size_t)t * row16;
+            float pv[8], gxv[8], nxt[8], d[8];
             unpack8(t > 0 ? x[i - row16] : shift[(size_t)b * row16 + c8], pv);
+            if (gx_add) unpack8(gx_add[i], gxv);
 #pragma unroll
-            for (int q = 0; q < 8; q++) { pv[q] -= xv[q]; gxv[q] = carry[q]; nxt[q] = 0.f; }
+            for (int q = 0; q < 8; q++) {
+                d[q] = pv[q] - xv[q];
+                gxv[q] = (gx_add ? gxv[q] : 0.f) + carry[q];
+                nxt[q] = 0.f;
+            }
 #pragma unroll
             for (int n = 0; n < NMIX; n++) {
-                float go[8], mv[8], gmv[8];
-                unpack8(gout[(size_t)n * tokens * row16 + i], go);
-                if (m) unpack8(m[(size_t)n * tokens * row16 + i], mv);
+                float go[8], a[8], gmv[8];
+                unpack8(gout[n * tokens16 + i], go);
+                maa.load(n, c8 * 8, a);
+                if (m) {
+                    float mv[8];
+                    unpack8(m[n * tokens16 + i], mv);
+#pragma unroll
+                    for (int q = 0; q < 8; q++) a[q] += mv[q];
+                }
 #pragma unroll
                 for (int q = 0; q < 8; q++) {
-                    const float a = mz[n][q] + (m ? mv[q] : 0.f);
-                    gmv[q] = go[q] * pv[q];
+                    gmv[q] = go[q] * d[q];
                     acc[n][q] += gmv[q];
-                    gxv[q] += go[q] * (1.f - a);
-                    nxt[q] += go[q] * a;
+                    gxv[q] += go[q] - go[q] * a[q];
+                    nxt[q] += go[q] * a[q];
                 }
-                if (gm) gm[(size_t)n * tokens * row16 + i] = pack8(gmv);
+                if (gm) gm[n * tokens16 + i] = pack8(gmv);
             }
             gx[i] = pack8(gxv);
 #pragma unroll
-            for (int q = 0; q < 8; q++) carry[q] = nxt[q];
+            for (int q = 0; q < 8; q++) { carry[q] = nxt[q]; xv[q] = pv[q]; }
         }
-        if (t0 == 0 && gshift_out) gshift_out[(size_t)b * row16 + c8] = pack8(carry);
-    }
-    // partial sums of gmaa per thread: [B*npiece, NMIX, C], folded by k_fold_maa
-    if (id < nthr) {
-        const size_t rowp = id / row16;
+        if (t0 == 0 && gshift_out) {
+            if (gshift_add) {
+                float add[8];
+                unpack8(gshift_add[(size_t)b * row16 + c8], add);
 #pragma unroll
-        for (int n = 0; n < NMIX; n++) {
-            float4 *dst = reinterpret_cast<float4 *>(part + (rowp * NMIX + n) * C + c8 * 8);
-            dst[0] = make_float4(acc[n][0], acc[n][1], acc[n][2], acc[n][3]);
-            dst[1] = make_float4(acc[n][4], acc[n][5], acc[n][6], acc[n][7]);
+                for (int q = 0; q < 8; q++) carry[q] += add[q];
+            }
+            gshift_out[(size_t)b * row16 + c8] = pack8(carry);
         }
     }
-}
-
-__global__ void __launch_bounds__(TPB)
-k_fold_maa(const float *__restrict__ part, int rows, int nmix, int C, float *__restrict__ gmaa) {
-    const int i = blockIdx.x * TPB + threadIdx.x;
-    if (i >= nmix * C) return;
-    float a = 0.f;
-    for (int r = 0; r < rows; r++) a += part[(size_t)r * nmix * C + i];
-    gmaa[i] = a;
+    // the CTA's sums of gm per mix: [B*npiece, NMIX, C], folded by k_fold_cols
+#pragma unroll 1
+    for (int n = 0; n < NMIX; n++) {
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < NMIX; k++)
+            if (k == n) {
+#pragma unroll
+                for (int q = 0; q < 8; q++) red[warp][(lane * 8 + q) ^ (lane & 7)] = acc[k][q];
+            }
+        __syncthreads();
+        const int c = cb * 256 + threadIdx.x, sw = (threadIdx.x) ^ ((threadIdx.x >> 3) & 7);
+        if (c < C) {
+            float a = 0.f;
+#pragma unroll
+            for (int w = 0; w < 8; w++) a += red[w][sw];
+            part[((size_t)rowp * NMIX + n) * C + c] = a;
+        }
+    }
 }
 
 Split make_split(int tokens, int C) {
     Split sp;
     sp.ncb = (C + 255) / 256;
-    int sms = 148, dev = 0;
-    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    int want = (sms * 8 + sp.ncb - 1) / sp.ncb;           // about 8 CTAs per SM
+    const int want = (device_sm_count() * 8 + sp.ncb - 1) / sp.ncb;      // about 8 CTAs per SM
     const int most = (tokens + 7) / 8;
     sp.nslot = want < most ? want : most;
     if (sp.nslot < 1) sp.nslot = 1;
     return sp;
 }
-constexpr int DDLERP_PIECE = 64;
+
+// tokens per warp of k_ddlerp_bwd: 8, or 2 when that leaves SMs without two CTAs
+int ddlerp_sub(int B, int T, int C) {
+    const long long ctas = (long long)B * ((T + 63) / 64) * ((C + 255) / 256);
+    return ctas >= 2 * device_sm_count() ? 8 : 2;
+}
+size_t ddlerp_rows(int B, int T, int C) {
+    const int piece = 8 * ddlerp_sub(B, T, C);
+    return (size_t)B * ((T + piece - 1) / piece);
+}
+
+int fold_cols(const float *part, size_t rows, int n, int C, void *const *out, int dtype, float sign, cudaStream_t s) {
+    GradPtrs g = {};
+    for (int i = 0; i < n; i++) g.p[i] = out[i];
+    return launch_chained(k_fold_cols, dim3((n * C + 31) / 32), dim3(TPB), 0, s, part, (int)rows, n, C, g, dtype, sign);
+}
+
+template <int NMIX>
+int ddlerp_bwd_launch(int B, int T, int C, const void *x, const void *shift, const MixPtrs &maa, const void *m, const void *gout,
+                      const void *gshift_in, const void *gx_add, const void *gshift_add, void *gx, void *gm, void *gshift_out,
+                      float *part, cudaStream_t s) {
+    const dim3 grid((unsigned)(ddlerp_rows(B, T, C) * ((C + 255) / 256)));
+    auto go = [&](auto kern) {
+        return launch_chained(kern, grid, dim3(TPB), 0, s, B, T, C, (const uint4 *)x, (const uint4 *)shift, maa, (const uint4 *)m,
+                              (const uint4 *)gout, (const uint4 *)gshift_in, (const uint4 *)gx_add, (const uint4 *)gshift_add, (uint4 *)gx,
+                              (uint4 *)gm, (uint4 *)gshift_out, part);
+    };
+    return ddlerp_sub(B, T, C) == 8 ? go(k_ddlerp_bwd<NMIX, 8>) : go(k_ddlerp_bwd<NMIX, 2>);
+}
+template <int NMIX>
+int ddlerp_fwd_launch(int B, int T, int C, const void *x, const void *shift, const MixPtrs &maa, const void *m, void *out, cudaStream_t s) {
+    const size_t total = (size_t)B * T * (C / 8);
+    size_t blocks = (total + TPB - 1) / TPB;
+    if (blocks > 148 * 16) blocks = 148 * 16;
+    return launch_chained(k_ddlerp_fwd<NMIX>, dim3((unsigned)blocks), dim3(TPB), 0, s, B, T, C, (const uint4 *)x, (const uint4 *)shift, maa,
+                          (const uint4 *)m, (uint4 *)out);
+}
+
+bool mixes_ok(int n) { return n == 1 || n == 3 || n == 4 || n == 5; }
+MixPtrs mix_ptrs(int n, const void *const *maa, int dtype, int one_minus) {
+    MixPtrs p = {};
+    for (int i = 0; i < n; i++) p.p[i] = maa[i];
+    p.dtype = dtype;
+    p.one_minus = one_minus;
+    return p;
+}
+bool all_aligned(std::initializer_list<const void *> ps) {
+    for (const void *p : ps)
+        if (p && !aligned16(p)) return false;
+    return true;
+}
 
 }  // namespace
 }  // namespace wkv
@@ -321,18 +465,21 @@ using namespace wkv;
 
 extern "C" {
 
-int wkv_lnx_gate_forward(int tokens, int H, const void *y, const void *g, const float *gamma, const float *beta,
-                         float eps, void *out, void *stream) {
+int wkvx_lnx_gate_forward(int tokens, int H, const void *y, const void *g, const void *gamma, const void *beta, int param_dtype,
+                          float eps, int silu, void *out, void *stream) {
     if (tokens < 0 || H < 0) return WKV_ERR_SHAPE;
     if (tokens == 0 || H == 0) return WKV_OK;
     if (!y || !g || !gamma || !beta || !out) return WKV_ERR_NULL;
-    for (const void *p : {y, g, (const void *)gamma, (const void *)beta, (const void *)out})
-        if (!aligned16(p)) return WKV_ERR_ALIGN;
+    if (!all_aligned({y, g, gamma, beta, out})) return WKV_ERR_ALIGN;
     const int C = H * HEAD;
     const Split sp = make_split(tokens, C);
-    k_lnx_gate_fwd<<<sp.ncb * sp.nslot, TPB, 0, (cudaStream_t)stream>>>(tokens, C, sp, (const uint4 *)y, (const uint4 *)g,
-                                                                      gamma, beta, eps, (uint4 *)out);
-    return launch_status();
+    return launch_chained(silu ? k_lnx_gate_fwd<true> : k_lnx_gate_fwd<false>, dim3(sp.ncb * sp.nslot), dim3(TPB), 0, (cudaStream_t)stream,
+                          tokens, C, sp, (const uint4 *)y, (const uint4 *)g, gamma, beta, param_dtype, eps, (uint4 *)out);
+}
+
+int wkv_lnx_gate_forward(int tokens, int H, const void *y, const void *g, const float *gamma, const float *beta,
+                         float eps, void *out, void *stream) {
+    return wkvx_lnx_gate_forward(tokens, H, y, g, gamma, beta, WKV_F32, eps, 0, out, stream);
 }
 
 size_t wkv_lnx_gate_backward_workspace(int tokens, int H) {
@@ -340,101 +487,112 @@ size_t wkv_lnx_gate_backward_workspace(int tokens, int H) {
     return (size_t)make_split(tokens, H * HEAD).nslot * 2 * H * HEAD * sizeof(float);
 }
 
-int wkv_lnx_gate_backward(int tokens, int H, const void *y, const void *g, const float *gamma, const float *beta,
-                          float eps, const void *gout, void *gy, void *gg, float *ggamma, float *gbeta,
-                          void *workspace, size_t workspace_bytes, void *stream) {
+int wkvx_lnx_gate_backward(int tokens, int H, const void *y, const void *g, const void *gamma, const void *beta, int param_dtype,
+                           float eps, int silu, const void *gout, void *gy, void *gg, void *ggamma, void *gbeta, void *workspace,
+                           size_t workspace_bytes, void *stream) {
     if (tokens < 0 || H < 0) return WKV_ERR_SHAPE;
     if (H == 0) return WKV_OK;
     if (!ggamma || !gbeta) return WKV_ERR_NULL;
     const int C = H * HEAD;
     cudaStream_t s = (cudaStream_t)stream;
     if (tokens == 0) {
-        if (cudaMemsetAsync(ggamma, 0, C * sizeof(float), s) != cudaSuccess ||
-            cudaMemsetAsync(gbeta, 0, C * sizeof(float), s) != cudaSuccess)
-            return WKV_ERR_LAUNCH;
+        const size_t n = (size_t)C * (param_dtype == WKV_F32 ? 4 : 2);
+        if (cudaMemsetAsync(ggamma, 0, n, s) != cudaSuccess || cudaMemsetAsync(gbeta, 0, n, s) != cudaSuccess) return WKV_ERR_LAUNCH;
         return WKV_OK;
     }
     if (!y || !g || !gamma || !beta || !gout || !gy || !gg) return WKV_ERR_NULL;
-    for (const void *p : {y, g, (const void *)gamma, (const void *)beta, gout, (const void *)gy, (const void *)gg})
-        if (!aligned16(p)) return WKV_ERR_ALIGN;
+    if (!all_aligned({y, g, gamma, beta, gout, gy, gg})) return WKV_ERR_ALIGN;
     if (!workspace || workspace_bytes < wkv_lnx_gate_backward_workspace(tokens, H)) return WKV_ERR_WORKSPACE;
     const Split sp = make_split(tokens, C);
-    k_lnx_gate_bwd<<<sp.ncb * sp.nslot, TPB, 0, s>>>(tokens, C, sp, (const uint4 *)y, (const uint4 *)g, gamma, beta, eps,
-                                                     (const uint4 *)gout, (uint4 *)gy, (uint4 *)gg, (float *)workspace);
-    k_fold_params<<<(C + TPB - 1) / TPB, TPB, 0, s>>>((const float *)workspace, sp.nslot, C, ggamma, gbeta);
-    return launch_status();
+    if (launch_chained(silu ? k_lnx_gate_bwd<true> : k_lnx_gate_bwd<false>, dim3(sp.ncb * sp.nslot), dim3(TPB), 0, s, tokens, C, sp,
+                       (const uint4 *)y, (const uint4 *)g, gamma, beta, param_dtype, eps, (const uint4 *)gout, (uint4 *)gy, (uint4 *)gg,
+                       (float *)workspace) != WKV_OK)
+        return WKV_ERR_LAUNCH;
+    void *out[2] = {ggamma, gbeta};
+    return fold_cols((const float *)workspace, sp.nslot, 2, C, out, param_dtype, 1.f, s);
+}
+
+int wkv_lnx_gate_backward(int tokens, int H, const void *y, const void *g, const float *gamma, const float *beta,
+                          float eps, const void *gout, void *gy, void *gg, float *ggamma, float *gbeta,
+                          void *workspace, size_t workspace_bytes, void *stream) {
+    return wkvx_lnx_gate_backward(tokens, H, y, g, gamma, beta, WKV_F32, eps, 0, gout, gy, gg, ggamma, gbeta, workspace, workspace_bytes, stream);
+}
+
+int wkvx_ddlerp_forward(int B, int T, int C, int nmix, const void *x, const void *shift, const void *const *maa, int maa_dtype,
+                        int one_minus, const void *m, void *out, void *stream) {
+    if (B < 0 || T < 0 || C < 0 || C % 8 != 0) return WKV_ERR_SHAPE;
+    if (!mixes_ok(nmix)) return WKV_ERR_UNSUPPORTED;
+    if (B == 0 || T == 0 || C == 0) return WKV_OK;
+    if (!x || !shift || !maa || !out) return WKV_ERR_NULL;
+    for (int i = 0; i < nmix; i++)
+        if (!maa[i]) return WKV_ERR_NULL;
+        else if (!aligned16(maa[i])) return WKV_ERR_ALIGN;
+    if (!all_aligned({x, shift, out, m})) return WKV_ERR_ALIGN;
+    const MixPtrs p = mix_ptrs(nmix, maa, maa_dtype, one_minus);
+    cudaStream_t s = (cudaStream_t)stream;
+    switch (nmix) {
+        case 5: return ddlerp_fwd_launch<5>(B, T, C, x, shift, p, m, out, s);
+        case 4: return ddlerp_fwd_launch<4>(B, T, C, x, shift, p, m, out, s);
+        case 3: return ddlerp_fwd_launch<3>(B, T, C, x, shift, p, m, out, s);
+        default: return ddlerp_fwd_launch<1>(B, T, C, x, shift, p, m, out, s);
+    }
 }
 
 int wkv_ddlerp_forward(int B, int T, int C, int nmix, const void *x, const void *shift, const float *maa,
                        const void *m, void *out, void *stream) {
-    if (B < 0 || T < 0 || C < 0 || C % 8 != 0) return WKV_ERR_SHAPE;
-    if (nmix != 1 && nmix != 3 && nmix != 4 && nmix != 5) return WKV_ERR_UNSUPPORTED;
-    if (B == 0 || T == 0 || C == 0) return WKV_OK;
-    if (!x || !shift || !maa || !out) return WKV_ERR_NULL;
-    for (const void *p : {x, shift, (const void *)maa, (const void *)out})
-        if (!aligned16(p)) return WKV_ERR_ALIGN;
-    if (m && !aligned16(m)) return WKV_ERR_ALIGN;
-    const size_t total = (size_t)B * T * (C / 8);
-    size_t blocks = (total + TPB - 1) / TPB;
-    if (blocks > 148 * 16) blocks = 148 * 16;
-    if (nmix == 5)
-        k_ddlerp_fwd<5><<<(unsigned)blocks, TPB, 0, (cudaStream_t)stream>>>(B, T, C, (const uint4 *)x, (const uint4 *)shift,
-                                                                           maa, (const uint4 *)m, (uint4 *)out);
-    else if (nmix == 4)
-        k_ddlerp_fwd<4><<<(unsigned)blocks, TPB, 0, (cudaStream_t)stream>>>(B, T, C, (const uint4 *)x, (const uint4 *)shift,
-                                                                           maa, (const uint4 *)m, (uint4 *)out);
-    else if (nmix == 3)
-        k_ddlerp_fwd<3><<<(unsigned)blocks, TPB, 0, (cudaStream_t)stream>>>(B, T, C, (const uint4 *)x, (const uint4 *)shift,
-                                                                           maa, (const uint4 *)m, (uint4 *)out);
-    else
-        k_ddlerp_fwd<1><<<(unsigned)blocks, TPB, 0, (cudaStream_t)stream>>>(B, T, C, (const uint4 *)x, (const uint4 *)shift,
-                                                                           maa, (const uint4 *)m, (uint4 *)out);
-    return launch_status();
+    const void *p[5] = {};
+    for (int i = 0; i < 5 && i < nmix; i++) p[i] = maa ? maa + (size_t)i * C : nullptr;
+    return wkvx_ddlerp_forward(B, T, C, nmix, x, shift, maa ? p : nullptr, WKV_F32, 0, m, out, stream);
 }
 
 size_t wkv_ddlerp_backward_workspace(int B, int T, int C, int nmix) {
     if (B <= 0 || T <= 0 || C <= 0) return 0;
-    const size_t npiece = (T + DDLERP_PIECE - 1) / DDLERP_PIECE;
-    return (size_t)B * npiece * nmix * C * sizeof(float);
+    return ddlerp_rows(B, T, C) * nmix * C * sizeof(float);
+}
+
+int wkvx_ddlerp_backward(int B, int T, int C, int nmix, const void *x, const void *shift, const void *const *maa, int maa_dtype,
+                         int one_minus, const void *m, const void *gout, const void *gshift_in, const void *gx_add,
+                         const void *gshift_add, void *gx, void *gm, void *gshift_out, void *const *gmaa, void *workspace,
+                         size_t workspace_bytes, void *stream) {
+    if (B < 0 || T < 0 || C < 0 || C % 8 != 0) return WKV_ERR_SHAPE;
+    if (!mixes_ok(nmix)) return WKV_ERR_UNSUPPORTED;
+    if (!gmaa) return WKV_ERR_NULL;
+    cudaStream_t s = (cudaStream_t)stream;
+    if (B == 0 || T == 0 || C == 0) {
+        for (int i = 0; i < nmix && C > 0; i++)
+            if (cudaMemsetAsync(gmaa[i], 0, (size_t)C * (maa_dtype == WKV_F32 ? 4 : 2), s) != cudaSuccess) return WKV_ERR_LAUNCH;
+        return WKV_OK;
+    }
+    if (!x || !shift || !maa || !gout || !gx || (m && !gm)) return WKV_ERR_NULL;
+    for (int i = 0; i < nmix; i++)
+        if (!maa[i]) return WKV_ERR_NULL;
+        else if (!aligned16(maa[i])) return WKV_ERR_ALIGN;
+    if (!all_aligned({x, shift, m, gout, gshift_in, gx_add, gshift_add, gx, gm, gshift_out})) return WKV_ERR_ALIGN;
+    if (!workspace || workspace_bytes < wkv_ddlerp_backward_workspace(B, T, C, nmix)) return WKV_ERR_WORKSPACE;
+    const MixPtrs p = mix_ptrs(nmix, maa, maa_dtype, one_minus);
+    float *part = (float *)workspace;
+    int err;
+    switch (nmix) {
+        case 5: err = ddlerp_bwd_launch<5>(B, T, C, x, shift, p, m, gout, gshift_in, gx_add, gshift_add, gx, gm, gshift_out, part, s); break;
+        case 4: err = ddlerp_bwd_launch<4>(B, T, C, x, shift, p, m, gout, gshift_in, gx_add, gshift_add, gx, gm, gshift_out, part, s); break;
+        case 3: err = ddlerp_bwd_launch<3>(B, T, C, x, shift, p, m, gout, gshift_in, gx_add, gshift_add, gx, gm, gshift_out, part, s); break;
+        default: err = ddlerp_bwd_launch<1>(B, T, C, x, shift, p, m, gout, gshift_in, gx_add, gshift_add, gx, gm, gshift_out, part, s);
+    }
+    if (err != WKV_OK) return err;
+    return fold_cols(part, ddlerp_rows(B, T, C), nmix, C, gmaa, maa_dtype, one_minus ? -1.f : 1.f, s);
 }
 
 int wkv_ddlerp_backward(int B, int T, int C, int nmix, const void *x, const void *shift, const float *maa, const void *m,
                         const void *gout, const void *gshift_in, void *gx, void *gm, void *gshift_out, float *gmaa,
                         void *workspace, size_t workspace_bytes, void *stream) {
-    if (B < 0 || T < 0 || C < 0 || C % 8 != 0) return WKV_ERR_SHAPE;
-    if (nmix != 1 && nmix != 3 && nmix != 4 && nmix != 5) return WKV_ERR_UNSUPPORTED;
-    if (!gmaa) return WKV_ERR_NULL;
-    cudaStream_t s = (cudaStream_t)stream;
-    if (B == 0 || T == 0 || C == 0) {
-        if (C > 0 && cudaMemsetAsync(gmaa, 0, (size_t)nmix * C * sizeof(float), s) != cudaSuccess) return WKV_ERR_LAUNCH;
-        return WKV_OK;
+    const void *p[5] = {};
+    void *g[5] = {};
+    for (int i = 0; i < 5 && i < nmix; i++) {
+        p[i] = maa ? maa + (size_t)i * C : nullptr;
+        g[i] = gmaa ? gmaa + (size_t)i * C : nullptr;
     }
-    if (!x || !shift || !maa || !gout || !gx) return WKV_ERR_NULL;
-    if (m && !gm) return WKV_ERR_NULL;
-    for (const void *p : {x, shift, (const void *)maa, gout, (const void *)gx})
-        if (!aligned16(p)) return WKV_ERR_ALIGN;
-    if (!workspace || workspace_bytes < wkv_ddlerp_backward_workspace(B, T, C, nmix)) return WKV_ERR_WORKSPACE;
-    const int npiece = (T + DDLERP_PIECE - 1) / DDLERP_PIECE;
-    const size_t nthr = (size_t)B * npiece * (C / 8);
-    const unsigned blocks = (unsigned)((nthr + TPB - 1) / TPB);
-    if (nmix == 5)
-        k_ddlerp_bwd<5><<<blocks, TPB, 0, s>>>(B, T, C, DDLERP_PIECE, (const uint4 *)x, (const uint4 *)shift, maa,
-                                               (const uint4 *)m, (const uint4 *)gout, (const uint4 *)gshift_in, (uint4 *)gx,
-                                               (uint4 *)gm, (uint4 *)gshift_out, (float *)workspace);
-    else if (nmix == 4)
-        k_ddlerp_bwd<4><<<blocks, TPB, 0, s>>>(B, T, C, DDLERP_PIECE, (const uint4 *)x, (const uint4 *)shift, maa,
-                                               (const uint4 *)m, (const uint4 *)gout, (const uint4 *)gshift_in, (uint4 *)gx,
-                                               (uint4 *)gm, (uint4 *)gshift_out, (float *)workspace);
-    else if (nmix == 3)
-        k_ddlerp_bwd<3><<<blocks, TPB, 0, s>>>(B, T, C, DDLERP_PIECE, (const uint4 *)x, (const uint4 *)shift, maa,
-                                               (const uint4 *)m, (const uint4 *)gout, (const uint4 *)gshift_in, (uint4 *)gx,
-                                               (uint4 *)gm, (uint4 *)gshift_out, (float *)workspace);
-    else
-        k_ddlerp_bwd<1><<<blocks, TPB, 0, s>>>(B, T, C, DDLERP_PIECE, (const uint4 *)x, (const uint4 *)shift, maa,
-                                               (const uint4 *)m, (const uint4 *)gout, (const uint4 *)gshift_in, (uint4 *)gx,
-                                               (uint4 *)gm, (uint4 *)gshift_out, (float *)workspace);
-    k_fold_maa<<<(nmix * C + TPB - 1) / TPB, TPB, 0, s>>>((const float *)workspace, B * npiece, nmix, C, gmaa);
-    return launch_status();
+    return wkvx_ddlerp_backward(B, T, C, nmix, x, shift, maa ? p : nullptr, WKV_F32, 0, m, gout, gshift_in, nullptr, nullptr, gx, gm,
+                                gshift_out, gmaa ? g : nullptr, workspace, workspace_bytes, stream);
 }
 
 }  // extern "C"

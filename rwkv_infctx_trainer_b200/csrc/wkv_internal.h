@@ -32,6 +32,22 @@ int wkv4x_backward(int B, int T, int C, int dtype, const void *time_decay, int d
                    const void *v, const float *state_in, const void *gy, const float *gstate_out, void *gw_sum, void *gu_sum,
                    int gu_dtype, void *gk, void *gv, float *gstate_in, void *workspace, const void *state_ckpt, void *stream);
 
+/* wkv_lnx_gate_* with parameters (and their gradients) in their own element type, and with silu != 0 the gate
+ * silu(g): g is then the pre-activation and gg its gradient. */
+int wkvx_lnx_gate_forward(int tokens, int H, const void *y, const void *g, const void *gamma, const void *beta, int param_dtype,
+                          float eps, int silu, void *out, void *stream);
+int wkvx_lnx_gate_backward(int tokens, int H, const void *y, const void *g, const void *gamma, const void *beta, int param_dtype,
+                           float eps, int silu, const void *gout, void *gy, void *gg, void *ggamma, void *gbeta, void *workspace,
+                           size_t workspace_bytes, void *stream);
+/* wkv_ddlerp_* with one pointer per mix, in their own element type; one_minus: the parameters p_i stand for maa_i = 1 - p_i
+ * (the gradients are w.r.t. p_i).  gx_add [B,T,C] and gshift_add [B,C] (or NULL) are added to gx and gshift_out. */
+int wkvx_ddlerp_forward(int B, int T, int C, int nmix, const void *x, const void *shift, const void *const *maa, int maa_dtype,
+                        int one_minus, const void *m, void *out, void *stream);
+int wkvx_ddlerp_backward(int B, int T, int C, int nmix, const void *x, const void *shift, const void *const *maa, int maa_dtype,
+                         int one_minus, const void *m, const void *gout, const void *gshift_in, const void *gx_add,
+                         const void *gshift_add, void *gx, void *gm, void *gshift_out, void *const *gmaa, void *workspace,
+                         size_t workspace_bytes, void *stream);
+
 #ifdef __cplusplus
 }
 #endif

@@ -10,8 +10,9 @@ Same constructor arguments, same parameter names and shapes (a state_dict of the
 module loads), same ``forward(x, last_state) -> (out, (shift_state, wkv_state))``.  What is
 different from the project's blocks:
 
-* token shift + (data-dependent) lerp, GroupNorm * gate are one fused kernel each
-  (``timemix.ddlerp``, ``timemix.lnx_gate``); the projections stay library GEMMs;
+* a block is one native call and one autograd node (csrc/native_blocks.cpp): token shift +
+  (data-dependent) lerp, the WKV op and GroupNorm * silu gate are kernels of the library, the
+  projections stay library GEMMs;
 * the WKV state is fp32 ``[B,H,64,64]`` indexed [key,value], per batch row, returned as a new
   tensor that carries its gradient: segments of one sequence can be chained without
   truncating back-propagation (the project's v6 block cannot: RWKV-v6/src/model.py:291-299);
@@ -22,14 +23,10 @@ from __future__ import annotations
 
 import torch
 import torch.nn as nn
-import torch.nn.functional as F
 
-from .timemix import ddlerp, lnx_gate
-from .wkv4 import wkv_op
-from .wkv5 import WKV5
-from .wkv6 import WKV6
+from . import _lib as L
+from . import wkv56
 
-BF16 = torch.bfloat16
 HEAD_SIZE_DIVISOR = 8
 
 
@@ -50,10 +47,6 @@ def _bonus(dim_att, r01):
     return r01 * (1.0 - n / max(dim_att - 1, 1)) + zigzag
 
 
-def _lin(x, layer):
-    return F.linear(x, layer.weight.to(x.dtype))
-
-
 class _TimeMixBase(nn.Module):
     def _common(self, layer_id, n_layer, n_embd, n_head, head_size, dim_att):
         if head_size != 64 or dim_att != n_head * head_size:
@@ -65,12 +58,6 @@ class _TimeMixBase(nn.Module):
         self.value = nn.Linear(n_embd, dim_att, bias=False)
         self.output = nn.Linear(dim_att, n_embd, bias=False)
         self.gate = nn.Linear(n_embd, dim_att, bias=False)
-
-    @staticmethod
-    def _inputs(x, last_state):
-        shift, wkv_state = last_state
-        x = x.to(BF16).contiguous()
-        return x, shift.to(BF16).contiguous(), wkv_state
 
 
 class RWKV_TimeMix6_0(_TimeMixBase):
@@ -102,22 +89,14 @@ class RWKV_TimeMix6_0(_TimeMixBase):
         self.ln_x = nn.GroupNorm(n_head, dim_att, eps=1e-5 * HEAD_SIZE_DIVISOR ** 2)
 
     def forward(self, x, last_state):
-        x, shift, wkv_state = self._inputs(x, last_state)
-        B, T, C = x.shape
-        H = self.n_head
-        # the five mixes: a first lerp feeds the low-rank map that makes them data-dependent
-        xxx = ddlerp(x, shift, self.time_maa_x.view(1, C))[0]
-        xxx = torch.tanh(xxx @ self.time_maa_w1.to(BF16)).view(B * T, 5, -1).transpose(0, 1)
-        m = torch.bmm(xxx, self.time_maa_w2.to(BF16)).view(5, B, T, C)
-        maa = torch.cat((self.time_maa_w, self.time_maa_k, self.time_maa_v, self.time_maa_r,
-                         self.time_maa_g), 0).view(5, C)
-        xw, xk, xv, xr, xg = ddlerp(x, shift, maa, m).unbind(0)
-        r, k, v = _lin(xr, self.receptance), _lin(xk, self.key), _lin(xv, self.value)
-        g = F.silu(_lin(xg, self.gate))
-        w = self.time_decay.to(BF16) + torch.tanh(xw @ self.time_decay_w1.to(BF16)) @ self.time_decay_w2.to(BF16)
-        y, wkv_state = WKV6.apply(B, T, self.dim_att, H, r, k, v, w, self.time_faaaa, wkv_state)
-        y = lnx_gate(y, g, self.ln_x.weight, self.ln_x.bias, self.ln_x.eps, H)
-        return _lin(y, self.output), (x[:, -1], wkv_state)
+        out, shift, wkv_state = L.native().block(
+            6, x, *last_state,
+            [self.time_maa_x, self.time_maa_w, self.time_maa_k, self.time_maa_v, self.time_maa_r, self.time_maa_g,
+             self.time_maa_w1, self.time_maa_w2, self.time_decay, self.time_decay_w1, self.time_decay_w2,
+             self.time_faaaa, self.receptance.weight, self.key.weight, self.value.weight, self.output.weight,
+             self.gate.weight, self.ln_x.weight, self.ln_x.bias],
+            self.n_head, self.ln_x.eps, wkv56.CHECK_STATUS)
+        return out, (shift, wkv_state)
 
 
 class RWKV_TimeMix(_TimeMixBase):
@@ -140,18 +119,14 @@ class RWKV_TimeMix(_TimeMixBase):
         self.ln_x = nn.GroupNorm(n_head, dim_att)
 
     def forward(self, x, last_state):
-        x, shift, wkv_state = self._inputs(x, last_state)
-        B, T, C = x.shape
-        H = self.n_head
-        # x*mix + x_prev*(1-mix)  =  x + (x_prev - x)*(1-mix)
-        maa = 1.0 - torch.cat((self.time_mix_k, self.time_mix_v, self.time_mix_r, self.time_mix_g), 0).view(4, C)
-        xk, xv, xr, xg = ddlerp(x, shift, maa).unbind(0)
-        r, k, v = _lin(xr, self.receptance), _lin(xk, self.key), _lin(xv, self.value)
-        g = F.silu(_lin(xg, self.gate))
-        y, wkv_state = WKV5.apply(B, T, self.dim_att, H, r, k, v, self.time_decay, self.time_faaaa, wkv_state)
         # ln_x(y / 8) with eps  ==  GroupNorm(y) with eps * 64
-        y = lnx_gate(y, g, self.ln_x.weight, self.ln_x.bias, self.ln_x.eps * HEAD_SIZE_DIVISOR ** 2, H)
-        return _lin(y, self.output), (x[:, -1], wkv_state)
+        out, shift, wkv_state = L.native().block(
+            5, x, *last_state,
+            [self.time_mix_k, self.time_mix_v, self.time_mix_r, self.time_mix_g, self.time_decay, self.time_faaaa,
+             self.receptance.weight, self.key.weight, self.value.weight, self.output.weight, self.gate.weight,
+             self.ln_x.weight, self.ln_x.bias],
+            self.n_head, self.ln_x.eps * HEAD_SIZE_DIVISOR ** 2, wkv56.CHECK_STATUS)
+        return out, (shift, wkv_state)
 
 
 class TimeMixState:
@@ -186,12 +161,8 @@ class RWKV_TimeMix_v4(nn.Module):
         self.output = nn.Linear(dim_att, n_embd, bias=False)
 
     def forward(self, x, last_state: TimeMixState):
-        x = x.to(BF16).contiguous()
-        C = x.shape[-1]
-        # x*mix + x_prev*(1-mix)  =  x + (x_prev - x)*(1-mix)
-        maa = 1.0 - torch.cat((self.time_mix_k, self.time_mix_v, self.time_mix_r), 0).view(3, C)
-        xk, xv, xr = ddlerp(x, last_state.shift_state.to(BF16).contiguous(), maa).unbind(0)
-        k, v = _lin(xk, self.key), _lin(xv, self.value)
-        sr = torch.sigmoid(_lin(xr, self.receptance))
-        y, new_wkv_state = wkv_op(self.time_decay, self.time_first.to(BF16), k, v, last_state.wkv_state)
-        return _lin(sr * y, self.output), TimeMixState(x[:, -1], new_wkv_state)
+        out, shift, wkv_state = L.native().block(
+            4, x, last_state.shift_state, last_state.wkv_state,
+            [self.time_mix_k, self.time_mix_v, self.time_mix_r, self.time_decay, self.time_first, self.key.weight,
+             self.value.weight, self.receptance.weight, self.output.weight], 0, 0.0, False)
+        return out, TimeMixState(shift, wkv_state)
