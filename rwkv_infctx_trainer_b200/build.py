@@ -17,7 +17,7 @@ CSRC = os.path.join(PKG, "csrc")
 LIB = os.path.join(PKG, "libwkv_b200.so")
 STAMP = LIB + ".digest"
 SOURCES = ["wkv_api.cu", "wkv4.cu", "wkv4_par.cu", "wkv56_scalar.cu", "wkv56_chunked.cu", "wkv56_chunked_bwd.cu",
-           "timemix_fused.cu"]
+           "timemix_fused.cu", "decode.cu"]
 NATIVE_NAME = "_wkv_native"
 NATIVE = os.path.join(PKG, NATIVE_NAME + ".so")
 NATIVE_SOURCES = ["native_ops.cpp", "native_timemix.cpp", "native_blocks.cpp"]

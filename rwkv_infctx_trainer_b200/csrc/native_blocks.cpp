@@ -117,6 +117,11 @@ struct Out {
     Tensor out, shift, state;
 };
 
+// whether decode.cu takes the call: one token of a few rows, widths its shared memory holds
+bool decode_fits(const Tensor &x, int64_t att) {
+    return x.size(1) == 1 && x.size(0) >= 1 && x.size(0) <= wkvx_decode_max_rows() && x.size(2) % 8 == 0 && x.size(2) <= 8192 && att <= 8192;
+}
+
 // ------------------------------------------------------------------------------ v6
 // params: time_maa_x, _w, _k, _v, _r, _g, time_maa_w1, w2, time_decay, time_decay_w1, w2, time_faaaa, receptance, key, value,
 // output, gate, ln_x.weight, ln_x.bias
@@ -127,6 +132,33 @@ Mixes five6(const variable_list &p) { return Mixes({p[P6_MW], p[P6_MK], p[P6_MV]
 
 Out forward6(const Tensor &x, const Tensor &shift, const Tensor &state, const variable_list &p, const Meta &me, variable_list *keep) {
     const int64_t B = x.size(0), T = x.size(1), C = x.size(2), M = B * T, H = me.H;
+    if (!keep && decode_fits(x, H * HEAD) && C == H * HEAD && p[P6_W2].dim() == 3 && p[P6_W2].size(1) == 32 && p[P6_D2].size(0) % 8 == 0) {
+        // one token of a few rows: the block's own kernels
+        const Mixes mx({p[P6_X], p[P6_MW], p[P6_MK], p[P6_MV], p[P6_MR], p[P6_MG]}, false);
+        const auto lt = param_type(p[P6_LW]);
+        const Tensor w1 = as_bf16(p[P6_W1]), w2 = as_bf16(p[P6_W2]), td = as_bf16(p[P6_DECAY]), d1 = as_bf16(p[P6_D1]), d2 = as_bf16(p[P6_D2]),
+                     u = as_bf16(p[P6_U]), lw = as_contig(p[P6_LW], lt), lb = as_contig(p[P6_LB], lt);
+        const Tensor proj[5] = {as_bf16(p[P6_R]), as_bf16(p[P6_K]), as_bf16(p[P6_V]), as_bf16(p[P6_G]), as_bf16(p[P6_O])};
+        const int64_t R = w2.size(1), DR = d2.size(0);
+        Tensor scratch = at::empty({10 * M * C + M * (5 * R + DR)}, x.options());
+        Out o{at::empty_like(x), at::empty_like(shift), at::empty_like(state)};
+        wkvx_decode6_t a = {};
+        a.M = (int)M; a.H = (int)H; a.rank = (int)R; a.decay_rank = (int)DR;
+        a.x = ptr(x); a.shift = ptr(shift);
+        a.maa_x = ptr(mx.t[0]);
+        for (int i = 0; i < 5; i++) a.maa[i] = ptr(mx.t[1 + i]);
+        a.maa_dtype = dtype_code(mx.type);
+        a.w1 = ptr(w1); a.w2 = ptr(w2); a.decay = ptr(td); a.d1 = ptr(d1); a.d2 = ptr(d2); a.u = ptr(u);
+        for (int i = 0; i < 5; i++) a.proj[i] = ptr(proj[i]);
+        a.ln_w = ptr(lw); a.ln_b = ptr(lb); a.ln_dtype = dtype_code(lt); a.eps = (float)me.eps;
+        a.state_in = (const float *)ptr(state); a.state_out = (float *)ptr(o.state);
+        char *q = (char *)ptr(scratch);
+        const int64_t n = M * C * 2;
+        a.xs = q; a.rkvg = q + 5 * n; a.normed = q + 9 * n; a.t1 = q + 10 * n; a.dd = q + 10 * n + M * 5 * R * 2;
+        a.out = ptr(o.out); a.new_shift = ptr(o.shift);
+        check(wkvx_decode6(&a, stream_of(x)), "decode6");
+        return o;
+    }
     // the five mixes: a first lerp feeds the low-rank map that makes them data-dependent
     const Tensor xxx = mix_forward(x, shift, first6(p), Tensor()).view({M, C});
     const Tensor w1 = as_bf16(p[P6_W1]), w2 = as_bf16(p[P6_W2]);
@@ -215,19 +247,42 @@ enum { P5_MK, P5_MV, P5_MR, P5_MG, P5_DECAY, P5_U, P5_R, P5_K, P5_V, P5_O, P5_G,
 Mixes four5(const variable_list &p) { return Mixes({p[P5_MK], p[P5_MV], p[P5_MR], p[P5_MG]}, true); }
 
 Out forward5(const Tensor &x, const Tensor &shift, const Tensor &state, const variable_list &p, const Meta &me, variable_list *keep) {
-    const int64_t B = x.size(0), T = x.size(1), C = x.size(2), M = B * T, H = me.H;
+    const int64_t B = x.size(0), T = x.size(1), C = x.size(2), M = B * T, H = me.H, A = H * HEAD;
+    if (!keep && decode_fits(x, A)) {
+        // one token of a few rows: the block's own kernels
+        const Mixes mx = four5(p);
+        const auto lt = param_type(p[P5_LW]);
+        const Tensor u = as_bf16(p[P5_U]), w = as_contig(p[P5_DECAY], param_type(p[P5_DECAY])), lw = as_contig(p[P5_LW], lt), lb = as_contig(p[P5_LB], lt);
+        const Tensor proj[5] = {as_bf16(p[P5_R]), as_bf16(p[P5_K]), as_bf16(p[P5_V]), as_bf16(p[P5_G]), as_bf16(p[P5_O])};
+        Tensor scratch = at::empty({5 * M * A}, x.options());
+        Out o{at::empty_like(x), at::empty_like(shift), at::empty_like(state)};
+        wkvx_decode5_t a = {};
+        a.M = (int)M; a.H = (int)H; a.C = (int)C;
+        a.x = ptr(x); a.shift = ptr(shift);
+        for (int i = 0; i < 4; i++) a.mix[i] = ptr(mx.t[i]);
+        a.mix_dtype = dtype_code(mx.type);
+        a.decay = ptr(w); a.decay_dtype = dtype_code(w.scalar_type()); a.u = ptr(u);
+        for (int i = 0; i < 5; i++) a.proj[i] = ptr(proj[i]);
+        a.ln_w = ptr(lw); a.ln_b = ptr(lb); a.ln_dtype = dtype_code(lt); a.eps = (float)me.eps;
+        a.state_in = (const float *)ptr(state); a.state_out = (float *)ptr(o.state);
+        char *q = (char *)ptr(scratch);
+        a.rkvg = q; a.normed = q + 4 * M * A * 2;
+        a.out = ptr(o.out); a.new_shift = ptr(o.shift);
+        check(wkvx_decode5(&a, stream_of(x)), "decode5");
+        return o;
+    }
     const Tensor xs = mix_forward(x, shift, four5(p), Tensor());
-    Tensor rkvg = at::empty({4, M, C}, x.options());
+    Tensor rkvg = at::empty({4, M, A}, x.options());
     linear_into(rkvg[0], xs[2], as_bf16(p[P5_R]));
     linear_into(rkvg[1], xs[0], as_bf16(p[P5_K]));
     linear_into(rkvg[2], xs[1], as_bf16(p[P5_V]));
     linear_into(rkvg[3], xs[3], as_bf16(p[P5_G]));
-    const auto btc = [&](const Tensor &t) { return t.view({B, T, C}); };
+    const auto btc = [&](const Tensor &t) { return t.view({B, T, A}); };
     const Tensor u = as_bf16(p[P5_U]), w = as_contig(p[P5_DECAY], at::kFloat);
     Fwd o = wkv56_forward(false, btc(rkvg[0]), btc(rkvg[1]), btc(rkvg[2]), w, u, state, WKV_W_RAW, WKV_STATE_KV, WKV_PATH_AUTO, Tensor(),
                           keep != nullptr, 0, Tensor(), WKV_GROUP_STATES_NONE, me.sync);
     const auto lt = param_type(p[P5_LW]);
-    const Tensor y = o.y.view({M, C}), n = norm_gate_forward(y, rkvg[3], as_contig(p[P5_LW], lt), as_contig(p[P5_LB], lt), me.eps, H);
+    const Tensor y = o.y.view({M, A}), n = norm_gate_forward(y, rkvg[3], as_contig(p[P5_LW], lt), as_contig(p[P5_LB], lt), me.eps, H);
     const Tensor out = at::mm(n, as_bf16(p[P5_O]).t());
     if (keep) *keep = {xs, rkvg, w, u, y, n, o.ckpt};
     return {out.view({B, T, C}), last_token(x), o.state_out};
@@ -235,9 +290,9 @@ Out forward5(const Tensor &x, const Tensor &shift, const Tensor &state, const va
 
 variable_list backward5(const Tensor &x, const Tensor &shift, const Tensor &state, const variable_list &p, const Meta &me,
                         const variable_list &kept, const Tensor &gout_, const Tensor &gshift_new, const Tensor &gstate, bool want_gs) {
-    const int64_t B = x.size(0), T = x.size(1), C = x.size(2), M = B * T, H = me.H;
+    const int64_t B = x.size(0), T = x.size(1), C = x.size(2), M = B * T, H = me.H, A = H * HEAD;
     const Tensor &xs = kept[0], &rkvg = kept[1], &w = kept[2], &u = kept[3], &y = kept[4], &n = kept[5], &ckpt = kept[6];
-    const auto btc = [&](const Tensor &t) { return t.view({B, T, C}); };
+    const auto btc = [&](const Tensor &t) { return t.view({B, T, A}); };
     variable_list gp(P5_N);
     const Tensor gout = gout_.view({M, C});
     gp[P5_O] = at::mm(gout.t(), n);
@@ -250,7 +305,7 @@ variable_list backward5(const Tensor &x, const Tensor &shift, const Tensor &stat
                            WKV_PATH_AUTO, want_gs, ckpt, 0, false, param_type(p[P5_U]), param_type(p[P5_DECAY]), me.sync);
     gp[P5_U] = o.gu;
     gp[P5_DECAY] = o.gw;
-    const Tensor gr = o.gr.view({M, C}), gk = o.gk.view({M, C}), gv = o.gv.view({M, C});
+    const Tensor gr = o.gr.view({M, A}), gk = o.gk.view({M, A}), gv = o.gv.view({M, A});
     gp[P5_R] = at::mm(gr.t(), xs[2]);
     gp[P5_K] = at::mm(gk.t(), xs[0]);
     gp[P5_V] = at::mm(gv.t(), xs[1]);

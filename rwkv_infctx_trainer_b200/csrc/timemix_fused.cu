@@ -293,11 +293,21 @@ k_ddlerp_bwd(int B, int T, int C, const uint4 *__restrict__ x, const uint4 *__re
     pdl_wait();
     pdl_trigger();
     __shared__ float red[8][256];
+    __shared__ __align__(16) float mixes[NMIX][256];      // maa of the CTA's channels
     const int row16 = C / 8, ncb = (C + 255) / 256, npiece = (T + 8 * SUB - 1) / (8 * SUB);
     const int cb = blockIdx.x % ncb, rowp = blockIdx.x / ncb, b = rowp / npiece, pc = rowp - b * npiece;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, c8 = cb * 32 + lane;
     const size_t tokens16 = (size_t)B * T * row16;
     const int t0 = pc * 8 * SUB + warp * SUB, t1 = min(T, t0 + SUB);
+    for (int k = threadIdx.x; k < NMIX * 32; k += TPB) {
+        const int n = k >> 5, l = k & 31;
+        if (cb * 32 + l < row16) maa.load(n, (cb * 32 + l) * 8, &mixes[n][l * 8]);
+    }
+    __syncthreads();
+    auto mix = [&](int n, float *a) {
+        const float4 p = *reinterpret_cast<const float4 *>(&mixes[n][lane * 8]), q = *reinterpret_cast<const float4 *>(&mixes[n][lane * 8 + 4]);
+        a[0] = p.x; a[1] = p.y; a[2] = p.z; a[3] = p.w; a[4] = q.x; a[5] = q.y; a[6] = q.z; a[7] = q.w;
+    };
     float acc[NMIX][8];
 #pragma unroll
     for (int n = 0; n < NMIX; n++)
@@ -315,7 +325,7 @@ k_ddlerp_bwd(int B, int T, int C, const uint4 *__restrict__ x, const uint4 *__re
             for (int n = 0; n < NMIX; n++) {
                 float go[8], a[8];
                 unpack8(gout[n * tokens16 + j], go);
-                maa.load(n, c8 * 8, a);
+                mix(n, a);
                 if (m) {
                     float mv[8];
                     unpack8(m[n * tokens16 + j], mv);
@@ -333,6 +343,13 @@ k_ddlerp_bwd(int B, int T, int C, const uint4 *__restrict__ x, const uint4 *__re
 #pragma unroll 1
         for (int t = t1 - 1; t >= t0; t--) {
             const size_t i = base + (size_t)t * row16;
+            // every load of the token goes out before the first is used
+            uint4 graw[NMIX], mraw[NMIX];
+#pragma unroll
+            for (int n = 0; n < NMIX; n++) {
+                graw[n] = gout[n * tokens16 + i];
+                if (m) mraw[n] = m[n * tokens16 + i];
+            }
             float pv[8], gxv[8], nxt[8], d[8];
             unpack8(t > 0 ? x[i - row16] : shift[(size_t)b * row16 + c8], pv);
             if (gx_add) unpack8(gx_add[i], gxv);
@@ -345,11 +362,11 @@ k_ddlerp_bwd(int B, int T, int C, const uint4 *__restrict__ x, const uint4 *__re
 #pragma unroll
             for (int n = 0; n < NMIX; n++) {
                 float go[8], a[8], gmv[8];
-                unpack8(gout[n * tokens16 + i], go);
-                maa.load(n, c8 * 8, a);
+                unpack8(graw[n], go);
+                mix(n, a);
                 if (m) {
                     float mv[8];
-                    unpack8(m[n * tokens16 + i], mv);
+                    unpack8(mraw[n], mv);
 #pragma unroll
                     for (int q = 0; q < 8; q++) a[q] += mv[q];
                 }

@@ -48,6 +48,47 @@ int wkvx_ddlerp_backward(int B, int T, int C, int nmix, const void *x, const voi
                          const void *gshift_add, void *gx, void *gm, void *gshift_out, void *const *gmaa, void *workspace,
                          size_t workspace_bytes, void *stream);
 
+/* One token of a time-mix block for M rows (1 .. wkvx_decode_max_rows()), forward only (decode.cu).  bf16 tensors;
+ * state fp32 [M,H,64,64] (key, value); C = H*64; scratch sizes beside the fields. */
+int wkvx_decode_max_rows(void);
+typedef struct wkvx_decode6 {
+    int M, H, rank, decay_rank;             /* rank: 32 */
+    const void *x, *shift;                  /* [M,C] */
+    const void *maa_x, *maa[5];             /* [C]; w, k, v, r, g */
+    int maa_dtype;
+    const void *w1, *w2;                    /* [C,5*rank], [5,rank,C] */
+    const void *decay, *d1, *d2;            /* [C], [C,decay_rank], [decay_rank,C] */
+    const void *u;                          /* [H,64] */
+    const void *proj[5];                    /* [C,C]: r, k, v, g, output */
+    const void *ln_w, *ln_b;
+    int ln_dtype;
+    float eps;
+    const float *state_in;
+    void *t1, *xs, *rkvg, *dd, *normed;     /* [M,5*rank], [5,M,C], [4,M,C], [M,decay_rank], [M,C] */
+    void *out, *new_shift;                  /* [M,C] */
+    float *state_out;
+} wkvx_decode6_t;
+int wkvx_decode6(const wkvx_decode6_t *a, void *stream);
+
+typedef struct wkvx_decode5 {
+    int M, H, C;                            /* C: width of x and out; the attention width is H*64 */
+    const void *x, *shift;                  /* [M,C] */
+    const void *mix[4];                     /* [C]; k, v, r, g: maa = 1 - mix */
+    int mix_dtype;
+    const void *decay;                      /* [H,64] time_decay */
+    int decay_dtype;
+    const void *u;                          /* [H,64] */
+    const void *proj[5];                    /* r, k, v, g [H*64,C], output [C,H*64] */
+    const void *ln_w, *ln_b;
+    int ln_dtype;
+    float eps;
+    const float *state_in;
+    void *rkvg, *normed;                    /* [4,M,H*64], [M,H*64] */
+    void *out, *new_shift;
+    float *state_out;
+} wkvx_decode5_t;
+int wkvx_decode5(const wkvx_decode5_t *a, void *stream);
+
 #ifdef __cplusplus
 }
 #endif
