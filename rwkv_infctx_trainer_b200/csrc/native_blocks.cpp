@@ -37,7 +37,7 @@ struct Mixes {
 
 Tensor mix_forward(const Tensor &x, const Tensor &shift, const Mixes &mx, const Tensor &m) {
     const int B = (int)x.size(0), T = (int)x.size(1), C = (int)x.size(2);
-    Tensor out = at::empty({mx.n(), B * (int64_t)T, C}, x.options());
+    Tensor out = fresh({mx.n(), B * (int64_t)T, C}, x.scalar_type(), x);
     const auto p = mx.ptrs();
     check(wkvx_ddlerp_forward(B, T, C, mx.n(), ptr(x), ptr(shift), p.data(), dtype_code(mx.type), mx.one_minus, ptr(m), ptr(out), stream_of(x)),
           "wkv_ddlerp_forward");
@@ -53,12 +53,12 @@ MixGrads mix_backward(const Tensor &x, const Tensor &shift, const Mixes &mx, con
                       const Tensor &gshift_in, const Tensor &gx_add, const Tensor &gshift_add) {
     const int B = (int)x.size(0), T = (int)x.size(1), C = (int)x.size(2);
     MixGrads g;
-    g.gx = at::empty_like(x);
-    if (m.defined()) g.gm = at::empty_like(m);
-    g.gshift = at::empty_like(shift);
+    g.gx = fresh_like(x);
+    if (m.defined()) g.gm = fresh_like(m);
+    g.gshift = fresh_like(shift);
     std::array<void *, 5> gp{};
     for (int i = 0; i < mx.n(); i++) {
-        g.gmaa.push_back(at::empty_like(mx.t[i]));
+        g.gmaa.push_back(fresh_like(mx.t[i]));
         gp[i] = ptr(g.gmaa[i]);
     }
     const size_t n = wkv_ddlerp_backward_workspace(B, T, C, mx.n());
@@ -73,7 +73,7 @@ MixGrads mix_backward(const Tensor &x, const Tensor &shift, const Mixes &mx, con
 
 // GroupNorm(y) * silu(g)
 Tensor norm_gate_forward(const Tensor &y, const Tensor &g, const Tensor &lw, const Tensor &lb, double eps, int64_t H) {
-    Tensor out = at::empty_like(y);
+    Tensor out = fresh_like(y);
     check(wkvx_lnx_gate_forward((int)y.size(0), (int)H, ptr(y), ptr(g), ptr(lw), ptr(lb), dtype_code(lw.scalar_type()), (float)eps, 1, ptr(out),
                                 stream_of(y)),
           "wkv_lnx_gate_forward");
@@ -83,7 +83,7 @@ struct NormGrads {
     Tensor gy, gg, glw, glb;
 };
 NormGrads norm_gate_backward(const Tensor &y, const Tensor &g, const Tensor &lw, const Tensor &lb, double eps, int64_t H, const Tensor &gout) {
-    NormGrads r{at::empty_like(y), at::empty_like(g), at::empty_like(lw), at::empty_like(lb)};
+    NormGrads r{fresh_like(y), fresh_like(g), fresh_like(lw), fresh_like(lb)};
     const int tokens = (int)y.size(0);
     const size_t n = wkv_lnx_gate_backward_workspace(tokens, (int)H);
     Tensor ws = bytes_like(y, n);
@@ -101,16 +101,6 @@ struct Meta {
 };
 
 Tensor last_token(const Tensor &x) { return x.select(1, x.size(1) - 1).contiguous(); }
-
-// gradients in the parameters' own types and shapes
-void finish(variable_list &grads, size_t first, const variable_list &params) {
-    for (size_t i = 0; i < params.size(); i++) {
-        Tensor &g = grads[first + i];
-        if (!g.defined()) continue;
-        if (g.scalar_type() != params[i].scalar_type()) g = g.to(params[i].scalar_type());
-        if (g.sizes() != params[i].sizes()) g = g.view(params[i].sizes());
-    }
-}
 
 // A forward pass of a block: with `keep` it also appends what the backward pass reads.
 struct Out {
@@ -140,8 +130,8 @@ Out forward6(const Tensor &x, const Tensor &shift, const Tensor &state, const va
                      u = as_bf16(p[P6_U]), lw = as_contig(p[P6_LW], lt), lb = as_contig(p[P6_LB], lt);
         const Tensor proj[5] = {as_bf16(p[P6_R]), as_bf16(p[P6_K]), as_bf16(p[P6_V]), as_bf16(p[P6_G]), as_bf16(p[P6_O])};
         const int64_t R = w2.size(1), DR = d2.size(0);
-        Tensor scratch = at::empty({10 * M * C + M * (5 * R + DR)}, x.options());
-        Out o{at::empty_like(x), at::empty_like(shift), at::empty_like(state)};
+        Tensor scratch = fresh({10 * M * C + M * (5 * R + DR)}, x.scalar_type(), x);
+        Out o{fresh_like(x), fresh_like(shift), fresh_like(state)};
         wkvx_decode6_t a = {};
         a.M = (int)M; a.H = (int)H; a.rank = (int)R; a.decay_rank = (int)DR;
         a.x = ptr(x); a.shift = ptr(shift);
@@ -166,7 +156,7 @@ Out forward6(const Tensor &x, const Tensor &shift, const Tensor &state, const va
     Tensor t1 = at::mm(xxx, w1).tanh_();
     const Tensor m = at::bmm(t1.view({M, 5, R}).transpose(0, 1), w2);
     const Tensor xs = mix_forward(x, shift, five6(p), m);
-    Tensor rkvg = at::empty({4, M, C}, x.options());
+    Tensor rkvg = fresh({4, M, C}, x.scalar_type(), x);
     linear_into(rkvg[0], xs[3], as_bf16(p[P6_R]));
     linear_into(rkvg[1], xs[1], as_bf16(p[P6_K]));
     linear_into(rkvg[2], xs[2], as_bf16(p[P6_V]));
@@ -207,7 +197,7 @@ variable_list backward6(const Tensor &x, const Tensor &shift, const Tensor &stat
     gp[P6_K] = at::mm(gk.t(), xs[1]);
     gp[P6_V] = at::mm(gv.t(), xs[2]);
     gp[P6_G] = at::mm(ng.gg.t(), xs[4]);
-    Tensor gxs = at::empty_like(xs);
+    Tensor gxs = fresh_like(xs);
     const auto into = [&](int i, const Tensor &a, const Tensor &b) { Tensor d = gxs[i]; at::mm_out(d, a, b); };
     into(3, gr, as_bf16(p[P6_R]));
     into(1, gk, as_bf16(p[P6_K]));
@@ -227,7 +217,7 @@ variable_list backward6(const Tensor &x, const Tensor &shift, const Tensor &stat
     const int64_t R = w2.size(1);
     const Tensor t5 = t1.view({M, 5, R});
     gp[P6_W2] = at::bmm(t5.permute({1, 2, 0}), mg.gm);
-    Tensor gt1 = at::empty_like(t1), gt5 = gt1.view({M, 5, R});
+    Tensor gt1 = fresh_like(t1), gt5 = gt1.view({M, 5, R});
     at::tanh_backward_out(gt5, at::bmm(mg.gm, w2.transpose(1, 2)).transpose(0, 1), t5);
     gp[P6_W1] = at::mm(xxx.t(), gt1);
     MixGrads m1 = mix_backward(x, shift, first6(p), Tensor(), at::mm(gt1, w1.t()), Tensor(), mg.gx, mg.gshift);
@@ -254,8 +244,8 @@ Out forward5(const Tensor &x, const Tensor &shift, const Tensor &state, const va
         const auto lt = param_type(p[P5_LW]);
         const Tensor u = as_bf16(p[P5_U]), w = as_contig(p[P5_DECAY], param_type(p[P5_DECAY])), lw = as_contig(p[P5_LW], lt), lb = as_contig(p[P5_LB], lt);
         const Tensor proj[5] = {as_bf16(p[P5_R]), as_bf16(p[P5_K]), as_bf16(p[P5_V]), as_bf16(p[P5_G]), as_bf16(p[P5_O])};
-        Tensor scratch = at::empty({5 * M * A}, x.options());
-        Out o{at::empty_like(x), at::empty_like(shift), at::empty_like(state)};
+        Tensor scratch = fresh({5 * M * A}, x.scalar_type(), x);
+        Out o{fresh_like(x), fresh_like(shift), fresh_like(state)};
         wkvx_decode5_t a = {};
         a.M = (int)M; a.H = (int)H; a.C = (int)C;
         a.x = ptr(x); a.shift = ptr(shift);
@@ -272,7 +262,7 @@ Out forward5(const Tensor &x, const Tensor &shift, const Tensor &state, const va
         return o;
     }
     const Tensor xs = mix_forward(x, shift, four5(p), Tensor());
-    Tensor rkvg = at::empty({4, M, A}, x.options());
+    Tensor rkvg = fresh({4, M, A}, x.scalar_type(), x);
     linear_into(rkvg[0], xs[2], as_bf16(p[P5_R]));
     linear_into(rkvg[1], xs[0], as_bf16(p[P5_K]));
     linear_into(rkvg[2], xs[1], as_bf16(p[P5_V]));
@@ -310,7 +300,7 @@ variable_list backward5(const Tensor &x, const Tensor &shift, const Tensor &stat
     gp[P5_K] = at::mm(gk.t(), xs[0]);
     gp[P5_V] = at::mm(gv.t(), xs[1]);
     gp[P5_G] = at::mm(ng.gg.t(), xs[3]);
-    Tensor gxs = at::empty_like(xs);
+    Tensor gxs = fresh_like(xs);
     const auto into = [&](int i, const Tensor &a, const Tensor &b) { Tensor d = gxs[i]; at::mm_out(d, a, b); };
     into(2, gr, as_bf16(p[P5_R]));
     into(0, gk, as_bf16(p[P5_K]));
@@ -333,7 +323,7 @@ Out forward4(const Tensor &x, const Tensor &shift, const Tensor &state, const va
     const int64_t B = x.size(0), T = x.size(1), C = x.size(2), M = B * T;
     const Tensor xs = mix_forward(x, shift, three4(p), Tensor());
     const int64_t A = p[P4_K].size(0);       // dim_att
-    Tensor kv = at::empty({2, M, A}, x.options());
+    Tensor kv = fresh({2, M, A}, x.scalar_type(), x);
     linear_into(kv[0], xs[0], as_bf16(p[P4_K]));
     linear_into(kv[1], xs[1], as_bf16(p[P4_V]));
     Tensor sr = at::mm(xs[2], as_bf16(p[P4_R]).t()).sigmoid_();
@@ -361,7 +351,7 @@ variable_list backward4(const Tensor &x, const Tensor &shift, const Tensor &stat
     gp[P4_K] = at::mm(gk.t(), xs[0]);
     gp[P4_V] = at::mm(gv.t(), xs[1]);
     gp[P4_R] = at::mm(gr.t(), xs[2]);
-    Tensor gxs = at::empty_like(xs);
+    Tensor gxs = fresh_like(xs);
     const auto into = [&](int i, const Tensor &a, const Tensor &b) { Tensor d = gxs[i]; at::mm_out(d, a, b); };
     into(0, gk, as_bf16(p[P4_K]));
     into(1, gv, as_bf16(p[P4_V]));
@@ -388,41 +378,23 @@ const Kind &kind_of(int64_t version) {
     return version == 4 ? k4 : version == 5 ? k5 : k6;
 }
 
-struct BlockFunction : torch::autograd::Function<BlockFunction> {
-    static variable_list forward(AutogradContext *ctx, int64_t version, const Tensor &x, const Tensor &shift, const Tensor &state,
-                                 at::TensorList params, int64_t H, double eps, bool sync) {
+struct BlockBackward : OpNode {
+    int64_t version;
+    Meta meta;
+    std::string name() const override { return "TimeMixBlockBackward"; }
+    variable_list apply(variable_list &&grads) override {
         at::AutoDispatchBelowADInplaceOrView below;
-        c10::cuda::OptionalCUDAGuard guard(x.device());
-        const variable_list p(params.begin(), params.end());
-        variable_list kept;
-        const Out o = kind_of(version).forward(x, shift, state, p, Meta{H, eps, sync}, &kept);
-        variable_list save = {x, shift, state};
-        save.insert(save.end(), p.begin(), p.end());
-        save.insert(save.end(), kept.begin(), kept.end());
-        ctx->save_for_backward(save);
-        ctx->saved_data["i"] = std::vector<int64_t>{version, H, (int64_t)sync};
-        ctx->saved_data["eps"] = eps;
-        ctx->set_materialize_grads(false);
-        return {o.out, o.shift, o.state};
-    }
-    static variable_list backward(AutogradContext *ctx, variable_list grads) {
-        at::AutoDispatchBelowADInplaceOrView below;
-        const variable_list st = ctx->get_saved_variables();
-        const auto i = ctx->saved_data["i"].toIntVector();
-        const Kind &k = kind_of(i[0]);
+        const variable_list st = unpack();
+        const Kind &k = kind_of(version);
         const Tensor &x = st[0], &shift = st[1], &state = st[2];
         c10::cuda::OptionalCUDAGuard guard(x.device());
         const variable_list p(st.begin() + 3, st.begin() + 3 + k.params), kept(st.begin() + 3 + k.params, st.end());
         const Tensor gout = grads[0].defined() ? as_contig(grads[0], BF16) : at::zeros_like(x);
         const Tensor gshift = grads[1].defined() ? as_contig(grads[1], BF16) : Tensor();
         const Tensor gstate = grads[2].defined() ? as_contig(grads[2], at::kFloat) : Tensor();
-        variable_list g = k.backward(x, shift, state, p, Meta{i[1], ctx->saved_data["eps"].toDouble(), i[2] != 0}, kept, gout, gshift, gstate,
-                                     ctx->needs_input_grad(2));
-        finish(g, 3, p);
-        variable_list r = {Tensor()};
-        r.insert(r.end(), g.begin(), g.end());
-        r.insert(r.end(), 3, Tensor());
-        return r;
+        variable_list g = k.backward(x, shift, state, p, meta, kept, gout, gshift, gstate, task_should_compute_output(2));
+        for (size_t i = 0; i < k.params; i++) g[3 + i] = as_input(g[3 + i], p[i].scalar_type(), p[i].sizes());
+        return g;
     }
 };
 
@@ -441,8 +413,25 @@ std::tuple<Tensor, Tensor, Tensor> block(int64_t version, const Tensor &x_, cons
     if (!grad && at::GradMode::is_enabled())
         for (const Tensor &p : params) grad |= p.requires_grad();
     if (grad) {
-        variable_list o = BlockFunction::apply(version, x, shift, state, at::TensorList(params), H, eps, sync);
-        return {o[0], o[1], o[2]};
+        variable_list in = {x, shift, state};
+        in.insert(in.end(), params.begin(), params.end());
+        auto node = make_node<BlockBackward>(in);
+        node->version = version;
+        node->meta = Meta{H, eps, sync};
+        Out o;
+        {
+            at::AutoDispatchBelowADInplaceOrView below;
+            c10::cuda::OptionalCUDAGuard guard(x.device());
+            variable_list kept;
+            o = k.forward(x, shift, state, params, node->meta, &kept);
+            node->saved.reserve(in.size() + kept.size());
+            for (const Tensor &t : in) node->keep({t});
+            for (const Tensor &t : kept) node->keep({t});
+        }
+        torch::autograd::set_history(o.out, node);
+        torch::autograd::set_history(o.shift, node);
+        torch::autograd::set_history(o.state, node);
+        return {o.out, o.shift, o.state};
     }
     at::AutoDispatchBelowADInplaceOrView below;
     c10::cuda::OptionalCUDAGuard guard(x.device());

@@ -89,9 +89,9 @@ Fwd wkv56_forward(bool v6, const Tensor &r, const Tensor &k, const Tensor &v, co
     raise_if_set(dev, status);
     c10::cuda::OptionalCUDAGuard guard(r.device());
     Fwd out;
-    out.y = at::empty_like(r);
+    out.y = fresh_like(r);
     wkv_args_t a = make_args(r, w_kind, layout, path, time_groups);
-    out.state_out = state_out.defined() ? state_out : at::empty({a.B, a.H, HEAD, HEAD}, r.options().dtype(at::kFloat));
+    out.state_out = state_out.defined() ? state_out : fresh({a.B, a.H, HEAD, HEAD}, at::kFloat, r);
     a.r = ptr(r); a.k = ptr(k); a.v = ptr(v); a.w = ptr(w); a.u = ptr(u);
     a.state_in = (const float *)ptr(state_in);
     a.y = ptr(out.y); a.state_out = (float *)ptr(out.state_out);
@@ -126,20 +126,19 @@ Bwd wkv56_backward(bool v6, const Tensor &r, const Tensor &k, const Tensor &v, c
     raise_if_set(dev, status);
     c10::cuda::OptionalCUDAGuard guard(r.device());
     wkv_args_t a = make_args(r, w_kind, layout, path, time_groups);
-    const auto f32 = r.options().dtype(at::kFloat);
     const int64_t B = a.B, H = a.H;
     Bwd g;
-    g.gr = at::empty_like(r); g.gk = at::empty_like(r); g.gv = at::empty_like(r);
+    g.gr = fresh_like(r); g.gk = fresh_like(r); g.gv = fresh_like(r);
     const bool empty = B == 0 || H == 0;
     if (per_batch) {
-        g.gu = at::empty({B, H * HEAD}, f32);
-        g.gw = v6 ? at::empty_like(r) : at::empty({B, H * HEAD}, f32);
+        g.gu = fresh({B, H * HEAD}, at::kFloat, r);
+        g.gw = v6 ? fresh_like(r) : fresh({B, H * HEAD}, at::kFloat, r);
     } else {
-        g.gu = empty ? at::zeros({H, HEAD}, r.options().dtype(u_type)) : at::empty({H, HEAD}, r.options().dtype(u_type));
-        g.gw = v6 ? at::empty_like(r)
-                  : (empty ? at::zeros({H, HEAD}, r.options().dtype(w_type)) : at::empty({H, HEAD}, r.options().dtype(w_type)));
+        g.gu = empty ? at::zeros({H, HEAD}, r.options().dtype(u_type)) : fresh({H, HEAD}, u_type, r);
+        g.gw = v6 ? fresh_like(r)
+                  : (empty ? at::zeros({H, HEAD}, r.options().dtype(w_type)) : fresh({H, HEAD}, w_type, r));
     }
-    if (want_gstate) g.gstate_in = at::empty({B, H, HEAD, HEAD}, f32);
+    if (want_gstate) g.gstate_in = fresh({B, H, HEAD, HEAD}, at::kFloat, r);
     a.r = ptr(r); a.k = ptr(k); a.v = ptr(v); a.w = ptr(w); a.u = ptr(u);
     a.state_in = (const float *)ptr(state_in);
     a.gy = ptr(gy); a.gstate_out = (const float *)ptr(gstate_out);
@@ -172,46 +171,22 @@ Bwd wkv56_backward(bool v6, const Tensor &r, const Tensor &k, const Tensor &v, c
 // ------------------------------------------------------------------------------ v5 / v6 autograd node
 namespace {
 
-struct Wkv56Function : torch::autograd::Function<Wkv56Function> {
-    // w: v6 in r's type, v5 fp32.  w_type / u_type: the element types the caller's parameters have.
-    static variable_list forward(AutogradContext *ctx, bool v6, const Tensor &r, const Tensor &k, const Tensor &v,
-                                 const Tensor &w, const Tensor &u, const Tensor &state, int64_t path, const Tensor *saved,
-                                 int64_t saved_mode, bool sync_check) {
-        const auto dt = r.scalar_type();
-        const Tensor rc = contig(r), kc = as_contig(k, dt), vc = as_contig(v, dt), uc = as_contig(u, dt),
-                     wc = as_contig(w, v6 ? dt : at::kFloat), sc = as_contig(state, at::kFloat);
-        Fwd o = wkv56_forward(v6, rc, kc, vc, wc, uc, sc, WKV_W_RAW, WKV_STATE_KV, (int)path, Tensor(), true, 0, *saved,
-                              (int)saved_mode, sync_check);
-        // (with a hand-over the backward pass does not need the initial state)
-        variable_list keep = {rc, kc, vc, wc, uc, sc};
-        if (o.ckpt.defined()) keep.push_back(o.ckpt);
-        ctx->save_for_backward(keep);
-        ctx->saved_data["v6"] = v6;
-        ctx->saved_data["path"] = path;
-        ctx->saved_data["sync"] = sync_check;
-        ctx->saved_data["types"] = std::vector<int64_t>{(int64_t)k.scalar_type(), (int64_t)v.scalar_type(), (int64_t)w.scalar_type(),
-                                                        (int64_t)u.scalar_type(), (int64_t)state.scalar_type()};
-        ctx->saved_data["w_shape"] = w.sizes().vec();
-        ctx->saved_data["u_shape"] = u.sizes().vec();
-        ctx->saved_data["s_shape"] = state.sizes().vec();
-        ctx->set_materialize_grads(false);
-        return {o.y, o.state_out};
-    }
-    static variable_list backward(AutogradContext *ctx, variable_list grads) {
-        const variable_list st = ctx->get_saved_variables();
+struct Wkv56Backward : OpNode {
+    bool v6, sync;
+    int path;
+    at::ScalarType k_type, v_type, w_type, u_type, s_type;
+    std::vector<int64_t> w_shape, u_shape, s_shape;
+    std::string name() const override { return "Wkv56Backward"; }
+    variable_list apply(variable_list &&grads) override {
+        at::AutoDispatchBelowADInplaceOrView below;
+        const variable_list st = unpack();
         const Tensor &r = st[0];
-        const bool v6 = ctx->saved_data["v6"].toBool();
-        const auto types = ctx->saved_data["types"].toIntVector();
-        const auto type = [&](int i) { return (at::ScalarType)types[i]; };
         const Tensor gy = grads[0].defined() ? as_contig(grads[0], r.scalar_type()) : at::zeros_like(r);
         const Tensor gs = grads[1].defined() ? as_contig(grads[1], at::kFloat) : Tensor();
-        Bwd g = wkv56_backward(v6, r, st[1], st[2], st[3], st[4], st[5], gy, gs, WKV_W_RAW, WKV_STATE_KV,
-                               (int)ctx->saved_data["path"].toInt(), ctx->needs_input_grad(5), st.size() > 6 ? st[6] : Tensor(), 0,
-                               false, type(3), v6 ? at::kFloat : type(2), ctx->saved_data["sync"].toBool());
-        Tensor gw = v6 ? g.gw.to(type(2)) : g.gw.view(ctx->saved_data["w_shape"].toIntVector());
-        Tensor gsi = g.gstate_in.defined() ? g.gstate_in.to(type(4)).view(ctx->saved_data["s_shape"].toIntVector()) : Tensor();
-        return {Tensor(), g.gr, g.gk.to(type(0)), g.gv.to(type(1)), gw, g.gu.view(ctx->saved_data["u_shape"].toIntVector()), gsi,
-                Tensor(), Tensor(), Tensor(), Tensor()};
+        Bwd g = wkv56_backward(v6, r, st[1], st[2], st[3], st[4], st[5], gy, gs, WKV_W_RAW, WKV_STATE_KV, path, task_should_compute_output(5),
+                               st[6], 0, false, u_type, v6 ? at::kFloat : w_type, sync);
+        return {g.gr, as_input(g.gk, k_type, g.gk.sizes()), as_input(g.gv, v_type, g.gv.sizes()), as_input(g.gw, w_type, w_shape),
+                as_input(g.gu, u_type, u_shape), as_input(g.gstate_in, s_type, s_shape)};
     }
 };
 
@@ -236,8 +211,23 @@ std::tuple<Tensor, Tensor> wkv56_apply(bool v6, int64_t B, int64_t T, int64_t C,
     check_shapes56(v6, B, T, C, H, r, k, v, w, u, state);
     const Tensor buf = saved.has_value() ? *saved : Tensor();
     if (wants_grad({&r, &k, &v, &w, &u, &state})) {
-        variable_list o = Wkv56Function::apply(v6, r, k, v, w, u, state, path, &buf, saved_mode, sync_check);
-        return {o[0], o[1]};
+        auto node = make_node<Wkv56Backward>({r, k, v, w, u, state});
+        node->v6 = v6; node->sync = sync_check; node->path = (int)path;
+        node->k_type = k.scalar_type(); node->v_type = v.scalar_type(); node->w_type = w.scalar_type();
+        node->u_type = u.scalar_type(); node->s_type = state.scalar_type();
+        node->w_shape = w.sizes().vec(); node->u_shape = u.sizes().vec(); node->s_shape = state.sizes().vec();
+        Fwd o;
+        {
+            at::AutoDispatchBelowADInplaceOrView below;
+            const auto dt = r.scalar_type();
+            const Tensor rc = contig(r), kc = as_contig(k, dt), vc = as_contig(v, dt), wc = as_contig(w, v6 ? dt : at::kFloat),
+                         uc = as_contig(u, dt), sc = as_contig(state, at::kFloat);
+            o = wkv56_forward(v6, rc, kc, vc, wc, uc, sc, WKV_W_RAW, WKV_STATE_KV, (int)path, Tensor(), true, 0, buf, (int)saved_mode, sync_check);
+            node->keep({rc, kc, vc, wc, uc, sc, o.ckpt});
+        }
+        torch::autograd::set_history(o.y, node);
+        torch::autograd::set_history(o.state_out, node);
+        return {o.y, o.state_out};
     }
     const auto dt = r.scalar_type();
     Fwd o = wkv56_forward(v6, contig(r), as_contig(k, dt), as_contig(v, dt), as_contig(w, v6 ? dt : at::kFloat),
@@ -251,44 +241,21 @@ std::tuple<Tensor, Tensor> wkv56_apply(bool v6, int64_t B, int64_t T, int64_t C,
 // place in the [value,key] layout and the gradient of the state after the call is taken as zero.
 namespace {
 
-struct DropinFunction : torch::autograd::Function<DropinFunction> {
-    static Tensor forward(AutogradContext *ctx, bool v6, const Tensor &r, const Tensor &k, const Tensor &v, const Tensor &w,
-                          const Tensor &u, const Tensor &state, bool save, bool sync_check) {
-        const Tensor wc = as_contig(w, v6 ? r.scalar_type() : at::kFloat);
-        const Tensor s32 = as_contig(state, at::kFloat);
-        // the chunked kernels hand the states over; the token-serial ones start backward from the state itself
-        wkv_args_t a = make_args(r, WKV_W_RAW, WKV_STATE_VK, WKV_PATH_AUTO, 0);
-        const Tensor s_in = save && !wkv56_uses_chunked(&a, v6) ? s32.clone() : Tensor();
-        Fwd o = wkv56_forward(v6, r, k, v, wc, u, s32, WKV_W_RAW, WKV_STATE_VK, WKV_PATH_AUTO, s32, save, 0, Tensor(),
-                              WKV_GROUP_STATES_NONE, sync_check);
-        if (s32.data_ptr() != state.data_ptr()) {
-            Tensor dst = state.detach();
-            dst.copy_(s32.view_as(state));
-        }
-        if (save) {
-            ctx->save_for_backward({r, k, v, wc, u, s_in, o.ckpt});
-            ctx->saved_data["v6"] = v6;
-            ctx->saved_data["sync"] = sync_check;
-            ctx->saved_data["types"] = std::vector<int64_t>{(int64_t)w.scalar_type(), (int64_t)state.scalar_type()};
-            ctx->saved_data["w_shape"] = w.sizes().vec();
-            ctx->saved_data["u_shape"] = u.sizes().vec();
-            ctx->saved_data["s_shape"] = state.sizes().vec();
-        }
-        return o.y;
-    }
-    static variable_list backward(AutogradContext *ctx, variable_list grads) {
-        const variable_list st = ctx->get_saved_variables();
+struct DropinBackward : OpNode {
+    bool v6, sync;
+    at::ScalarType w_type, s_type;
+    std::vector<int64_t> w_shape, u_shape, s_shape;
+    std::string name() const override { return "WkvDropinBackward"; }
+    variable_list apply(variable_list &&grads) override {
+        if (!grads[0].defined()) return variable_list(6);
+        at::AutoDispatchBelowADInplaceOrView below;
+        const variable_list st = unpack();
         const Tensor &r = st[0];
-        const bool v6 = ctx->saved_data["v6"].toBool();
-        const auto types = ctx->saved_data["types"].toIntVector();
         // (the v5 wrapper gives its state no gradient)
-        const bool want_gs = v6 && ctx->needs_input_grad(5);
+        const bool want_gs = v6 && task_should_compute_output(5);
         Bwd g = wkv56_backward(v6, r, st[1], st[2], st[3], st[4], st[5], as_contig(grads[0], r.scalar_type()), Tensor(), WKV_W_RAW,
-                               WKV_STATE_VK, WKV_PATH_AUTO, want_gs, st[6], 0, false, r.scalar_type(), (at::ScalarType)types[0],
-                               ctx->saved_data["sync"].toBool());
-        Tensor gw = v6 ? g.gw.to((at::ScalarType)types[0]) : g.gw.view(ctx->saved_data["w_shape"].toIntVector());
-        Tensor gs = want_gs ? g.gstate_in.to((at::ScalarType)types[1]).view(ctx->saved_data["s_shape"].toIntVector()) : Tensor();
-        return {Tensor(), g.gr, g.gk, g.gv, gw, g.gu.view(ctx->saved_data["u_shape"].toIntVector()), gs, Tensor(), Tensor()};
+                               WKV_STATE_VK, WKV_PATH_AUTO, want_gs, st[6], 0, false, r.scalar_type(), w_type, sync);
+        return {g.gr, g.gk, g.gv, as_input(g.gw, w_type, w_shape), as_input(g.gu, r.scalar_type(), u_shape), as_input(g.gstate_in, s_type, s_shape)};
     }
 };
 
@@ -303,7 +270,32 @@ Tensor wkv56_dropin(bool v6, int64_t B, int64_t T, int64_t C, int64_t H, const T
         TORCH_CHECK_TYPE(state.scalar_type() == at::kFloat && w.scalar_type() == at::kFloat, "state and w must be float32");
     dtype_code(dt);
     check_shapes56(v6, B, T, C, H, r, k, v, w, u, state);
-    return DropinFunction::apply(v6, r, k, v, w, u, state, wants_grad({&r, &k, &v, &w, &u, &state}), sync_check);
+    const bool save = wants_grad({&r, &k, &v, &w, &u, &state});
+    std::shared_ptr<DropinBackward> node;
+    if (save) {
+        node = make_node<DropinBackward>({r, k, v, w, u, state});
+        node->v6 = v6; node->sync = sync_check;
+        node->w_type = w.scalar_type(); node->s_type = state.scalar_type();
+        node->w_shape = w.sizes().vec(); node->u_shape = u.sizes().vec(); node->s_shape = state.sizes().vec();
+    }
+    Tensor y;
+    {
+        at::AutoDispatchBelowADInplaceOrView below;
+        const Tensor wc = as_contig(w, v6 ? dt : at::kFloat), s32 = as_contig(state, at::kFloat);
+        // the chunked kernels hand the states over; the token-serial ones start backward from the state itself
+        const wkv_args_t a = make_args(r, WKV_W_RAW, WKV_STATE_VK, WKV_PATH_AUTO, 0);
+        const Tensor s_in = save && !wkv56_uses_chunked(&a, v6) ? s32.clone() : Tensor();
+        Fwd o = wkv56_forward(v6, r, k, v, wc, u, s32, WKV_W_RAW, WKV_STATE_VK, WKV_PATH_AUTO, s32, save, 0, Tensor(),
+                              WKV_GROUP_STATES_NONE, sync_check);
+        if (s32.data_ptr() != state.data_ptr()) {
+            Tensor dst = state.detach();
+            dst.copy_(s32.view_as(state));
+        }
+        y = o.y;
+        if (save) node->keep({r, k, v, wc, u, s_in, o.ckpt});
+    }
+    if (save) torch::autograd::set_history(y, node);
+    return y;
 }
 
 // ------------------------------------------------------------------------------ v4
@@ -311,8 +303,8 @@ Fwd4 wkv4_forward(const Tensor &w, const Tensor &u, const Tensor &k, const Tenso
     const int B = (int)k.size(0), T = (int)k.size(1), C = (int)k.size(2);
     c10::cuda::OptionalCUDAGuard guard(k.device());
     Fwd4 o;
-    o.y = at::empty_like(k);
-    o.state_out = at::empty_like(state);
+    o.y = fresh_like(k);
+    o.state_out = fresh_like(state);
     o.ckpt = bytes_like(k, save ? wkv4_state_ckpt_bytes(B, T, C) : 0);
     check(wkv4x_forward(B, T, C, dtype_code(k.scalar_type()), ptr(w), dtype_code(w.scalar_type()), ptr(u), ptr(k), ptr(v),
                         (const float *)ptr(state), ptr(o.y), (float *)ptr(o.state_out), ptr(o.ckpt), stream_of(k)),
@@ -325,11 +317,11 @@ Bwd4 wkv4_backward(const Tensor &w, const Tensor &u, const Tensor &k, const Tens
     const int B = (int)k.size(0), T = (int)k.size(1), C = (int)k.size(2);
     c10::cuda::OptionalCUDAGuard guard(k.device());
     Bwd4 g;
-    g.gw = B ? at::empty_like(w) : at::zeros_like(w);
-    g.gu = B ? at::empty({C}, u.options().dtype(u_type)) : at::zeros({C}, u.options().dtype(u_type));
-    g.gk = at::empty_like(k);
-    g.gv = at::empty_like(v);
-    if (want_gstate) g.gstate = at::empty_like(state);
+    g.gw = B ? fresh_like(w) : at::zeros_like(w);
+    g.gu = B ? fresh({C}, u_type, u) : at::zeros({C}, u.options().dtype(u_type));
+    g.gk = fresh_like(k);
+    g.gv = fresh_like(v);
+    if (want_gstate) g.gstate = fresh_like(state);
     Tensor ws = bytes_like(k, wkv4x_backward_workspace(B, T, C, ckpt.defined()));
     check(wkv4x_backward(B, T, C, dtype_code(k.scalar_type()), ptr(w), dtype_code(w.scalar_type()), ptr(u), ptr(k), ptr(v),
                          (const float *)ptr(state), ptr(gy), (const float *)ptr(gstate_out), ptr(g.gw), ptr(g.gu), dtype_code(u_type),
@@ -341,31 +333,19 @@ Bwd4 wkv4_backward(const Tensor &w, const Tensor &u, const Tensor &k, const Tens
 namespace {
 
 // RWKV-v4neo/cuda/wkv_op_bf16.cpp:13-92
-struct Wkv4Function : torch::autograd::Function<Wkv4Function> {
-    static variable_list forward(AutogradContext *ctx, const Tensor &raw_w, const Tensor &raw_u, const Tensor &raw_k,
-                                 const Tensor &raw_v, const Tensor &raw_state, bool save) {
-        const auto dt = raw_k.scalar_type();
-        const Tensor w = as_contig(raw_w, param_type(raw_w)), u = as_contig(raw_u, dt), k = contig(raw_k), v = as_contig(raw_v, dt),
-                     state = as_contig(raw_state, at::kFloat);
-        Fwd4 o = wkv4_forward(w, u, k, v, state, save);
-        if (save) {
-            ctx->save_for_backward({w, u, k, v, state, o.ckpt});
-            ctx->saved_data["types"] = std::vector<int64_t>{(int64_t)raw_w.scalar_type(), (int64_t)raw_u.scalar_type(),
-                                                            (int64_t)raw_v.scalar_type(), (int64_t)raw_state.scalar_type(),
-                                                            (int64_t)param_type(raw_u)};
-            ctx->set_materialize_grads(false);
-        }
-        return {o.y, o.state_out};
-    }
-    static variable_list backward(AutogradContext *ctx, variable_list grads) {
-        const variable_list st = ctx->get_saved_variables();
+struct Wkv4Backward : OpNode {
+    at::ScalarType w_type, u_type, v_type, s_type;
+    std::string name() const override { return "Wkv4Backward"; }
+    variable_list apply(variable_list &&grads) override {
+        at::AutoDispatchBelowADInplaceOrView below;
+        const variable_list st = unpack();
         const Tensor &k = st[2];
-        const auto types = ctx->saved_data["types"].toIntVector();
-        const auto type = [&](int i) { return (at::ScalarType)types[i]; };
         const Tensor gy = grads[0].defined() ? as_contig(grads[0], k.scalar_type()) : at::zeros_like(k);
         const Tensor gs = grads[1].defined() ? as_contig(grads[1], at::kFloat) : Tensor();
-        Bwd4 g = wkv4_backward(st[0], st[1], k, st[3], st[4], st[5], gy, gs, type(4), ctx->needs_input_grad(4));
-        return {g.gw.to(type(0)), g.gu.to(type(1)), g.gk, g.gv.to(type(2)), g.gstate.defined() ? g.gstate.to(type(3)) : Tensor(), Tensor()};
+        Bwd4 g = wkv4_backward(st[0], st[1], k, st[3], st[4], st[5], gy, gs, u_type == at::kDouble ? at::kFloat : u_type,
+                               task_should_compute_output(4));
+        return {as_input(g.gw, w_type, g.gw.sizes()), as_input(g.gu, u_type, g.gu.sizes()), g.gk, as_input(g.gv, v_type, g.gv.sizes()),
+                as_input(g.gstate, s_type, st[4].sizes())};
     }
 };
 
@@ -380,7 +360,26 @@ std::vector<Tensor> wkv4(const Tensor &w, const Tensor &u, const Tensor &k, cons
                       "last_state must be [B,C,3]");
     require_cuda({&w, &u, &k, &v, &state});
     dtype_code(k.scalar_type());
-    return Wkv4Function::apply(w, u, k, v, state, wants_grad({&w, &u, &k, &v, &state}));
+    const bool save = wants_grad({&w, &u, &k, &v, &state});
+    std::shared_ptr<Wkv4Backward> node;
+    if (save) {
+        node = make_node<Wkv4Backward>({w, u, k, v, state});
+        node->w_type = w.scalar_type(); node->u_type = u.scalar_type(); node->v_type = v.scalar_type(); node->s_type = state.scalar_type();
+    }
+    Fwd4 o;
+    {
+        at::AutoDispatchBelowADInplaceOrView below;
+        const auto dt = k.scalar_type();
+        const Tensor wc = as_contig(w, param_type(w)), uc = as_contig(u, dt), kc = contig(k), vc = as_contig(v, dt),
+                     sc = as_contig(state, at::kFloat);
+        o = wkv4_forward(wc, uc, kc, vc, sc, save);
+        if (save) node->keep({wc, uc, kc, vc, sc, o.ckpt});
+    }
+    if (save) {
+        torch::autograd::set_history(o.y, node);
+        torch::autograd::set_history(o.state_out, node);
+    }
+    return {o.y, o.state_out};
 }
 
 }  // namespace wkv_native

@@ -22,7 +22,7 @@ struct LnxGate : torch::autograd::Function<LnxGate> {
         c10::cuda::OptionalCUDAGuard guard(y_.device());
         const auto pt = weight.scalar_type() == bias.scalar_type() ? param_type(weight) : at::kFloat;
         const Tensor y = contig(y_), g = contig(g_), ga = as_contig(weight, pt), be = as_contig(bias, pt);
-        Tensor out = at::empty_like(y);
+        Tensor out = fresh_like(y);
         const int tokens = (int)(y.numel() / (H * HEAD));
         check(wkvx_lnx_gate_forward(tokens, (int)H, ptr(y), ptr(g), ptr(ga), ptr(be), dtype_code(pt), (float)eps, 0, ptr(out), stream_of(y)),
               "wkv_lnx_gate_forward");
@@ -40,7 +40,7 @@ struct LnxGate : torch::autograd::Function<LnxGate> {
         const int H = (int)ctx->saved_data["H"].toInt(), C = H * (int)HEAD, tokens = (int)(y.numel() / C);
         c10::cuda::OptionalCUDAGuard guard(y.device());
         const Tensor gout = as_contig(grads[0], at::kBFloat16);
-        Tensor gy = at::empty_like(y), gg = at::empty_like(g), gga = at::empty({C}, ga.options()), gbe = at::empty({C}, be.options());
+        Tensor gy = fresh_like(y), gg = fresh_like(g), gga = fresh({C}, ga.scalar_type(), ga), gbe = fresh({C}, be.scalar_type(), be);
         const size_t n = wkv_lnx_gate_backward_workspace(tokens, H);
         Tensor ws = bytes_like(y, n);
         check(wkvx_lnx_gate_backward(tokens, H, ptr(y), ptr(g), ptr(ga), ptr(be), dtype_code(ga.scalar_type()),
@@ -58,7 +58,7 @@ struct DDLerp : torch::autograd::Function<DDLerp> {
         c10::cuda::OptionalCUDAGuard guard(x_.device());
         const Tensor x = contig(x_), sh = contig(shift_), m = m_.has_value() ? contig(*m_) : Tensor(), ma = as_contig(maa, param_type(maa));
         const int B = (int)x.size(0), T = (int)x.size(1), C = (int)x.size(2), n = (int)ma.size(0);
-        Tensor out = at::empty({n, B, T, C}, x.options());
+        Tensor out = fresh({n, B, T, C}, x.scalar_type(), x);
         const auto p = rows_of(ma);
         check(wkvx_ddlerp_forward(B, T, C, n, ptr(x), ptr(sh), p.data(), dtype_code(ma.scalar_type()), 0, ptr(m), ptr(out), stream_of(x)),
               "wkv_ddlerp_forward");
@@ -72,8 +72,8 @@ struct DDLerp : torch::autograd::Function<DDLerp> {
         const int B = (int)x.size(0), T = (int)x.size(1), C = (int)x.size(2), n = (int)ma.size(0);
         c10::cuda::OptionalCUDAGuard guard(x.device());
         const Tensor gout = as_contig(grads[0], at::kBFloat16);
-        Tensor gx = at::empty_like(x), gm = m.defined() ? at::empty_like(m) : Tensor(), gsh = at::empty_like(sh),
-               gma = at::empty({n, C}, ma.options());
+        Tensor gx = fresh_like(x), gm = m.defined() ? fresh_like(m) : Tensor(), gsh = fresh_like(sh),
+               gma = fresh({n, C}, ma.scalar_type(), ma);
         const size_t nb = wkv_ddlerp_backward_workspace(B, T, C, n);
         Tensor ws = bytes_like(x, nb);
         const auto p = rows_of(ma), gp = rows_of(gma);
