@@ -61,29 +61,8 @@ __device__ __forceinline__ float rcp(float x) {
 }
 
 // ---- two channels at a time
-typedef float2 f2;
 // keeps loads of later tokens from being hoisted above this point: all eight at once do not fit the registers
 __device__ __forceinline__ void no_hoist() { asm volatile("" ::: "memory"); }
-__device__ __forceinline__ unsigned long long bits(const f2 &a) { return *reinterpret_cast<const unsigned long long *>(&a); }
-__device__ __forceinline__ f2 from_bits(unsigned long long v) { return *reinterpret_cast<f2 *>(&v); }
-__device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c) {
-    unsigned long long r;
-    asm("fma.rn.ftz.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(bits(a)), "l"(bits(b)), "l"(bits(c)));
-    return from_bits(r);
-}
-__device__ __forceinline__ f2 mul2(f2 a, f2 b) {
-    unsigned long long r;
-    asm("mul.rn.ftz.f32x2 %0, %1, %2;" : "=l"(r) : "l"(bits(a)), "l"(bits(b)));
-    return from_bits(r);
-}
-__device__ __forceinline__ f2 add2(f2 a, f2 b) {
-    unsigned long long r;
-    asm("add.rn.ftz.f32x2 %0, %1, %2;" : "=l"(r) : "l"(bits(a)), "l"(bits(b)));
-    return from_bits(r);
-}
-__device__ __forceinline__ f2 both(float x) { return make_float2(x, x); }
-__device__ __forceinline__ f2 sub2(f2 a, f2 b) { return fma2(b, both(-1.f), a); }
-__device__ __forceinline__ f2 neg2(f2 a) { return make_float2(-a.x, -a.y); }
 __device__ __forceinline__ f2 max2(f2 a, f2 b) { return make_float2(fmaxf(a.x, b.x), fmaxf(a.y, b.y)); }
 __device__ __forceinline__ f2 min2(f2 a, f2 b) { return make_float2(fminf(a.x, b.x), fminf(a.y, b.y)); }
 __device__ __forceinline__ f2 ex2_2(f2 a) { return make_float2(ex2(a.x), ex2(a.y)); }

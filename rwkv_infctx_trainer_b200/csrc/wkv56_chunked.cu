@@ -298,7 +298,7 @@ k_chunk_fwd(const __grid_constant__ CUtensorMap map_r, const __grid_constant__ C
             Tile *in = s.in[j & 1];
             Tile &khat = s.khat[j & 1];
             float c[4][4];
-            DecayT<4> D;
+            Decay D;
             float other_l2[4];
             bool mild;
             if (!PER_TOKEN && (jg + 1) * CH <= P.T) {
@@ -369,14 +369,12 @@ k_chunk_fwd(const __grid_constant__ CUtensorMap map_r, const __grid_constant__ C
                         float r[4], k[4], rt[4], rh[4];
                         unpack4(ld_tile4(in[0], t, cc, hf), r);
                         unpack4(ld_tile4(in[1], t, cc, hf), k);
-                        float dsum = 0.f;
-#pragma unroll
-                        for (int ch = 0; ch < 4; ch++) {
-                            rt[ch] = r[ch] * fa[ch];
-                            rh[ch] = rt[ch] * cr[ch];
-                            dsum += r[ch] * uu[ch] * k[ch];
-                            fa[ch] *= D.w[i][ch];
-                        }
+                        vmul<4>(rt, r, fa);
+                        vmul<4>(rh, rt, cr);
+                        vmul<4>(fa, fa, D.w[i]);
+                        f2 d2 = mul2(mul2(make_float2(r[0], r[1]), make_float2(uu[0], uu[1])), make_float2(k[0], k[1]));
+                        d2 = fma2(mul2(make_float2(r[2], r[3]), make_float2(uu[2], uu[3])), make_float2(k[2], k[3]), d2);
+                        float dsum = d2.x + d2.y;
                         st_tile4(in[0], t, cc, hf, pack4(rt));
                         st_tile4(in[3], t, cc, hf, pack4(rh));
                         dsum += __shfl_xor_sync(0xffffffffu, dsum, 1);
@@ -389,11 +387,9 @@ k_chunk_fwd(const __grid_constant__ CUtensorMap map_r, const __grid_constant__ C
                         const int t = tok0 + i;
                         float r[4], rh[4];
                         unpack4(ld_tile4(in[0], t, cc, hf), r);
-#pragma unroll
-                        for (int ch = 0; ch < 4; ch++) {
-                            rh[ch] = r[ch] * fa[ch] * cr[ch];
-                            fa[ch] *= D.w[i][ch];
-                        }
+                        vmul<4>(rh, r, fa);
+                        vmul<4>(rh, rh, cr);
+                        vmul<4>(fa, fa, D.w[i]);
                         st_tile4(in[3], t, cc, hf, pack4(rh));
                     }
                 }
@@ -404,12 +400,9 @@ k_chunk_fwd(const __grid_constant__ CUtensorMap map_r, const __grid_constant__ C
                     const int t = tok0 + i;
                     float k[4], kt[4], kh[4];
                     unpack4(ld_tile4(in[1], t, cc, hf), k);
-#pragma unroll
-                    for (int ch = 0; ch < 4; ch++) {
-                        kt[ch] = k[ch] * fa[ch];
-                        kh[ch] = kt[ch] * ck[ch];
-                        fa[ch] *= D.w[i][ch];
-                    }
+                    vmul<4>(kt, k, fa);
+                    vmul<4>(kh, kt, ck);
+                    vmul<4>(fa, fa, D.w[i]);
                     if (full) st_tile4(in[1], t, cc, hf, pack4(kt));
                     st_tile4(khat, t, cc, hf, pack4(kh));
                 }
@@ -559,8 +552,7 @@ k_chunk_fwd(const __grid_constant__ CUtensorMap map_r, const __grid_constant__ C
                 tmem_ld_wait();
                 const float d = s.dvec[j & 1][row];
                 if (summary) dprod *= d;
-#pragma unroll
-                for (int q = 0; q < 16; q++) S[q] = fmaf(d, S[q], uacc[q]);
+                vaxpy<16>(S, d, S, uacc);
             }
             publish_state(j + 1);
             // (M) masked scores of chunk j+1: lo lanes own columns 0..31 of token row t, hi lanes 32..63;

@@ -41,14 +41,7 @@ __device__ __forceinline__ void st_tile(Tile &t, int row, int chunk, const uint4
 }
 
 // ---------------------------------------------------------------------------
-// Per-chunk decay bookkeeping.  Thread layout of the operand passes (128 threads):
-//   warp  = 2*blk + cch     blk: which 32-token block of the chunk, cch: upper/lower 4
-//                           of the 8 16-byte columns of a tile row
-//   lane  = 4*tgl + ccl     tgl: group of 4 consecutive tokens inside the block (0..7),
-//                           ccl: column inside the group of 4
-// so a thread owns tokens 32*blk + 4*tgl .. +3 of channels 8*(4*cch+ccl) .. +7.  With the
-// 128-byte swizzle every 8 consecutive lanes then touch 8 different 16-byte bank groups:
-// the tile loads and stores are free of bank conflicts.
+// Per-chunk decay bookkeeping.
 //
 // All decay arithmetic is done in the log2 domain (one ex2 per exponential, no
 // extra multiply): l2 = log2(decay) per token, c = running sum of l2 from the start
@@ -69,43 +62,13 @@ __device__ __forceinline__ float log2_decay(float x, int w_kind, bool &live) {
     return fmaxf(l2, L2_FLOOR);
 }
 
-template <int NCH>
-struct DecayT {
-    float w[4][NCH];   // decay of each of the thread's 4 tokens (1 past the segment end)
-    float cp0[NCH];    // log2-decay accumulated from the block start to before the thread's first token
-    float c3[NCH];     // ... up to and including its last token
-    float m[NCH];      // ... up to and including token 15 of the block (the block midpoint reference)
-    float e[NCH];      // the whole block
+struct Decay {           // of a thread's 4 tokens x 4 channels
+    float w[4][4];   // decay of each of the tokens (1 past the segment end)
+    float cp0[4];    // log2-decay accumulated from the block start to before the thread's first token
+    float c3[4];     // ... up to and including its last token
+    float m[4];      // ... up to and including token 15 of the block (the block midpoint reference)
+    float e[4];      // the whole block
 };
-using Decay = DecayT<8>;
-
-// In: l2[i][ch] per-token log2-decay.  Out: l2 holds the block-local inclusive sums c
-// (local scan + scan over the 8 threads that share a column, which sit 4 lanes apart).
-template <int NCH>
-__device__ __forceinline__ void decay_scan(float (&l2)[4][NCH], int lane, DecayT<NCH> &D) {
-    const int tgl = lane >> 2, ccl = lane & 3;
-#pragma unroll
-    for (int ch = 0; ch < NCH; ch++) {
-#pragma unroll
-        for (int i = 0; i < 4; i++) D.w[i][ch] = exp2f(l2[i][ch]);
-        const float first = l2[0][ch];
-#pragma unroll
-        for (int i = 1; i < 4; i++) l2[i][ch] += l2[i - 1][ch];
-        float tot = l2[3][ch];
-#pragma unroll
-        for (int off = 1; off < 8; off <<= 1) {
-            const float o = __shfl_up_sync(0xffffffffu, tot, 4 * off);
-            if (tgl >= off) tot += o;
-        }
-        const float excl = tot - l2[3][ch];
-#pragma unroll
-        for (int i = 0; i < 4; i++) l2[i][ch] += excl;
-        D.cp0[ch] = l2[0][ch] - first;
-        D.c3[ch] = l2[3][ch];
-        D.m[ch] = __shfl_sync(0xffffffffu, l2[3][ch], ccl + 12);   // tgl = 3: token 15 of the block
-        D.e[ch] = __shfl_sync(0xffffffffu, l2[3][ch], ccl + 28);   // tgl = 7: token 31
-    }
-}
 
 // Operand-pass layout for kernels with eight compute warps (256 threads):
 //   warp w owns tokens 8w .. 8w+7 of the chunk (so warps 0..3 are block 0, warps 4..7 block 1);
@@ -113,8 +76,8 @@ __device__ __forceinline__ void decay_scan(float (&l2)[4][NCH], int lane, DecayT
 // i.e. a thread owns 4 tokens x 4 channels and reads or writes 8 bytes of a tile row at a time.
 // The 16 lanes of a half-warp then cover one whole 128-byte row: free of bank conflicts.
 //
-// In: l2[i][ch] per-token log2-decay.  Out: l2 holds the block-local inclusive sums c; D as in
-// decay_scan; other_l2 = log2-decay total of the other block.  The totals of the eight warps go
+// In: l2[i][ch] per-token log2-decay.  Out: l2 holds the block-local inclusive sums c; D;
+// other_l2 = log2-decay total of the other block.  The totals of the eight warps go
 // through `wtot` ([8][CH] floats of shared memory); `sync(pred)` is the barrier of the 256 threads,
 // returning the OR of `pred` over them.
 //
@@ -124,48 +87,56 @@ __device__ __forceinline__ void decay_scan(float (&l2)[4][NCH], int lane, DecayT
 // blocks is not needed.
 constexpr float MILD_L2_PER_8 = -30.f;
 template <class Sync>
-__device__ __forceinline__ bool decay_scan8(float (&l2)[4][4], int warp, int lane, float *wtot, DecayT<4> &D,
+__device__ __forceinline__ bool decay_scan8(float (&l2)[4][4], int warp, int lane, float *wtot, Decay &D,
                                             float (&other_l2)[4], Sync sync) {
     const int r = lane >> 4, ch0 = (lane & 15) * 4, blk = warp >> 2, wb = warp & 3;
-    float tot[4], first[4];
+    float tot[4], first[4], o[4];
     bool steep = false;
 #pragma unroll
     for (int ch = 0; ch < 4; ch++) {
 #pragma unroll
         for (int i = 0; i < 4; i++) D.w[i][ch] = exp2f(l2[i][ch]);
         first[ch] = l2[0][ch];
-#pragma unroll
-        for (int i = 1; i < 4; i++) l2[i][ch] += l2[i - 1][ch];
-        const float o = __shfl_xor_sync(0xffffffffu, l2[3][ch], 16);
-        tot[ch] = l2[3][ch] + o;
-        steep |= tot[ch] < MILD_L2_PER_8;
-        if (r) {
-#pragma unroll
-            for (int i = 0; i < 4; i++) l2[i][ch] += o;
-        }
     }
+#pragma unroll
+    for (int i = 1; i < 4; i++) vadd<4>(l2[i], l2[i], l2[i - 1]);
+#pragma unroll
+    for (int ch = 0; ch < 4; ch++) o[ch] = __shfl_xor_sync(0xffffffffu, l2[3][ch], 16);
+    vadd<4>(tot, l2[3], o);
+#pragma unroll
+    for (int ch = 0; ch < 4; ch++) steep |= tot[ch] < MILD_L2_PER_8;
     if (r) *reinterpret_cast<float4 *>(wtot + warp * CH + ch0) = make_float4(tot[0], tot[1], tot[2], tot[3]);
     const bool mild = !sync(steep);
     const float *own = wtot + 4 * blk * CH + ch0, *oth = wtot + 4 * (blk ^ 1) * CH + ch0;
-    float base[4] = {0.f, 0.f, 0.f, 0.f}, m[4], e[4];
+    // what lies in the block before the thread's tokens: its warp's other half and the earlier warps
+    float base[4], m[4], e[4];
+#pragma unroll
+    for (int ch = 0; ch < 4; ch++) base[ch] = r ? o[ch] : 0.f;
 #pragma unroll
     for (int q = 0; q < 4; q++) {
         const float4 a4 = *reinterpret_cast<const float4 *>(own + q * CH);
         const float4 b4 = *reinterpret_cast<const float4 *>(oth + q * CH);
         const float a[4] = {a4.x, a4.y, a4.z, a4.w}, b[4] = {b4.x, b4.y, b4.z, b4.w};
+        if (q == 0) {
 #pragma unroll
-        for (int ch = 0; ch < 4; ch++) {
-            if (q == 0) { m[ch] = a[ch]; other_l2[ch] = b[ch]; }
-            else if (q == 1) { m[ch] += a[ch]; e[ch] = m[ch]; other_l2[ch] += b[ch]; }     // m: through token 15 of the block
-            else { e[ch] += a[ch]; other_l2[ch] += b[ch]; }                                // e: the whole block
-            if (wb > q) base[ch] += a[ch];
+            for (int ch = 0; ch < 4; ch++) { m[ch] = a[ch]; other_l2[ch] = b[ch]; }
+        } else {
+            vadd<4>(other_l2, other_l2, b);
+            if (q == 1) {                                    // m: through token 15 of the block
+                vadd<4>(m, m, a);
+#pragma unroll
+                for (int ch = 0; ch < 4; ch++) e[ch] = m[ch];
+            } else {                                         // e: the whole block
+                vadd<4>(e, e, a);
+            }
         }
+        if (wb > q) vadd<4>(base, base, a);
     }
 #pragma unroll
-    for (int ch = 0; ch < 4; ch++) {
+    for (int i = 0; i < 4; i++) vadd<4>(l2[i], l2[i], base);
+    vsub<4>(D.cp0, l2[0], first);
 #pragma unroll
-        for (int i = 0; i < 4; i++) l2[i][ch] += base[ch];
-        D.cp0[ch] = l2[0][ch] - first[ch];
+    for (int ch = 0; ch < 4; ch++) {
         D.c3[ch] = l2[3][ch];
         D.m[ch] = m[ch];
         D.e[ch] = e[ch];
@@ -177,7 +148,7 @@ __device__ __forceinline__ bool decay_scan8(float (&l2)[4][4], int warp, int lan
 // every token of channel ch decays by lw[ch] (log2), so nothing has to be scanned or exchanged.
 // w[ch] = 2^{lw[ch]}; tok0 = first of the thread's 4 tokens (0..63).
 __device__ __forceinline__ void decay_static(const float (&lw)[4], const float (&w)[4], int tok0, float (&l2)[4][4],
-                                             DecayT<4> &D, float (&other_l2)[4]) {
+                                             Decay &D, float (&other_l2)[4]) {
     const float t0 = (float)(tok0 & (HB - 1));
 #pragma unroll
     for (int ch = 0; ch < 4; ch++) {

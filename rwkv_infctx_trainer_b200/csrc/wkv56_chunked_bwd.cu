@@ -188,15 +188,17 @@ k_chunk_dscan(const __grid_constant__ CUtensorMap map_rh, const __grid_constant_
             if (!mbar_wait(&s.load_bar[st], load_parity(i), LIM)) { fail = 1; break; }
             // with D_{j+1} in hand: its checkpoint and E_{j+1} ...
             if (!summary) {
-                float dot[4] = {0.f, 0.f, 0.f, 0.f};
+                f2 dot[2] = {both(0.f), both(0.f)};
 #pragma unroll
                 for (int c8 = 0; c8 < 4; c8++) {
                     float sv[8];
                     unpack8(ld_tile(in[2], row, (vcol0 >> 3) + c8), sv);
 #pragma unroll
-                    for (int q = 0; q < 8; q++) dot[c8] += sv[q] * v[8 * c8 + q];
+                    for (int q = 0; q < 8; q += 2)
+                        dot[c8 & 1] = fma2(make_float2(sv[q], sv[q + 1]), make_float2(v[8 * c8 + q], v[8 * c8 + q + 1]), dot[c8 & 1]);
                 }
-                float e = (dot[0] + dot[1]) + (dot[2] + dot[3]);
+                dot[0] = add2(dot[0], dot[1]);
+                float e = dot[0].x + dot[0].y;
                 e += __shfl_xor_sync(0xffffffffu, e, 16);
                 if (active) P.e0[((size_t)bh * (N + 1) + (j + 1)) * 64 + row] = e;
             }
@@ -226,8 +228,7 @@ k_chunk_dscan(const __grid_constant__ CUtensorMap map_rh, const __grid_constant_
                 tmem_ld_wait();
                 const float d = s.dvec[st][row];
                 dprod *= d;
-#pragma unroll
-                for (int q = 0; q < 32; q++) v[q] = fmaf(d, v[q], u[q]);
+                vaxpy<32>(v, d, v, u);
             }
             // this warp is done with the product buffer and with the stage
             tc_fence_before();
@@ -338,6 +339,11 @@ __device__ __forceinline__ float halving_sum8(const float *v, int l16) {
 // reaches token 31.  (Walking group 1 backward from the chunk-end constant would need no offset,
 // but that constant comes from a separately rounded bf16 state and the small residuals of
 // strongly decaying channels do not survive the mismatch.)
+//
+// What bounds it is the issue of CUDA-core instructions (two CTAs, four warps per scheduler), so the arithmetic is done on
+// channel pairs by packed fp32 instructions and the token scan of the decay gradient owns channel pairs too (one
+// load, store or conversion for two channels, tile addresses constants of the unrolled loop): 4 rows of 4096 tokens x
+// 64 heads 660 -> 608 us.
 //
 // The body is compiled twice.  MILD_ONLY = true: the chunk is known to be mild (the forward kernel
 // said so), every cross-block code path is left out -- a smaller, leaner kernel (96 instead of 125
@@ -459,7 +465,7 @@ bwd_chunk(const CUtensorMap &map_r, const CUtensorMap &map_k, const CUtensorMap 
     bool mild = false;
     {
         float c[4][4];
-        DecayT<4> D;
+        Decay D;
         unsigned livebits[4];
         // the warps' decay totals are exchanged through the first bytes of the A~ tile (unused until the mask pass)
         float *wtot = reinterpret_cast<float *>(s.atil.b);
@@ -506,18 +512,21 @@ bwd_chunk(const CUtensorMap &map_r, const CUtensorMap &map_k, const CUtensorMap 
             // (the barrier inside: every w value has been read, so its slot may take the table)
             mild = decay_scan8(c, warp, lane, wtot, D, other_l2, [](bool p) { return __syncthreads_or(p) != 0; });
         }
+        float before[4];      // log2-decay of the block before the thread's own
 #pragma unroll
-        for (int ch = 0; ch < 4; ch++) other[ch] = exp2f(other_l2[ch]);
+        for (int ch = 0; ch < 4; ch++) {
+            other[ch] = exp2f(other_l2[ch]);
+            before[ch] = pblk ? other_l2[ch] : 0.f;
+        }
 #pragma unroll
         for (int i = 0; i < 4; i++) {
             const int t = ptok0 + i;
-            float cv[4];      // cumulative log2-decay counted from the chunk start; its lowest mantissa
+            float cabs[4], cv[4];      // cumulative log2-decay counted from the chunk start; its lowest mantissa
                               // bit is replaced by the "decay above the floor" flag of the token
+            vadd<4>(cabs, c[i], before);
 #pragma unroll
-            for (int ch = 0; ch < 4; ch++) {
-                const float cabs = pblk ? c[i][ch] + other_l2[ch] : c[i][ch];
-                cv[ch] = __uint_as_float((__float_as_uint(cabs) & ~1u) | ((livebits[i] >> ch) & 1u));
-            }
+            for (int ch = 0; ch < 4; ch++)
+                cv[ch] = __uint_as_float((__float_as_uint(cabs[ch]) & ~1u) | ((livebits[i] >> ch) & 1u));
             *ctab_ptr4(s.in[T_W], s.ctab_hi, t, ch0 >> 2) = make_float4(cv[0], cv[1], cv[2], cv[3]);
         }
         // r-side operands, walking forward:  fa = 2^{cp - m};  block 1 also x = r 2^{cp}  (block-local cp)
@@ -533,11 +542,8 @@ bwd_chunk(const CUtensorMap &map_r, const CUtensorMap &map_k, const CUtensorMap 
             const int t = ptok0 + i;
             float r[4], rt[4], xx[4];
             unpack4(ld_tile4(s.in[T_R], t, pcc, phf), r);
-#pragma unroll
-            for (int ch = 0; ch < 4; ch++) {
-                rt[ch] = r[ch] * fa[ch];
-                fa[ch] *= D.w[i][ch];
-            }
+            vmul<4>(rt, r, fa);
+            vmul<4>(fa, fa, D.w[i]);
             st_tile4(s.rt, t, pcc, phf, pack4(rt));
             if (pblk && !mild) {
 #pragma unroll
@@ -564,12 +570,9 @@ bwd_chunk(const CUtensorMap &map_r, const CUtensorMap &map_k, const CUtensorMap 
                 const int t = ptok0 + i;
                 float k[4], kt[4], kh[4];
                 unpack4(ld_tile4(s.in[T_K], t, pcc, phf), k);
-#pragma unroll
-                for (int ch = 0; ch < 4; ch++) {
-                    kt[ch] = k[ch] * fa[ch];
-                    kh[ch] = kt[ch] * ck[ch];
-                    fa[ch] *= D.w[i][ch];
-                }
+                vmul<4>(kt, k, fa);
+                vmul<4>(kh, kt, ck);
+                vmul<4>(fa, fa, D.w[i]);
                 st_tile4(s.kt, t, pcc, phf, pack4(kt));
                 st_tile4(s.khat, t, pcc, phf, pack4(kh));
             }
@@ -627,6 +630,7 @@ bwd_chunk(const CUtensorMap &map_r, const CUtensorMap &map_k, const CUtensorMap 
     const bool diag_warp = (w4 >= 2) == (wg == 1), cross_warp = wg == 0 && w4 >= 2;
     float diag = 0.f;
     if (diag_warp) {
+        f2 d2 = both(0.f);
 #pragma unroll
         for (int c = 0; c < 4; c++) {
             const int c8 = (lo ? 0 : 4) + c;
@@ -638,8 +642,10 @@ bwd_chunk(const CUtensorMap &map_r, const CUtensorMap &map_k, const CUtensorMap 
                 uq[0] = u0.x; uq[1] = u0.y; uq[2] = u0.z; uq[3] = u0.w; uq[4] = u1.x; uq[5] = u1.y; uq[6] = u1.z; uq[7] = u1.w;
             }
 #pragma unroll
-            for (int q = 0; q < 8; q++) diag += a[q] * uq[q] * d[q];
+            for (int q = 0; q < 8; q += 2)
+                d2 = fma2(mul2(make_float2(a[q], a[q + 1]), make_float2(uq[q], uq[q + 1])), make_float2(d[q], d[q + 1]), d2);
         }
+        diag = d2.x + d2.y;
         diag += __shfl_xor_sync(0xffffffffu, diag, 16);
     }
     if (!abort1 && !(mbar_wait(&s.bar_early, 0, LIM) && mbar_wait(&s.bar_score, 0, LIM))) fail = 1;
@@ -773,11 +779,12 @@ bwd_chunk(const CUtensorMap &map_r, const CUtensorMap &map_k, const CUtensorMap 
     const int t = row, hh = lane >> 4, l16 = lane & 15;
     const float ptt_t = s.ptt[t];
     const bool tvalid = j * CH + t < P.T;
-    // [4][64] totals of the token scan, and [4][64] partial sums for gu / the static gw.  General build:
-    // per warp, in the v tile.  Mild-only build: per quarter of the chunk's tokens, in the A~ tile (free
-    // once gv is done; the v tile holds part of the a/b exchange there).
+    // [NPART][64] totals of the token scan, and as many partial sums for gu / the static gw.  General build: per 16
+    // tokens, in the v tile.  Mild-only build: per 8 tokens, in the A~ tile (free once gv is done; the v tile
+    // holds part of the a/b exchange there).
+    constexpr int NPART = MILD_ONLY ? 8 : 4;
     float *wtot = reinterpret_cast<float *>(MILD_ONLY ? s.atil.b : s.in[T_V].b);
-    float *gup = wtot + 4 * CH, *gwp = gup + 4 * CH;
+    float *gup = wtot + NPART * CH, *gwp = gup + NPART * CH;
     float keep[16];   // (general build) group 0: a_t of its first 16 channels; group 1: b_t of its last 16 channels
 
     // decay-gradient constant sum_v S[k,v] D[k,v] at the chunk start (consumed after two more barriers)
@@ -828,25 +835,35 @@ bwd_chunk(const CUtensorMap &map_r, const CUtensorMap &map_k, const CUtensorMap 
             }
             tmem_ld_wait();
             float out[8], ab[8], gue[8];
+            {
+                float f1[8], fS[8], sgs[8];
+                if (GR) vsub<8>(f1, z, mb); else vsub<8>(f1, mb, z);
+                if (!GR) vsub<8>(fS, e1r, z);
+#pragma unroll
+                for (int q = 0; q < 8; q++) {
+                    f1[q] = exp2f(f1[q]);
+                    fS[q] = exp2f(GR ? z[q] : fS[q]);
+                }
+                vmul<8>(sgs, fS, gs);
+                vfma<8>(out, f1, g1, sgs);
+                vmul<8>(ab, raw, sgs);
+                vfma<8>(ab, own, g1, ab);
+                vmul<8>(uu, uu, oth);
+                vaxpy<8>(out, ptt_t, uu, out);
+            }
 #pragma unroll
             for (int q = 0; q < 8; q++) {
-                const float f1 = GR ? exp2f(z[q] - mb[q]) : exp2f(mb[q] - z[q]);
-                const float fS = GR ? exp2f(z[q]) : exp2f(e1r[q] - z[q]);
-                const float sgs = fS * gs[q];
-                float o = f1 * g1[q] + sgs + ptt_t * uu[q] * oth[q];
-                float qq = own[q] * g1[q] + raw[q] * sgs;
                 if (has2) {
                     const float f3 = GR ? exp2f(z[q] - e0r[q]) : exp2f(e0r[q] - z[q]);
-                    o += f3 * g2[q];
-                    qq += xx[q] * g2[q];
+                    out[q] += f3 * g2[q];
+                    ab[q] += xx[q] * g2[q];
                 }
-                out[q] = o;
-                ab[q] = GR ? -qq : qq;
+                if (GR && !MILD_ONLY) ab[q] = -ab[q];
                 if (!GR && !MILD_ONLY) gue[q] = ptt_t * raw[q] * oth[q];
             }
             st_tile(o_main, t, c8, pack8(out));
             if constexpr (MILD_ONLY) {
-                // a_t (gr side) / b_t (gk side) of the lane half's 32 channels: one fp32 row of a tile of
+                // -a_t (gr side) / b_t (gk side) of the lane half's 32 channels: one fp32 row of a tile of
                 // their own (a: S and P~ tiles, b: v and x tiles -- all consumed by now), read back
                 // channel-major by the token scan below
                 Tile &dstt = GR ? (hh ? s.ptil : s.in[T_S]) : (hh ? s.x : s.in[T_V]);
@@ -881,65 +898,69 @@ bwd_chunk(const CUtensorMap &map_r, const CUtensorMap &map_k, const CUtensorMap 
     } else {
         if (wg == 0) side_pass(std::true_type{}, std::false_type{}); else side_pass(std::false_type{}, std::false_type{});
     }
-    if (wg == 0) {
-        // gv: accumulator [s, v]
+    {
+        // gv: accumulator [s, v]; each group takes half of the columns
         if (!abort2 && !mbar_wait(&s.bar_gv, 0, LIM)) fail = 1;
         tc_fence_after();
-        float gv[32];
-        tmem_ld16(tmem_addr(tm, lane_base, C_GV), gv);
-        tmem_ld16(tmem_addr(tm, lane_base, C_GV + 16), gv + 16);
+        float gv[16];
+        tmem_ld16(tmem_addr(tm, lane_base, C_GV + 16 * wg), gv);
         tmem_ld_wait();
 #pragma unroll
-        for (int c8 = 0; c8 < 4; c8++) st_tile(o_gv, t, 4 * hh + c8, pack8(gv + 8 * c8));
+        for (int c8 = 0; c8 < 2; c8++) st_tile(o_gv, t, 4 * hh + 2 * wg + c8, pack8(gv + 8 * c8));
     }
     __syncthreads();
     if constexpr (MILD_ONLY) {
-        // Token scan, channel-major: thread = one channel c and one quarter q4 of the chunk's tokens.
-        // a and b of its 16 tokens come from the exchange tiles (a warp reads 32 consecutive floats of
-        // a row: no bank conflict); the exclusive prefix of z = a + b is a serial sum in registers, the
-        // quarters meet through `wtot`.  gu's partial sum p_tt r k rides along.
-        const int c = tid & 63, q4 = tid >> 6, cl = c & 31;
-        const Tile &ta = (c & 32) ? s.ptil : s.in[T_S], &tb = (c & 32) ? s.x : s.in[T_V];
-        float av[16], pre[16];
-        float run = 0.f, gus = 0.f;
-#pragma unroll
-        for (int i = 0; i < 16; i++) {
-            const int tt = 16 * q4 + i;
-            const uint32_t off = tile_off(tt, cl >> 2) + (cl & 3) * 4;
-            const float a = *reinterpret_cast<const float *>(ta.b + off);
-            const float b = *reinterpret_cast<const float *>(tb.b + off);
-            av[i] = a;
-            pre[i] = run;
-            run += a + b;
-            const uint32_t boff = tile_off(tt, c >> 3) + (c & 7) * 2;
-            const float rr = __bfloat162float(*reinterpret_cast<const __nv_bfloat16 *>(s.in[T_R].b + boff));
-            const float kk = __bfloat162float(*reinterpret_cast<const __nv_bfloat16 *>(s.in[T_K].b + boff));
-            gus = fmaf(s.ptt[tt] * rr, kk, gus);
+        // Token scan, channel-major: lane = two adjacent channels, warp = 8 consecutive tokens (so that a tile row's
+        // swizzle is a constant of the unrolled loop, and every load, store and packed instruction serves two
+        // channels).  -a and b come from the exchange tiles (a half-warp reads 128 consecutive bytes of a row: no
+        // bank conflict); the exclusive prefix of z = a + b is a serial sum in registers, the warps meet through
+        // `wtot`.  gu's partial sum p_tt r k rides along.
+        const int t8 = 8 * warp, l16b = lane & 15;
+        const unsigned char *pa = (lane & 16 ? s.ptil : s.in[T_S]).b + t8 * 128 + (l16b & 1) * 8,
+                            *pb = (lane & 16 ? s.x : s.in[T_V]).b + t8 * 128 + (l16b & 1) * 8;
+        const unsigned rowoff = t8 * 128 + (lane & 3) * 4;       // bf16 tiles: 16-byte column lane >> 2
+        float pt[8];
+        {
+            const float4 p0 = *reinterpret_cast<const float4 *>(s.ptt + t8), p1 = *reinterpret_cast<const float4 *>(s.ptt + t8 + 4);
+            pt[0] = p0.x; pt[1] = p0.y; pt[2] = p0.z; pt[3] = p0.w; pt[4] = p1.x; pt[5] = p1.y; pt[6] = p1.z; pt[7] = p1.w;
         }
-        wtot[q4 * CH + c] = run;
-        gup[q4 * CH + c] = gus;
+        f2 glw[8], run = both(0.f), gus = both(0.f);
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+            const int o32 = i * 128 + (((l16b >> 1) ^ i) << 4), o16 = i * 128 + (((lane >> 2) ^ i) << 4);
+            const f2 na = *reinterpret_cast<const f2 *>(pa + o32), bb = *reinterpret_cast<const f2 *>(pb + o32);
+            glw[i] = sub2(run, na);
+            run = add2(run, sub2(bb, na));
+            const uint32_t r2 = *reinterpret_cast<const uint32_t *>(s.in[T_R].b + rowoff + o16),
+                           k2 = *reinterpret_cast<const uint32_t *>(s.in[T_K].b + rowoff + o16);
+            const f2 rr = make_float2(__uint_as_float(r2 << 16), __uint_as_float(r2 & 0xFFFF0000u)),
+                     kk = make_float2(__uint_as_float(k2 << 16), __uint_as_float(k2 & 0xFFFF0000u));
+            gus = fma2(mul2(both(pt[i]), rr), kk, gus);
+        }
+        *reinterpret_cast<f2 *>(wtot + warp * CH + 2 * lane) = run;
+        *reinterpret_cast<f2 *>(gup + warp * CH + 2 * lane) = gus;
         __syncthreads();
-        float base = s.kb[c];      // the constant of the chunk start plus the earlier quarters' totals
-        for (int w = 0; w < q4; w++) base += wtot[w * CH + c];
+        f2 base = *reinterpret_cast<const f2 *>(s.kb + 2 * lane);      // the constant of the chunk start plus the earlier warps' totals
+        for (int w = 0; w < warp; w++) base = add2(base, *reinterpret_cast<const f2 *>(wtot + w * CH + 2 * lane));
         if (PER_TOKEN) {
             // times the floored log-decay of the token, zero where the floor was hit (no gradient)
-            auto ctab1 = [&](int tt) { return reinterpret_cast<const float *>(ctab_ptr4(ct_lo, ct_hi, tt, c >> 2))[c & 3]; };
-            float cprev = q4 ? ctab1(16 * q4 - 1) : 0.f;
+            const unsigned char *pc = (warp < 4 ? ct_lo : ct_hi).b + (t8 & 31) * 256 + (lane & 1) * 8;
+            f2 cprev = warp ? *reinterpret_cast<const f2 *>(reinterpret_cast<const float *>(ctab_ptr4(ct_lo, ct_hi, t8 - 1, lane >> 1)) + 2 * (lane & 1))
+                            : both(0.f);
 #pragma unroll
-            for (int i = 0; i < 16; i++) {
-                const int tt = 16 * q4 + i;
-                const float cc = ctab1(tt);
-                const float glw = base + pre[i] + av[i];
-                const float o = (__float_as_uint(cc) & 1u) ? glw * (cc - cprev) * LN2 : 0.f;
+            for (int i = 0; i < 8; i++) {
+                const f2 cc = *reinterpret_cast<const f2 *>(pc + i * 256 + (((lane >> 1) ^ i) << 4));
+                const f2 o = mul2(mul2(add2(base, glw[i]), both(LN2)), sub2(cc, cprev));
                 cprev = cc;
-                *reinterpret_cast<__nv_bfloat16 *>(o_gw.b + tile_off(tt, c >> 3) + (c & 7) * 2) = __float2bfloat16_rn(o);
+                *reinterpret_cast<uint32_t *>(o_gw.b + rowoff + i * 128 + (((lane >> 2) ^ i) << 4)) =
+                    pack2((__float_as_uint(cc.x) & 1u) ? o.x : 0.f, (__float_as_uint(cc.y) & 1u) ? o.y : 0.f);
             }
         } else {
-            float tot = 0.f;
+            f2 tot = both(0.f);
 #pragma unroll
-            for (int i = 0; i < 16; i++)
-                if (j * CH + 16 * q4 + i < P.T) tot += base + pre[i] + av[i];
-            gwp[q4 * CH + c] = tot;
+            for (int i = 0; i < 8; i++)
+                if (j * CH + t8 + i < P.T) tot = add2(tot, add2(base, glw[i]));
+            *reinterpret_cast<f2 *>(gwp + warp * CH + 2 * lane) = tot;
         }
     } else {
         // the token scan of z = a + b for this thread's 16 channels: 32*hh + 16*wg .. +15
@@ -1033,12 +1054,17 @@ bwd_chunk(const CUtensorMap &map_r, const CUtensorMap &map_k, const CUtensorMap 
     // per-chunk partials, folded later in a fixed order
     if (tid >= 64 && tid < 128) {
         const int k = tid - 64;
-        P.gu_part[((size_t)bh * n + j) * 64 + k] = gup[k] + gup[CH + k] + gup[2 * CH + k] + gup[3 * CH + k];
+        float tot = gup[k];
+#pragma unroll
+        for (int q = 1; q < NPART; q++) tot += gup[q * CH + k];
+        P.gu_part[((size_t)bh * n + j) * 64 + k] = tot;
     } else if (!PER_TOKEN && tid >= 128 && tid < 192) {
         const int k = tid - 128;
         bool live;
         const float lw = log2_decay(P.wvec[h * 64 + k], P.w_kind, live) * LN2;
-        const float tot = gwp[k] + gwp[CH + k] + gwp[2 * CH + k] + gwp[3 * CH + k];
+        float tot = gwp[k];
+#pragma unroll
+        for (int q = 1; q < NPART; q++) tot += gwp[q * CH + k];
         P.gw_part[((size_t)bh * n + j) * 64 + k] = live ? tot * lw : 0.f;
     }
     if (!abort3 && tid == 0) tma_store_wait_read();   // the tiles must outlive the reads of the bulk stores

@@ -25,6 +25,71 @@ template <> struct Elem<__half> {
     static __device__ __forceinline__ void st(__half *p, float x) { *p = __float2half_rn(x); }
 };
 
+// Two fp32 values per instruction (fma.f32x2): half the issue slots of the scalar forms, same rounding.
+typedef float2 f2;
+__device__ __forceinline__ unsigned long long bits(const f2 &a) { return *reinterpret_cast<const unsigned long long *>(&a); }
+__device__ __forceinline__ f2 from_bits(unsigned long long v) { return *reinterpret_cast<f2 *>(&v); }
+__device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c) {
+    unsigned long long r;
+    asm("fma.rn.ftz.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(bits(a)), "l"(bits(b)), "l"(bits(c)));
+    return from_bits(r);
+}
+__device__ __forceinline__ f2 mul2(f2 a, f2 b) {
+    unsigned long long r;
+    asm("mul.rn.ftz.f32x2 %0, %1, %2;" : "=l"(r) : "l"(bits(a)), "l"(bits(b)));
+    return from_bits(r);
+}
+__device__ __forceinline__ f2 add2(f2 a, f2 b) {
+    unsigned long long r;
+    asm("add.rn.ftz.f32x2 %0, %1, %2;" : "=l"(r) : "l"(bits(a)), "l"(bits(b)));
+    return from_bits(r);
+}
+__device__ __forceinline__ f2 both(float x) { return make_float2(x, x); }
+__device__ __forceinline__ f2 sub2(f2 a, f2 b) { return fma2(b, both(-1.f), a); }
+__device__ __forceinline__ f2 neg2(f2 a) { return make_float2(-a.x, -a.y); }
+// the same on arrays, N even
+template <int N>
+__device__ __forceinline__ void vmul(float *o, const float *a, const float *b) {
+#pragma unroll
+    for (int i = 0; i < N; i += 2) {
+        const f2 r = mul2(make_float2(a[i], a[i + 1]), make_float2(b[i], b[i + 1]));
+        o[i] = r.x; o[i + 1] = r.y;
+    }
+}
+template <int N>
+__device__ __forceinline__ void vadd(float *o, const float *a, const float *b) {
+#pragma unroll
+    for (int i = 0; i < N; i += 2) {
+        const f2 r = add2(make_float2(a[i], a[i + 1]), make_float2(b[i], b[i + 1]));
+        o[i] = r.x; o[i + 1] = r.y;
+    }
+}
+template <int N>
+__device__ __forceinline__ void vsub(float *o, const float *a, const float *b) {
+#pragma unroll
+    for (int i = 0; i < N; i += 2) {
+        const f2 r = sub2(make_float2(a[i], a[i + 1]), make_float2(b[i], b[i + 1]));
+        o[i] = r.x; o[i + 1] = r.y;
+    }
+}
+template <int N>
+__device__ __forceinline__ void vfma(float *o, const float *a, const float *b, const float *c) {
+#pragma unroll
+    for (int i = 0; i < N; i += 2) {
+        const f2 r = fma2(make_float2(a[i], a[i + 1]), make_float2(b[i], b[i + 1]), make_float2(c[i], c[i + 1]));
+        o[i] = r.x; o[i + 1] = r.y;
+    }
+}
+// o = s * a + c
+template <int N>
+__device__ __forceinline__ void vaxpy(float *o, float s, const float *a, const float *c) {
+#pragma unroll
+    for (int i = 0; i < N; i += 2) {
+        const f2 r = fma2(both(s), make_float2(a[i], a[i + 1]), make_float2(c[i], c[i + 1]));
+        o[i] = r.x; o[i + 1] = r.y;
+    }
+}
+
 inline bool aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
 inline int launch_status() { return cudaGetLastError() == cudaSuccess ? WKV_OK : WKV_ERR_LAUNCH; }
