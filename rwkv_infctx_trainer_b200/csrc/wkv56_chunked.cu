@@ -182,7 +182,7 @@ k_chunk_fwd(const __grid_constant__ CUtensorMap map_r, const __grid_constant__ C
                                d_kh = make_desc(smem_u32(&s.khat[st]));
                 if (!mbar_wait_or_abort(&s.ops_bar[c & 1], (uint32_t)((c >> 1) & 1), &s.abort_flag, P.wait_limit)) { fail = 1; break; }
                 tc_fence_after();
-                // the per-chunk backward kernel comes in two builds: tell it which one this chunk needs
+                // the per-chunk backward kernel comes in two bodies: tell it which one this chunk needs
                 // (written from here: this lane has time, the compute warps do not)
                 if (P.dchunk)
                     P.mildflag[bh * P.nchunk + j0 + c] = *reinterpret_cast<volatile int *>(&s.mild_flag[c & 1]) != 0;

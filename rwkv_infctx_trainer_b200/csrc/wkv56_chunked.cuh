@@ -182,7 +182,7 @@ __device__ __forceinline__ void st_tile4(Tile &t, int row, int chunk, int half, 
 //   sck     bf16 [B*H, nchunk+1, 64, 64]  state at the start of every chunk (key rows, value columns)
 //   rhat    bf16 [B, T, C]                r_t * (decay accumulated from the chunk start to before t)
 //   dchunk  fp32 [B*H, nchunk, 64]        decay of each whole chunk per key channel
-//   mild    u8   [B*H * nchunk]           1 = the chunk is mild (see decay_scan8), 0 = steep: which build of
+//   mild    u8   [B*H * nchunk]           1 = the chunk is mild (see decay_scan8), 0 = steep: which body of
 //                                         the per-chunk backward kernel the chunk needs
 struct CkptLayout {
     size_t sck, rhat, dchunk, mild, total;

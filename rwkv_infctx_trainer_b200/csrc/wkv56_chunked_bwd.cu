@@ -270,7 +270,7 @@ struct BwdSmem {
     uint64_t bar_grad;         // phase 2 except gv
     uint64_t bar_gv;           // gv
     uint32_t tmem_base;
-    int not_mine;              // mild-only build: the chunk turned out to be a steep one
+    int is_mild;               // which of the two bodies the chunk takes
 };
 
 static_assert(sizeof(BwdSmem) <= 115712, "two CTAs per SM need <= 113 KiB each");
@@ -345,79 +345,23 @@ __device__ __forceinline__ float halving_sum8(const float *v, int l16) {
 // load, store or conversion for two channels, tile addresses constants of the unrolled loop): 4 rows of 4096 tokens x
 // 64 heads 660 -> 608 us.
 //
-// The body is compiled twice.  MILD_ONLY = true: the chunk is known to be mild (the forward kernel
-// said so), every cross-block code path is left out -- a smaller, leaner kernel (96 instead of 125
-// registers) that serves every chunk of ordinary data.  MILD_ONLY = false: the general body, run
-// only for the chunks the forward kernel listed as steep.
+// The body is compiled twice, and a CTA takes one of the two by the flag the forward kernel left for its chunk.
+// MILD_ONLY = true: the chunk is known to be mild, every cross-block code path is left out (all chunks of ordinary
+// data).  MILD_ONLY = false: the general body.  (Both stay within the 128 registers that two CTAs per SM leave; a
+// kernel of its own for the steep chunks cost every call a launch that usually found none.)
 template <bool PER_TOKEN, bool MILD_ONLY>
 __device__ __forceinline__ void
-bwd_chunk(const CUtensorMap &map_r, const CUtensorMap &map_k, const CUtensorMap &map_v, const CUtensorMap &map_w,
-          const CUtensorMap &map_gy, const CUtensorMap &map_s, const CUtensorMap &map_d, const CUtensorMap &map_gr,
-          const CUtensorMap &map_gk, const CUtensorMap &map_gv, const CUtensorMap &map_gw, const BwdParams &P,
-          const int chunk_id) {
-    extern __shared__ __align__(1024) unsigned char smem_raw[];
-    BwdSmem &s = *reinterpret_cast<BwdSmem *>(smem_raw);
+bwd_chunk(const CUtensorMap &map_gr, const CUtensorMap &map_gk, const CUtensorMap &map_gv, const CUtensorMap &map_gw,
+          const BwdParams &P, BwdSmem &s, const uint32_t tm, const int warp) {
     const int tid = threadIdx.x, lane = tid & 31;
-    const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);   // tells the compiler it is uniform across the warp
     const int wg = warp >> 2, w4 = warp & 3;
-    const int n = P.nchunk;
+    const int n = P.nchunk, chunk_id = (int)blockIdx.x;
     const int bh = chunk_id / n, j = chunk_id % n, b = bh / P.H, h = bh % P.H;
     const bool lo = (lane & 16) == 0;
     const int row = w4 * 16 + (lane & 15);   // accumulator row owned (token in phase 1, channel in phase 2)
     const uint32_t lane_base = (uint32_t)(w4 * 32);
-
-    // the swizzled tiles need a 1024-byte aligned base; refuse to run otherwise
-    if ((smem_u32(smem_raw) & 1023u) != 0) {
-        if (tid == 0 && P.status) atomicOr(P.status, 8);
-        return;
-    }
     const uint32_t LIM = P.wait_limit;
-    if (tid == 0) {
-        mbar_init(&s.load_bar, 1);
-        // lane 0 of every warp commits to every barrier, whether or not it issued a share of the group
-        mbar_init(&s.bar_early, 8); mbar_init(&s.bar_score, 8); mbar_init(&s.bar_grad, 8); mbar_init(&s.bar_gv, 8);
-        fence_mbar_init();
-        if (j != P.skip_load) {
-            mbar_expect_tx(&s.load_bar, (PER_TOKEN ? 7 : 6) * TILE_BYTES);
-            tma_load_3d(&s.in[T_R], &map_r, &s.load_bar, h * 64, j * CH, b);
-            tma_load_3d(&s.in[T_K], &map_k, &s.load_bar, h * 64, j * CH, b);
-            tma_load_3d(&s.in[T_V], &map_v, &s.load_bar, h * 64, j * CH, b);
-            if (PER_TOKEN) tma_load_3d(&s.in[T_W], &map_w, &s.load_bar, h * 64, j * CH, b);
-            tma_load_3d(&s.in[T_GY], &map_gy, &s.load_bar, h * 64, j * CH, b);
-            tma_load_3d(&s.in[T_S], &map_s, &s.load_bar, 0, 0, bh * (n + 1) + j);
-            tma_load_3d(&s.in[T_D], &map_d, &s.load_bar, 0, 0, bh * (n + 1) + j + 1);
-        }
-    }
-    if (MILD_ONLY && tid == 32) {
-        // the CTA that will take this one's place on the SM finds its tiles in L2
-        const int nb = chunk_id + P.prefetch_dist;
-        if (nb < (int)gridDim.x) {
-            const int bh2 = nb / n, j2 = nb % n, b2 = bh2 / P.H, h2 = bh2 % P.H;
-            tma_prefetch_l2_3d(&map_r, h2 * 64, j2 * CH, b2);
-            tma_prefetch_l2_3d(&map_k, h2 * 64, j2 * CH, b2);
-            tma_prefetch_l2_3d(&map_v, h2 * 64, j2 * CH, b2);
-            if (PER_TOKEN) tma_prefetch_l2_3d(&map_w, h2 * 64, j2 * CH, b2);
-            tma_prefetch_l2_3d(&map_gy, h2 * 64, j2 * CH, b2);
-            tma_prefetch_l2_3d(&map_s, 0, 0, bh2 * (n + 1) + j2);
-            tma_prefetch_l2_3d(&map_d, 0, 0, bh2 * (n + 1) + j2 + 1);
-        }
-    }
-    // (the flag is read while the loads are in flight: asking first would put a DRAM round trip in front of them)
-    if (MILD_ONLY && tid == 64) s.not_mine = P.mildflag[chunk_id] == 0;
-    if (tid >= 128 && tid < 128 + CH) s.uf[tid - 128] = __bfloat162float(P.u[h * 64 + tid - 128]);
-    if (warp == 0) { tmem_alloc(&s.tmem_base, BWD_TMEM_COLS); tmem_relinquish(); }
-    tc_fence_before();
-    __syncthreads();
-    tc_fence_after();
-    const uint32_t tm = s.tmem_base;
     const uint32_t tm_lo = tm, tm_hi = tm + (16u << 16);
-    if (MILD_ONLY && s.not_mine) {
-        // a steep chunk: the other kernel computes it.  Let this CTA's loads land, give the tensor memory back.
-        if (tid == 0 && chunk_id % P.nchunk != P.skip_load) mbar_wait(&s.load_bar, 0, LIM);
-        __syncthreads();
-        if (warp == 0) tmem_dealloc(tm, BWD_TMEM_COLS);
-        return;
-    }
 
     // operand-pass coordinates (see decay_scan8): 4 tokens x 4 channels per thread, a half-warp per tile row
     const int pblk = warp >> 2, pcc = (lane & 15) >> 1, phf = lane & 1, ptok0 = 8 * warp + 4 * (lane >> 4);
@@ -1073,8 +1017,6 @@ bwd_chunk(const CUtensorMap &map_r, const CUtensorMap &map_k, const CUtensorMap 
         mbar_wait(&s.bar_early, 0); mbar_wait(&s.bar_score, 0); mbar_wait(&s.bar_grad, 0); mbar_wait(&s.bar_gv, 0);
         if (P.status) atomicOr(P.status, 4);
     }
-    __syncthreads();
-    if (warp == 0) tmem_dealloc(tm, BWD_TMEM_COLS);
 }
 
 #define BWD_MAPS                                                                                              \
@@ -1084,38 +1026,67 @@ bwd_chunk(const CUtensorMap &map_r, const CUtensorMap &map_k, const CUtensorMap 
         const __grid_constant__ CUtensorMap map_d, const __grid_constant__ CUtensorMap map_gr,               \
         const __grid_constant__ CUtensorMap map_gk, const __grid_constant__ CUtensorMap map_gv,              \
         const __grid_constant__ CUtensorMap map_gw
-#define BWD_MAP_ARGS map_r, map_k, map_v, map_w, map_gy, map_s, map_d, map_gr, map_gk, map_gv, map_gw
 
-// one CTA per (batch, head, chunk); CTAs of steep chunks leave early (the other kernel has them)
+// one CTA per (batch, head, chunk)
 template <bool PER_TOKEN>
 __global__ void __launch_bounds__(256, 2) k_chunk_bwd(BWD_MAPS, const BwdParams P) {
     pdl_wait();
     pdl_trigger();
-    bwd_chunk<PER_TOKEN, true>(BWD_MAP_ARGS, P, (int)blockIdx.x);
-}
+    extern __shared__ __align__(1024) unsigned char smem_raw[];
+    BwdSmem &s = *reinterpret_cast<BwdSmem *>(smem_raw);
+    const int tid = threadIdx.x, lane = tid & 31;
+    const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);   // tells the compiler it is uniform across the warp
+    const int n = P.nchunk, chunk_id = (int)blockIdx.x;
+    const int bh = chunk_id / n, j = chunk_id % n, b = bh / P.H, h = bh % P.H;
 
-// A fixed, small grid that looks through the mild flags for steep chunks (usually there is none and
-// every CTA leaves after one load) and runs the general body on them.  CTA c looks at chunks
-// c, c + grid, c + 2 grid, ...: 256 of them per round, one flag per thread.
-// One CTA per SM: the general body inside a loop wants more than the 128 registers two CTAs leave.
-template <bool PER_TOKEN>
-__global__ void __launch_bounds__(256, 1) k_chunk_bwd_steep(BWD_MAPS, const BwdParams P, const int total) {
-    pdl_wait();
-    pdl_trigger();
-    __shared__ unsigned char is_steep[256];
-    for (int base = blockIdx.x; base < total; base += 256 * gridDim.x) {
-        const int mine = base + threadIdx.x * gridDim.x;
-        const bool steep = mine < total && P.mildflag[mine] == 0;
-        is_steep[threadIdx.x] = steep ? 1 : 0;
-        if (!__syncthreads_or(steep)) continue;
-        for (int t = 0; t < 256; t++) {
-            if (is_steep[t]) {      // (the same for every thread of the CTA)
-                bwd_chunk<PER_TOKEN, false>(BWD_MAP_ARGS, P, base + t * gridDim.x);
-                __syncthreads();    // the barriers and the tensor memory of this chunk are done with
-            }
-        }
-        __syncthreads();
+    // the swizzled tiles need a 1024-byte aligned base; refuse to run otherwise
+    if ((smem_u32(smem_raw) & 1023u) != 0) {
+        if (tid == 0 && P.status) atomicOr(P.status, 8);
+        return;
     }
+    if (tid == 0) {
+        mbar_init(&s.load_bar, 1);
+        // lane 0 of every warp commits to every barrier, whether or not it issued a share of the group
+        mbar_init(&s.bar_early, 8); mbar_init(&s.bar_score, 8); mbar_init(&s.bar_grad, 8); mbar_init(&s.bar_gv, 8);
+        fence_mbar_init();
+        if (j != P.skip_load) {
+            mbar_expect_tx(&s.load_bar, (PER_TOKEN ? 7 : 6) * TILE_BYTES);
+            tma_load_3d(&s.in[T_R], &map_r, &s.load_bar, h * 64, j * CH, b);
+            tma_load_3d(&s.in[T_K], &map_k, &s.load_bar, h * 64, j * CH, b);
+            tma_load_3d(&s.in[T_V], &map_v, &s.load_bar, h * 64, j * CH, b);
+            if (PER_TOKEN) tma_load_3d(&s.in[T_W], &map_w, &s.load_bar, h * 64, j * CH, b);
+            tma_load_3d(&s.in[T_GY], &map_gy, &s.load_bar, h * 64, j * CH, b);
+            tma_load_3d(&s.in[T_S], &map_s, &s.load_bar, 0, 0, bh * (n + 1) + j);
+            tma_load_3d(&s.in[T_D], &map_d, &s.load_bar, 0, 0, bh * (n + 1) + j + 1);
+        }
+    }
+    if (tid == 32) {
+        // the CTA that will take this one's place on the SM finds its tiles in L2
+        const int nb = chunk_id + P.prefetch_dist;
+        if (nb < (int)gridDim.x) {
+            const int bh2 = nb / n, j2 = nb % n, b2 = bh2 / P.H, h2 = bh2 % P.H;
+            tma_prefetch_l2_3d(&map_r, h2 * 64, j2 * CH, b2);
+            tma_prefetch_l2_3d(&map_k, h2 * 64, j2 * CH, b2);
+            tma_prefetch_l2_3d(&map_v, h2 * 64, j2 * CH, b2);
+            if (PER_TOKEN) tma_prefetch_l2_3d(&map_w, h2 * 64, j2 * CH, b2);
+            tma_prefetch_l2_3d(&map_gy, h2 * 64, j2 * CH, b2);
+            tma_prefetch_l2_3d(&map_s, 0, 0, bh2 * (n + 1) + j2);
+            tma_prefetch_l2_3d(&map_d, 0, 0, bh2 * (n + 1) + j2 + 1);
+        }
+    }
+    // (the flag is read while the loads are in flight: asking first would put a DRAM round trip in front of them)
+    if (tid == 64) s.is_mild = P.mildflag[chunk_id];
+    if (tid >= 128 && tid < 128 + CH) s.uf[tid - 128] = __bfloat162float(P.u[h * 64 + tid - 128]);
+    if (warp == 0) { tmem_alloc(&s.tmem_base, BWD_TMEM_COLS); tmem_relinquish(); }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tm = s.tmem_base;
+    // (through a shuffle: the compiler then knows that the branch is uniform across the warp)
+    if (__shfl_sync(0xffffffffu, s.is_mild, 0)) bwd_chunk<PER_TOKEN, true>(map_gr, map_gk, map_gv, map_gw, P, s, tm, warp);
+    else bwd_chunk<PER_TOKEN, false>(map_gr, map_gk, map_gv, map_gw, P, s, tm, warp);
+    __syncthreads();
+    if (warp == 0) tmem_dealloc(tm, BWD_TMEM_COLS);
 }
 
 // sum the per-chunk partials: out[bh*64 + k] = sum_j part[(bh*n + j)*64 + k]
@@ -1236,20 +1207,10 @@ int chunked_backward(const wkv_args_t *a0, bool per_token_w, const CallOpts &opt
         p.mildflag = (const unsigned char *)(fwd_ck + CL.mild);
         const size_t smem = sizeof(BwdSmem);
         auto kern = per_token_w ? k_chunk_bwd<true> : k_chunk_bwd<false>;
-        auto kern_steep = per_token_w ? k_chunk_bwd_steep<true> : k_chunk_bwd_steep<false>;
-        static unsigned char attr_done[2][2][64];
-        const int pt = per_token_w ? 1 : 0;
-        if (!set_max_smem_once(kern, (int)smem, attr_done[0][pt]) ||
-            !set_max_smem_once(kern_steep, (int)smem, attr_done[1][pt]))
-            return WKV_ERR_LAUNCH;
-        // every chunk the forward kernel found mild (all of them, on ordinary data) ...
+        static unsigned char attr_done[2][64];
+        if (!set_max_smem_once(kern, (int)smem, attr_done[per_token_w ? 1 : 0])) return WKV_ERR_LAUNCH;
         if (launch_chained(kern, dim3(BH * n), dim3(256), smem, stream, mr, mk, mv, mw, mgy, ms, md, mgr, mgk, mgv,
                            mgw, p) != WKV_OK)
-            return WKV_ERR_LAUNCH;
-        // ... and the ones it flagged as steep
-        const int steep_grid = BH * n < device_sm_count() ? BH * n : device_sm_count();
-        if (launch_chained(kern_steep, dim3(steep_grid), dim3(256), smem, stream, mr, mk, mv, mw, mgy, ms, md, mgr,
-                           mgk, mgv, mgw, p, BH * n) != WKV_OK)
             return WKV_ERR_LAUNCH;
     }
     // 4. fold the per-chunk partial sums: over the chunks and the batch, or over the chunks alone
