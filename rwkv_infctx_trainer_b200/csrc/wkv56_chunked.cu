@@ -19,10 +19,11 @@
 //
 // Time groups.  A segment's chunks are a serial chain per (batch, head).  When there are
 // too few chains to fill the device the chain is cut into G groups of consecutive
-// chunks and the forward runs as three launches:
+// chunks and the forward runs as two or three launches:
 //   A. per (chain, group), from a zero state: the group's own contribution U_g and the
 //      decay d_g of the whole group (no y, no scores -- a "summary" pass);
-//   B. k_group_scan: S_start[g+1] = d_g * S_start[g] + U_g, elementwise over the groups;
+//   B. S_start[g+1] = d_g * S_start[g] + U_g, elementwise over the groups: by k_group_scan when there are many,
+//      else in the prologue of
 //   C. per (chain, group), from S_start[g]: the full pass.
 // With G = 1 only C runs, from the caller's state.
 
@@ -69,11 +70,13 @@ struct FwdParams {
     int G, L;                 // time groups per chain, chunks per group (the last group may be shorter)
     const __nv_bfloat16 *u;
     const float *wvec;        // v5: per-channel decay parameter [H*64]
-    const float *state_in;    // G == 1: the caller's state (layout `layout`)
-    const float *gstart;      // G > 1, pass C: [B*H*G, 64, 64] state at the start of every group ([key,value])
+    const float *state_in;    // the caller's state (layout `layout`)
+    const float *gstart;      // or NULL: [B*H*G, 64*64] state at the start of every group (order: carried_at)
+    const float *grestart;    // or NULL: the same from an earlier call ([key,value])
+    int fold;                 // pass C without gstart: start from state_in and the gU, gD of the groups before
     float *state_out;         // written by the CTA whose group ends the segment
-    float *gU;                // pass A: [B*H*G, 64, 64] state a group builds from zero ([key,value])
-    float *gD;                // pass A: [B*H*G, 64] decay of a whole group per key channel
+    float *gU;                // [B*H*G, 64*64] state a group builds from zero (order: carried_at): pass A writes,
+    float *gD;                // [B*H*G, 64] decay of a whole group per key channel           pass C may read
     float *gsave;             // or NULL: [B*H, ceil(nchunk/Lsave), 64, 64] fp32 state at the start of every
     int Lsave;                // Lsave-th chunk ([key,value]), for a later call that restarts from them
     __nv_bfloat16 *y;
@@ -272,12 +275,11 @@ k_chunk_fwd(const __grid_constant__ CUtensorMap map_r, const __grid_constant__ C
         const size_t sbase = (size_t)bh * 64 * 64;
         float S[16];
 #pragma unroll
-        for (int q = 0; q < 16; q++) {
-            const int vc = vcol0 + q;
-            const size_t idx = P.layout == WKV_STATE_KV ? (size_t)row * 64 + vc : (size_t)vc * 64 + row;
-            if (P.gstart) S[q] = P.gstart[(size_t)unit * 4096 + row * 64 + vc];
-            else S[q] = (P.state_in && !summary) ? P.state_in[sbase + idx] : 0.f;
-        }
+        for (int q = 0; q < 16; q++) S[q] = 0.f;
+        if (P.grestart) load_state_row<16>(S, P.grestart + (size_t)unit * 4096, WKV_STATE_KV, row, vcol0);
+        else if (P.state_in && !summary) load_state_row<16>(S, P.state_in + sbase, P.layout, row, vcol0);
+        if (!summary && P.gstart) load_carried<16>(S, P.gstart + (size_t)unit * 4096, 4 * wg, tid & 127);
+        if (!summary && P.fold) fold_groups<16>(S, P.gU, P.gD, (size_t)bh * P.G, 1, grp, row, 4 * wg, tid & 127);
         float dprod = 1.f;      // summary pass: decay of the whole group for key channel `row`
         float lwc[4], wc[4];
         bool steep_static = false;
@@ -593,17 +595,10 @@ k_chunk_fwd(const __grid_constant__ CUtensorMap map_r, const __grid_constant__ C
                 if (P.status) atomicOr(P.status, 1);
             }
         } else if (summary) {
-            float4 *dst = reinterpret_cast<float4 *>(P.gU + (size_t)unit * 4096 + row * 64 + vcol0);
-#pragma unroll
-            for (int q = 0; q < 4; q++) dst[q] = make_float4(S[4 * q], S[4 * q + 1], S[4 * q + 2], S[4 * q + 3]);
+            store_carried<16>(S, P.gU + (size_t)unit * 4096, 4 * wg, tid & 127);
             if (vcol0 == 0) P.gD[(size_t)unit * 64 + row] = dprod;
         } else if (P.state_out && j0 + n == P.nchunk) {
-#pragma unroll
-            for (int q = 0; q < 16; q++) {
-                const int vc = vcol0 + q;
-                const size_t idx = P.layout == WKV_STATE_KV ? (size_t)row * 64 + vc : (size_t)vc * 64 + row;
-                P.state_out[sbase + idx] = S[q];
-            }
+            store_state_row<16>(S, P.state_out + sbase, P.layout, row, vcol0);
         }
     }
     tc_fence_before();
@@ -615,23 +610,38 @@ static_assert(sizeof(FwdSmem) + 1024 <= 115712, "two CTAs per SM need <= 113 KiB
 
 // Pass B of the time-group scheme: for every chain the elementwise recurrence over its groups,
 //   S <- init;  for each group g (forward order, or reverse for the gradient):  starts[g] = S;  S = d_g * S + U_g
-// and the final S.  One thread per state element; the loads do not depend on S, so the compiler
-// is free to run them ahead.  `init` / `final_out` are in the caller's state layout (NULL init = zeros).
+// (the last group's U_g is not formed).  One thread per state element; the loads do not depend on S and run ahead.
+// `init` is in the caller's state layout (NULL = zeros).
 __global__ void __launch_bounds__(256)
 k_group_scan(const float *__restrict__ U, const float *__restrict__ dG, const float *__restrict__ init,
-             float *__restrict__ starts, float *__restrict__ final_out, int G, int layout, int reverse) {
+             float *__restrict__ starts, int G, int layout, int reverse) {
     pdl_wait();
     pdl_trigger();
-    const int idx = blockIdx.x * 256 + threadIdx.x, bh = idx >> 12, e = idx & 4095, row = e >> 6, vc = e & 63;
-    const size_t lidx = (size_t)bh * 4096 + (layout == WKV_STATE_KV ? e : vc * 64 + row);
+    const int idx = blockIdx.x * 256 + threadIdx.x, bh = idx >> 12, e = idx & 4095, row = carried_row(e), vc = carried_col(e);
+    const size_t lidx = (size_t)bh * 4096 + (layout == WKV_STATE_KV ? row * 64 + vc : vc * 64 + row);
     float S = init ? init[lidx] : 0.f;
+    const ptrdiff_t dir = reverse ? -1 : 1;
+    size_t u = (size_t)bh * G + (reverse ? G - 1 : 0);
+    int step = 0;
+    for (; step + 16 < G; step += 16) {
+        float d[16], add[16];
+#pragma unroll
+        for (int i = 0; i < 16; i++) {
+            d[i] = dG[(u + i * dir) * 64 + row];
+            add[i] = U[(u + i * dir) * 4096 + e];
+        }
+#pragma unroll
+        for (int i = 0; i < 16; i++, u += dir) {
+            starts[u * 4096 + e] = S;
+            S = fmaf(d[i], S, add[i]);
+        }
+    }
 #pragma unroll 4
-    for (int step = 0; step < G; step++) {
-        const size_t u = (size_t)bh * G + (reverse ? G - 1 - step : step);
+    for (; step < G - 1; step++, u += dir) {
         starts[u * 4096 + e] = S;
         S = fmaf(dG[u * 64 + row], S, U[u * 4096 + e]);
     }
-    if (final_out) final_out[lidx] = S;
+    starts[u * 4096 + e] = S;
 }
 
 // Self-test of the bounded waits: one CTA, one mbarrier on which nobody ever arrives.  Warp 0
@@ -765,12 +775,12 @@ GroupLayout group_layout(size_t units) {
     return L;
 }
 
-int launch_group_scan(const void *group_ws, int BH, int G, const float *init, float *final_out, int layout,
-                      bool reverse, cudaStream_t stream) {
+int launch_group_scan(const void *group_ws, int BH, int G, const float *init, int layout, bool reverse,
+                      cudaStream_t stream) {
     const GroupLayout GL = group_layout((size_t)BH * G);
     const char *g = (const char *)group_ws;
     return launch_chained(k_group_scan, dim3(BH * 16), dim3(256), 0, stream, (const float *)(g + GL.gU),
-                          (const float *)(g + GL.gD), init, (float *)(g + GL.gstart), final_out, G, layout,
+                          (const float *)(g + GL.gD), init, (float *)(g + GL.gstart), G, layout,
                           reverse ? 1 : 0);
 }
 
@@ -829,23 +839,27 @@ int chunked_forward_impl(const wkv_args_t *a, bool per_token_w, void *state_ckpt
     if (gp.G > 1 && !restart) {
         // A: what every group adds to the state, from zero
         if (!set_max_smem_once(kerns[pt][FWD_SUMMARY], (int)smem, attr_done[pt][FWD_SUMMARY])) return WKV_ERR_LAUNCH;
-        p.state_in = nullptr; p.gstart = nullptr; p.state_out = nullptr;
+        p.state_in = nullptr; p.gstart = p.grestart = nullptr; p.state_out = nullptr; p.fold = 0;
         p.gU = (float *)(g + GL.gU); p.gD = (float *)(g + GL.gD);
         p.y = nullptr; p.ckpt = nullptr; p.dchunk = nullptr;
-        if (launch_chained(kerns[pt][FWD_SUMMARY], dim3(gp.G, BH), dim3(FWD_THREADS), smem, stream, mr, mk, mv, mw,
+        // (nothing needs what the last group adds)
+        if (launch_chained(kerns[pt][FWD_SUMMARY], dim3(gp.G - 1, BH), dim3(FWD_THREADS), smem, stream, mr, mk, mv, mw,
                            mrh, p) != WKV_OK)
             return WKV_ERR_LAUNCH;
         // B: the state at the start of every group.  (The state after the segment is left to the last
         // group of pass C, so that a later restart from saved states reproduces it bit for bit.)
-        if (launch_group_scan(g, BH, gp.G, a->state_in, nullptr, a->state_layout, false, stream) != WKV_OK)
+        if (gp.G > GROUP_FOLD_MAX &&
+            launch_group_scan(g, BH, gp.G, a->state_in, a->state_layout, false, stream) != WKV_OK)
             return WKV_ERR_LAUNCH;
     }
     // C (or the whole job when the chains are not split)
     if (!set_max_smem_once(kerns[pt][mode], (int)smem, attr_done[pt][mode])) return WKV_ERR_LAUNCH;
-    p.state_in = a->state_in;
-    p.gstart = restart ? (const float *)a->group_states : gp.G > 1 ? (const float *)(g + GL.gstart) : nullptr;
+    p.grestart = restart ? (const float *)a->group_states : nullptr;
+    p.gstart = !restart && gp.G > GROUP_FOLD_MAX ? (const float *)(g + GL.gstart) : nullptr;
+    p.state_in = p.gstart ? nullptr : a->state_in;
+    p.fold = !restart && gp.G > 1 && gp.G <= GROUP_FOLD_MAX;
     p.state_out = a->state_out;      // written by the group that ends the segment
-    p.gU = nullptr; p.gD = nullptr;
+    if (!p.fold) { p.gU = nullptr; p.gD = nullptr; }
     p.y = (__nv_bfloat16 *)a->y;
     const CkptLayout CL = ckpt_layout(B, T, H);
     p.ckpt = nullptr; p.dchunk = nullptr;

@@ -54,11 +54,12 @@ struct DscanParams {
     int G, L;             // time groups per chain, chunks per group (see wkv56_chunked.cu)
     int summary;          // pass A: zero start, the only outputs are gU / gD
     const float *dchunk;  // [B*H, nchunk, 64] decay of each whole chunk (from the forward kernel)
-    const float *gstate_out;   // G == 1: the caller's gradient w.r.t. the state after the segment
-    const float *gstart;       // G > 1, pass C: [B*H*G, 64, 64] gradient at the END of every group ([key,value])
-    float *gstate_in;          // G == 1 only (with G > 1 the group scan writes it)
-    float *gU;                 // pass A: [B*H*G, 64, 64] gradient a group builds from zero
-    float *gD;                 // pass A: [B*H*G, 64] decay of a whole group per key channel
+    const float *gstate_out;   // the caller's gradient w.r.t. the state after the segment
+    const float *gstart;       // or NULL: [B*H*G, 64*64] gradient at the END of every group (order: carried_at)
+    int fold;                  // pass C without gstart: start from gstate_out and the gU, gD of the groups after
+    float *gstate_in;
+    float *gU;                 // [B*H*G, 64*64] gradient a group builds from zero: pass A writes,
+    float *gD;                 // [B*H*G, 64] decay of a whole group per key channel: pass C may read
     __nv_bfloat16 *dck;  // [B*H, nchunk+1, 64, 64]; entry j+1 = dL/dS at the end of chunk j
     float *e0;           // [B*H, nchunk+1, 64]; entry j = sum_v S_j[k,v] D_j[k,v] at chunk boundary j
     int *status;
@@ -95,7 +96,9 @@ k_chunk_dscan(const __grid_constant__ CUtensorMap map_rh, const __grid_constant_
     // behind `s` is shared memory and uses shared-memory loads and stores for the tiles.
     DscanSmem &s = *reinterpret_cast<DscanSmem *>(smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u));
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int unit = blockIdx.x, bh = unit / P.G, grp = unit - bh * P.G, b = bh / P.H, h = bh % P.H;
+    // one CTA per (chain, group); a summary pass leaves out group 0, which nothing needs
+    const int skip = P.summary ? 1 : 0, bh = blockIdx.x / (P.G - skip), grp = blockIdx.x - bh * (P.G - skip) + skip;
+    const int unit = bh * P.G + grp, b = bh / P.H, h = bh % P.H;
     const int j0 = grp * P.L, n = min(P.L, P.nchunk - j0), N = P.nchunk;
     const bool summary = P.summary != 0;
     const int nsteps = n + ((!summary && grp == 0) ? 1 : 0);    // + the closing step
@@ -175,12 +178,10 @@ k_chunk_dscan(const __grid_constant__ CUtensorMap map_rh, const __grid_constant_
         const size_t sbase = (size_t)bh * 64 * 64;
         float v[32];     // D, this thread's key row and half of the value columns
 #pragma unroll
-        for (int q = 0; q < 32; q++) {
-            const int vc = vcol0 + q;
-            const size_t idx = P.layout == WKV_STATE_KV ? (size_t)row * 64 + vc : (size_t)vc * 64 + row;
-            if (P.gstart) v[q] = P.gstart[(size_t)unit * 4096 + row * 64 + vc];
-            else v[q] = (P.gstate_out && !summary) ? P.gstate_out[sbase + idx] : 0.f;
-        }
+        for (int q = 0; q < 32; q++) v[q] = 0.f;
+        if (P.gstate_out) load_state_row<32>(v, P.gstate_out + sbase, P.layout, row, vcol0);
+        if (P.gstart) load_carried<32>(v, P.gstart + (size_t)unit * 4096, 0, tid);
+        if (P.fold) fold_groups<32>(v, P.gU, P.gD, (size_t)bh * P.G + P.G - 1, -1, P.G - 1 - grp, row, 0, tid);
         float dprod = 1.f;      // summary pass: decay of the whole group for key channel `row`
         for (int i = 0; i < nsteps; i++) {
             const int st = i % DS_STAGES, j = j0 + n - 1 - i;       // global chunk of step i
@@ -203,14 +204,7 @@ k_chunk_dscan(const __grid_constant__ CUtensorMap map_rh, const __grid_constant_
                 if (active) P.e0[((size_t)bh * (N + 1) + (j + 1)) * 64 + row] = e;
             }
             if (i == n) {   // closing step: D_0 is the state gradient
-                if (P.gstate_in && P.G == 1) {
-#pragma unroll
-                    for (int q = 0; q < 32; q++) {
-                        const int vc = vcol0 + q;
-                        const size_t idx = P.layout == WKV_STATE_KV ? (size_t)row * 64 + vc : (size_t)vc * 64 + row;
-                        P.gstate_in[sbase + idx] = v[q];
-                    }
-                }
+                if (P.gstate_in) store_state_row<32>(v, P.gstate_in + sbase, P.layout, row, vcol0);
                 break;
             }
             if (!summary) {
@@ -238,9 +232,7 @@ k_chunk_dscan(const __grid_constant__ CUtensorMap map_rh, const __grid_constant_
         if (fail) {
             if (lane == 0 && P.status) atomicOr(P.status, 2);
         } else if (summary) {
-            float4 *dst = reinterpret_cast<float4 *>(P.gU + (size_t)unit * 4096 + row * 64 + vcol0);
-#pragma unroll
-            for (int q = 0; q < 8; q++) dst[q] = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+            store_carried<32>(v, P.gU + (size_t)unit * 4096, 0, tid);
             if (active) P.gD[(size_t)unit * 64 + row] = dprod;
         }
     }
@@ -1179,18 +1171,20 @@ int chunked_backward(const wkv_args_t *a0, bool per_token_w, const CallOpts &opt
         if (!set_max_smem_once(k_chunk_dscan, (int)smem, attr_done)) return WKV_ERR_LAUNCH;
         if (gp.G > 1) {
             p.summary = 1;
-            p.gstate_out = nullptr; p.gstart = nullptr; p.gstate_in = nullptr;
+            p.gstate_out = nullptr; p.gstart = nullptr; p.gstate_in = nullptr; p.fold = 0;
             p.gU = (float *)(g + GL.gU); p.gD = (float *)(g + GL.gD);
-            if (launch_chained(k_chunk_dscan, dim3(BH * gp.G), dim3(160), smem, stream, mrh, mgy, ms, p) != WKV_OK)
+            if (launch_chained(k_chunk_dscan, dim3(BH * (gp.G - 1)), dim3(160), smem, stream, mrh, mgy, ms, p) != WKV_OK)
                 return WKV_ERR_LAUNCH;
-            if (launch_group_scan(g, BH, gp.G, a->gstate_out, a->gstate_in, a->state_layout, true, stream) != WKV_OK)
+            if (gp.G > GROUP_FOLD_MAX &&
+                launch_group_scan(g, BH, gp.G, a->gstate_out, a->state_layout, true, stream) != WKV_OK)
                 return WKV_ERR_LAUNCH;
         }
         p.summary = 0;
-        p.gstate_out = a->gstate_out;
-        p.gstart = gp.G > 1 ? (const float *)(g + GL.gstart) : nullptr;
-        p.gstate_in = gp.G > 1 ? nullptr : a->gstate_in;
-        p.gU = nullptr; p.gD = nullptr;
+        p.gstart = gp.G > GROUP_FOLD_MAX ? (const float *)(g + GL.gstart) : nullptr;
+        p.gstate_out = p.gstart ? nullptr : a->gstate_out;
+        p.fold = gp.G > 1 && gp.G <= GROUP_FOLD_MAX;
+        p.gstate_in = a->gstate_in;
+        if (!p.fold) { p.gU = nullptr; p.gD = nullptr; }
         if (launch_chained(k_chunk_dscan, dim3(BH * gp.G), dim3(160), smem, stream, mrh, mgy, ms, p) != WKV_OK)
             return WKV_ERR_LAUNCH;
     }
