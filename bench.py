@@ -212,7 +212,6 @@ class Runner:
     the C ABI and nothing else on the host; events around every forward and backward call."""
 
     def __init__(self, wl, seg_tensors, u, device):
-        import ctypes
         import rwkv_infctx_trainer_b200 as W
         from rwkv_infctx_trainer_b200 import wkv56
         self.W, self.wkv56, self.wl, self.device = W, wkv56, wl, device
@@ -230,13 +229,6 @@ class Runner:
                                        ckpt=f.ckpt, gstate_in=gstates[i])
             self.fwd.append(f); self.bwd.append(b)
         self.bwd_events, self.fwd_events = [], []
-        self.launches = 0
-        # kernels per call: k_chunk_fwd ; k_chunk_dscan, k_chunk_bwd, k_reduce_partials
-        # -- and, when the library cuts the chains into time groups (few chains per GPU), a summary pass
-        # and a group scan more for the forward and for the dS scan
-        a = wkv56._args("wkv6", B, wl["seg"], H, torch.bfloat16, W.WKV_W_RAW, W.WKV_STATE_KV, W.WKV_PATH_AUTO)
-        split = W._lib.load().wkv6_forward_workspace(ctypes.byref(a)) > 256
-        self.fwd_launches, self.bwd_launches = (3, 5) if split else (1, 3)
 
     def step(self, record=False):
         for f in self.fwd:
@@ -247,7 +239,6 @@ class Runner:
             if record:
                 e1.record()
                 self.fwd_events.append((e0, e1))
-            self.launches += self.fwd_launches
         for b in reversed(self.bwd):
             if record:
                 e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
@@ -256,7 +247,6 @@ class Runner:
             if record:
                 e1.record()
                 self.bwd_events.append((e0, e1))
-            self.launches += self.bwd_launches
 
     def status(self) -> int:
         """OR of the status words of every call (0 = no device-side wait ran out)"""
@@ -315,7 +305,8 @@ def run_ours(args):
     for _ in range(args.warmup):
         runner.step()
     barrier()
-    runner.launches = 0
+    launched = runner.W._lib.load().wkvx_launch_count     # kernels of the library, counted where it launches them
+    launches = launched()
     sampler = None
     if rank == 0:
         sampler = NvmlSampler(local)
@@ -339,7 +330,7 @@ def run_ours(args):
     ms = t_start.elapsed_time(t_end)
     if runner.status() != 0:
         raise SystemExit("a device-side wait ran out during the timed region: the results are invalid")
-    launches = runner.launches
+    launches = launched() - launches
     bwd_ms = [a.elapsed_time(b) for a, b in runner.bwd_events]
     fwd_ms = [a.elapsed_time(b) for a, b in runner.fwd_events]
 

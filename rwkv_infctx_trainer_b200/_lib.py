@@ -98,6 +98,7 @@ def load() -> ctypes.CDLL:
     lib.wkv_error_string.restype = ctypes.c_char_p
     lib.wkv_error_string.argtypes = [ctypes.c_int]
     lib.wkv_version.restype = ctypes.c_char_p
+    lib.wkvx_launch_count.restype = ctypes.c_ulonglong
     i, f = ctypes.c_int, _vp
     lib.wkv4_forward_workspace.restype = ctypes.c_size_t
     lib.wkv4_forward_workspace.argtypes = [i, i, i]

@@ -168,6 +168,8 @@ const char *wkv_error_string(int code) {
 
 int wkv56_uses_chunked(const wkv_args_t *a, int per_token_w);
 
+unsigned long long wkvx_launch_count(void) { return launch_count.load(std::memory_order_relaxed); }
+
 const char *wkv_version(void) { return "wkv_b200 2 sm_100a"; }
 
 size_t wkv56_group_states_bytes(const wkv_args_t *a) {

@@ -5,6 +5,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
+
 #include "../../include/wkv_b200.h"
 
 namespace wkv {
@@ -105,6 +107,8 @@ inline int launch_status() { return cudaGetLastError() == cudaSuccess ? WKV_OK :
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
+inline std::atomic<unsigned long long> launch_count{0};     // launches of this process
+
 template <typename... KArgs, typename... Args>
 inline int launch_chained(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
                           Args &&...args) {
@@ -118,6 +122,7 @@ inline int launch_chained(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t 
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
+    launch_count.fetch_add(1, std::memory_order_relaxed);
     return cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...) == cudaSuccess ? WKV_OK : WKV_ERR_LAUNCH;
 }
 

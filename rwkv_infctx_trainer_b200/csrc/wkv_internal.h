@@ -9,6 +9,9 @@
 extern "C" {
 #endif
 
+/* kernels this process has launched through the library */
+unsigned long long wkvx_launch_count(void);
+
 /* wkv5/6_forward and _backward (per_token_w: 0 = v5, 1 = v6) with the status word at `status`
  * instead of the start of the workspace.  It may be mapped host memory; it is only ever written
  * when a device-side wait runs out and is not cleared by the call, so that a binding keeps one
