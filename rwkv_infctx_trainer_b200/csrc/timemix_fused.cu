@@ -14,6 +14,7 @@
 // Parameters come in their own element type and from their own tensors (a block's mixes are
 // separate parameters), and their gradients go back the same way.
 #include <initializer_list>
+#include <type_traits>
 
 #include "wkv_common.cuh"
 #include "wkv_internal.h"
@@ -121,34 +122,50 @@ k_lnx_gate_fwd(int tokens, int C, Split sp, const uint4 *__restrict__ y, const u
 
 // gy, gg and per-CTA partial sums of the gradients of gamma and beta ([nslot, 2, C])
 template <bool SILU>
-__global__ void __launch_bounds__(TPB)
+__global__ void __launch_bounds__(TPB, 3)
 k_lnx_gate_bwd(int tokens, int C, Split sp, const uint4 *__restrict__ y, const uint4 *__restrict__ g,
                const void *__restrict__ gamma, const void *__restrict__ beta, int pdtype, float eps,
                const uint4 *__restrict__ gout, uint4 *__restrict__ gy, uint4 *__restrict__ gg,
                float *__restrict__ part) {
     pdl_wait();
     pdl_trigger();
-    __shared__ float red[8][2][256];
+    __shared__ __align__(16) float red[8][2][256];
     const int cb = blockIdx.x % sp.ncb, slot = blockIdx.x / sp.ncb, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int c0 = cb * 256 + lane * 8;
     const bool live = c0 < C;
-    float ga[8], be[8], dga[8], dbe[8];
+    float dga[8], dbe[8];
 #pragma unroll
-    for (int q = 0; q < 8; q++) { dga[q] = 0.f; dbe[q] = 0.f; ga[q] = 0.f; be[q] = 0.f; }
+    for (int q = 0; q < 8; q++) { dga[q] = 0.f; dbe[q] = 0.f; }
     {
         // (every lane runs the loop, lanes past the last channel on zeros: the shuffles name all 32 lanes)
-        if (live) {
-            load8(gamma, pdtype, c0, ga);
-            load8(beta, pdtype, c0, be);
+        // gamma and beta wait in shared memory, each warp's own copy: the registers go to the loads ahead
+        float *gab = &red[warp][0][lane * 8], *beb = &red[warp][1][lane * 8];
+        {
+            float ga[8], be[8];
+#pragma unroll
+            for (int q = 0; q < 8; q++) { ga[q] = 0.f; be[q] = 0.f; }
+            if (live) {
+                load8(gamma, pdtype, c0, ga);
+                load8(beta, pdtype, c0, be);
+            }
+#pragma unroll
+            for (int q = 0; q < 8; q++) { gab[q] = ga[q]; beb[q] = be[q]; }
         }
         const int stride = sp.nslot * 8, row16 = C / 8;
+        const uint4 zero4 = make_uint4(0u, 0u, 0u, 0u);
+        uint4 raw[3] = {zero4, zero4, zero4};       // the next token's, on their way while this one is worked on
+        auto fetch = [&](int t) {
+            const size_t i = (size_t)t * row16 + (c0 >> 3);
+            if (live && t < tokens) { raw[0] = y[i]; raw[1] = g[i]; raw[2] = gout[i]; }
+        };
+        fetch(slot * 8 + warp);
         for (int t = slot * 8 + warp; t < tokens; t += stride) {
             const size_t i = (size_t)t * row16 + (c0 >> 3);
             float yv[8], gv[8], go[8];
-            const uint4 zero4 = make_uint4(0u, 0u, 0u, 0u);
-            unpack8(live ? y[i] : zero4, yv);
-            unpack8(live ? g[i] : zero4, gv);
-            unpack8(live ? gout[i] : zero4, go);
+            unpack8(raw[0], yv);
+            unpack8(raw[1], gv);
+            unpack8(raw[2], go);
+            fetch(t + stride);
             float dsilu[8];
             if (SILU) {
 #pragma unroll
@@ -166,7 +183,13 @@ k_lnx_gate_bwd(int tokens, int C, Split sp, const uint4 *__restrict__ y, const u
 #pragma unroll
             for (int q = 0; q < 8; q++) { yv[q] -= mean; v += yv[q] * yv[q]; }
             const float rstd = rsqrtf(head_sum(v) * (1.f / 64.f) + eps);
-            float dg[8], dy[8], s1 = 0.f, s2 = 0.f;
+            float dg[8], dy[8], s1 = 0.f, s2 = 0.f, ga[8], be[8];
+#pragma unroll
+            for (int q = 0; q < 8; q += 4) {
+                const float4 p = *reinterpret_cast<const float4 *>(gab + q), r = *reinterpret_cast<const float4 *>(beb + q);
+                ga[q] = p.x; ga[q + 1] = p.y; ga[q + 2] = p.z; ga[q + 3] = p.w;
+                be[q] = r.x; be[q + 1] = r.y; be[q + 2] = r.z; be[q + 3] = r.w;
+            }
 #pragma unroll
             for (int q = 0; q < 8; q++) {
                 const float xh = yv[q] * rstd;               // normalised value
@@ -279,119 +302,154 @@ k_ddlerp_fwd(int B, int T, int C, const uint4 *__restrict__ x, const uint4 *__re
 //   gx_t = sum_i gout_i,t (1 - a_i,t)  +  sum_i gout_i,t+1 a_i,t+1     (the second term: token t is
 //   the predecessor of t+1; for a row's last token it comes from the next segment, `gshift_in`),
 //   gshift_out = sum_i gout_i,0 a_i,0   (gradient w.r.t. `shift`).
-// A warp walks SUB consecutive tokens of 256 channels backward, so that the t+1 term is carried in registers and
-// recomputed once per SUB tokens; the 8 warps of a CTA take 8*SUB consecutive tokens of the same channels and pool
-// their sums of gm for gmaa.  (One thread per 64 tokens, as before, left half the SMs without a CTA: 191 us for
-// 4096 x 2560 tokens and 5 mixes, 17 tensors of 21 MB.)
+// A warp walks `sub` consecutive tokens of 256 channels backward, so that the t+1 term is carried in registers; the 8
+// warps of a CTA take 8*sub consecutive tokens of the same channels, hand that term on through shared memory (only the
+// CTA's last warp forms its first one from the token after it) and pool their sums of gm for gmaa.  HBM-bound: the
+// loads of K tokens go out before the first is used, and `sub` is chosen so that the grid is one wave, or as
+// few as possible (ddlerp_sub).  4096 x 2560 tokens, 5 mixes, 17 tensors of 21 MB, of which 64-token CTAs
+// in 2.2 waves took 116 us: 81 us; one mix, 4 tensors: 36 -> 21 us.
 // gx_add, gshift_add: gradients of x and shift from elsewhere, added.
-template <int NMIX, int SUB>
-__global__ void __launch_bounds__(TPB, 2)
-k_ddlerp_bwd(int B, int T, int C, const uint4 *__restrict__ x, const uint4 *__restrict__ shift, const MixPtrs maa,
+constexpr int MIX_CTAS = 2;       // per SM
+template <int NMIX>
+__global__ void __launch_bounds__(TPB, MIX_CTAS)
+k_ddlerp_bwd(int B, int T, int C, int sub, const uint4 *__restrict__ x, const uint4 *__restrict__ shift, const MixPtrs maa,
              const uint4 *__restrict__ m, const uint4 *__restrict__ gout, const uint4 *__restrict__ gshift_in,
              const uint4 *__restrict__ gx_add, const uint4 *__restrict__ gshift_add, uint4 *__restrict__ gx,
              uint4 *__restrict__ gm, uint4 *__restrict__ gshift_out, float *__restrict__ part) {
     pdl_wait();
     pdl_trigger();
-    __shared__ float red[8][256];
+    constexpr int K = NMIX == 1 ? 4 : 1;
+    __shared__ __align__(16) float red[8][256];
+    __shared__ __align__(16) float last[8][256];          // gx of a warp's last token without the term from its successor
     __shared__ __align__(16) float mixes[NMIX][256];      // maa of the CTA's channels
-    const int row16 = C / 8, ncb = (C + 255) / 256, npiece = (T + 8 * SUB - 1) / (8 * SUB);
+    const int row16 = C / 8, ncb = (C + 255) / 256, npiece = (T + 8 * sub - 1) / (8 * sub);
     const int cb = blockIdx.x % ncb, rowp = blockIdx.x / ncb, b = rowp / npiece, pc = rowp - b * npiece;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, c8 = cb * 32 + lane;
-    const size_t tokens16 = (size_t)B * T * row16;
-    const int t0 = pc * 8 * SUB + warp * SUB, t1 = min(T, t0 + SUB);
+    const size_t tokens16 = (size_t)B * T * row16, base = (size_t)b * T * row16 + c8;
+    const int t0 = pc * 8 * sub + warp * sub, t1 = min(T, t0 + sub);
+    const bool act = c8 < row16 && t0 < T;
     for (int k = threadIdx.x; k < NMIX * 32; k += TPB) {
         const int n = k >> 5, l = k & 31;
         if (cb * 32 + l < row16) maa.load(n, (cb * 32 + l) * 8, &mixes[n][l * 8]);
     }
     __syncthreads();
-    auto mix = [&](int n, float *a) {
-        const float4 p = *reinterpret_cast<const float4 *>(&mixes[n][lane * 8]), q = *reinterpret_cast<const float4 *>(&mixes[n][lane * 8 + 4]);
+    auto lds8 = [&](const float *row, float *a) {
+        const float4 p = *reinterpret_cast<const float4 *>(row + lane * 8), q = *reinterpret_cast<const float4 *>(row + lane * 8 + 4);
         a[0] = p.x; a[1] = p.y; a[2] = p.z; a[3] = p.w; a[4] = q.x; a[5] = q.y; a[6] = q.z; a[7] = q.w;
     };
-    float acc[NMIX][8];
+    auto sts8 = [&](float *row, const float *a) {
+        *reinterpret_cast<float4 *>(row + lane * 8) = make_float4(a[0], a[1], a[2], a[3]);
+        *reinterpret_cast<float4 *>(row + lane * 8 + 4) = make_float4(a[4], a[5], a[6], a[7]);
+    };
+    float acc[NMIX][8], carry[8];
 #pragma unroll
-    for (int n = 0; n < NMIX; n++)
+    for (int q = 0; q < 8; q++) {
+        carry[q] = 0.f;
 #pragma unroll
-        for (int q = 0; q < 8; q++) acc[n][q] = 0.f;
-    if (c8 < row16 && t0 < T) {
-        const size_t base = (size_t)b * T * row16 + c8;
-        // carry: what token t1 (the first after this warp's) sends back to token t1-1
-        float carry[8];
+        for (int n = 0; n < NMIX; n++) acc[n][q] = 0.f;
+    }
+    if (act) {
+        uint4 xraw = x[base + (size_t)(t1 - 1) * row16];
+        auto walk = [&](int t, auto count) {         // tokens t, t-1, ...
+            constexpr int N = decltype(count)::value;
+            uint4 graw[N][NMIX], mraw[N][NMIX], praw[N], araw[N];
 #pragma unroll
-        for (int q = 0; q < 8; q++) carry[q] = 0.f;
-        if (t1 < T) {
+            for (int k = 0; k < N; k++) {
+                const size_t i = base + (size_t)(t - k) * row16;
+#pragma unroll
+                for (int n = 0; n < NMIX; n++) {
+                    graw[k][n] = gout[n * tokens16 + i];
+                    if (m) mraw[k][n] = m[n * tokens16 + i];
+                }
+                praw[k] = t - k > 0 ? x[i - row16] : shift[(size_t)b * row16 + c8];
+                if (NMIX == 1 && gx_add) araw[k] = gx_add[i];
+            }
+#pragma unroll
+            for (int k = 0; k < N; k++) {
+                const size_t i = base + (size_t)(t - k) * row16;
+                float xv[8], d[8], gxv[8], nxt[8];
+                unpack8(xraw, xv);
+                unpack8(praw[k], d);
+                vsub<8>(d, d, xv);
+                if (gx_add) {
+                    unpack8(NMIX == 1 ? araw[k] : gx_add[i], gxv);
+                    vadd<8>(gxv, gxv, carry);
+                } else {
+#pragma unroll
+                    for (int q = 0; q < 8; q++) gxv[q] = carry[q];
+                }
+#pragma unroll
+                for (int q = 0; q < 8; q++) nxt[q] = 0.f;
+#pragma unroll
+                for (int n = 0; n < NMIX; n++) {
+                    float go[8], a[8], gmv[8];
+                    unpack8(graw[k][n], go);
+                    lds8(mixes[n], a);
+                    if (m) {
+                        float mv[8];
+                        unpack8(mraw[k][n], mv);
+                        vadd<8>(a, a, mv);
+                    }
+                    vmul<8>(gmv, go, d);
+                    vadd<8>(acc[n], acc[n], gmv);
+                    vmul<8>(a, a, go);
+                    vadd<8>(nxt, nxt, a);
+                    vsub<8>(a, go, a);
+                    vadd<8>(gxv, gxv, a);
+                    if (gm) gm[n * tokens16 + i] = pack8(gmv);
+                }
+                if (t - k == t1 - 1) sts8(last[warp], gxv);
+                else gx[i] = pack8(gxv);
+#pragma unroll
+                for (int q = 0; q < 8; q++) carry[q] = nxt[q];
+                xraw = praw[k];
+            }
+        };
+        int t = t1 - 1;
+        if (K > 1) {
+#pragma unroll 1
+            for (; t - K + 1 >= t0; t -= K) walk(t, std::integral_constant<int, K>());
+        }
+#pragma unroll 1
+        for (; t >= t0; t--) walk(t, std::integral_constant<int, 1>());
+        if (t0 == 0 && gshift_out) {
+            float out[8], add[8];
+            if (gshift_add) unpack8(gshift_add[(size_t)b * row16 + c8], add);
+#pragma unroll
+            for (int q = 0; q < 8; q++) out[q] = carry[q] + (gshift_add ? add[q] : 0.f);
+            gshift_out[(size_t)b * row16 + c8] = pack8(out);
+        }
+    }
+    // what the warp's first token sends back goes to the warp before; each finishes its last token
+    sts8(red[warp], carry);
+    __syncthreads();
+    if (act) {
+        float end[8];
+        lds8(last[warp], end);
+        if (t1 < T && warp < 7) {
+            float g[8];
+            lds8(red[warp + 1], g);
+            vadd<8>(end, end, g);
+        } else if (t1 < T) {
             const size_t j = base + (size_t)t1 * row16;
 #pragma unroll
             for (int n = 0; n < NMIX; n++) {
                 float go[8], a[8];
                 unpack8(gout[n * tokens16 + j], go);
-                mix(n, a);
+                lds8(mixes[n], a);
                 if (m) {
                     float mv[8];
                     unpack8(m[n * tokens16 + j], mv);
-#pragma unroll
-                    for (int q = 0; q < 8; q++) a[q] += mv[q];
+                    vadd<8>(a, a, mv);
                 }
-#pragma unroll
-                for (int q = 0; q < 8; q++) carry[q] += go[q] * a[q];
+                vfma<8>(end, go, a, end);
             }
         } else if (gshift_in) {
-            unpack8(gshift_in[(size_t)b * row16 + c8], carry);
+            float g[8];
+            unpack8(gshift_in[(size_t)b * row16 + c8], g);
+            vadd<8>(end, end, g);
         }
-        float xv[8];
-        unpack8(x[base + (size_t)(t1 - 1) * row16], xv);
-#pragma unroll 1
-        for (int t = t1 - 1; t >= t0; t--) {
-            const size_t i = base + (size_t)t * row16;
-            // every load of the token goes out before the first is used
-            uint4 graw[NMIX], mraw[NMIX];
-#pragma unroll
-            for (int n = 0; n < NMIX; n++) {
-                graw[n] = gout[n * tokens16 + i];
-                if (m) mraw[n] = m[n * tokens16 + i];
-            }
-            float pv[8], gxv[8], nxt[8], d[8];
-            unpack8(t > 0 ? x[i - row16] : shift[(size_t)b * row16 + c8], pv);
-            if (gx_add) unpack8(gx_add[i], gxv);
-#pragma unroll
-            for (int q = 0; q < 8; q++) {
-                d[q] = pv[q] - xv[q];
-                gxv[q] = (gx_add ? gxv[q] : 0.f) + carry[q];
-                nxt[q] = 0.f;
-            }
-#pragma unroll
-            for (int n = 0; n < NMIX; n++) {
-                float go[8], a[8], gmv[8];
-                unpack8(graw[n], go);
-                mix(n, a);
-                if (m) {
-                    float mv[8];
-                    unpack8(mraw[n], mv);
-#pragma unroll
-                    for (int q = 0; q < 8; q++) a[q] += mv[q];
-                }
-#pragma unroll
-                for (int q = 0; q < 8; q++) {
-                    gmv[q] = go[q] * d[q];
-                    acc[n][q] += gmv[q];
-                    gxv[q] += go[q] - go[q] * a[q];
-                    nxt[q] += go[q] * a[q];
-                }
-                if (gm) gm[n * tokens16 + i] = pack8(gmv);
-            }
-            gx[i] = pack8(gxv);
-#pragma unroll
-            for (int q = 0; q < 8; q++) { carry[q] = nxt[q]; xv[q] = pv[q]; }
-        }
-        if (t0 == 0 && gshift_out) {
-            if (gshift_add) {
-                float add[8];
-                unpack8(gshift_add[(size_t)b * row16 + c8], add);
-#pragma unroll
-                for (int q = 0; q < 8; q++) carry[q] += add[q];
-            }
-            gshift_out[(size_t)b * row16 + c8] = pack8(carry);
-        }
+        gx[base + (size_t)(t1 - 1) * row16] = pack8(end);
     }
     // the CTA's sums of gm per mix: [B*npiece, NMIX, C], folded by k_fold_cols
 #pragma unroll 1
@@ -414,20 +472,35 @@ k_ddlerp_bwd(int B, int T, int C, const uint4 *__restrict__ x, const uint4 *__re
     }
 }
 
-Split make_split(int tokens, int C) {
+// ctas: per SM.  Forward: 8.  Backward: as many as are resident at once (its tokens come through a loop that loads ahead,
+// and every CTA leaves a row of partials to fold): 4096 x 2560 tokens 37 + 10 -> 28 + 8 us.
+constexpr int LNX_FWD_CTAS = 8, LNX_BWD_CTAS = 3;
+Split make_split(int tokens, int C, int ctas) {
     Split sp;
     sp.ncb = (C + 255) / 256;
-    const int want = (device_sm_count() * 8 + sp.ncb - 1) / sp.ncb;      // about 8 CTAs per SM
+    const int want = ctas == LNX_FWD_CTAS ? (device_sm_count() * ctas + sp.ncb - 1) / sp.ncb : device_sm_count() * ctas / sp.ncb;
     const int most = (tokens + 7) / 8;
     sp.nslot = want < most ? want : most;
     if (sp.nslot < 1) sp.nslot = 1;
     return sp;
 }
 
-// tokens per warp of k_ddlerp_bwd: 8, or 2 when that leaves SMs without two CTAs
+// How k_ddlerp_bwd cuts a row: tokens per warp.  All CTAs of a wave walk side by side, so a grid a little over one
+// wave costs two; of one to eight waves the cut with the fewest token steps (and two for a CTA's start and end).
 int ddlerp_sub(int B, int T, int C) {
-    const long long ctas = (long long)B * ((T + 63) / 64) * ((C + 255) / 256);
-    return ctas >= 2 * device_sm_count() ? 8 : 2;
+    const long long cols = (long long)B * ((C + 255) / 256), slots = (long long)device_sm_count() * MIX_CTAS;
+    int best = 0;
+    long long least = 0;
+    for (int w = 1; w <= 8; w++) {
+        long long pieces = w * slots / cols;
+        if (pieces < 1) pieces = 1;
+        long long sub = (T + 8 * pieces - 1) / (8 * pieces);
+        if (sub < 2) sub = 2;
+        const long long ctas = cols * ((T + 8 * sub - 1) / (8 * sub)), cost = (ctas + slots - 1) / slots * (sub + 2);
+        if (best == 0 || cost < least) { best = (int)sub; least = cost; }
+        if (sub == 2) break;
+    }
+    return best;
 }
 size_t ddlerp_rows(int B, int T, int C) {
     const int piece = 8 * ddlerp_sub(B, T, C);
@@ -445,12 +518,9 @@ int ddlerp_bwd_launch(int B, int T, int C, const void *x, const void *shift, con
                       const void *gshift_in, const void *gx_add, const void *gshift_add, void *gx, void *gm, void *gshift_out,
                       float *part, cudaStream_t s) {
     const dim3 grid((unsigned)(ddlerp_rows(B, T, C) * ((C + 255) / 256)));
-    auto go = [&](auto kern) {
-        return launch_chained(kern, grid, dim3(TPB), 0, s, B, T, C, (const uint4 *)x, (const uint4 *)shift, maa, (const uint4 *)m,
-                              (const uint4 *)gout, (const uint4 *)gshift_in, (const uint4 *)gx_add, (const uint4 *)gshift_add, (uint4 *)gx,
-                              (uint4 *)gm, (uint4 *)gshift_out, part);
-    };
-    return ddlerp_sub(B, T, C) == 8 ? go(k_ddlerp_bwd<NMIX, 8>) : go(k_ddlerp_bwd<NMIX, 2>);
+    return launch_chained(k_ddlerp_bwd<NMIX>, grid, dim3(TPB), 0, s, B, T, C, ddlerp_sub(B, T, C), (const uint4 *)x, (const uint4 *)shift,
+                          maa, (const uint4 *)m, (const uint4 *)gout, (const uint4 *)gshift_in, (const uint4 *)gx_add,
+                          (const uint4 *)gshift_add, (uint4 *)gx, (uint4 *)gm, (uint4 *)gshift_out, part);
 }
 template <int NMIX>
 int ddlerp_fwd_launch(int B, int T, int C, const void *x, const void *shift, const MixPtrs &maa, const void *m, void *out, cudaStream_t s) {
@@ -489,7 +559,7 @@ int wkvx_lnx_gate_forward(int tokens, int H, const void *y, const void *g, const
     if (!y || !g || !gamma || !beta || !out) return WKV_ERR_NULL;
     if (!all_aligned({y, g, gamma, beta, out})) return WKV_ERR_ALIGN;
     const int C = H * HEAD;
-    const Split sp = make_split(tokens, C);
+    const Split sp = make_split(tokens, C, LNX_FWD_CTAS);
     return launch_chained(silu ? k_lnx_gate_fwd<true> : k_lnx_gate_fwd<false>, dim3(sp.ncb * sp.nslot), dim3(TPB), 0, (cudaStream_t)stream,
                           tokens, C, sp, (const uint4 *)y, (const uint4 *)g, gamma, beta, param_dtype, eps, (uint4 *)out);
 }
@@ -501,7 +571,7 @@ int wkv_lnx_gate_forward(int tokens, int H, const void *y, const void *g, const 
 
 size_t wkv_lnx_gate_backward_workspace(int tokens, int H) {
     if (tokens <= 0 || H <= 0) return 0;
-    return (size_t)make_split(tokens, H * HEAD).nslot * 2 * H * HEAD * sizeof(float);
+    return (size_t)make_split(tokens, H * HEAD, LNX_BWD_CTAS).nslot * 2 * H * HEAD * sizeof(float);
 }
 
 int wkvx_lnx_gate_backward(int tokens, int H, const void *y, const void *g, const void *gamma, const void *beta, int param_dtype,
@@ -520,7 +590,7 @@ int wkvx_lnx_gate_backward(int tokens, int H, const void *y, const void *g, cons
     if (!y || !g || !gamma || !beta || !gout || !gy || !gg) return WKV_ERR_NULL;
     if (!all_aligned({y, g, gamma, beta, gout, gy, gg})) return WKV_ERR_ALIGN;
     if (!workspace || workspace_bytes < wkv_lnx_gate_backward_workspace(tokens, H)) return WKV_ERR_WORKSPACE;
-    const Split sp = make_split(tokens, C);
+    const Split sp = make_split(tokens, C, LNX_BWD_CTAS);
     if (launch_chained(silu ? k_lnx_gate_bwd<true> : k_lnx_gate_bwd<false>, dim3(sp.ncb * sp.nslot), dim3(TPB), 0, s, tokens, C, sp,
                        (const uint4 *)y, (const uint4 *)g, gamma, beta, param_dtype, eps, (const uint4 *)gout, (uint4 *)gy, (uint4 *)gg,
                        (float *)workspace) != WKV_OK)
@@ -564,6 +634,7 @@ int wkv_ddlerp_forward(int B, int T, int C, int nmix, const void *x, const void 
 
 size_t wkv_ddlerp_backward_workspace(int B, int T, int C, int nmix) {
     if (B <= 0 || T <= 0 || C <= 0) return 0;
+    if (!mixes_ok(nmix)) return 0;
     return ddlerp_rows(B, T, C) * nmix * C * sizeof(float);
 }
 
