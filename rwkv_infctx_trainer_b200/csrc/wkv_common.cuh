@@ -6,6 +6,7 @@
 #include <stdint.h>
 
 #include <atomic>
+#include <utility>
 
 #include "../../include/wkv_b200.h"
 
@@ -109,8 +110,9 @@ __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.lau
 
 inline std::atomic<unsigned long long> launch_count{0};     // launches of this process
 
+// early: whether the kernel may be scheduled before the one in front of it has finished
 template <typename... KArgs, typename... Args>
-inline int launch_chained(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
+inline int launch_kernel(bool early, void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
                           Args &&...args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
@@ -119,11 +121,16 @@ inline int launch_chained(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t 
     cfg.stream = stream;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[0].val.programmaticStreamSerializationAllowed = early ? 1 : 0;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     launch_count.fetch_add(1, std::memory_order_relaxed);
     return cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...) == cudaSuccess ? WKV_OK : WKV_ERR_LAUNCH;
+}
+template <typename... KArgs, typename... Args>
+inline int launch_chained(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
+                          Args &&...args) {
+    return launch_kernel(true, kern, grid, block, smem, stream, std::forward<Args>(args)...);
 }
 
 // cudaFuncAttributeMaxDynamicSharedMemorySize is a per-device property of a kernel: set it on
