@@ -405,10 +405,20 @@ std::tuple<Tensor, Tensor, Tensor> block(int64_t version, const Tensor &x_, cons
     const Kind &k = kind_of(version);
     TORCH_CHECK_VALUE(params.size() == k.params, "wrong number of parameters");
     TORCH_CHECK_VALUE(x_.dim() == 3 && x_.size(1) > 0, "x must be [B,T,C] with T > 0");
-    require_cuda({&x_, &shift_, &state_, &params[0]});
     const int64_t B = x_.size(0), C = x_.size(2);
     TORCH_CHECK_VALUE(shift_.dim() == 2 && shift_.size(0) == B && shift_.size(1) == C, "the shift state must be [B,C]");
-    const Tensor x = x_.to(BF16).contiguous(), shift = shift_.to(BF16).contiguous(), state = state_.to(at::kFloat).contiguous();
+    // (nothing is launched before the state is known to fit: the kernels read it, and write its successor, by B and H)
+    if (version == 4) {
+        const int64_t A = params[P4_DECAY].numel();
+        TORCH_CHECK_VALUE(state_.dim() == 3 && state_.size(0) == B && state_.size(1) == A && state_.size(2) == 3,
+                          "the wkv state must be [", B, ",", A, ",3], got ", state_.sizes());
+    } else {
+        TORCH_CHECK_VALUE(state_.numel() == B * H * HEAD * HEAD, "the wkv state must be [", B, ",", H, ",64,64], got ", state_.sizes());
+    }
+    require_cuda({&x_, &shift_, &state_, &params[0]});
+    const Tensor x = x_.to(BF16).contiguous(), shift = shift_.to(BF16).contiguous();
+    Tensor state = state_.to(at::kFloat).contiguous();
+    if (version != 4 && state.dim() != 4) state = state.view({B, H, HEAD, HEAD});
     bool grad = wants_grad({&x, &shift, &state});
     if (!grad && at::GradMode::is_enabled())
         for (const Tensor &p : params) grad |= p.requires_grad();

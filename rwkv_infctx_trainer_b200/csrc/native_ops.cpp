@@ -64,16 +64,24 @@ void check_btc(const Tensor &r, const Tensor &t, const char *name) {
     TORCH_CHECK_VALUE(t.sizes() == r.sizes(), name, " must have shape ", r.sizes(), ", got ", t.sizes());
     TORCH_CHECK_VALUE(t.is_contiguous(), name, " must be contiguous (a [:, t0:t1] view of a longer tensor is not)");
 }
-void check_contig(const Tensor &t, const char *name) {
-    TORCH_CHECK_VALUE(!t.defined() || t.is_contiguous(), name, " must be contiguous");
+// a parameter or a state: `n` elements of type `dt`
+void check_flat(const Tensor &t, int64_t n, at::ScalarType dt, const char *name) {
+    if (!t.defined()) return;
+    TORCH_CHECK_VALUE(t.numel() == n, name, " must have ", n, " elements, got ", t.sizes());
+    TORCH_CHECK_VALUE(t.scalar_type() == dt, name, " must be ", dt, ", got ", t.scalar_type());
+    TORCH_CHECK_VALUE(t.is_contiguous(), name, " must be contiguous");
 }
 // the kernels take raw pointers: everything has to have the element type and size they assume
 void check_call(bool v6, const Tensor &r, const Tensor &k, const Tensor &v, const Tensor &w, const Tensor &u,
                 const Tensor &state, int w_kind) {
     TORCH_CHECK_VALUE(r.dim() == 3 && r.size(2) % HEAD == 0, "r must be [B,T,H*64]");
+    const auto dt = r.scalar_type();
     check_btc(r, r, "r"); check_btc(r, k, "k"); check_btc(r, v, "v");
     if (v6) check_btc(r, w, "w");
-    check_contig(u, "u"); check_contig(state, "state_in");
+    check_flat(k, r.numel(), dt, "k"); check_flat(v, r.numel(), dt, "v");
+    check_flat(w, v6 ? r.numel() : r.size(2), v6 && w_kind == WKV_W_RAW ? dt : at::kFloat, "w");
+    check_flat(u, r.size(2), dt, "u");
+    check_flat(state, r.size(0) * r.size(2) * HEAD, at::kFloat, "the state");
 }
 
 }  // namespace
@@ -81,9 +89,9 @@ void check_call(bool v6, const Tensor &r, const Tensor &k, const Tensor &v, cons
 Fwd wkv56_forward(bool v6, const Tensor &r, const Tensor &k, const Tensor &v, const Tensor &w, const Tensor &u,
                   const Tensor &state_in, int w_kind, int layout, int path, const Tensor &state_out, bool save_ckpt,
                   int time_groups, const Tensor &saved, int saved_mode, bool sync_check) {
-    require_cuda({&r, &k, &v, &w, &u, &state_in});
     check_call(v6, r, k, v, w, u, state_in, w_kind);
-    check_contig(state_out, "state_out");
+    require_cuda({&r, &k, &v, &w, &u, &state_in, &state_out});
+    check_flat(state_out, r.size(0) * r.size(2) * HEAD, at::kFloat, "state_out");
     const int dev = r.device().index();
     int *status = status_word(dev);
     raise_if_set(dev, status);
@@ -117,10 +125,11 @@ Bwd wkv56_backward(bool v6, const Tensor &r, const Tensor &k, const Tensor &v, c
                    const Tensor &state_in, const Tensor &gy, const Tensor &gstate_out, int w_kind, int layout, int path,
                    bool want_gstate, const Tensor &ckpt, int time_groups, bool per_batch, at::ScalarType u_type,
                    at::ScalarType w_type, bool sync_check) {
-    require_cuda({&r, &k, &v, &w, &u, &state_in, &gy, &gstate_out});
     check_call(v6, r, k, v, w, u, state_in, w_kind);
+    require_cuda({&r, &k, &v, &w, &u, &state_in, &gy, &gstate_out});
     check_btc(r, gy, "gy");
-    check_contig(gstate_out, "gstate_out");
+    check_flat(gy, r.numel(), r.scalar_type(), "gy");
+    check_flat(gstate_out, r.size(0) * r.size(2) * HEAD, at::kFloat, "gstate_out");
     const int dev = r.device().index();
     int *status = status_word(dev);
     raise_if_set(dev, status);
@@ -299,7 +308,19 @@ Tensor wkv56_dropin(bool v6, int64_t B, int64_t T, int64_t C, int64_t H, const T
 }
 
 // ------------------------------------------------------------------------------ v4
+namespace {
+void check_wkv4(const Tensor &w, const Tensor &u, const Tensor &k, const Tensor &v, const Tensor &state) {
+    TORCH_CHECK_VALUE(k.dim() == 3, "k must be [B,T,C]");
+    const int64_t C = k.size(2);
+    TORCH_CHECK_VALUE(w.dim() == 1 && w.size(0) == C && u.dim() == 1 && u.size(0) == C, "time_decay and time_first must be [C]");
+    TORCH_CHECK_VALUE(v.sizes() == k.sizes(), "v must match k");
+    TORCH_CHECK_VALUE(state.dim() == 3 && state.size(0) == k.size(0) && state.size(1) == C && state.size(2) == 3,
+                      "last_state must be [B,C,3]");
+}
+}  // namespace
+
 Fwd4 wkv4_forward(const Tensor &w, const Tensor &u, const Tensor &k, const Tensor &v, const Tensor &state, bool save) {
+    check_wkv4(w, u, k, v, state);
     const int B = (int)k.size(0), T = (int)k.size(1), C = (int)k.size(2);
     c10::cuda::OptionalCUDAGuard guard(k.device());
     Fwd4 o;
@@ -352,12 +373,7 @@ struct Wkv4Backward : OpNode {
 }  // namespace
 
 std::vector<Tensor> wkv4(const Tensor &w, const Tensor &u, const Tensor &k, const Tensor &v, const Tensor &state) {
-    TORCH_CHECK_VALUE(k.dim() == 3, "k must be [B,T,C]");
-    const int64_t C = k.size(2);
-    TORCH_CHECK_VALUE(w.dim() == 1 && w.size(0) == C && u.dim() == 1 && u.size(0) == C, "time_decay and time_first must be [C]");
-    TORCH_CHECK_VALUE(v.sizes() == k.sizes(), "v must match k");
-    TORCH_CHECK_VALUE(state.dim() == 3 && state.size(0) == k.size(0) && state.size(1) == C && state.size(2) == 3,
-                      "last_state must be [B,C,3]");
+    check_wkv4(w, u, k, v, state);
     require_cuda({&w, &u, &k, &v, &state});
     dtype_code(k.scalar_type());
     const bool save = wants_grad({&w, &u, &k, &v, &state});

@@ -1,0 +1,38 @@
+"""The time-mix blocks look at their arguments before they launch anything.  Shapes are looked at before
+devices, so most of this runs without a GPU: a call that would read or write out of range raises ValueError."""
+import pytest
+import torch
+
+BLOCKS = {4: "RWKV_TimeMix_v4", 5: "RWKV_TimeMix", 6: "RWKV_TimeMix6_0"}
+C, H, B = 128, 2, 3
+
+
+def make(version, device="cpu"):
+    import rwkv_infctx_trainer_b200 as W
+    torch.manual_seed(version)
+    cls = getattr(W, BLOCKS[version])
+    return (cls(1, 4, C, C) if version == 4 else cls(1, 4, C, H, 64, C)).to(device)
+
+
+def call(version, blk, x, shift, state):
+    import rwkv_infctx_trainer_b200 as W
+    return blk(x, W.TimeMixState(shift, state) if version == 4 else (shift, state))
+
+
+def good_state(version, device="cpu"):
+    return torch.zeros((B, C, 3) if version == 4 else (B, H, 64, 64), device=device)
+
+
+@pytest.mark.parametrize("version", [4, 5, 6])
+@pytest.mark.parametrize("T", [1, 20])
+@pytest.mark.parametrize("grad", [False, True])
+def test_state_of_another_size_is_refused(version, T, grad):
+    blk = make(version)
+    x, shift = torch.zeros((B, T, C)), torch.zeros((B, C))
+    ok = good_state(version)
+    with torch.set_grad_enabled(grad):
+        for bad in (ok[:1], torch.cat((ok, ok)), ok[:, :1], ok[..., :1]):
+            with pytest.raises(ValueError, match="wkv state"):
+                call(version, blk, x, shift, bad)
+        with pytest.raises(RuntimeError, match="CUDA"):      # the right one gets as far as the device check
+            call(version, blk, x, shift, ok)
