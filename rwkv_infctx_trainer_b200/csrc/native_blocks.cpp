@@ -367,13 +367,56 @@ variable_list backward4(const Tensor &x, const Tensor &shift, const Tensor &stat
 typedef Out (*ForwardFn)(const Tensor &, const Tensor &, const Tensor &, const variable_list &, const Meta &, variable_list *);
 typedef variable_list (*BackwardFn)(const Tensor &, const Tensor &, const Tensor &, const variable_list &, const Meta &,
                                     const variable_list &, const Tensor &, const Tensor &, const Tensor &, bool);
+typedef void (*CheckFn)(const variable_list &, int64_t C, int64_t H);
 struct Kind {
     ForwardFn forward;
     BackwardFn backward;
+    CheckFn check;
     size_t params;
 };
+
+// The parameters' sizes against the width of x and the head count: the kernels take pointers, and some of them run
+// before (decode: instead of) any library call that would notice.
+void check_vec(const Tensor &t, int64_t n, const char *name) {
+    TORCH_CHECK_VALUE(t.numel() == n, name, " must have ", n, " elements for this input, got ", t.sizes());
+}
+void check_mat(const Tensor &t, int64_t rows, int64_t cols, const char *name) {
+    TORCH_CHECK_VALUE(t.dim() == 2 && t.size(0) == rows && t.size(1) == cols, name, " must be [", rows, ",", cols, "] for this input, got ", t.sizes());
+}
+void check6(const variable_list &p, int64_t C, int64_t H) {
+    TORCH_CHECK_VALUE(C == H * HEAD, "x must be [B,T,H*64] with H = ", H, ", got a width of ", C);
+    static const char *const mixes[] = {"time_maa_x", "time_maa_w", "time_maa_k", "time_maa_v", "time_maa_r", "time_maa_g"};
+    for (int i = P6_X; i <= P6_MG; i++) check_vec(p[i], C, mixes[i]);
+    const Tensor &w1 = p[P6_W1], &w2 = p[P6_W2], &d1 = p[P6_D1], &d2 = p[P6_D2];
+    TORCH_CHECK_VALUE(w2.dim() == 3 && w2.size(0) == 5 && w2.size(2) == C, "time_maa_w2 must be [5,rank,", C, "] for this input, got ", w2.sizes());
+    check_mat(w1, C, 5 * w2.size(1), "time_maa_w1");
+    check_vec(p[P6_DECAY], C, "time_decay");
+    TORCH_CHECK_VALUE(d2.dim() == 2 && d2.size(1) == C, "time_decay_w2 must be [rank,", C, "] for this input, got ", d2.sizes());
+    check_mat(d1, C, d2.size(0), "time_decay_w1");
+    check_vec(p[P6_U], C, "time_faaaa");
+    static const char *const proj[] = {"receptance", "key", "value", "output", "gate"};
+    for (int i = 0; i < 5; i++) check_mat(p[P6_R + i], C, C, proj[i]);
+    check_vec(p[P6_LW], C, "ln_x.weight"); check_vec(p[P6_LB], C, "ln_x.bias");
+}
+void check5(const variable_list &p, int64_t C, int64_t H) {
+    const int64_t A = H * HEAD;
+    static const char *const mixes[] = {"time_mix_k", "time_mix_v", "time_mix_r", "time_mix_g"};
+    for (int i = P5_MK; i <= P5_MG; i++) check_vec(p[i], C, mixes[i]);
+    check_vec(p[P5_DECAY], A, "time_decay"); check_vec(p[P5_U], A, "time_faaaa");
+    check_mat(p[P5_R], A, C, "receptance"); check_mat(p[P5_K], A, C, "key"); check_mat(p[P5_V], A, C, "value"); check_mat(p[P5_G], A, C, "gate");
+    check_mat(p[P5_O], C, A, "output");
+    check_vec(p[P5_LW], A, "ln_x.weight"); check_vec(p[P5_LB], A, "ln_x.bias");
+}
+void check4(const variable_list &p, int64_t C, int64_t) {
+    const int64_t A = p[P4_DECAY].numel();      // dim_att
+    static const char *const mixes[] = {"time_mix_k", "time_mix_v", "time_mix_r"};
+    for (int i = P4_MK; i <= P4_MR; i++) check_vec(p[i], C, mixes[i]);
+    check_vec(p[P4_U], A, "time_first");
+    check_mat(p[P4_K], A, C, "key"); check_mat(p[P4_V], A, C, "value"); check_mat(p[P4_R], A, C, "receptance");
+    check_mat(p[P4_O], C, A, "output");
+}
 const Kind &kind_of(int64_t version) {
-    static const Kind k4{forward4, backward4, P4_N}, k5{forward5, backward5, P5_N}, k6{forward6, backward6, P6_N};
+    static const Kind k4{forward4, backward4, check4, P4_N}, k5{forward5, backward5, check5, P5_N}, k6{forward6, backward6, check6, P6_N};
     TORCH_CHECK_VALUE(version >= 4 && version <= 6, "unknown block version");
     return version == 4 ? k4 : version == 5 ? k5 : k6;
 }
@@ -415,7 +458,9 @@ std::tuple<Tensor, Tensor, Tensor> block(int64_t version, const Tensor &x_, cons
     } else {
         TORCH_CHECK_VALUE(state_.numel() == B * H * HEAD * HEAD, "the wkv state must be [", B, ",", H, ",64,64], got ", state_.sizes());
     }
-    require_cuda({&x_, &shift_, &state_, &params[0]});
+    k.check(params, C, H);
+    require_cuda({&x_, &shift_, &state_});
+    for (const Tensor &p : params) require_cuda({&x_, &p});
     const Tensor x = x_.to(BF16).contiguous(), shift = shift_.to(BF16).contiguous();
     Tensor state = state_.to(at::kFloat).contiguous();
     if (version != 4 && state.dim() != 4) state = state.view({B, H, HEAD, HEAD});

@@ -36,3 +36,45 @@ def test_state_of_another_size_is_refused(version, T, grad):
                 call(version, blk, x, shift, bad)
         with pytest.raises(RuntimeError, match="CUDA"):      # the right one gets as far as the device check
             call(version, blk, x, shift, ok)
+
+
+def _param(blk, name):
+    owner, _, leaf = name.rpartition(".")
+    return (blk.get_submodule(owner) if owner else blk), leaf
+
+
+@pytest.mark.parametrize("version", [4, 5, 6])
+@pytest.mark.parametrize("T", [1, 20])
+def test_width_or_parameter_of_another_size_is_refused(version, T):
+    blk = make(version)
+    state = good_state(version)
+    with torch.no_grad():
+        for width in (C - 64, C + 64, C + 1):        # an input of another width than the parameters
+            with pytest.raises(ValueError):
+                call(version, blk, torch.zeros((B, T, width)), torch.zeros((B, width)), state)
+        x, shift = torch.zeros((B, T, C)), torch.zeros((B, C))
+        for name, p in list(blk.named_parameters()):  # one parameter with an element (or row) missing
+            owner, leaf = _param(blk, name)
+            flat = p.dim() < 2 or p.shape[0] == 1 or name == "time_faaaa" or (version == 5 and name == "time_decay")
+            setattr(owner, leaf, torch.nn.Parameter(p.detach().flatten()[1:] if flat else p.detach()[1:]))
+            with pytest.raises(ValueError):
+                call(version, blk, x, shift, state)
+            setattr(owner, leaf, p)
+        with pytest.raises(RuntimeError, match="CUDA"):
+            call(version, blk, x, shift, state)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("version", [4, 5, 6])
+def test_parameter_on_another_device_is_refused(version):
+    """every parameter, not the first alone: one left on the host raises before any kernel sees its address"""
+    blk = make(version, "cuda")
+    x, shift, state = torch.zeros((B, 1, C), device="cuda"), torch.zeros((B, C), device="cuda"), good_state(version, "cuda")
+    with torch.no_grad():
+        for name, p in list(blk.named_parameters()):
+            owner, leaf = _param(blk, name)
+            setattr(owner, leaf, torch.nn.Parameter(p.detach().cpu()))
+            with pytest.raises(RuntimeError, match="CUDA"):
+                call(version, blk, x, shift, state)
+            setattr(owner, leaf, p)
+        call(version, blk, x, shift, state)
