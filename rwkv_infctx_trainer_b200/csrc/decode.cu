@@ -396,6 +396,9 @@ int wkvx_decode_max_rows(void) { return 8; }
 
 int wkvx_decode6(const wkvx_decode6_t *a, void *stream) {
     if (!a || a->M < 1 || a->M > 8 || a->H < 1 || a->H > 128 || a->rank != 32 || a->decay_rank % 8) return WKV_ERR_SHAPE;
+    if (!all_aligned({a->x, a->shift, a->w1, a->w2, a->d1, a->proj[0], a->proj[1], a->proj[2], a->proj[3], a->proj[4], a->state_in, a->xs, a->rkvg,
+                      a->normed, a->new_shift, a->state_out}))
+        return WKV_ERR_ALIGN;
     const int M = a->M, C = a->H * 64;
     cudaStream_t s = (cudaStream_t)stream;
     typedef const __nv_bfloat16 *cb;
@@ -435,6 +438,9 @@ int wkvx_decode6(const wkvx_decode6_t *a, void *stream) {
 
 int wkvx_decode5(const wkvx_decode5_t *a, void *stream) {
     if (!a || a->M < 1 || a->M > 8 || a->H < 1 || a->H > 128 || a->C < 8 || a->C % 8 || a->C > 8192) return WKV_ERR_SHAPE;
+    if (!all_aligned({a->x, a->shift, a->proj[0], a->proj[1], a->proj[2], a->proj[3], a->proj[4], a->state_in, a->rkvg, a->normed, a->new_shift,
+                      a->state_out}))
+        return WKV_ERR_ALIGN;
     const int M = a->M, A = a->H * 64;
     cudaStream_t s = (cudaStream_t)stream;
     typedef const __nv_bfloat16 *cb;

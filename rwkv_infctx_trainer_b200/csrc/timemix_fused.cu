@@ -547,12 +547,6 @@ MixPtrs mix_ptrs(int n, const void *const *maa, int dtype, int one_minus) {
     p.one_minus = one_minus;
     return p;
 }
-bool all_aligned(std::initializer_list<const void *> ps) {
-    for (const void *p : ps)
-        if (p && !aligned16(p)) return false;
-    return true;
-}
-
 }  // namespace
 }  // namespace wkv
 

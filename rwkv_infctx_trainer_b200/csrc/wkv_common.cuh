@@ -6,6 +6,7 @@
 #include <stdint.h>
 
 #include <atomic>
+#include <initializer_list>
 #include <utility>
 
 #include "../../include/wkv_b200.h"
@@ -94,6 +95,11 @@ __device__ __forceinline__ void vaxpy(float *o, float s, const float *a, const f
 }
 
 inline bool aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
+inline bool all_aligned(std::initializer_list<const void *> ps) {      // (NULL counts as aligned)
+    for (const void *p : ps)
+        if (!aligned16(p)) return false;
+    return true;
+}
 
 inline int launch_status() { return cudaGetLastError() == cudaSuccess ? WKV_OK : WKV_ERR_LAUNCH; }
 
