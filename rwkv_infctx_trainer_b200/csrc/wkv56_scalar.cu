@@ -192,7 +192,8 @@ serial_role(const SerialParams &P, Stage (&stage)[STAGES], const F *a_, const F 
         typedef typename Two<F>::raw R2;
         typedef typename Two<typename WElem<F, WSRC>::type>::raw W2;
         const int c = 2 * lane;
-        const float2 u2 = Two<F>::f(*reinterpret_cast<const R2 *>((const F *)P.u + h * N + c));
+        // (u may start at any element: two loads)
+        const float2 u2 = make_float2(Elem<F>::ld((const F *)P.u + h * N + c), Elem<F>::ld((const F *)P.u + h * N + c + 1));
         float ws[2] = {0.f, 0.f};
         if (WSRC == W_STATIC) {
 #pragma unroll

@@ -35,3 +35,27 @@ def test_short_bf16_forward_matches_the_floored_oracle(T):
     want = CG.floored_oracle("v6", q)
     TL.assert_close("y", y, want["y"], 2e-2)
     TL.assert_close("state_out", s, want["state_out"], 2e-2 if T > 48 else 1e-3)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("variant", ["v5", "v6"])
+def test_bonus_that_starts_on_an_odd_element(variant, dtype):
+    """u is [H,64] wherever the caller keeps it: as a slice of a larger buffer it need not start on a pair of elements;
+    same numbers, so the same bits"""
+    import rwkv_infctx_trainer_b200 as W
+    from rwkv_infctx_trainer_b200 import wkv56
+    q = TL.case56(variant, 2, 11, 3, dtype, seed=730)
+    d = {n: TL.to_dev(q[n], dtype) for n in ("r", "k", "v", "u", "gy")}
+    w = TL.to_dev(q["x"], dtype if variant == "v6" else torch.float32)
+    s, gs = TL.to_dev(q["state_in"], torch.float32), TL.to_dev(q["gstate_out"], torch.float32)
+    buf = torch.zeros(d["u"].numel() + 8, dtype=dtype, device="cuda")
+    odd = buf[1:1 + d["u"].numel()].view_as(d["u"])
+    odd.copy_(d["u"])
+    kw = dict(w_kind=W.WKV_W_RAW, path=W.WKV_PATH_SCALAR)
+    name = "wkv6" if variant == "v6" else "wkv5"
+    runs = []
+    for u in (d["u"], odd):
+        y, s1 = wkv56.forward(name, d["r"], d["k"], d["v"], w, u, s, **kw)
+        runs.append((y, s1) + tuple(wkv56.backward(name, d["r"], d["k"], d["v"], w, u, s, d["gy"], gs, **kw)))
+    for a, b in zip(*runs):
+        assert torch.equal(a, b)
