@@ -303,6 +303,8 @@ template <bool ASYNC> struct Place {
         if (ASYNC) return Pair<F>::ld(p + o + ch);
         return make_float2(Elem<F>::ld(p + o + ch), Elem<F>::ld(p + o + ch1));
     }
+    // of a [C] vector that may start at any element
+    template <typename F> __device__ __forceinline__ f2 elements(const F *p) const { return make_float2(Elem<F>::ld(p + ch), Elem<F>::ld(p + ch1)); }
     // `p` points at channel ch
     template <typename F> __device__ __forceinline__ void st(F *p, f2 v) const {
         if (ASYNC) {
@@ -343,7 +345,7 @@ template <typename F, int NT, bool ASYNC, bool STATES, class S>
 __device__ __noinline__ void slow_forward(const Par &P, S &sm) {
     const Place<ASYNC> L(P);
     const int c = L.c, i = L.i, T = L.T, C = L.C, n8 = (T + TK - 1) / TK, n64 = (T + COARSE - 1) / COARSE;
-    const f2 w = make_float2(P.w.at(L.ch) * V4_LOG2E, P.w.at(L.ch1) * V4_LOG2E), u = mul2(L.ld((const F *)P.u, 0), both(V4_LOG2E));
+    const f2 w = make_float2(P.w.at(L.ch) * V4_LOG2E, P.w.at(L.ch1) * V4_LOG2E), u = mul2(L.elements((const F *)P.u), both(V4_LOG2E));
     const F *const k = (const F *)P.k + L.row, *const v = (const F *)P.v + L.row;
     if (i == 0) sm.carry[0][c] = L.ext_state(P.state_in);
     for (int s = 0; s < P.nslab; s++) {
@@ -379,7 +381,7 @@ __global__ void __launch_bounds__(NT * CP, NT == 8 ? 8 : NT == 16 ? 4 : 2) k_v4_
     const Place<ASYNC> L(P);
     const int c = L.c, i = L.i, T = L.T, C = L.C;
     const Copy<F, NT> cp(threadIdx.x, L.c0, C);
-    const f2 w = make_float2(P.w.at(L.ch) * V4_LOG2E, P.w.at(L.ch1) * V4_LOG2E), u = mul2(L.ld((const F *)P.u, 0), both(V4_LOG2E));
+    const f2 w = make_float2(P.w.at(L.ch) * V4_LOG2E, P.w.at(L.ch1) * V4_LOG2E), u = mul2(L.elements((const F *)P.u), both(V4_LOG2E));
     const F *const src[2] = {(const F *)P.k + L.row, (const F *)P.v + L.row};
     if (i == 0) sm.carry[0][c] = L.ext_state(P.state_in);
     if (ASYNC) { fetch_slab<F, NT, 2>(sm, cp, 0, src, T, C, 0); cp_commit(); }
@@ -484,7 +486,7 @@ template <typename F, int NT, bool ASYNC, bool FINE, class S>
 __device__ __noinline__ void slow_walk_back(const Par &P, S &sm, f2 &gw, f2 &gu) {
     const Place<ASYNC> L(P);
     const int c = L.c, i = L.i, T = L.T, C = L.C, n8 = (T + TK - 1) / TK, n64 = (T + COARSE - 1) / COARSE, last = P.nslab - 1;
-    const f2 w = make_float2(P.w.at(L.ch) * V4_LOG2E, P.w.at(L.ch1) * V4_LOG2E), u = mul2(L.ld((const F *)P.u, 0), both(V4_LOG2E));
+    const f2 w = make_float2(P.w.at(L.ch) * V4_LOG2E, P.w.at(L.ch1) * V4_LOG2E), u = mul2(L.elements((const F *)P.u), both(V4_LOG2E));
     const F *const k = (const F *)P.k + L.row, *const v = (const F *)P.v + L.row, *const gy = (const F *)P.gy + L.row;
     F *const gk = (F *)P.gk + L.row, *const gv = (F *)P.gv + L.row;
     if (i == 0) sm.carry[last & 1][c] = L.ext_gradient(P.gstate_out);
@@ -527,7 +529,7 @@ __global__ void __launch_bounds__(NT * CP, NT == 8 ? 7 : NT == 16 ? 3 : 1) k_v4_
     const Place<ASYNC> L(P);
     const int c = L.c, i = L.i, T = L.T, C = L.C;
     const Copy<F, NT> cp(threadIdx.x, L.c0, C);
-    const f2 w = make_float2(P.w.at(L.ch) * V4_LOG2E, P.w.at(L.ch1) * V4_LOG2E), u = mul2(L.ld((const F *)P.u, 0), both(V4_LOG2E));
+    const f2 w = make_float2(P.w.at(L.ch) * V4_LOG2E, P.w.at(L.ch1) * V4_LOG2E), u = mul2(L.elements((const F *)P.u), both(V4_LOG2E));
     const F *const src[3] = {(const F *)P.k + L.row, (const F *)P.v + L.row, (const F *)P.gy + L.row};
     const int n8 = (T + TK - 1) / TK, n64 = (T + COARSE - 1) / COARSE, last = P.nslab - 1;
     if (i == 0) sm.carry[last & 1][c] = L.ext_gradient(P.gstate_out);
@@ -716,10 +718,11 @@ int launch_bwd(Par P, cudaStream_t s) {
                   : launch(k_v4_par_bwd<F, NT, ASYNC, false>, smem, done[1], P, NT, s);
 }
 
-// 16-byte copies need rows that start on 16 bytes; other widths load element by element
+// 16-byte copies and accesses of channel pairs need rows that start on 16 bytes, in every tensor; what does not is read
+// and written element by element
 template <typename F>
 bool rows_aligned(const Par &P) {
-    return (size_t)P.C * sizeof(F) % 16 == 0 && aligned16(P.k) && aligned16(P.v) && (!P.gy || aligned16(P.gy));
+    return (size_t)P.C * sizeof(F) % 16 == 0 && all_aligned({P.k, P.v, P.gy, P.y, P.gk, P.gv, P.gw, P.gu, P.fine, P.coarse});
 }
 
 template <typename F>
@@ -733,7 +736,7 @@ int forward_as(const Par &P, bool states, cudaStream_t s) {
 }
 template <typename F>
 int backward_as(Par P, float *scratch, cudaStream_t s) {
-    const bool aligned = rows_aligned<F>(P);
+    const bool aligned = rows_aligned<F>(P) && aligned16(scratch);
     const int nt = aligned ? pick_tiles(P.B, P.T, P.C) : 16;
     if (!P.fine && P.T > nt * TK) {
         // nothing was handed over and there is more than one slab: the states every 64 tokens first

@@ -67,3 +67,45 @@ def test_v4_matches_oracle(B, T, C, dtype, how):
     for n, a, b in (("gw", gw, g["gw"]), ("gu", gu, g["gu"]), ("gk", o["gk"], g["gk"]), ("gv", o["gv"], g["gv"]),
                     ("gstate", state(gsi), state(g["gstate_in"]))):
         TL.assert_close("no hand-over " + n, a, b, tol)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("T", [20, 200])
+def test_tensors_that_start_on_an_odd_element(dtype, T):
+    """any one tensor of a call (the bonus, an input, an output, the hand-over) off its 16-byte boundary: the same result
+    as with all of them on it, up to the order of fp32 operations"""
+    from rwkv_infctx_trainer_b200 import _lib as L
+    B, C = 2, 48
+    lib, st, code = L.load(), torch.cuda.current_stream().cuda_stream, L.DTYPE_CODE[dtype]
+    c = inputs.wkv4_case(B, T, C, seed=850 + T)
+    src = {n: TL.to_dev(c[n], dtype) for n in ("u", "k", "v", "gy")}
+    w = TL.to_dev(-np.exp(c["td"]), torch.float32)
+    nck, nws = lib.wkv4_state_ckpt_bytes(B, T, C), lib.wkv4_backward_workspace(B, T, C)
+    nfw = lib.wkv4_forward_workspace(B, T, C)
+
+    def place(t, odd):
+        buf = torch.empty(t.numel() + 8, device="cuda", dtype=t.dtype)
+        out = buf[1:1 + t.numel()] if odd else buf[:t.numel()]
+        out.copy_(t.flatten())
+        return out
+
+    def run(odd):
+        t = {n: place(x, n == odd) for n, x in src.items()}
+        o = {n: place(torch.zeros_like(src["k"]), n == odd) for n in ("y", "gk", "gv")}
+        o.update({n: place(torch.zeros((B, C), device="cuda"), n == odd) for n in ("gw", "gu")})
+        ck = place(torch.zeros(max(nck // 4, 1), device="cuda"), odd == "ckpt")
+        ws = place(torch.zeros(max(nws, nfw) // 4, device="cuda"), odd == "ws")
+        p = lambda x: x.data_ptr()
+        hand = [(p(ck), nck)] if nck else []
+        for args in hand + [(None, 0)]:          # with a hand-over, then without
+            assert lib.wkv4_forward_ckpt(B, T, C, code, p(w), p(t["u"]), p(t["k"]), p(t["v"]), None, p(o["y"]), None, p(ws), ws.numel() * 4, *args, st) == 0
+            assert lib.wkv4_backward_ckpt(B, T, C, code, p(w), p(t["u"]), p(t["k"]), p(t["v"]), None, p(t["gy"]), None, p(o["gw"]), p(o["gu"]), p(o["gk"]),
+                                          p(o["gv"]), None, p(ws), ws.numel() * 4, *args, st) == 0
+            yield {n: x.clone() for n, x in o.items()}
+
+    # fp32 values: a chain of T steps of about four roundings of 2^-24 each; bf16: one rounding may fall the other way
+    tol = {True: 4 * 200 * 2.0 ** -24, False: 2.0 ** -7}
+    for odd in ("u", "k", "v", "gy", "y", "gk", "gv", "gw", "gu", "ckpt", "ws"):
+        for a, b in zip(run(odd), run(None)):
+            for n in a:
+                TL.assert_close(f"{n} with {odd} moved", a[n], TL.back(b[n]), tol[dtype == torch.float32 or n in ("gw", "gu")])
