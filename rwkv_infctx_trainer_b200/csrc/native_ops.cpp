@@ -183,7 +183,7 @@ namespace {
 struct Wkv56Backward : OpNode {
     bool v6, sync;
     int path;
-    at::ScalarType k_type, v_type, w_type, u_type, s_type;
+    at::ScalarType k_type, v_type, w_type, u_type, s_type;      // of the caller's tensors
     std::vector<int64_t> w_shape, u_shape, s_shape;
     std::string name() const override { return "Wkv56Backward"; }
     variable_list apply(variable_list &&grads) override {
@@ -193,7 +193,7 @@ struct Wkv56Backward : OpNode {
         const Tensor gy = grads[0].defined() ? as_contig(grads[0], r.scalar_type()) : at::zeros_like(r);
         const Tensor gs = grads[1].defined() ? as_contig(grads[1], at::kFloat) : Tensor();
         Bwd g = wkv56_backward(v6, r, st[1], st[2], st[3], st[4], st[5], gy, gs, WKV_W_RAW, WKV_STATE_KV, path, task_should_compute_output(5),
-                               st[6], 0, false, u_type, v6 ? at::kFloat : w_type, sync);
+                               st[6], 0, false, abi_type(u_type), abi_type(w_type), sync);
         return {g.gr, as_input(g.gk, k_type, g.gk.sizes()), as_input(g.gv, v_type, g.gv.sizes()), as_input(g.gw, w_type, w_shape),
                 as_input(g.gu, u_type, u_shape), as_input(g.gstate_in, s_type, s_shape)};
     }
@@ -363,7 +363,7 @@ struct Wkv4Backward : OpNode {
         const Tensor &k = st[2];
         const Tensor gy = grads[0].defined() ? as_contig(grads[0], k.scalar_type()) : at::zeros_like(k);
         const Tensor gs = grads[1].defined() ? as_contig(grads[1], at::kFloat) : Tensor();
-        Bwd4 g = wkv4_backward(st[0], st[1], k, st[3], st[4], st[5], gy, gs, u_type == at::kDouble ? at::kFloat : u_type,
+        Bwd4 g = wkv4_backward(st[0], st[1], k, st[3], st[4], st[5], gy, gs, abi_type(u_type),
                                task_should_compute_output(4));
         return {as_input(g.gw, w_type, g.gw.sizes()), as_input(g.gu, u_type, g.gu.sizes()), g.gk, as_input(g.gv, v_type, g.gv.sizes()),
                 as_input(g.gstate, s_type, st[4].sizes())};

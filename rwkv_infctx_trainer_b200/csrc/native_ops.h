@@ -34,7 +34,8 @@ struct Bwd4 {
 Bwd4 wkv4_backward(const Tensor &w, const Tensor &u, const Tensor &k, const Tensor &v, const Tensor &state, const Tensor &ckpt,
                    const Tensor &gy, const Tensor &gstate_out, at::ScalarType u_type, bool want_gstate);
 
-// an element type of the ABI for a parameter (double is taken as float)
-inline at::ScalarType param_type(const Tensor &t) { return t.scalar_type() == at::kDouble ? at::kFloat : t.scalar_type(); }
+// the element type the ABI takes a parameter of this type in, and gives its gradient in (double: float)
+inline at::ScalarType abi_type(at::ScalarType t) { return t == at::kBFloat16 || t == at::kHalf ? t : at::kFloat; }
+inline at::ScalarType param_type(const Tensor &t) { return abi_type(t.scalar_type()); }
 
 }  // namespace wkv_native

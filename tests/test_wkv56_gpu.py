@@ -280,3 +280,32 @@ def test_bad_arguments_raise_not_crash():
         f = torch.zeros((1, 4, 64), device="cuda", dtype=torch.float32)
         wkv56.forward("wkv6", f, f, f, f, f[0, 0], s, w_kind=W.WKV_W_RAW, path=W.WKV_PATH_CHUNKED)
     torch.cuda.synchronize()
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("variant", ["v5", "v6"])
+@pytest.mark.parametrize("frozen", [False, True])
+def test_parameters_of_another_type_than_the_kernels_take(variant, dtype, frozen):
+    """u (and v5's decay) in float64: computed as float32 and the gradient handed back in float64; with the parameters
+    frozen the backward pass runs just the same"""
+    W = _pkg()
+    B, T, H = 2, 70, 2
+    q = TL.case56(variant, B, T, H, dtype, seed=77)
+    gy, gs = TL.to_dev(q["gy"], dtype), TL.to_dev(q["gstate_out"], torch.float32)
+
+    def run(ptype):
+        t = {n: TL.to_dev(q[n], dtype).requires_grad_(True) for n in ("r", "k", "v")}
+        t["u"] = TL.to_dev(q["u"], torch.float32).to(ptype).requires_grad_(not frozen)
+        t["x"] = TL.to_dev(q["x"], dtype if variant == "v6" else torch.float32)
+        t["x"] = t["x"].to(ptype).requires_grad_(not frozen) if variant == "v5" else t["x"].requires_grad_(True)
+        t["s"] = TL.to_dev(q["state_in"], torch.float32).requires_grad_(True)
+        y, s = (W.WKV6 if variant == "v6" else W.WKV5).apply(B, T, H * 64, H, t["r"], t["k"], t["v"], t["x"], t["u"], t["s"])
+        torch.autograd.backward((y, s), (gy, gs))
+        return t
+
+    a, b = run(torch.float64), run(torch.float32)
+    for n in a:
+        assert (a[n].grad is None) == (b[n].grad is None) == (not a[n].requires_grad)
+        if a[n].requires_grad:
+            assert a[n].grad.dtype == a[n].dtype
+            assert torch.equal(a[n].grad.float(), b[n].grad.float()), n
