@@ -25,7 +25,7 @@ struct Mixes {
         type = param_type(*ps.begin());
         for (const Tensor &p : ps)
             if (param_type(p) != type) type = at::kFloat;
-        for (const Tensor &p : ps) t.push_back(as_contig(p, type));
+        for (const Tensor &p : ps) t.push_back(as_param(p, type));
     }
     int n() const { return (int)t.size(); }
     std::array<const void *, 5> ptrs() const {
@@ -127,7 +127,7 @@ Out forward6(const Tensor &x, const Tensor &shift, const Tensor &state, const va
         const Mixes mx({p[P6_X], p[P6_MW], p[P6_MK], p[P6_MV], p[P6_MR], p[P6_MG]}, false);
         const auto lt = param_type(p[P6_LW]);
         const Tensor w1 = as_bf16(p[P6_W1]), w2 = as_bf16(p[P6_W2]), td = as_bf16(p[P6_DECAY]), d1 = as_bf16(p[P6_D1]), d2 = as_bf16(p[P6_D2]),
-                     u = as_bf16(p[P6_U]), lw = as_contig(p[P6_LW], lt), lb = as_contig(p[P6_LB], lt);
+                     u = as_bf16(p[P6_U]), lw = as_param(p[P6_LW], lt), lb = as_param(p[P6_LB], lt);
         const Tensor proj[5] = {as_bf16(p[P6_R]), as_bf16(p[P6_K]), as_bf16(p[P6_V]), as_bf16(p[P6_G]), as_bf16(p[P6_O])};
         const int64_t R = w2.size(1), DR = d2.size(0);
         Tensor scratch = fresh({10 * M * C + M * (5 * R + DR)}, x.scalar_type(), x);
@@ -172,7 +172,7 @@ Out forward6(const Tensor &x, const Tensor &shift, const Tensor &state, const va
     Fwd o = wkv56_forward(true, btc(rkvg[0]), btc(rkvg[1]), btc(rkvg[2]), btc(w), u, state, WKV_W_RAW, WKV_STATE_KV, WKV_PATH_AUTO, Tensor(),
                           keep != nullptr, 0, Tensor(), WKV_GROUP_STATES_NONE, me.sync);
     const auto lt = param_type(p[P6_LW]);
-    const Tensor y = o.y.view({M, C}), n = norm_gate_forward(y, rkvg[3], as_contig(p[P6_LW], lt), as_contig(p[P6_LB], lt), me.eps, H);
+    const Tensor y = o.y.view({M, C}), n = norm_gate_forward(y, rkvg[3], as_param(p[P6_LW], lt), as_param(p[P6_LB], lt), me.eps, H);
     const Tensor out = at::mm(n, as_bf16(p[P6_O]).t());
     if (keep) *keep = {xxx, t1, m, xs, rkvg, dd, w, u, y, n, o.ckpt};
     return {out.view({B, T, C}), last_token(x), o.state_out};
@@ -190,7 +190,7 @@ variable_list backward6(const Tensor &x, const Tensor &shift, const Tensor &stat
     gp[P6_O] = at::mm(gout.t(), n);
     const Tensor gn = at::mm(gout, as_bf16(p[P6_O]));
     const auto lt = param_type(p[P6_LW]);
-    NormGrads ng = norm_gate_backward(y, rkvg[3], as_contig(p[P6_LW], lt), as_contig(p[P6_LB], lt), me.eps, H, gn);
+    NormGrads ng = norm_gate_backward(y, rkvg[3], as_param(p[P6_LW], lt), as_param(p[P6_LB], lt), me.eps, H, gn);
     gp[P6_LW] = ng.glw;
     gp[P6_LB] = ng.glb;
     Bwd o = wkv56_backward(true, btc(rkvg[0]), btc(rkvg[1]), btc(rkvg[2]), btc(w), u, state, btc(ng.gy), gstate, WKV_W_RAW, WKV_STATE_KV,
@@ -246,7 +246,7 @@ Out forward5(const Tensor &x, const Tensor &shift, const Tensor &state, const va
         // one token of a few rows: the block's own kernels
         const Mixes mx = four5(p);
         const auto lt = param_type(p[P5_LW]);
-        const Tensor u = as_bf16(p[P5_U]), w = as_contig(p[P5_DECAY], param_type(p[P5_DECAY])), lw = as_contig(p[P5_LW], lt), lb = as_contig(p[P5_LB], lt);
+        const Tensor u = as_bf16(p[P5_U]), w = as_contig(p[P5_DECAY], param_type(p[P5_DECAY])), lw = as_param(p[P5_LW], lt), lb = as_param(p[P5_LB], lt);
         const Tensor proj[5] = {as_bf16(p[P5_R]), as_bf16(p[P5_K]), as_bf16(p[P5_V]), as_bf16(p[P5_G]), as_bf16(p[P5_O])};
         Tensor scratch = fresh({5 * M * A}, x.scalar_type(), x);
         Out o{fresh_like(x), fresh_like(shift), fresh_like(state)};
@@ -279,7 +279,7 @@ Out forward5(const Tensor &x, const Tensor &shift, const Tensor &state, const va
     Fwd o = wkv56_forward(false, btc(rkvg[0]), btc(rkvg[1]), btc(rkvg[2]), w, u, state, WKV_W_RAW, WKV_STATE_KV, WKV_PATH_AUTO, Tensor(),
                           keep != nullptr, 0, Tensor(), WKV_GROUP_STATES_NONE, me.sync);
     const auto lt = param_type(p[P5_LW]);
-    const Tensor y = o.y.view({M, A}), n = norm_gate_forward(y, rkvg[3], as_contig(p[P5_LW], lt), as_contig(p[P5_LB], lt), me.eps, H);
+    const Tensor y = o.y.view({M, A}), n = norm_gate_forward(y, rkvg[3], as_param(p[P5_LW], lt), as_param(p[P5_LB], lt), me.eps, H);
     const Tensor out = at::mm(n, as_bf16(p[P5_O]).t());
     if (keep) *keep = {xs, rkvg, w, u, y, n, o.ckpt};
     return {out.view({B, T, C}), last_token(x), o.state_out};
@@ -295,7 +295,7 @@ variable_list backward5(const Tensor &x, const Tensor &shift, const Tensor &stat
     gp[P5_O] = at::mm(gout.t(), n);
     const Tensor gn = at::mm(gout, as_bf16(p[P5_O]));
     const auto lt = param_type(p[P5_LW]);
-    NormGrads ng = norm_gate_backward(y, rkvg[3], as_contig(p[P5_LW], lt), as_contig(p[P5_LB], lt), me.eps, H, gn);
+    NormGrads ng = norm_gate_backward(y, rkvg[3], as_param(p[P5_LW], lt), as_param(p[P5_LB], lt), me.eps, H, gn);
     gp[P5_LW] = ng.glw;
     gp[P5_LB] = ng.glb;
     Bwd o = wkv56_backward(false, btc(rkvg[0]), btc(rkvg[1]), btc(rkvg[2]), w, u, state, btc(ng.gy), gstate, WKV_W_RAW, WKV_STATE_KV,

@@ -34,6 +34,12 @@ inline void *ptr(const Tensor &t) { return t.defined() ? t.data_ptr() : nullptr;
 inline void *stream_of(const Tensor &t) { return at::cuda::getCurrentCUDAStream(t.device().index()).stream(); }
 inline Tensor contig(const Tensor &t) { return t.is_contiguous() ? t : t.contiguous(); }
 inline Tensor as_contig(const Tensor &t, at::ScalarType dt) { return t.scalar_type() == dt ? contig(t) : t.to(dt).contiguous(); }
+// a parameter as the kernels that read 16 bytes at a time take it (a copy when it starts elsewhere: parameters may be slices
+// of one flat buffer)
+inline Tensor as_param(const Tensor &t, at::ScalarType dt) {
+    const Tensor c = as_contig(t, dt);
+    return (reinterpret_cast<uintptr_t>(c.data_ptr()) & 15u) == 0 ? c : c.clone();
+}
 inline void require_cuda(std::initializer_list<const Tensor *> ts) {
     const Tensor *first = nullptr;
     for (const Tensor *t : ts) {

@@ -21,7 +21,7 @@ struct LnxGate : torch::autograd::Function<LnxGate> {
                           double eps, int64_t H) {
         c10::cuda::OptionalCUDAGuard guard(y_.device());
         const auto pt = weight.scalar_type() == bias.scalar_type() ? param_type(weight) : at::kFloat;
-        const Tensor y = contig(y_), g = contig(g_), ga = as_contig(weight, pt), be = as_contig(bias, pt);
+        const Tensor y = contig(y_), g = contig(g_), ga = as_param(weight, pt), be = as_param(bias, pt);
         Tensor out = fresh_like(y);
         const int tokens = (int)(y.numel() / (H * HEAD));
         check(wkvx_lnx_gate_forward(tokens, (int)H, ptr(y), ptr(g), ptr(ga), ptr(be), dtype_code(pt), (float)eps, 0, ptr(out), stream_of(y)),
@@ -56,7 +56,7 @@ struct LnxGate : torch::autograd::Function<LnxGate> {
 struct DDLerp : torch::autograd::Function<DDLerp> {
     static Tensor forward(AutogradContext *ctx, const Tensor &x_, const Tensor &shift_, const Tensor &maa, const OptTensor &m_) {
         c10::cuda::OptionalCUDAGuard guard(x_.device());
-        const Tensor x = contig(x_), sh = contig(shift_), m = m_.has_value() ? contig(*m_) : Tensor(), ma = as_contig(maa, param_type(maa));
+        const Tensor x = contig(x_), sh = contig(shift_), m = m_.has_value() ? contig(*m_) : Tensor(), ma = as_param(maa, param_type(maa));
         const int B = (int)x.size(0), T = (int)x.size(1), C = (int)x.size(2), n = (int)ma.size(0);
         Tensor out = fresh({n, B, T, C}, x.scalar_type(), x);
         const auto p = rows_of(ma);

@@ -78,3 +78,31 @@ def test_parameter_on_another_device_is_refused(version):
                 call(version, blk, x, shift, state)
             setattr(owner, leaf, p)
         call(version, blk, x, shift, state)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("version", [4, 5, 6])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_parameters_that_are_slices_of_a_flat_buffer(version, dtype):
+    """every parameter one element past a 16-byte boundary: a training segment gives what it gives with the
+    parameters in buffers of their own"""
+    x, gy = torch.randn((B, 20, C), device="cuda").bfloat16(), torch.randn((B, 20, C), device="cuda").bfloat16()
+    shift, state = torch.randn((B, C), device="cuda").bfloat16(), torch.ones_like(good_state(version, "cuda"))
+    blk = make(version, "cuda").to(dtype)
+
+    def run():
+        out = call(version, blk, x, shift, state)[0]
+        params = [p for _, p in sorted(blk.named_parameters())]
+        return [out] + list(torch.autograd.grad(out, params, gy))
+
+    want = run()
+    for name, p in list(blk.named_parameters()):
+        owner, leaf = _param(blk, name)
+        buf = torch.empty(p.numel() + 8, device="cuda", dtype=dtype)
+        odd = buf[1:1 + p.numel()].view(p.shape)
+        odd.copy_(p.detach())
+        setattr(owner, leaf, torch.nn.Parameter(odd))
+        assert getattr(owner, leaf).data_ptr() % 16 != 0
+    rel = lambda a, b: float((a.float() - b.float()).norm() / b.float().norm().clamp_min(1e-30))
+    for a, b in zip(run(), want):
+        assert a.shape == b.shape and rel(a.detach(), b.detach()) < 1e-2      # (a library GEMM may pick another kernel for such an operand)
