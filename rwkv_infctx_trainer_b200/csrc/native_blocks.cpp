@@ -93,6 +93,19 @@ NormGrads norm_gate_backward(const Tensor &y, const Tensor &g, const Tensor &lw,
     return r;
 }
 
+// Which gradients a backward pass is asked for: x, the shift state, the wkv state, then the parameters.  What nobody asks
+// for is not formed -- the weight gradients of frozen projections are a third of a block's GEMM work.
+struct Wanted {
+    std::vector<char> w;
+    bool shared(int i) const { return w[i]; }           // 0 x, 1 shift, 2 state
+    bool operator()(int i) const { return w[3 + i]; }
+    bool any(int first, int last) const {
+        for (int i = first; i <= last; i++)
+            if (w[3 + i]) return true;
+        return false;
+    }
+};
+
 // what every block's Function is given and keeps besides its tensors
 struct Meta {
     int64_t H = 0;
@@ -179,57 +192,64 @@ Out forward6(const Tensor &x, const Tensor &shift, const Tensor &state, const va
 }
 
 variable_list backward6(const Tensor &x, const Tensor &shift, const Tensor &state, const variable_list &p, const Meta &me,
-                        const variable_list &kept, const Tensor &gout_, const Tensor &gshift_new, const Tensor &gstate, bool want_gs) {
+                        const variable_list &kept, const Tensor &gout_, const Tensor &gshift_new, const Tensor &gstate, const Wanted &want) {
     const int64_t B = x.size(0), T = x.size(1), C = x.size(2), M = B * T, H = me.H;
     const Tensor &xxx = kept[0], &t1 = kept[1], &m = kept[2], &xs = kept[3], &rkvg = kept[4], &dd = kept[5], &w = kept[6], &u = kept[7],
                  &y = kept[8], &n = kept[9], &ckpt = kept[10];
     const auto btc = [&](const Tensor &t) { return t.view({B, T, C}); };
     variable_list g(3 + P6_N);
-    variable_list gp(P6_N);
+    const auto param = [&](int i) -> Tensor & { return g[3 + i]; };
+    // through the low-rank map of the mixes; through the mixes; through the WKV op; through norm and gate
+    const bool first = want.shared(0) || want.shared(1) || want(P6_X), mixes = first || want.any(P6_MW, P6_W2),
+               wkv = mixes || want.shared(2) || want.any(P6_DECAY, P6_V), norm = wkv || want.any(P6_G, P6_LB);
     const Tensor gout = gout_.view({M, C});
-    gp[P6_O] = at::mm(gout.t(), n);
+    if (want(P6_O)) param(P6_O) = at::mm(gout.t(), n);
+    if (!norm) return g;
     const Tensor gn = at::mm(gout, as_bf16(p[P6_O]));
     const auto lt = param_type(p[P6_LW]);
     NormGrads ng = norm_gate_backward(y, rkvg[3], as_param(p[P6_LW], lt), as_param(p[P6_LB], lt), me.eps, H, gn);
-    gp[P6_LW] = ng.glw;
-    gp[P6_LB] = ng.glb;
+    param(P6_LW) = ng.glw;
+    param(P6_LB) = ng.glb;
+    if (want(P6_G)) param(P6_G) = at::mm(ng.gg.t(), xs[4]);
+    if (!wkv) return g;
     Bwd o = wkv56_backward(true, btc(rkvg[0]), btc(rkvg[1]), btc(rkvg[2]), btc(w), u, state, btc(ng.gy), gstate, WKV_W_RAW, WKV_STATE_KV,
-                           WKV_PATH_AUTO, want_gs, ckpt, 0, false, param_type(p[P6_U]), at::kFloat, me.sync);
-    gp[P6_U] = o.gu;
+                           WKV_PATH_AUTO, want.shared(2), ckpt, 0, false, param_type(p[P6_U]), at::kFloat, me.sync);
+    param(P6_U) = o.gu;
+    g[2] = o.gstate_in;
     const Tensor gr = o.gr.view({M, C}), gk = o.gk.view({M, C}), gv = o.gv.view({M, C}), gw = o.gw.view({M, C});
-    gp[P6_R] = at::mm(gr.t(), xs[3]);
-    gp[P6_K] = at::mm(gk.t(), xs[1]);
-    gp[P6_V] = at::mm(gv.t(), xs[2]);
-    gp[P6_G] = at::mm(ng.gg.t(), xs[4]);
+    if (want(P6_R)) param(P6_R) = at::mm(gr.t(), xs[3]);
+    if (want(P6_K)) param(P6_K) = at::mm(gk.t(), xs[1]);
+    if (want(P6_V)) param(P6_V) = at::mm(gv.t(), xs[2]);
+    // the decay's low-rank map
+    const Tensor d1 = as_bf16(p[P6_D1]), d2 = as_bf16(p[P6_D2]);
+    if (want(P6_DECAY)) param(P6_DECAY) = gw.sum(0);
+    if (want(P6_D2)) param(P6_D2) = at::mm(dd.t(), gw);
+    const Tensor gdd = mixes || want(P6_D1) ? at::tanh_backward(at::mm(gw, d2.t()), dd) : Tensor();
+    if (want(P6_D1)) param(P6_D1) = at::mm(xs[0].t(), gdd);
+    if (!mixes) return g;
     Tensor gxs = fresh_like(xs);
     const auto into = [&](int i, const Tensor &a, const Tensor &b) { Tensor d = gxs[i]; at::mm_out(d, a, b); };
     into(3, gr, as_bf16(p[P6_R]));
     into(1, gk, as_bf16(p[P6_K]));
     into(2, gv, as_bf16(p[P6_V]));
     into(4, ng.gg, as_bf16(p[P6_G]));
-    // the decay's low-rank map
-    const Tensor d1 = as_bf16(p[P6_D1]), d2 = as_bf16(p[P6_D2]);
-    gp[P6_DECAY] = gw.sum(0);
-    gp[P6_D2] = at::mm(dd.t(), gw);
-    const Tensor gdd = at::tanh_backward(at::mm(gw, d2.t()), dd);
-    gp[P6_D1] = at::mm(xs[0].t(), gdd);
     into(0, gdd, d1.t());
     MixGrads mg = mix_backward(x, shift, five6(p), m, gxs, gshift_new, Tensor(), Tensor());
-    for (int i = 0; i < 5; i++) gp[P6_MW + i] = mg.gmaa[i];
+    for (int i = 0; i < 5; i++) param(P6_MW + i) = mg.gmaa[i];
     // the mixes' low-rank map
     const Tensor w1 = as_bf16(p[P6_W1]), w2 = as_bf16(p[P6_W2]);
     const int64_t R = w2.size(1);
     const Tensor t5 = t1.view({M, 5, R});
-    gp[P6_W2] = at::bmm(t5.permute({1, 2, 0}), mg.gm);
+    if (want(P6_W2)) param(P6_W2) = at::bmm(t5.permute({1, 2, 0}), mg.gm);
+    if (!first && !want(P6_W1)) return g;
     Tensor gt1 = fresh_like(t1), gt5 = gt1.view({M, 5, R});
     at::tanh_backward_out(gt5, at::bmm(mg.gm, w2.transpose(1, 2)).transpose(0, 1), t5);
-    gp[P6_W1] = at::mm(xxx.t(), gt1);
+    if (want(P6_W1)) param(P6_W1) = at::mm(xxx.t(), gt1);
+    if (!first) return g;
     MixGrads m1 = mix_backward(x, shift, first6(p), Tensor(), at::mm(gt1, w1.t()), Tensor(), mg.gx, mg.gshift);
-    gp[P6_X] = m1.gmaa[0];
+    param(P6_X) = m1.gmaa[0];
     g[0] = m1.gx;
     g[1] = m1.gshift;
-    g[2] = o.gstate_in;
-    for (int i = 0; i < P6_N; i++) g[3 + i] = gp[i];
     return g;
 }
 
@@ -286,27 +306,34 @@ Out forward5(const Tensor &x, const Tensor &shift, const Tensor &state, const va
 }
 
 variable_list backward5(const Tensor &x, const Tensor &shift, const Tensor &state, const variable_list &p, const Meta &me,
-                        const variable_list &kept, const Tensor &gout_, const Tensor &gshift_new, const Tensor &gstate, bool want_gs) {
+                        const variable_list &kept, const Tensor &gout_, const Tensor &gshift_new, const Tensor &gstate, const Wanted &want) {
     const int64_t B = x.size(0), T = x.size(1), C = x.size(2), M = B * T, H = me.H, A = H * HEAD;
     const Tensor &xs = kept[0], &rkvg = kept[1], &w = kept[2], &u = kept[3], &y = kept[4], &n = kept[5], &ckpt = kept[6];
     const auto btc = [&](const Tensor &t) { return t.view({B, T, A}); };
-    variable_list gp(P5_N);
+    variable_list g(3 + P5_N);
+    const auto param = [&](int i) -> Tensor & { return g[3 + i]; };
+    const bool mixes = want.shared(0) || want.shared(1) || want.any(P5_MK, P5_MG), wkv = mixes || want.shared(2) || want.any(P5_DECAY, P5_V),
+               norm = wkv || want.any(P5_G, P5_LB);
     const Tensor gout = gout_.view({M, C});
-    gp[P5_O] = at::mm(gout.t(), n);
+    if (want(P5_O)) param(P5_O) = at::mm(gout.t(), n);
+    if (!norm) return g;
     const Tensor gn = at::mm(gout, as_bf16(p[P5_O]));
     const auto lt = param_type(p[P5_LW]);
     NormGrads ng = norm_gate_backward(y, rkvg[3], as_param(p[P5_LW], lt), as_param(p[P5_LB], lt), me.eps, H, gn);
-    gp[P5_LW] = ng.glw;
-    gp[P5_LB] = ng.glb;
+    param(P5_LW) = ng.glw;
+    param(P5_LB) = ng.glb;
+    if (want(P5_G)) param(P5_G) = at::mm(ng.gg.t(), xs[3]);
+    if (!wkv) return g;
     Bwd o = wkv56_backward(false, btc(rkvg[0]), btc(rkvg[1]), btc(rkvg[2]), w, u, state, btc(ng.gy), gstate, WKV_W_RAW, WKV_STATE_KV,
-                           WKV_PATH_AUTO, want_gs, ckpt, 0, false, param_type(p[P5_U]), param_type(p[P5_DECAY]), me.sync);
-    gp[P5_U] = o.gu;
-    gp[P5_DECAY] = o.gw;
+                           WKV_PATH_AUTO, want.shared(2), ckpt, 0, false, param_type(p[P5_U]), param_type(p[P5_DECAY]), me.sync);
+    param(P5_U) = o.gu;
+    param(P5_DECAY) = o.gw;
+    g[2] = o.gstate_in;
     const Tensor gr = o.gr.view({M, A}), gk = o.gk.view({M, A}), gv = o.gv.view({M, A});
-    gp[P5_R] = at::mm(gr.t(), xs[2]);
-    gp[P5_K] = at::mm(gk.t(), xs[0]);
-    gp[P5_V] = at::mm(gv.t(), xs[1]);
-    gp[P5_G] = at::mm(ng.gg.t(), xs[3]);
+    if (want(P5_R)) param(P5_R) = at::mm(gr.t(), xs[2]);
+    if (want(P5_K)) param(P5_K) = at::mm(gk.t(), xs[0]);
+    if (want(P5_V)) param(P5_V) = at::mm(gv.t(), xs[1]);
+    if (!mixes) return g;
     Tensor gxs = fresh_like(xs);
     const auto into = [&](int i, const Tensor &a, const Tensor &b) { Tensor d = gxs[i]; at::mm_out(d, a, b); };
     into(2, gr, as_bf16(p[P5_R]));
@@ -314,9 +341,9 @@ variable_list backward5(const Tensor &x, const Tensor &shift, const Tensor &stat
     into(1, gv, as_bf16(p[P5_V]));
     into(3, ng.gg, as_bf16(p[P5_G]));
     MixGrads mg = mix_backward(x, shift, four5(p), Tensor(), gxs, gshift_new, Tensor(), Tensor());
-    for (int i = 0; i < 4; i++) gp[P5_MK + i] = mg.gmaa[i];
-    variable_list g = {mg.gx, mg.gshift, o.gstate_in};
-    g.insert(g.end(), gp.begin(), gp.end());
+    for (int i = 0; i < 4; i++) param(P5_MK + i) = mg.gmaa[i];
+    g[0] = mg.gx;
+    g[1] = mg.gshift;
     return g;
 }
 
@@ -342,38 +369,44 @@ Out forward4(const Tensor &x, const Tensor &shift, const Tensor &state, const va
 }
 
 variable_list backward4(const Tensor &x, const Tensor &shift, const Tensor &state, const variable_list &p, const Meta &,
-                        const variable_list &kept, const Tensor &gout_, const Tensor &gshift_new, const Tensor &gstate, bool want_gs) {
+                        const variable_list &kept, const Tensor &gout_, const Tensor &gshift_new, const Tensor &gstate, const Wanted &want) {
     const int64_t B = x.size(0), T = x.size(1), C = x.size(2), M = B * T;
     const Tensor &xs = kept[0], &kv = kept[1], &sr = kept[2], &w = kept[3], &u = kept[4], &y = kept[5], &sy = kept[6], &ckpt = kept[7];
     const int64_t A = kv.size(2);
-    variable_list gp(P4_N);
+    variable_list g(3 + P4_N);
+    const auto param = [&](int i) -> Tensor & { return g[3 + i]; };
+    const bool mixes = want.shared(0) || want.shared(1) || want.any(P4_MK, P4_MR), wkv = mixes || want.shared(2) || want.any(P4_DECAY, P4_V);
     const Tensor gout = gout_.view({M, C});
-    gp[P4_O] = at::mm(gout.t(), sy);
-    const Tensor gsy = at::mm(gout, as_bf16(p[P4_O]));
-    const Tensor gr = at::sigmoid_backward(at::mul(gsy, y), sr), gy = at::mul(gsy, sr);
-    Bwd4 o = wkv4_backward(w, u, kv[0].view({B, T, A}), kv[1].view({B, T, A}), state, ckpt, gy.view({B, T, A}), gstate, param_type(p[P4_U]), want_gs);
-    gp[P4_DECAY] = o.gw;
-    gp[P4_U] = o.gu;
+    if (want(P4_O)) param(P4_O) = at::mm(gout.t(), sy);
+    if (!wkv && !want(P4_R)) return g;
+    const Tensor gsy = at::mm(gout, as_bf16(p[P4_O])), gr = mixes || want(P4_R) ? at::sigmoid_backward(at::mul(gsy, y), sr) : Tensor();
+    if (want(P4_R)) param(P4_R) = at::mm(gr.t(), xs[2]);
+    if (!wkv) return g;
+    Bwd4 o = wkv4_backward(w, u, kv[0].view({B, T, A}), kv[1].view({B, T, A}), state, ckpt, at::mul(gsy, sr).view({B, T, A}), gstate,
+                           param_type(p[P4_U]), want.shared(2));
+    param(P4_DECAY) = o.gw;
+    param(P4_U) = o.gu;
+    g[2] = o.gstate;
     const Tensor gk = o.gk.view({M, A}), gv = o.gv.view({M, A});
-    gp[P4_K] = at::mm(gk.t(), xs[0]);
-    gp[P4_V] = at::mm(gv.t(), xs[1]);
-    gp[P4_R] = at::mm(gr.t(), xs[2]);
+    if (want(P4_K)) param(P4_K) = at::mm(gk.t(), xs[0]);
+    if (want(P4_V)) param(P4_V) = at::mm(gv.t(), xs[1]);
+    if (!mixes) return g;
     Tensor gxs = fresh_like(xs);
     const auto into = [&](int i, const Tensor &a, const Tensor &b) { Tensor d = gxs[i]; at::mm_out(d, a, b); };
     into(0, gk, as_bf16(p[P4_K]));
     into(1, gv, as_bf16(p[P4_V]));
     into(2, gr, as_bf16(p[P4_R]));
     MixGrads mg = mix_backward(x, shift, three4(p), Tensor(), gxs, gshift_new, Tensor(), Tensor());
-    for (int i = 0; i < 3; i++) gp[P4_MK + i] = mg.gmaa[i];
-    variable_list g = {mg.gx, mg.gshift, o.gstate};
-    g.insert(g.end(), gp.begin(), gp.end());
+    for (int i = 0; i < 3; i++) param(P4_MK + i) = mg.gmaa[i];
+    g[0] = mg.gx;
+    g[1] = mg.gshift;
     return g;
 }
 
 // ------------------------------------------------------------------------------ the node
 typedef Out (*ForwardFn)(const Tensor &, const Tensor &, const Tensor &, const variable_list &, const Meta &, variable_list *);
 typedef variable_list (*BackwardFn)(const Tensor &, const Tensor &, const Tensor &, const variable_list &, const Meta &,
-                                    const variable_list &, const Tensor &, const Tensor &, const Tensor &, bool);
+                                    const variable_list &, const Tensor &, const Tensor &, const Tensor &, const Wanted &);
 typedef void (*CheckFn)(const variable_list &, int64_t C, int64_t H);
 struct Kind {
     ForwardFn forward;
@@ -442,7 +475,9 @@ struct BlockBackward : OpNode {
         const Tensor gout = grads[0].defined() ? as_contig(grads[0], BF16) : at::zeros_like(x);
         const Tensor gshift = grads[1].defined() ? as_contig(grads[1], BF16) : Tensor();
         const Tensor gstate = grads[2].defined() ? as_contig(grads[2], at::kFloat) : Tensor();
-        variable_list g = k.backward(x, shift, state, p, meta, kept, gout, gshift, gstate, task_should_compute_output(2));
+        Wanted want;
+        for (size_t i = 0; i < 3 + k.params; i++) want.w.push_back(task_should_compute_output(i));
+        variable_list g = k.backward(x, shift, state, p, meta, kept, gout, gshift, gstate, want);
         for (size_t i = 0; i < k.params; i++) g[3 + i] = as_input(g[3 + i], p[i].scalar_type(), p[i].sizes());
         return g;
     }
