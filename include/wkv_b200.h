@@ -177,7 +177,7 @@ typedef struct wkv_args {
                            wkv6state_cuda_v1.cu:290).  v5: [B,C] fp32 per-batch
                            partials of the gradient w.r.t. time_decay */
     float *gu;          /* [B,C] fp32 per-batch partials */
-    float *gstate_in;   /* [B,H,N,N] fp32; may be NULL */
+    float *gstate_in;   /* [B,H,N,N] fp32; may be NULL; must not alias gstate_out */
     /* scratch */
     void *workspace;
     size_t workspace_bytes;

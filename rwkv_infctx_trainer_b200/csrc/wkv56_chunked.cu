@@ -25,7 +25,9 @@
 //   B. S_start[g+1] = d_g * S_start[g] + U_g, elementwise over the groups: by k_group_scan when there are many,
 //      else in the prologue of
 //   C. per (chain, group), from S_start[g]: the full pass.
-// With G = 1 only C runs, from the caller's state.
+// With G = 1 only C runs, from the caller's state.  With more, C does not touch the caller's initial state: state_out may
+// be the same memory, and the CTA of a chain's last group writes it without waiting for the others.  What the fold in C's
+// prologue starts from is a copy that A leaves in the last group's place of gU (A forms nothing for that group).
 
 #include "wkv56_chunked.cuh"
 
@@ -70,10 +72,10 @@ struct FwdParams {
     int G, L;                 // time groups per chain, chunks per group (the last group may be shorter)
     const __nv_bfloat16 *u;
     const float *wvec;        // v5: per-channel decay parameter [H*64]
-    const float *state_in;    // the caller's state (layout `layout`)
+    const float *state_in;    // the caller's state (layout `layout`); pass C with `fold`: only whether there is one
     const float *gstart;      // or NULL: [B*H*G, 64*64] state at the start of every group (order: carried_at)
     const float *grestart;    // or NULL: the same from an earlier call ([key,value])
-    int fold;                 // pass C without gstart: start from state_in and the gU, gD of the groups before
+    int fold;                 // pass C without gstart: start from the copy of state_in and the gU, gD of the groups before
     float *state_out;         // written by the CTA whose group ends the segment
     float *gU;                // [B*H*G, 64*64] state a group builds from zero (order: carried_at): pass A writes,
     float *gD;                // [B*H*G, 64] decay of a whole group per key channel           pass C may read
@@ -276,10 +278,24 @@ k_chunk_fwd(const __grid_constant__ CUtensorMap map_r, const __grid_constant__ C
         float S[16];
 #pragma unroll
         for (int q = 0; q < 16; q++) S[q] = 0.f;
-        if (P.grestart) load_state_row<16>(S, P.grestart + (size_t)unit * 4096, WKV_STATE_KV, row, vcol0);
-        else if (P.state_in && !summary) load_state_row<16>(S, P.state_in + sbase, P.layout, row, vcol0);
-        if (!summary && P.gstart) load_carried<16>(S, P.gstart + (size_t)unit * 4096, 4 * wg, tid & 127);
-        if (!summary && P.fold) fold_groups<16>(S, P.gU, P.gD, (size_t)bh * P.G, 1, grp, row, 4 * wg, tid & 127);
+        const size_t init = ((size_t)bh * P.G + P.G - 1) * 4096;     // where gU holds the copy of state_in (time groups)
+        if (summary) {
+            if (P.state_in && grp == 0) {
+                load_state_row<16>(S, P.state_in + sbase, P.layout, row, vcol0);
+                store_carried<16>(S, P.gU + init, 4 * wg, tid & 127);
+#pragma unroll
+                for (int q = 0; q < 16; q++) S[q] = 0.f;
+            }
+        } else if (P.grestart) {
+            load_state_row<16>(S, P.grestart + (size_t)unit * 4096, WKV_STATE_KV, row, vcol0);
+        } else if (P.gstart) {
+            load_carried<16>(S, P.gstart + (size_t)unit * 4096, 4 * wg, tid & 127);
+        } else if (P.fold) {
+            if (P.state_in) load_carried<16>(S, P.gU + init, 4 * wg, tid & 127);
+            fold_groups<16>(S, P.gU, P.gD, (size_t)bh * P.G, 1, grp, row, 4 * wg, tid & 127);
+        } else if (P.state_in) {
+            load_state_row<16>(S, P.state_in + sbase, P.layout, row, vcol0);
+        }
         float dprod = 1.f;      // summary pass: decay of the whole group for key channel `row`
         float lwc[4], wc[4];
         bool steep_static = false;
@@ -839,7 +855,8 @@ int chunked_forward_impl(const wkv_args_t *a, bool per_token_w, void *state_ckpt
     if (gp.G > 1 && !restart) {
         // A: what every group adds to the state, from zero
         if (!set_max_smem_once(kerns[pt][FWD_SUMMARY], (int)smem, attr_done[pt][FWD_SUMMARY])) return WKV_ERR_LAUNCH;
-        p.state_in = nullptr; p.gstart = p.grestart = nullptr; p.state_out = nullptr; p.fold = 0;
+        p.state_in = gp.G <= GROUP_FOLD_MAX ? a->state_in : nullptr;     // (copied for pass C)
+        p.gstart = p.grestart = nullptr; p.state_out = nullptr; p.fold = 0;
         p.gU = (float *)(g + GL.gU); p.gD = (float *)(g + GL.gD);
         p.y = nullptr; p.ckpt = nullptr; p.dchunk = nullptr;
         // (nothing needs what the last group adds)
