@@ -45,7 +45,13 @@ __device__ __forceinline__ float param(const void *p, int dtype, size_t i) {
     return dtype == WKV_F32 ? ((const float *)p)[i] : dtype == WKV_BF16 ? __bfloat162float(((const bf16 *)p)[i]) : __half2float(((const __half *)p)[i]);
 }
 __device__ __forceinline__ float sigmoidf(float x) { return __fdividef(1.f, 1.f + __expf(-x)); }
-__device__ __forceinline__ float tanh_fast(float x) { return 1.f - __fdividef(2.f, 1.f + __expf(2.f * x)); }
+// tanh to a few fp32 roundings of its value for every x (1 - 2 / (1 + e^{2x}) is that close to 1 only: for small x the
+// difference cancels, and under 6e-8 it is zero; low-rank maps start out with such values).  With E = e^{-2|x|} - 1:
+// tanh|x| = -E / (2 + E).
+__device__ __forceinline__ float tanh_full(float x) {
+    const float e = expm1f(-2.f * fabsf(x));
+    return copysignf(__fdividef(-e, 2.f + e), x);
+}
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
@@ -99,7 +105,7 @@ __device__ __forceinline__ void strip(const bf16 *W, int ldw, int n0, const bf16
         float s = 0.f;
 #pragma unroll
         for (int g = 0; g < 8; g++) s += red[g][m][q];
-        if (m < M) out[(size_t)m * ldw + n0 + q] = __float2bfloat16_rn(tanh_fast(rbf(s)));
+        if (m < M) out[(size_t)m * ldw + n0 + q] = __float2bfloat16_rn(tanh_full(rbf(s)));
     }
 }
 
