@@ -13,9 +13,10 @@ std::atomic<int *> g_status[MAX_DEVICES];
 std::mutex g_status_lock;
 
 void raise_if_set(int device, int *word) {
-    const int code = *reinterpret_cast<volatile int *>(word);
-    if (code == 0) return;
-    *reinterpret_cast<volatile int *>(word) = 0;      // reported once
+    if (__atomic_load_n(word, __ATOMIC_ACQUIRE) == 0) return;
+    // reported once; taken and cleared in one step, so that a bit a kernel sets meanwhile is reported by this look or the next
+    const int code = __atomic_exchange_n(word, 0, __ATOMIC_ACQ_REL);
+    if (code == 0) return;      // (another thread reports it)
     TORCH_CHECK(false, "a v5/v6 call on cuda:", device, ": a device-side wait ran out (status ", code,
                 "); the outputs of that call are invalid");
 }
@@ -419,7 +420,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     m.def("wkv56_apply", &wkv56_apply);
     m.def("wkv56_dropin", &wkv56_dropin);
     m.def("wkv4", &wkv4);
-    m.def("poll_status", &poll_status);
+    m.def("poll_status", &poll_status, py::call_guard<py::gil_scoped_release>());     // (it may wait for the device)
+    m.def("status_word", [](int device) { return (uintptr_t)status_word(device); });      // its address (tests)
     m.def("wkv56_forward",
           [](bool v6, const Tensor &r, const Tensor &k, const Tensor &v, const Tensor &w, const Tensor &u, const OptTensor &s,
              int w_kind, int layout, int path, const OptTensor &s_out, bool save_ckpt, int time_groups, const OptTensor &saved,

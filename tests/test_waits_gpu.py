@@ -5,6 +5,7 @@ it waits for (a host-side decision passed to the kernel) and by cutting the numb
 from 4e6 to a few thousand.  The kernels must return, report through the status word, free
 their tensor memory, and leave the context usable -- the next call must work."""
 import ctypes
+import time
 
 import pytest
 import torch
@@ -67,25 +68,63 @@ def test_kernels_unwind_when_a_load_never_arrives(kernel, backward, bit):
 
 
 def test_status_word_reaches_the_host_without_a_sync():
-    """in normal use (CHECK_STATUS off) a call whose kernel gave up is reported by the next call on
-    that device, or by poll_status()"""
+    """in normal use (CHECK_STATUS off) a call whose kernel gave up is reported by the next call on that device, or by
+    poll_status(): the kernels write one word per device in mapped host memory, and this test writes it in their place"""
     import rwkv_infctx_trainer_b200 as W
-    from rwkv_infctx_trainer_b200 import wkv56
+    from rwkv_infctx_trainer_b200 import _lib as L, wkv56
     wkv56.CHECK_STATUS = False
     try:
         B, T, H = 1, 128, 1
         q = TL.case56("v6", B, T, H, BF, seed=92)
-        d = {n: TL.to_dev(q[n], BF) for n in ("r", "k", "v", "u", "x")}
+        d = {n: TL.to_dev(q[n], BF).requires_grad_(True) for n in ("r", "k", "v", "u", "x")}
         s_in = TL.to_dev(q["state_in"], torch.float32)
-        wkv56.forward("wkv6", d["r"], d["k"], d["v"], d["x"], d["u"], s_in, w_kind=W.WKV_W_RAW)
+        call = lambda: W.WKV6.apply(B, T, H * 64, H, d["r"], d["k"], d["v"], d["x"], d["u"], s_in)
+        y, _ = call()
         wkv56.poll_status(wait=True)          # a healthy call: nothing raised
-        # a word that says "gave up", queued the way a call queues its own
-        ev = torch.cuda.Event(); ev.record()
-        word = torch.full((1,), 4, dtype=torch.int32).pin_memory()
-        wkv56._pending.setdefault(0, []).append((ev, word, "wkv6_backward"))
-        torch.cuda.synchronize()
-        with pytest.raises(RuntimeError, match="device-side wait ran out"):
-            wkv56.forward("wkv6", d["r"], d["k"], d["v"], d["x"], d["u"], s_in, w_kind=W.WKV_W_RAW)
-        wkv56.poll_status(wait=True)          # reported once, then cleared
+        word = ctypes.c_int.from_address(L.native().status_word(0))
+        backward = lambda: torch.autograd.grad(y, d["r"], torch.ones_like(y), retain_graph=True)
+        for look in (call, lambda: wkv56.poll_status(), lambda: wkv56.poll_status("cuda:0", wait=True),
+                     lambda: wkv56.forward("wkv6", *(d[n].detach() for n in ("r", "k", "v", "x", "u")), s_in, w_kind=W.WKV_W_RAW),
+                     backward):
+            torch.cuda.synchronize()
+            word.value = 4
+            with pytest.raises(RuntimeError, match=r"device-side wait ran out \(status 4\)"):
+                look()
+            assert word.value == 0            # reported once, then cleared
+            backward()
     finally:
         wkv56.CHECK_STATUS = True
+
+
+def test_status_word_set_while_it_is_looked_at_is_not_lost():
+    """two threads look, at the same time, while the word is set over and over: every value is reported exactly once"""
+    import sys
+    import threading
+    from rwkv_infctx_trainer_b200 import _lib as L
+    native = L.native()
+    word = ctypes.c_int.from_address(native.status_word(0))
+    reports, stop = [], threading.Event()
+
+    def look():
+        while not stop.is_set():
+            try:
+                native.poll_status(0, False)
+            except RuntimeError:
+                reports.append(1)
+
+    threads = [threading.Thread(target=look) for _ in range(2)]
+    for t in threads:
+        t.start()
+    n, interval = 1000, sys.getswitchinterval()
+    sys.setswitchinterval(1e-5)
+    try:
+        for _ in range(n):
+            word.value = 1
+            while word.value != 0:
+                time.sleep(0)
+    finally:
+        stop.set()
+        sys.setswitchinterval(interval)
+        for t in threads:
+            t.join()
+    assert len(reports) == n
