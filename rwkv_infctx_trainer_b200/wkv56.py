@@ -16,35 +16,16 @@ HEAD_SIZE = 64
 # before returning (tests do that).
 CHECK_STATUS = False
 
-_pending = {}      # device index -> list of (event, pinned int32 tensor, description): words of a caller's
-                   # own C-ABI calls, looked at in the same places
-
 
 def poll_status(device=None, wait=False):
     """Raise if a chunked-kernel call on ``device`` (default: all devices) reported a device-side
     wait that ran out.  ``wait=True`` first waits for the calls issued so far."""
     index = None if device is None else (torch.device(device).index or 0)
     L.native().poll_status(-1 if index is None else index, wait)
-    for key in list(_pending) if index is None else [index]:
-        still = []
-        for ev, word, what in _pending.get(key, []):
-            if wait:
-                ev.synchronize()
-            if ev.query():
-                code = int(word.item())
-                if code != 0:
-                    _pending[key] = []
-                    raise RuntimeError(f"{what}: a device-side wait ran out (status {code}); "
-                                       "the outputs of that call are invalid")
-            else:
-                still.append((ev, word, what))
-        _pending[key] = still
 
 
 def apply(variant, B, T, C, H, r, k, v, w, u, state_in, path, saved):
     """``WKV5.apply`` / ``WKV6.apply``"""
-    if _pending:
-        poll_status(r.device)
     if saved is None:
         return L.native().wkv56_apply(variant == "wkv6", B, T, C, H, r, k, v, w, u, state_in, path, None, 0,
                                       CHECK_STATUS)
@@ -56,8 +37,6 @@ def apply(variant, B, T, C, H, r, k, v, w, u, state_in, path, saved):
 
 def apply_dropin(variant, B, T, C, H, r, k, v, w, u, state):
     """``WKV5_CUDA.apply`` / ``WKV6STATE_CUDA.apply``: ``state`` [B,H,value,key] updated in place"""
-    if _pending:
-        poll_status(r.device)
     return L.native().wkv56_dropin(variant == "wkv6", B, T, C, H, r, k, v, w, u, state, CHECK_STATUS)
 
 
@@ -98,8 +77,6 @@ def forward(variant: str, r, k, v, w, u, state_in, *, w_kind, layout=L.WKV_STATE
     ``time_groups``: see ``wkv_args_t.time_groups`` (0 = the library decides).
     ``saved``: a ``SavedStates``; empty, the call fills it; filled (by a call with the same
     inputs), the call restarts from it instead of scanning over T."""
-    if _pending:
-        poll_status(r.device)
     mode, buf = (0, None) if saved is None else saved._attach(variant, r, path, w_kind, layout)
     y, state_out, ckpt = L.native().wkv56_forward(variant == "wkv6", r, k, v, w, u, state_in, w_kind, layout, path,
                                                   state_out, save_ckpt, time_groups, buf, mode, CHECK_STATUS)
@@ -113,8 +90,6 @@ def backward(variant: str, r, k, v, w, u, state_in, gy, gstate_out, *, w_kind,
              time_groups=0):
     """Launch wkv5_backward / wkv6_backward.  Returns gr, gk, gv, gw, gu, gstate_in with
     gw = [B,T,C] (v6, activation dtype) or [B,C] fp32 per-batch partials (v5); gu [B,C] fp32."""
-    if _pending:
-        poll_status(r.device)
     return L.native().wkv56_backward(variant == "wkv6", r, k, v, w, u, state_in, gy, gstate_out, w_kind, layout, path,
                                      want_gstate, ckpt, time_groups, CHECK_STATUS)
 
