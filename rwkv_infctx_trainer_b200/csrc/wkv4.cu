@@ -141,9 +141,8 @@ template <typename F>
 int fwd(int B, int T, int C, const Decay4 &w, const void *u, const void *k, const void *v,
         const float *si, void *y, float *so, cudaStream_t s) {
     const int n = B * C;
-    k_v4_fwd<F><<<(n + THREADS - 1) / THREADS, THREADS, 0, s>>>(
-        B, T, C, w, (const F *)u, (const F *)k, (const F *)v, si, (F *)y, so);
-    return launch_status();
+    return launch_kernel(false, k_v4_fwd<F>, dim3((n + THREADS - 1) / THREADS), dim3(THREADS), 0, s, B, T, C, w, (const F *)u, (const F *)k,
+                         (const F *)v, si, (F *)y, so);
 }
 
 template <typename F>
@@ -151,10 +150,8 @@ int bwd(int B, int T, int C, const Decay4 &w, const void *u, const void *k, cons
         const float *si, const void *gy, const float *gso, float *gw, float *gu, void *gk,
         void *gv, float *gsi, float *ws, cudaStream_t s) {
     const int n = B * C;
-    k_v4_bwd<F><<<(n + THREADS - 1) / THREADS, THREADS, 0, s>>>(
-        B, T, C, w, (const F *)u, (const F *)k, (const F *)v, si, (const F *)gy, gso, gw, gu,
-        (F *)gk, (F *)gv, gsi, ws);
-    return launch_status();
+    return launch_kernel(false, k_v4_bwd<F>, dim3((n + THREADS - 1) / THREADS), dim3(THREADS), 0, s, B, T, C, w, (const F *)u, (const F *)k,
+                         (const F *)v, si, (const F *)gy, gso, gw, gu, (F *)gk, (F *)gv, gsi, ws);
 }
 
 // Segments shorter than this run on the kernels above: with two tiles of 8 tokens there is little to

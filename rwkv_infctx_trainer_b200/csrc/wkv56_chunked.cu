@@ -689,8 +689,7 @@ __global__ void __launch_bounds__(64) k_selftest_wait(int *status, uint32_t limi
 
 int selftest_wait(int *status, uint32_t limit, cudaStream_t stream) {
     if (limit == 0 || limit > 100000u) return WKV_ERR_SHAPE;     // a test: keep it short
-    k_selftest_wait<<<1, 64, 0, stream>>>(status, limit);
-    return launch_status();
+    return launch_kernel(false, k_selftest_wait, dim3(1), dim3(64), 0, stream, status, limit);
 }
 
 // ---------------------------------------------------------------------------

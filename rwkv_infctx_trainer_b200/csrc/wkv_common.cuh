@@ -101,8 +101,6 @@ inline bool all_aligned(std::initializer_list<const void *> ps) {      // (NULL 
     return true;
 }
 
-inline int launch_status() { return cudaGetLastError() == cudaSuccess ? WKV_OK : WKV_ERR_LAUNCH; }
-
 // Programmatic dependent launch.  A kernel launched through launch_chained() may be scheduled
 // while the kernel before it in the stream is still running, which hides its launch latency
 // behind that kernel's last CTAs.  pdl_wait() returns once every earlier kernel of the stream

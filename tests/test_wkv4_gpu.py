@@ -187,3 +187,19 @@ def test_v4_handover_equals_recompute(dtype):
     for i in (0, 1):      # (gp,gq,go) stands for (gp,gq)*e^go
         x, y = (TL.back(o[4]) for o in outs)
         TL.assert_close("gstate_in", x[..., i] * np.exp(x[..., 2]), y[..., i] * np.exp(y[..., 2]), tol)
+
+
+@pytest.mark.parametrize("T,forward,backward", [(4, 1, 2), (200, 1, 2)])
+def test_every_launch_is_counted(T, forward, backward):
+    """the count a program reads from the library (wkvx_launch_count) on both sides of the length where the kernels change:
+    one kernel forward, one and the parameter fold backward"""
+    import rwkv_infctx_trainer_b200 as W
+    from rwkv_infctx_trainer_b200 import _lib as L
+    count = L.load().wkvx_launch_count
+    k, v = (torch.randn((2, T, 64), device="cuda").requires_grad_(True) for _ in range(2))
+    td, u = torch.zeros(64, device="cuda"), torch.zeros(64, device="cuda")
+    a = count()
+    y, _ = W.wkv_op(td, u, k, v, torch.ones((2, 64, 3), device="cuda"))
+    b = count()
+    torch.autograd.grad(y, k, torch.ones_like(y))
+    assert (b - a, count() - b) == (forward, backward)
