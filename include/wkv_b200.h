@@ -88,8 +88,9 @@ const char *wkv_error_string(int code);
  *   gstate_*   fp32 [B,C,3] = (gp,gq,go) in the exponent-scaled convention of
  *              wkv_cuda_bf16.cu:116-152; gstate_out may be NULL (= none)
  * No compile-time limit on T (the project needs T <= Tmax).  Segments of 16 tokens or more
- * run in tiles of 8 tokens in parallel (tile summaries are folded per channel).  The workspace
- * must be at least what wkv4_*_workspace() says.
+ * run in tiles of 8 tokens in parallel (tile summaries are folded per channel).  The backward workspace
+ * must be at least what wkv4_backward_workspace() says.  The forward kernels use none: the argument may be NULL, and
+ * wkv4_forward_workspace() stays for callers that size one by it.
  */
 size_t wkv4_forward_workspace(int B, int T, int C);
 

@@ -158,7 +158,7 @@ int bwd(int B, int T, int C, const Decay4 &w, const void *u, const void *k, cons
 // parallelise, and the time-parallel kernels' barriers cost more than the chain.
 constexpr int PAR_MIN_T = 16;
 // Segments of at least this many tokens hand tile states from forward to backward (part of the ABI, as are the
-// workspace sizes below, which the kernels use only a part of).
+// workspace sizes below: the backward kernels use a part of theirs, the forward kernels none).
 constexpr int CKPT_MIN_T = 128;
 constexpr int PIECE = 64;
 
@@ -252,12 +252,9 @@ extern "C" int wkv4_forward_ckpt(int B, int T, int C, int dtype, const float *w,
     if (!w || !u) return WKV_ERR_NULL;
     if (T > 0 && (!k || !v || !y)) return WKV_ERR_NULL;
     if (dtype != WKV_F32 && dtype != WKV_BF16 && dtype != WKV_F16) return WKV_ERR_DTYPE;
-    if (T >= CKPT_MIN_T) {
-        if (!workspace || workspace_bytes < wkv4_forward_workspace(B, T, C)) return WKV_ERR_WORKSPACE;
-        if (state_ckpt && state_ckpt_bytes < wkv4_state_ckpt_bytes(B, T, C)) return WKV_ERR_WORKSPACE;
-    } else {
-        state_ckpt = nullptr;
-    }
+    (void)workspace; (void)workspace_bytes;      // (no forward kernel uses one)
+    if (T < CKPT_MIN_T) state_ckpt = nullptr;
+    else if (state_ckpt && state_ckpt_bytes < wkv4_state_ckpt_bytes(B, T, C)) return WKV_ERR_WORKSPACE;
     return run_forward(B, T, C, dtype, Decay4{w, -1}, u, k, v, state_in, y, state_out, (float *)state_ckpt, (cudaStream_t)stream);
 }
 

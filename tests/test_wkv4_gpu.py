@@ -203,3 +203,26 @@ def test_every_launch_is_counted(T, forward, backward):
     b = count()
     torch.autograd.grad(y, k, torch.ones_like(y))
     assert (b - a, count() - b) == (forward, backward)
+
+
+@pytest.mark.parametrize("T", [20, 300])
+def test_forward_needs_no_workspace(T):
+    """the C ABI's forward call with none, with a hand-over buffer and without: what it gives with the size it names"""
+    from rwkv_infctx_trainer_b200 import _lib as L
+    lib, st = L.load(), torch.cuda.current_stream().cuda_stream
+    B, C = 2, 40
+    k, v = (torch.randn((B, T, C), device="cuda") for _ in range(2))
+    w, u = -torch.rand(C, device="cuda") - 0.1, torch.randn(C, device="cuda")
+    nck, n = lib.wkv4_state_ckpt_bytes(B, T, C), lib.wkv4_forward_workspace(B, T, C)
+
+    def run(size, handover):
+        y, s1 = torch.empty_like(k), torch.empty((B, C, 3), device="cuda")
+        ws = torch.empty(max(size, 16), dtype=torch.uint8, device="cuda")
+        ck = torch.zeros(max(nck, 16), dtype=torch.uint8, device="cuda")
+        assert lib.wkv4_forward_ckpt(B, T, C, L.WKV_F32, w.data_ptr(), u.data_ptr(), k.data_ptr(), v.data_ptr(), None, y.data_ptr(), s1.data_ptr(),
+                                     ws.data_ptr() if size else None, size, ck.data_ptr() if handover else None, nck if handover else 0, st) == 0
+        return y, s1, ck
+
+    for handover in (False, True):
+        for a, b in zip(run(0, handover), run(n, handover)):
+            assert torch.equal(a, b)
