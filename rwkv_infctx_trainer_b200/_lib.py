@@ -57,17 +57,18 @@ _native = None
 
 
 def native():
-    """The PyTorch binding (``_native.so``, csrc/native_*.cpp): argument checks, allocation and the
-    autograd nodes of the ops, on top of libwkv_b200.so."""
+    """The PyTorch binding (``_wkv_native.so``, csrc/native_*.cpp): argument checks, allocation and the
+    autograd nodes of the ops, on top of libwkv_b200.so.  It is compiled against one torch and one Python: a file
+    that was built from other sources or against others is rebuilt (g++), and never loaded."""
     global _native
     if _native is None:
         load()
         path = _build.NATIVE
         if not _build.native_is_current():
-            if _build.have_nvcc():
-                path = _build.build_native()
-            elif not os.path.exists(path):
-                raise ImportError(f"{path} is missing and there is no compiler to build it")
+            if not _build.have_cxx():
+                raise ImportError(f"{path} is missing, or was built from other sources or against another torch or "
+                                  "Python, and there is no g++ to build it")
+            path = _build.build_native()
         spec = importlib.util.spec_from_file_location(_build.NATIVE_NAME, path)
         mod = importlib.util.module_from_spec(spec)
         spec.loader.exec_module(mod)

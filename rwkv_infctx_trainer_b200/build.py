@@ -29,6 +29,10 @@ def have_nvcc() -> bool:
     return bool(shutil.which("nvcc")) or os.path.exists("/usr/local/cuda/bin/nvcc")
 
 
+def have_cxx() -> bool:
+    return bool(shutil.which("g++"))
+
+
 def _digest(files, *more: str) -> str:
     """sha256 over the names and contents of the files and over the other strings"""
     h = hashlib.sha256()
@@ -54,7 +58,7 @@ def _native_digest() -> str:
     return _digest(files, torch.__version__, sys.version, *NATIVE_FLAGS)
 
 
-NATIVE_FLAGS = ["-O2", "-std=c++17", "-fPIC", "-w", f"-DTORCH_EXTENSION_NAME={NATIVE_NAME}"]
+NATIVE_FLAGS = ["-O2", "-std=c++17", "-fPIC", "-Wall", "-Wextra", f"-DTORCH_EXTENSION_NAME={NATIVE_NAME}"]
 
 
 def native_is_current() -> bool:
@@ -70,7 +74,8 @@ def build_native(force: bool = False) -> str:
         return NATIVE
     import torch
     from torch.utils import cpp_extension
-    incs = [f"-I{p}" for p in cpp_extension.include_paths()] + ["-I/usr/local/cuda/include", f"-I{sysconfig.get_paths()['include']}"]
+    # (-isystem: warnings are for this package's own sources)
+    incs = [f"-isystem{p}" for p in [*cpp_extension.include_paths(), "/usr/local/cuda/include", sysconfig.get_paths()["include"]]]
     bdir = os.path.join(PKG, "build")
     os.makedirs(bdir, exist_ok=True)
     procs, objs = [], []
@@ -84,6 +89,8 @@ def build_native(force: bool = False) -> str:
         out = p.communicate()[0].decode()
         if p.returncode != 0:
             raise RuntimeError(f"g++ failed on {s}:\n{out}")
+        if out:
+            print(out, file=sys.stderr)
     tmp = f"{NATIVE}.{os.getpid()}.tmp"
     tlib = os.path.join(os.path.dirname(torch.__file__), "lib")
     subprocess.check_call(["g++", "-shared", "-o", tmp, *objs, f"-L{PKG}", "-l:libwkv_b200.so", f"-L{tlib}", "-lc10", "-lc10_cuda",

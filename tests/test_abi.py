@@ -82,3 +82,22 @@ def test_handover_buffer_size_without_gpu():
     assert lib.wkv56_state_ckpt_bytes(ctypes.byref(a), 1) == want
     a.dtype = L.WKV_F32          # fp32 I/O runs on the token-serial kernels: nothing to hand over
     assert lib.wkv56_state_ckpt_bytes(ctypes.byref(a), 1) == 0
+
+
+def test_binding_of_another_build_is_not_loaded(monkeypatch):
+    """_wkv_native.so is compiled against one torch: with a digest that does not match it is rebuilt where there is a
+    compiler, whether or not nvcc is there, and refused where there is none"""
+    import pytest
+    build = L._build
+    L.load()
+    rebuilt = []
+    monkeypatch.setattr(L, "_native", None)
+    monkeypatch.setattr(build, "native_is_current", lambda: False)
+    monkeypatch.setattr(build, "have_nvcc", lambda: False)
+    monkeypatch.setattr(build, "build_native", lambda: rebuilt.append(1) or build.NATIVE)
+    monkeypatch.setattr(build, "have_cxx", lambda: False, raising=False)
+    with pytest.raises(ImportError, match="another torch"):
+        L.native()
+    monkeypatch.setattr(build, "have_cxx", lambda: True)
+    L.native()
+    assert rebuilt == [1]
