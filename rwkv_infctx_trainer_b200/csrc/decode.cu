@@ -3,7 +3,8 @@
 // With up to 8 rows every projection is a matrix-vector product: the weights (5 C^2 bf16 for v5/v6) are read once and
 // everything else is small, so the floor is their HBM time (C = 2560: 65 MB, 10 us) and the enemy is the chain's
 // latency: as separate library calls the projections took 8 us each and the block fifteen launches (72 us of GPU
-// time, 126 us in all; now 40).  Here:
+// time, 126 us in all; now 38).  The rows cost shared-memory reads for every output row; how many are taken at which
+// width, and what both sides measure, stands at decode_fits() in native_blocks.cpp.  Here:
 //
 //   v6   strip (x, W1 -> tanh)  ->  mix5 (W2 -> the five mixed inputs)  ->  linear (r, k, v, g and the decay's W1)
 //        ->  step (decay, WKV, group norm, silu gate)  ->  linear (output)
@@ -371,7 +372,10 @@ int strip_launch(const Strip &P, cudaStream_t s) {
 }
 template <int MT>
 int linear_launch(const Linear &P, int ctas, cudaStream_t s) {
-    // (10 chunks of 8 x 32 weights: rows of up to 2560; wider rows prefetch the same and stream the rest)
+    // 10 chunks of 8 x 32 weights: rows of up to 2560 are prefetched whole, wider rows stream the rest.  One row, us with 3 / 6 /
+    // 10 / 16 chunks ahead: v6 C = 768 19.4 / 19.5 / 19.4 / 20.8, C = 2560 38.3 / 36.8 / 36.6 / 41.7, C = 4096 59.3 / 57.7 / 62.5 /
+    // 60.9; v5 8.9 / 9.0 / 9.4 / 11.1, 27.3 / 25.7 / 23.7 / 31.0, 46.3 / 44.5 / 51.6 / 47.8.  (A row that does not fit is better off with
+    // 6: registers it cannot use up cost warps.)
     static unsigned char done[64];
     if (!set_max_smem_once(k_dec_linear<MT, 10>, MAX_SMEM, done)) return WKV_ERR_LAUNCH;
     return launch_chained(k_dec_linear<MT, 10>, dim3(ctas), dim3(256), (size_t)MT * P.C * 2, s, P);

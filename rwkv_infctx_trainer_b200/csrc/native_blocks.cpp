@@ -120,9 +120,21 @@ struct Out {
     Tensor out, shift, state;
 };
 
-// whether decode.cu takes the call: one token of a few rows, widths its shared memory holds
+// Whether decode.cu takes the call: one token of a few rows, at widths where its matrix-vector kernel beats the library's
+// GEMMs.  It reads the input rows from shared memory again for every output row (1, 2, 4 or 8 of them, the next that
+// holds M), so the line falls with the width.  One block of a chain over cold weights, us, decode kernels / library path,
+// as a CUDA graph (called from Python the library path is 13 to 80 us longer, the decode kernels 3):
+//             v6  M=1        M=2        M=4        M=8           v5  M=1        M=2        M=4        M=8
+//   C = 768       19 / 49    22 / 49    24 / 49    30 / 50           10 / 33    10 / 33    12 / 32    16 / 33
+//   C = 2048                            38 / 69    53 / 69                                 31 / 48    49 / 48
+//   C = 2560      37 / 76    42 / 73    49 / 74    76 / 74           24 / 54    28 / 54    39 / 53    75 / 53
+//   C = 4096      62 / 108   66 / 105   84 / 105   138 / 106         52 / 83    59 / 80    85 / 79    167 / 82
+//   C = 6144     101 / 114  116 / 120  163 / 121   291 / 125         92 / 89   117 / 90   181 / 91    405 / 95
+//   C = 8192     162 / 171  197 / 174  268 / 174                    162 / 138  202 / 138  322 / 137
+// (M = 5 takes what 8 takes: the rule is by the kernels' row counts.)
 bool decode_fits(const Tensor &x, int64_t att) {
-    return x.size(1) == 1 && x.size(0) >= 1 && x.size(0) <= wkvx_decode_max_rows() && x.size(2) % 8 == 0 && x.size(2) <= 8192 && att <= 8192;
+    const int64_t M = x.size(0), width = std::max(x.size(2), att);
+    return x.size(1) == 1 && M >= 1 && M <= wkvx_decode_max_rows() && x.size(2) % 8 == 0 && width <= (M == 1 ? 6144 : M <= 4 ? 4096 : 2048);
 }
 
 // ------------------------------------------------------------------------------ v6

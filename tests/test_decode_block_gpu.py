@@ -37,3 +37,23 @@ def test_decode_steps_match_the_same_tokens_in_one_call(cls, B, H, dtype):
     assert rel(got, want) < 1e-2
     assert rel(state[1], wk) < 5e-3
     assert torch.equal(state[0], ws)
+
+
+@pytest.mark.parametrize("cls", ["RWKV_TimeMix6_0", "RWKV_TimeMix"])
+@pytest.mark.parametrize("B,H,own", [(1, 96, True), (1, 97, False), (2, 64, True), (2, 65, False), (4, 64, True), (4, 65, False), (5, 32, True),
+                                     (5, 33, False), (8, 32, True), (8, 33, False), (9, 2, False)])
+def test_rows_and_widths_on_both_sides_of_the_rule(cls, B, H, own):
+    """which call runs on the decode kernels (no library product at all), and that both sides give what the same token gives
+    as the first of two"""
+    C = 64 * H
+    blk = _block(cls, C, H, torch.bfloat16)
+    x = torch.randn((B, 2, C), device="cuda").bfloat16()
+    state = (torch.randn((B, C), device="cuda").bfloat16(), torch.randn((B, H, 64, 64), device="cuda"))
+    rel = lambda a, b: float((a.float() - b.float()).norm() / b.float().norm())
+    with torch.no_grad(), torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CPU]) as prof:
+        got, _ = blk(x[:, :1], state)
+    products = sum(e.count for e in prof.key_averages() if e.key in ("aten::mm", "aten::addmm", "aten::bmm"))
+    assert (products == 0) == own
+    with torch.no_grad():
+        want, _ = blk(x, state)
+    assert rel(got, want[:, :1]) < 1e-2
