@@ -418,13 +418,22 @@ SerialParams make_params(const wkv_args_t *a) {
     return P;
 }
 
-// Which shape, from the number of chains (heads x rows x roles) an SM gets: with one-warp CTAs of NC = 1 a
-// chain costs the SM's shared-memory port 8 x 48 cycles a token, with NC = 2 half, with NC = 4 a quarter;
-// alone, they take about 100, 130 and 250 cycles a token.
+// Which shape, from the heads x rows the SMs get: with one-warp CTAs of NC = 1 a chain costs the SM's shared-memory port
+// 8 x 48 cycles a token, with NC = 2 half, with NC = 4 a quarter; alone, they take about 100, 130 and 250 cycles a token.
+// Measured, us for the shapes 1 / 2 / 4:
+//   forward, 128 tokens fp32   37 heads 14.0 / 19.8 / 33.1     74: 20.7 / 20.0 / 33.2    100: 37.7 / 28.9 / 33.2
+//                             256: 76.0 / 35.6 / 48.7         296: 77.8 / 36.2 / 48.9    340: 96.1 / 53.5 / 54.3
+//   forward, bf16              60 heads 4.7 / 5.1 / 6.3 (T = 16), 3.7 / 3.7 / 4.3 (T = 8), 3.4 / 3.1 / 3.3 (T = 4)
+//                             256: 14.2 / 7.6 / 8.2 (T = 16), 10.2 / 5.5 / 5.4 (T = 8), 9.4 / 4.5 / 4.2 (T = 4), 7.0 / 3.7 / 3.1 (T = 1)
+//   backward, 128 tokens fp32  10 heads 26.2 / 30.1 / 34.6     12: 31.3 / 29.9 / 34.6     60: 75.9 / 45.7 / 65.3
+//                             148: 147 / 79.1 / 87.1          296: 289 / 123 / 125       340: 334 / 159 / 134
+// so NC = 1 up to half a head per SM forward and a fourteenth backward (three roles, and both rows and columns of the
+// state to read), NC = 2 up to two heads per SM, but not for calls so short that the state is most of the work.
 enum { SHAPE_1, SHAPE_2, SHAPE_4 };
-int pick_shape(const wkv_args_t *a, int roles) {
-    const long long chains = (long long)a->B * a->H * roles, sms = device_sm_count();
-    return chains * 2 <= sms ? SHAPE_1 : chains * 5 <= sms * 6 ? SHAPE_2 : SHAPE_4;
+int pick_shape(const wkv_args_t *a, bool backward) {
+    const long long heads = (long long)a->B * a->H, sms = device_sm_count();
+    if (heads * (backward ? 14 : 2) <= sms) return SHAPE_1;
+    return heads <= 2 * sms && (backward || a->T >= 12) ? SHAPE_2 : SHAPE_4;
 }
 
 template <typename F, int WSRC>
@@ -432,7 +441,7 @@ int launch_fwd(const wkv_args_t *a, bool floor, cudaStream_t s) {
     SerialParams P = make_params(a);
     P.floor = floor;
     const int bh = a->B * a->H;
-    switch (pick_shape(a, 1)) {
+    switch (pick_shape(a, false)) {
         case SHAPE_1: return launch_chained(k_serial_fwd<F, WSRC, 1, 1>, dim3(bh * 8), dim3(64), 0, s, P);
         case SHAPE_2: return launch_chained(k_serial_fwd<F, WSRC, 2, 2>, dim3(bh * 2), dim3(96), 0, s, P);
         default: return launch_chained(k_serial_fwd<F, WSRC, 4, 2>, dim3(bh), dim3(96), 0, s, P);
@@ -455,7 +464,7 @@ int launch_bwd(const wkv_args_t *a, cudaStream_t s) {
     P.q = (float *)a->workspace; P.p = P.q + n; P.eT = P.p + n;
     const int bh = a->B * a->H;
     int err;
-    switch (pick_shape(a, 3)) {
+    switch (pick_shape(a, true)) {
         case SHAPE_1: err = launch_chained(k_serial_bwd<F, WSRC, 1, 1>, dim3(bh * 8, 3), dim3(64), 0, s, P); break;
         case SHAPE_2: err = launch_chained(k_serial_bwd<F, WSRC, 2, 2>, dim3(bh * 2, 3), dim3(96), 0, s, P); break;
         default: err = launch_chained(k_serial_bwd<F, WSRC, 4, 2>, dim3(bh, 3), dim3(96), 0, s, P);

@@ -12,10 +12,12 @@ import test_wkv56_gpu as TW
 pytestmark = pytest.mark.gpu
 
 
-# 8 heads x rows: one-warp shape; 80 and 120 chains forward: two-column shape; 200: four-column shape
+# up to 10 heads x rows: the one-warp shape both ways; 80 to 200: the two-column shape (forward from 12 tokens on, under that
+# the four-column shape); 300: the four-column shape
 @pytest.mark.parametrize("variant,B,T,H,layout", [
     ("v6", 1, 1, 1, 0), ("v6", 2, 7, 4, 1), ("v6", 1, 8, 8, 0), ("v5", 1, 9, 8, 1), ("v6", 1, 33, 2, 0), ("v5", 2, 41, 2, 0),
-    ("v6", 4, 17, 20, 0), ("v6", 4, 9, 30, 1), ("v5", 4, 10, 20, 0), ("v6", 5, 19, 40, 1), ("v5", 5, 9, 40, 0)])
+    ("v6", 4, 17, 20, 0), ("v6", 4, 9, 30, 1), ("v5", 4, 10, 20, 0), ("v6", 5, 19, 40, 1), ("v5", 5, 9, 40, 0),
+    ("v6", 6, 11, 50, 0), ("v5", 6, 13, 50, 1), ("v6", 4, 12, 30, 0), ("v6", 1, 12, 11, 1)])
 def test_serial_kernels_match_oracle(variant, B, T, H, layout):
     import rwkv_infctx_trainer_b200 as W
     q = TL.case56(variant, B, T, H, torch.float32, seed=700 + T)
