@@ -19,8 +19,8 @@
 // the state at the start of every tile (3 floats per 8 tokens).  gw needs no running derivative across
 // tiles: with the true gradient at its own tile's end a tile's contribution is complete.
 //
-// The CTAs (B * C/16 of them) are all resident at once at the sizes that matter (7 CTAs of 64 threads per SM), so
-// nothing waits for a second wave; with few of them the slab is made longer (NT 16, 32) and the walk shorter.
+// The slab is as long as leaves the CTAs (B * C/16 of them) all resident at once (see pick_tiles), so that nothing waits for a
+// second wave and the walk is short.
 // Issue slots and HBM time are of the same size here, so the inner loops work on channel pairs: the packed fp32
 // instructions (fma.f32x2) take two channels each, and so does every address, load and store.
 //
@@ -684,12 +684,25 @@ __global__ void __launch_bounds__(NT * CP, NT == 8 ? 7 : NT == 16 ? 3 : 1) k_v4_
     }
 }
 
-// Tiles per slab: 8 (7 CTAs of 64 threads per SM) once the CTAs alone fill the SMs; else longer slabs, and never
-// much longer than the segment.
-int pick_tiles(int B, int T, int C) {
+// Tiles per slab.  Longer slabs make the walk over the row shorter and the barriers fewer, and put fewer CTAs on an SM (8, 4
+// or 2 of 8, 16 or 32 tiles forward; 7, 3 or 1 backward); a slab much longer than the segment is idle.  The longest that
+// has its CTAs resident at once, then -- except that backward beyond 256 tokens is better off in several waves of 16 than of
+// 8, which have twice the barriers and carried states per token.  us for 8 / 16 / 32 tiles, fp32, C = 2048:
+//              T = 64        128           256           1024               T = 64      128          256          1024
+//   fwd B = 1  3.5/4.1/4.5   5.1/4.1/4.7   8.2/5.7/4.6   26/16/11    bwd    7.2/9.5/11  7.8/4.9/5.9  14/7.3/5.9   48/22/15
+//       B = 2                5.9/5.1/6.7   8.9/7.1/6.9   27/19/16                       8.6/6.5/12   15/9.1/12    60/27/31
+//       B = 4  5.0/6.5/11    6.7/6.7/11    10/9.6/12     32/27/32           9.3/22/42   10/11/22     17/17/21     77/53/60
+//       B = 8  6.3/11/19     8.8/11/20     14/17/21      84/87/98 *         12/32/72    14/17/38     27/28/42     199/153/189 *
+// (* T = 2048.  bf16 has the same order, within a percent, at each of them.)
+int pick_tiles(int B, int T, int C, bool backward) {
     const long long ctas = (long long)B * ((C + CT - 1) / CT), sms = device_sm_count();
-    if (ctas >= 4 * sms || T <= 64) return 8;
-    return ctas >= 2 * sms || T <= 128 ? 16 : 32;
+    if (T <= 64) return 8;
+    if (backward) {
+        if (ctas <= sms && T > 128) return 32;
+        return ctas <= 3 * sms || T > 256 ? 16 : 8;
+    }
+    if (ctas <= 2 * sms && T > 128) return 32;
+    return ctas <= 4 * sms ? 16 : 8;
 }
 
 template <class K>
@@ -728,7 +741,7 @@ bool rows_aligned(const Par &P) {
 template <typename F>
 int forward_as(const Par &P, bool states, cudaStream_t s) {
     if (!rows_aligned<F>(P)) return launch_fwd<F, 16, false>(P, states, s);
-    switch (pick_tiles(P.B, P.T, P.C)) {
+    switch (pick_tiles(P.B, P.T, P.C, false)) {
         case 8: return launch_fwd<F, 8, true>(P, states, s);
         case 16: return launch_fwd<F, 16, true>(P, states, s);
         default: return launch_fwd<F, 32, true>(P, states, s);
@@ -737,7 +750,7 @@ int forward_as(const Par &P, bool states, cudaStream_t s) {
 template <typename F>
 int backward_as(Par P, float *scratch, cudaStream_t s) {
     const bool aligned = rows_aligned<F>(P) && aligned16(scratch);
-    const int nt = aligned ? pick_tiles(P.B, P.T, P.C) : 16;
+    const int nt = aligned ? pick_tiles(P.B, P.T, P.C, true) : 16;
     if (!P.fine && P.T > nt * TK) {
         // nothing was handed over and there is more than one slab: the states every 64 tokens first
         P.coarse = scratch;

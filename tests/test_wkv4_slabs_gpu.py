@@ -26,7 +26,8 @@ def spread(c, how):
 @pytest.mark.parametrize("B,T,C,dtype", [
     (1, 16, 16, torch.float32), (2, 17, 24, torch.bfloat16), (1, 63, 40, torch.float32), (2, 64, 20, torch.bfloat16),
     (1, 65, 7, torch.float32), (1, 129, 9, torch.float32), (1, 127, 16, torch.float32), (1, 128, 32, torch.bfloat16), (3, 257, 48, torch.float32),
-    (1, 511, 16, torch.bfloat16), (2, 300, 1, torch.float32), (4, 200, 1264, torch.float32), (8, 136, 1200, torch.bfloat16)])
+    (1, 511, 16, torch.bfloat16), (2, 300, 1, torch.float32), (4, 200, 1264, torch.float32), (8, 136, 1200, torch.bfloat16),
+    (8, 260, 960, torch.float32), (8, 256, 960, torch.bfloat16), (4, 130, 2384, torch.float32)])
 def test_v4_matches_oracle(B, T, C, dtype, how):
     import rwkv_infctx_trainer_b200 as W
     from rwkv_infctx_trainer_b200 import _lib as L
