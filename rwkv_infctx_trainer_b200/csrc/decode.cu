@@ -26,37 +26,15 @@ namespace {
 typedef __nv_bfloat16 bf16;
 constexpr float LOG_FLOOR = -5.298317367f;   // log(0.005), as in the chunked WKV kernels
 
-__device__ __forceinline__ void unpack8(const uint4 &q, float *f) {
-    const uint32_t w[4] = {q.x, q.y, q.z, q.w};
-#pragma unroll
-    for (int i = 0; i < 4; i++) {
-        f[2 * i] = __uint_as_float(w[i] << 16);
-        f[2 * i + 1] = __uint_as_float(w[i] & 0xFFFF0000u);
-    }
-}
-__device__ __forceinline__ uint32_t pack2(float a, float b) {
-    __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
-    return *reinterpret_cast<uint32_t *>(&h);
-}
-__device__ __forceinline__ uint4 pack8(const float *f) {
-    return make_uint4(pack2(f[0], f[1]), pack2(f[2], f[3]), pack2(f[4], f[5]), pack2(f[6], f[7]));
-}
-__device__ __forceinline__ float rbf(float x) { return __bfloat162float(__float2bfloat16_rn(x)); }
 __device__ __forceinline__ float param(const void *p, int dtype, size_t i) {
     return dtype == WKV_F32 ? ((const float *)p)[i] : dtype == WKV_BF16 ? __bfloat162float(((const bf16 *)p)[i]) : __half2float(((const __half *)p)[i]);
 }
-__device__ __forceinline__ float sigmoidf(float x) { return __fdividef(1.f, 1.f + __expf(-x)); }
 // tanh to a few fp32 roundings of its value for every x (1 - 2 / (1 + e^{2x}) is that close to 1 only: for small x the
 // difference cancels, and under 6e-8 it is zero; low-rank maps start out with such values).  With E = e^{-2|x|} - 1:
 // tanh|x| = -E / (2 + E).
 __device__ __forceinline__ float tanh_full(float x) {
     const float e = expm1f(-2.f * fabsf(x));
     return copysignf(__fdividef(-e, 2.f + e), x);
-}
-__device__ __forceinline__ float warp_sum(float v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    return v;
 }
 
 // x + (shift - x) * maa for 8 channels; one_minus: the parameter is 1 - maa
@@ -106,7 +84,7 @@ __device__ __forceinline__ void strip(const bf16 *W, int ldw, int n0, const bf16
         float s = 0.f;
 #pragma unroll
         for (int g = 0; g < 8; g++) s += red[g][m][q];
-        if (m < M) out[(size_t)m * ldw + n0 + q] = __float2bfloat16_rn(tanh_full(rbf(s)));
+        if (m < M) out[(size_t)m * ldw + n0 + q] = __float2bfloat16_rn(tanh_full(bf16_round(s)));
     }
 }
 
@@ -190,7 +168,7 @@ __global__ void __launch_bounds__(128) k_dec_mix5(const Mix5 P) {
 #pragma unroll
         for (int q = 0; q < 8; q++) {
             const int i = lane * 8 + q;
-            const float md = rbf((part[0][m][i] + part[1][m][i]) + (part[2][m][i] + part[3][m][i]));
+            const float md = bf16_round((part[0][m][i] + part[1][m][i]) + (part[2][m][i] + part[3][m][i]));
             x[q] += (s[q] - x[q]) * (param(P.maa[n], P.dtype, c + q) + md);
         }
         *reinterpret_cast<uint4 *>(P.out + ((size_t)n * P.M + m) * P.C + c) = pack8(x);
@@ -322,7 +300,7 @@ __global__ void __launch_bounds__(256) k_dec_step(const Step P) {
     __syncthreads();
     if (g4 == 0) {
         float x;
-        if (V6) x = rbf(param(P.decay, P.decay_dtype, h * 64 + c) + ((wpart[0][c] + wpart[1][c]) + (wpart[2][c] + wpart[3][c])));
+        if (V6) x = bf16_round(param(P.decay, P.decay_dtype, h * 64 + c) + ((wpart[0][c] + wpart[1][c]) + (wpart[2][c] + wpart[3][c])));
         else x = param(P.decay, P.decay_dtype, h * 64 + c);
         sw[c] = __expf(fmaxf(-__expf(x), LOG_FLOOR));
     }
@@ -349,7 +327,7 @@ __global__ void __launch_bounds__(256) k_dec_step(const Step P) {
         float y = 0.f;
 #pragma unroll
         for (int j = 0; j < 16; j++) y += part[j][c];
-        y = rbf(y);
+        y = bf16_round(y);
         // the 64 channels sit in two warps
         const float s = warp_sum(y);
         if ((tid & 31) == 0) red[tid >> 5] = s;
@@ -359,7 +337,7 @@ __global__ void __launch_bounds__(256) k_dec_step(const Step P) {
         asm volatile("bar.sync 1, 64;" ::: "memory");
         const float rstd = rsqrtf((red[2] + red[3]) * (1.f / 64.f) + P.eps), gr = __bfloat162float(P.g[at]);
         const float o = d * rstd * param(P.lw, P.ln_dtype, h * 64 + c) + param(P.lb, P.ln_dtype, h * 64 + c);
-        P.out[at] = __float2bfloat16_rn(o * rbf(gr * sigmoidf(gr)));
+        P.out[at] = __float2bfloat16_rn(o * bf16_round(gr * sigmoidf(gr)));
     }
 }
 

@@ -24,21 +24,6 @@ namespace {
 
 constexpr int TPB = 256;
 
-__device__ __forceinline__ void unpack8(const uint4 &q, float *f) {
-    const uint32_t w[4] = {q.x, q.y, q.z, q.w};
-#pragma unroll
-    for (int i = 0; i < 4; i++) {
-        f[2 * i] = __uint_as_float(w[i] << 16);
-        f[2 * i + 1] = __uint_as_float(w[i] & 0xFFFF0000u);
-    }
-}
-__device__ __forceinline__ uint32_t pack2(float a, float b) {
-    __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
-    return *reinterpret_cast<uint32_t *>(&h);
-}
-__device__ __forceinline__ uint4 pack8(const float *f) {
-    return make_uint4(pack2(f[0], f[1]), pack2(f[2], f[3]), pack2(f[4], f[5]), pack2(f[6], f[7]));
-}
 // sum over the 8 lanes that hold one head's 64 channels
 __device__ __forceinline__ float head_sum(float v) {
     v += __shfl_xor_sync(0xffffffffu, v, 1);
@@ -60,13 +45,6 @@ __device__ __forceinline__ void load8(const void *p, int dtype, size_t at, float
         for (int i = 0; i < 4; i++) { const float2 v = __half22float2(q[i]); f[2 * i] = v.x; f[2 * i + 1] = v.y; }
     }
 }
-__device__ __forceinline__ void store_as(void *p, int dtype, size_t i, float x) {
-    if (dtype == WKV_F32) ((float *)p)[i] = x;
-    else if (dtype == WKV_BF16) ((__nv_bfloat16 *)p)[i] = __float2bfloat16_rn(x);
-    else ((__half *)p)[i] = __float2half_rn(x);
-}
-__device__ __forceinline__ float sigmoidf(float x) { return __fdividef(1.f, 1.f + __expf(-x)); }
-__device__ __forceinline__ float bf16_round(float x) { return __bfloat162float(__float2bfloat16_rn(x)); }
 
 // Work split shared by the kernels: the C channels are cut into column blocks of 256 (a warp's
 // 32 lanes x 8 channels = 4 heads); blockIdx.x = column block + ncb * token slot; the 8 warps of

@@ -163,11 +163,6 @@ constexpr int CKPT_MIN_T = 128;
 constexpr int PIECE = 64;
 
 // gw_sum, gu_sum [C]: the per-batch partials [B,C] summed over the batch, in the parameters' element types
-__device__ __forceinline__ void store_as(void *p, int dtype, int i, float x) {
-    if (dtype == WKV_F32) ((float *)p)[i] = x;
-    else if (dtype == WKV_BF16) ((__nv_bfloat16 *)p)[i] = __float2bfloat16_rn(x);
-    else ((__half *)p)[i] = __float2half_rn(x);
-}
 __global__ void __launch_bounds__(THREADS)
 k_v4_fold(const float *__restrict__ gw, const float *__restrict__ gu, void *gw_sum, int gw_dtype, void *gu_sum, int gu_dtype,
           int B, int C) {

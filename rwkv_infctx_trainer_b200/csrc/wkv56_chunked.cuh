@@ -18,21 +18,6 @@ constexpr float LW_FLOOR = -5.298317367f;  // log(0.005)
 
 struct __align__(16) Tile { unsigned char b[TILE_BYTES]; };
 
-__device__ __forceinline__ uint32_t pack2(float a, float b) {
-    __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
-    return *reinterpret_cast<uint32_t *>(&h);
-}
-__device__ __forceinline__ void unpack8(const uint4 &q, float *f) {
-    const uint32_t w[4] = {q.x, q.y, q.z, q.w};
-#pragma unroll
-    for (int i = 0; i < 4; i++) {
-        f[2 * i] = __uint_as_float(w[i] << 16);
-        f[2 * i + 1] = __uint_as_float(w[i] & 0xFFFF0000u);
-    }
-}
-__device__ __forceinline__ uint4 pack8(const float *f) {
-    return make_uint4(pack2(f[0], f[1]), pack2(f[2], f[3]), pack2(f[4], f[5]), pack2(f[6], f[7]));
-}
 __device__ __forceinline__ uint4 ld_tile(const Tile &t, int row, int chunk) {
     return *reinterpret_cast<const uint4 *>(t.b + tile_off(row, chunk));
 }

@@ -97,12 +97,6 @@ template <> struct Two<__half> {
     static __device__ __forceinline__ float2 f(__half2 v) { return __half22float2(v); }
 };
 
-__device__ __forceinline__ float warp_sum(float v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    return v;
-}
-
 // element (i of 16, n of NC) of the state: reduced index 16*(i/4) + 4*q + i%4, other index o0 + n
 __device__ __forceinline__ int red_index(int i, int q) { return 16 * (i >> 2) + 4 * q + (i & 3); }
 

@@ -8,12 +8,6 @@
 namespace wkv {
 namespace {
 
-__device__ __forceinline__ void store_as(void *p, int dtype, int i, float x) {
-    if (dtype == WKV_F32) ((float *)p)[i] = x;
-    else if (dtype == WKV_BF16) ((__nv_bfloat16 *)p)[i] = __float2bfloat16_rn(x);
-    else ((__half *)p)[i] = __float2half_rn(x);
-}
-
 // One CTA per (head, parameter): 16 groups of 64 threads (a channel each) take every 16th of the
 // B*n rows, the groups meet in shared memory in a fixed order.  Latency-bound (a few hundred KB from
 // L2): the width is there to have many loads in flight.

@@ -29,6 +29,35 @@ template <> struct Elem<__half> {
     static __device__ __forceinline__ void st(__half *p, float x) { *p = __float2half_rn(x); }
 };
 
+// ---- bf16 values in 32-bit words, element types chosen at run time, sums over a warp
+__device__ __forceinline__ void unpack8(const uint4 &q, float *f) {
+    const uint32_t w[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        f[2 * i] = __uint_as_float(w[i] << 16);
+        f[2 * i + 1] = __uint_as_float(w[i] & 0xFFFF0000u);
+    }
+}
+__device__ __forceinline__ uint32_t pack2(float a, float b) {
+    __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
+    return *reinterpret_cast<uint32_t *>(&h);
+}
+__device__ __forceinline__ uint4 pack8(const float *f) {
+    return make_uint4(pack2(f[0], f[1]), pack2(f[2], f[3]), pack2(f[4], f[5]), pack2(f[6], f[7]));
+}
+__device__ __forceinline__ float bf16_round(float x) { return __bfloat162float(__float2bfloat16_rn(x)); }
+__device__ __forceinline__ void store_as(void *p, int dtype, size_t i, float x) {
+    if (dtype == WKV_F32) ((float *)p)[i] = x;
+    else if (dtype == WKV_BF16) ((__nv_bfloat16 *)p)[i] = __float2bfloat16_rn(x);
+    else ((__half *)p)[i] = __float2half_rn(x);
+}
+__device__ __forceinline__ float warp_sum(float v) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+__device__ __forceinline__ float sigmoidf(float x) { return __fdividef(1.f, 1.f + __expf(-x)); }
+
 // Two fp32 values per instruction (fma.f32x2): half the issue slots of the scalar forms, same rounding.
 typedef float2 f2;
 __device__ __forceinline__ unsigned long long bits(const f2 &a) { return *reinterpret_cast<const unsigned long long *>(&a); }
