@@ -517,7 +517,7 @@ std::tuple<Tensor, Tensor, Tensor> block(int64_t version, const Tensor &x_, cons
     for (const Tensor &p : params) require_cuda({&x_, &p});
     const Tensor x = x_.to(BF16).contiguous(), shift = shift_.to(BF16).contiguous();
     Tensor state = state_.to(at::kFloat).contiguous();
-    if (version != 4 && state.dim() != 4) state = state.view({B, H, HEAD, HEAD});
+    if (version != 4 && state.sizes() != at::IntArrayRef({B, H, HEAD, HEAD})) state = state.view({B, H, HEAD, HEAD});
     bool grad = wants_grad({&x, &shift, &state});
     if (!grad && at::GradMode::is_enabled())
         for (const Tensor &p : params) grad |= p.requires_grad();

@@ -106,3 +106,24 @@ def test_parameters_that_are_slices_of_a_flat_buffer(version, dtype):
     rel = lambda a, b: float((a.float() - b.float()).norm() / b.float().norm().clamp_min(1e-30))
     for a, b in zip(run(), want):
         assert a.shape == b.shape and rel(a.detach(), b.detach()) < 1e-2      # (a library GEMM may pick another kernel for such an operand)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("version", [5, 6])
+@pytest.mark.parametrize("T", [1, 20])
+@pytest.mark.parametrize("shape", [(B * H, 64, 64), (B * H, 1, 64, 64), (B, H * 64 * 64)])
+def test_state_of_the_same_size_in_another_shape(version, T, shape):
+    """the state is taken by its elements; what comes back is [B,H,64,64], and its gradient has the shape it was given in"""
+    blk = make(version, "cuda").bfloat16()
+    x, shift = torch.randn((B, T, C), device="cuda").bfloat16(), torch.randn((B, C), device="cuda").bfloat16()
+    state = torch.randn((B, H, 64, 64), device="cuda")
+    with torch.no_grad():
+        want, (_, ws) = call(version, blk, x, shift, state)
+        got, (_, s) = call(version, blk, x, shift, state.view(shape))
+        assert s.shape == ws.shape == (B, H, 64, 64) and torch.equal(got, want) and torch.equal(s, ws)
+    grads = []
+    for st in (state, state.view(shape)):
+        leaf = st.clone().requires_grad_(True)
+        out, (_, s) = call(version, blk, x, shift, leaf)
+        grads += torch.autograd.grad((out, s), leaf, (torch.ones_like(out), torch.ones_like(s)))
+    assert grads[1].shape == shape and torch.equal(grads[0].view(shape), grads[1])
