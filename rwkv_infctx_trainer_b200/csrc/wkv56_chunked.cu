@@ -72,10 +72,10 @@ struct FwdParams {
     int G, L;                 // time groups per chain, chunks per group (the last group may be shorter)
     const __nv_bfloat16 *u;
     const float *wvec;        // v5: per-channel decay parameter [H*64]
-    const float *state_in;    // the caller's state (layout `layout`); pass C with `fold`: only whether there is one
-    const float *gstart;      // or NULL: [B*H*G, 64*64] state at the start of every group (order: carried_at)
+    const float *state_in;    // the caller's state (layout `layout`), or NULL
+    const float *gstart;      // or NULL: [B*H*G, 64*64] state at the start of every group, or (fold) of the chain (order: carried_at)
     const float *grestart;    // or NULL: the same from an earlier call ([key,value])
-    int fold;                 // pass C without gstart: start from the copy of state_in and the gU, gD of the groups before
+    int fold;                 // pass C: from the chain's start, by the gU, gD of the groups before
     float *state_out;         // written by the CTA whose group ends the segment
     float *gU;                // [B*H*G, 64*64] state a group builds from zero (order: carried_at): pass A writes,
     float *gD;                // [B*H*G, 64] decay of a whole group per key channel           pass C may read
@@ -278,23 +278,16 @@ k_chunk_fwd(const __grid_constant__ CUtensorMap map_r, const __grid_constant__ C
         float S[16];
 #pragma unroll
         for (int q = 0; q < 16; q++) S[q] = 0.f;
-        const size_t init = ((size_t)bh * P.G + P.G - 1) * 4096;     // where gU holds the copy of state_in (time groups)
-        if (summary) {
-            if (P.state_in && grp == 0) {
-                load_state_row<16>(S, P.state_in + sbase, P.layout, row, vcol0);
-                store_carried<16>(S, P.gU + init, 4 * wg, tid & 127);
-#pragma unroll
-                for (int q = 0; q < 16; q++) S[q] = 0.f;
-            }
-        } else if (P.grestart) {
-            load_state_row<16>(S, P.grestart + (size_t)unit * 4096, WKV_STATE_KV, row, vcol0);
-        } else if (P.gstart) {
-            load_carried<16>(S, P.gstart + (size_t)unit * 4096, 4 * wg, tid & 127);
-        } else if (P.fold) {
-            if (P.state_in) load_carried<16>(S, P.gU + init, 4 * wg, tid & 127);
-            fold_groups<16>(S, P.gU, P.gD, (size_t)bh * P.G, 1, grp, row, 4 * wg, tid & 127);
-        } else if (P.state_in) {
+        if (P.grestart) load_state_row<16>(S, P.grestart + (size_t)unit * 4096, WKV_STATE_KV, row, vcol0);
+        else if (P.state_in && !summary) load_state_row<16>(S, P.state_in + sbase, P.layout, row, vcol0);
+        // (with the fold the start is one for the whole chain: the last group's place)
+        if (!summary && P.gstart) load_carried<16>(S, P.gstart + (size_t)(P.fold ? bh * P.G + P.G - 1 : unit) * 4096, 4 * wg, tid & 127);
+        if (!summary && P.fold) fold_groups<16>(S, P.gU, P.gD, (size_t)bh * P.G, 1, grp, row, 4 * wg, tid & 127);
+        if (summary && P.state_in && grp == 0) {
             load_state_row<16>(S, P.state_in + sbase, P.layout, row, vcol0);
+            store_carried<16>(S, P.gU + (size_t)(bh * P.G + P.G - 1) * 4096, 4 * wg, tid & 127);
+#pragma unroll
+            for (int q = 0; q < 16; q++) S[q] = 0.f;
         }
         float dprod = 1.f;      // summary pass: decay of the whole group for key channel `row`
         float lwc[4], wc[4];
@@ -871,9 +864,9 @@ int chunked_forward_impl(const wkv_args_t *a, bool per_token_w, void *state_ckpt
     // C (or the whole job when the chains are not split)
     if (!set_max_smem_once(kerns[pt][mode], (int)smem, attr_done[pt][mode])) return WKV_ERR_LAUNCH;
     p.grestart = restart ? (const float *)a->group_states : nullptr;
-    p.gstart = !restart && gp.G > GROUP_FOLD_MAX ? (const float *)(g + GL.gstart) : nullptr;
-    p.state_in = p.gstart ? nullptr : a->state_in;
     p.fold = !restart && gp.G > 1 && gp.G <= GROUP_FOLD_MAX;
+    p.gstart = restart ? nullptr : gp.G > GROUP_FOLD_MAX ? (const float *)(g + GL.gstart) : p.fold && a->state_in ? (const float *)(g + GL.gU) : nullptr;
+    p.state_in = gp.G > 1 ? nullptr : a->state_in;
     p.state_out = a->state_out;      // written by the group that ends the segment
     if (!p.fold) { p.gU = nullptr; p.gD = nullptr; }
     p.y = (__nv_bfloat16 *)a->y;
