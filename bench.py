@@ -345,7 +345,7 @@ def run_ours(args):
     # Software pipeline over steps: while step s computes, the inputs of step s+1 are copied
     # in on one side stream and the results of step s-1 are copied out on another (PCIe is
     # full duplex).  Every step's host->device and device->host copies are inside the timed
-    # region; the ops are called through the public autograd Function.
+    # region; the ops are called through the public autograd ops.
     in_s, out_s = torch.cuda.Stream(device), torch.cuda.Stream(device)
     names_in, names_g = ("r", "k", "v", "w", "gy"), ("gr", "gk", "gv", "gw")
 
