@@ -47,12 +47,13 @@ using namespace chunked;
 // the chunk's own contribution U_j = khat_j^T V_j, which does not depend on the state, so the
 // serial chain per chunk is one fused multiply-add per state element.
 struct FwdSmem {
-    Tile in[2][4];     // per stage: r, k, v, w  (r,k,w are overwritten in place by
-                       // r*fr, k*fk, r*e^{cp})
-    Tile x, khat[2], atil, sbf;   // khat is double-buffered: chunk j+1 is prepared while the
+    Tile in[2][4];     // per stage: r, k, v, w  (r and k are overwritten in place by the operands of the
+                       // scores, in a steep chunk w by r*e^{cp})
+    Tile x, khat[2], atil, sbf;   // x: steep chunks.  khat is double-buffered: chunk j+1 is prepared while the
                                   // state product of chunk j may still read khat of chunk j
     float dpart[4][CH];    // score-diagonal partials per token
     float dvec[2][CH];     // decay of the whole chunk per key channel, by chunk parity
+    float hvec[2][CH];     // scale of the chunk-start state that is left for the backward pass (see CkptLayout)
     float wtot[8][CH];     // log2-decay total of each warp's 8 tokens, per channel
     __align__(16) float uf[CH];   // the head's bonus u in fp32
     uint64_t load_bar[2];  // TMA: a stage has landed
@@ -83,7 +84,7 @@ struct FwdParams {
     int Lsave;                // Lsave-th chunk ([key,value]), for a later call that restarts from them
     __nv_bfloat16 *y;
     __nv_bfloat16 *ckpt;      // [B,H,nchunk+1,64,64] chunk-start states, or NULL
-    float *dchunk;            // [B*H,nchunk,64] decay of each whole chunk, or NULL; with it the
+    float *dchunk;            // [B*H,nchunk,64] decay of each whole chunk (see ChunkDecay), or NULL; with it the
                               // kernel also stores r e^{cp} of every chunk through map_rh
     unsigned char *mildflag;  // with dchunk: [B*H*nchunk], 1 = the chunk is mild
     int *status;
@@ -100,16 +101,6 @@ struct FwdParams {
 //   Y       lo 128..159   y[:, 0..31]                  hi 128..159   y[:, 32..63]
 enum { COL_U = 0, COL_A1A = 64, COL_A2 = 96, COL_Y = 128, FWD_TMEM_COLS = 256 };
 constexpr int FWD_THREADS = 288;
-
-// barrier of the 256 compute threads that also ORs a predicate over them
-__device__ __forceinline__ bool compute_sync_or(bool pred) {
-    uint32_t any;
-    asm volatile("{\n.reg .pred p, q;\nsetp.ne.u32 q, %1, 0;\nbar.red.or.pred p, 1, 256, q;\nselp.u32 %0, 1, 0, p;\n}"
-                 : "=r"(any) : "r"((uint32_t)pred) : "memory");
-    return any != 0;
-}
-// barrier of the 256 compute threads
-__device__ __forceinline__ void compute_sync() { asm volatile("bar.sync 1, 256;" ::: "memory"); }
 
 // MODE: what the launch is for (compiled separately so that the full pass does not carry the others' state)
 enum { FWD_FULL = 0,      // y, state_out and, when asked for, the hand-over to the backward pass
@@ -183,19 +174,20 @@ k_chunk_fwd(const __grid_constant__ CUtensorMap map_r, const __grid_constant__ C
             for (int c = 0; c < n; c++) {
                 const int st = c & 1;
                 const uint64_t d_r = make_desc(smem_u32(&s.in[st][0])), d_k = make_desc(smem_u32(&s.in[st][1])),
-                               d_v = make_desc(smem_u32(&s.in[st][2])), d_rh = make_desc(smem_u32(&s.in[st][3])),
-                               d_kh = make_desc(smem_u32(&s.khat[st]));
+                               d_v = make_desc(smem_u32(&s.in[st][2]));
                 if (!mbar_wait_or_abort(&s.ops_bar[c & 1], (uint32_t)((c >> 1) & 1), &s.abort_flag, P.wait_limit)) { fail = 1; break; }
                 tc_fence_after();
                 // the per-chunk backward kernel comes in two bodies: tell it which one this chunk needs
                 // (written from here: this lane has time, the compute warps do not)
-                if (P.dchunk)
-                    P.mildflag[bh * P.nchunk + j0 + c] = *reinterpret_cast<volatile int *>(&s.mild_flag[c & 1]) != 0;
+                const bool mild = *reinterpret_cast<volatile int *>(&s.mild_flag[c & 1]) != 0;
+                if (P.dchunk) P.mildflag[bh * P.nchunk + j0 + c] = mild;
+                // r's operand of the state product: a mild chunk's is that of its scores
+                Tile *rh = mild ? &s.in[st][0] : &s.in[st][3];
+                const uint64_t d_rh = make_desc(smem_u32(rh)), d_kh = make_desc(smem_u32(&s.khat[st]));
                 if (full) {
                     // scores: A1 = Rt Kt^T (column halves), A2 = X X[0:32]^T.  In a mild chunk Rt and Kt are
                     // scaled around one point, A1's rows 32..63 of columns 0..31 ARE the cross-block scores:
                     // that half goes where A2 would have gone and A2 is not formed.
-                    const bool mild = *reinterpret_cast<volatile int *>(&s.mild_flag[c & 1]) != 0;
                     const uint32_t a1a = tm + (mild ? COL_A2 : COL_A1A);
 #pragma unroll
                     for (int k = 0; k < 4; k++) mma_ss(a1a, d_r + k * KSTEP, d_k + k * KSTEP, id32, k > 0);
@@ -216,9 +208,9 @@ k_chunk_fwd(const __grid_constant__ CUtensorMap map_r, const __grid_constant__ C
                                id_mm32, k > 0);
                 mma_commit(&s.u_bar[c & 1]);
                 pending = c;
-                // r e^{cp} of this chunk goes out for the backward pass
+                // r e^{cp} (a mild chunk: rt) goes out for the backward pass
                 if (P.dchunk) {
-                    tma_store_3d(&map_rh, &s.in[st][3], h * 64, (j0 + c) * CH, b);
+                    tma_store_3d(&map_rh, rh, h * 64, (j0 + c) * CH, b);
                     tma_store_commit();
                 }
                 if (full) {
@@ -356,38 +348,35 @@ k_chunk_fwd(const __grid_constant__ CUtensorMap map_r, const __grid_constant__ C
                 for (int ch = 0; ch < 4; ch++) {
                     const float d = exp2f(D.e[ch]) * other[ch];
                     s.dvec[j & 1][ch0 + ch] = d;
-                    if (P.dchunk) P.dchunk[((size_t)bh * P.nchunk + jg) * 64 + ch0 + ch] = d;
+                    const float e = chunk_decay_entry(D.e[ch] + other_l2[ch], mild);
+                    s.hvec[j & 1][ch0 + ch] = chunk_decay(e).hs;
+                    if (P.dchunk) P.dchunk[((size_t)bh * P.nchunk + jg) * 64 + ch0 + ch] = e;
                 }
             }
             if (mild) {
-                // One reference point (the end of block 0) for the whole chunk.  With it the state-term
-                // factors are the score factors times a per-channel constant:
-                //   block 0:  rt = r 2^{cp - e0},  rhat = rt 2^{e0};   kt = k 2^{e0 - c},  khat = kt 2^{total of block 1}
-                //   block 1:  rt = r 2^{cp},       rhat = rt 2^{e0};   kt = k 2^{-c},      khat = kt 2^{total of block 1}
-                // (cp, c counted from the thread's block start) -- one running factor per side instead of two.
-                float fa[4], cr[4], ck[4];
+                // One reference point m for the whole chunk, half of its log-decay c:  rt = r 2^{cp - m},  kt = k 2^{m - c_t}.
+                // rt is the operand of the state too:  r e^{cp} S = rt (2^m S);  khat = kt 2^{c - m}.
+                float fa[4], ref[4], ck[4];         // ref: m counted from the thread's block start
 #pragma unroll
                 for (int ch = 0; ch < 4; ch++) {
-                    const float own = exp2f(D.e[ch]);
-                    cr[ch] = blk ? other[ch] : own;
-                    ck[ch] = blk ? own : other[ch];
-                    fa[ch] = exp2f(D.cp0[ch] - (blk ? 0.f : D.e[ch]));
+                    const float c = D.e[ch] + other_l2[ch], m = rintf(chunk_decay_entry(c, true));
+                    ref[ch] = m - (blk ? other_l2[ch] : 0.f);
+                    ck[ch] = exp2f(c - m);
+                    fa[ch] = exp2f(D.cp0[ch] - ref[ch]);
                 }
                 if (full) {
 #pragma unroll
                     for (int i = 0; i < 4; i++) {
                         const int t = tok0 + i;
-                        float r[4], k[4], rt[4], rh[4];
+                        float r[4], k[4], rt[4];
                         unpack4(ld_tile4(in[0], t, cc, hf), r);
                         unpack4(ld_tile4(in[1], t, cc, hf), k);
                         vmul<4>(rt, r, fa);
-                        vmul<4>(rh, rt, cr);
                         vmul<4>(fa, fa, D.w[i]);
                         f2 d2 = mul2(mul2(make_float2(r[0], r[1]), make_float2(uu[0], uu[1])), make_float2(k[0], k[1]));
                         d2 = fma2(mul2(make_float2(r[2], r[3]), make_float2(uu[2], uu[3])), make_float2(k[2], k[3]), d2);
                         float dsum = d2.x + d2.y;
                         st_tile4(in[0], t, cc, hf, pack4(rt));
-                        st_tile4(in[3], t, cc, hf, pack4(rh));
                         dsum += __shfl_xor_sync(0xffffffffu, dsum, 1);
                         dsum += __shfl_xor_sync(0xffffffffu, dsum, 2);
                         if ((lane & 3) == 0) s.dpart[(lane & 15) >> 2][t] = dsum;
@@ -396,16 +385,15 @@ k_chunk_fwd(const __grid_constant__ CUtensorMap map_r, const __grid_constant__ C
 #pragma unroll
                     for (int i = 0; i < 4; i++) {
                         const int t = tok0 + i;
-                        float r[4], rh[4];
+                        float r[4], rt[4];
                         unpack4(ld_tile4(in[0], t, cc, hf), r);
-                        vmul<4>(rh, r, fa);
-                        vmul<4>(rh, rh, cr);
+                        vmul<4>(rt, r, fa);
                         vmul<4>(fa, fa, D.w[i]);
-                        st_tile4(in[3], t, cc, hf, pack4(rh));
+                        st_tile4(in[0], t, cc, hf, pack4(rt));
                     }
                 }
 #pragma unroll
-                for (int ch = 0; ch < 4; ch++) fa[ch] = exp2f((blk ? 0.f : D.e[ch]) - D.c3[ch]);
+                for (int ch = 0; ch < 4; ch++) fa[ch] = exp2f(ref[ch] - D.c3[ch]);
 #pragma unroll
                 for (int i = 3; i >= 0; i--) {
                     const int t = tok0 + i;
@@ -505,10 +493,18 @@ k_chunk_fwd(const __grid_constant__ CUtensorMap map_r, const __grid_constant__ C
             *reinterpret_cast<volatile int *>(&s.abort_flag) = 1;
             return false;
         };
-        // bf16 copy of the state at the start of chunk jn: operand of rhat*S, checkpoint
+        // bf16 copy of the state at the start of chunk jn, times the chunk's 2^m: operand of the y product, checkpoint
         // (jn local; the state at the end of a group is the next group's first checkpoint, written there)
         auto publish_state = [&](int jn) {
-            const uint4 q0 = pack8(S), q1 = pack8(S + 8);
+            // (the state after the segment has no chunk behind it, and no reader)
+            const float hs = jn < n ? s.hvec[jn & 1][row] : 1.f;
+            float Sh[16];
+#pragma unroll
+            for (int q = 0; q < 16; q += 2) {
+                const f2 v = mul2(both(hs), make_float2(S[q], S[q + 1]));
+                Sh[q] = v.x; Sh[q + 1] = v.y;
+            }
+            const uint4 q0 = pack8(Sh), q1 = pack8(Sh + 8);
             if (full && jn < n) {
                 st_tile(s.sbf, row, (vcol0 >> 3), q0);
                 st_tile(s.sbf, row, (vcol0 >> 3) + 1, q1);

@@ -25,6 +25,15 @@ __device__ __forceinline__ void st_tile(Tile &t, int row, int chunk, const uint4
     *reinterpret_cast<uint4 *>(t.b + tile_off(row, chunk)) = v;
 }
 
+// named barrier `id` of `threads` threads (by default the 256 compute threads of a kernel) that also ORs a predicate over them
+__device__ __forceinline__ bool compute_sync_or(bool pred, int id = 1, int threads = 256) {
+    uint32_t any;
+    asm volatile("{\n.reg .pred p, q;\nsetp.ne.u32 q, %1, 0;\nbar.red.or.pred p, %2, %3, q;\nselp.u32 %0, 1, 0, p;\n}"
+                 : "=r"(any) : "r"((uint32_t)pred), "r"(id), "r"(threads) : "memory");
+    return any != 0;
+}
+__device__ __forceinline__ void compute_sync(int id = 1, int threads = 256) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
+
 // ---------------------------------------------------------------------------
 // Per-chunk decay bookkeeping.
 //
@@ -36,6 +45,7 @@ __device__ __forceinline__ void st_tile(Tile &t, int row, int chunk, const uint4
 // per-token decay w = 2^{l2}.  Everything a block needs from the other block is that
 // block's total, exchanged through shared memory.
 constexpr float LOG2E = 1.4426950408889634f;
+constexpr float LOG2_LOG2E = 0.5287663729448977f;
 constexpr float LN2 = 0.6931471805599453f;
 constexpr float L2_FLOOR = LW_FLOOR * LOG2E;
 
@@ -66,11 +76,11 @@ struct Decay {           // of a thread's 4 tokens x 4 channels
 // through `wtot` ([8][CH] floats of shared memory); `sync(pred)` is the barrier of the 256 threads,
 // returning the OR of `pred` over them.
 //
-// Returns true when the chunk is "mild": no 8 consecutive tokens decay by more than 2^-30 in any
-// channel, so that the whole chunk can be factored around ONE reference point, the end of block 0
-// (both halves then stay within 2^+-120), and the separate treatment of the pairs across the two
-// blocks is not needed.
-constexpr float MILD_L2_PER_8 = -30.f;
+// Returns true when the chunk is "mild": no 8 consecutive tokens decay by more than 2^-28 in any
+// channel, so that the whole chunk can be factored around ONE reference point, half of the chunk's total log-decay
+// (every factor then stays within 2^+-113, which leaves operands 13 bits above the smallest normal number), and the
+// separate treatment of the pairs across the two blocks is not needed.
+constexpr float MILD_L2_PER_8 = -28.f;
 template <class Sync>
 __device__ __forceinline__ bool decay_scan8(float (&l2)[4][4], int warp, int lane, float *wtot, Decay &D,
                                             float (&other_l2)[4], Sync sync) {
@@ -164,11 +174,17 @@ __device__ __forceinline__ void st_tile4(Tile &t, int row, int chunk, int half, 
 }
 
 // What the forward kernel hands to the backward kernels (wkv_args_t.state_ckpt):
-//   sck     bf16 [B*H, nchunk+1, 64, 64]  state at the start of every chunk (key rows, value columns)
-//   rhat    bf16 [B, T, C]                r_t * (decay accumulated from the chunk start to before t)
-//   dchunk  fp32 [B*H, nchunk, 64]        decay of each whole chunk per key channel
+//   sck     bf16 [B*H, nchunk+1, 64, 64]  state at the start of every chunk (key rows, value columns); of a mild
+//                                         chunk times 2^m per key row
+//   rhat    bf16 [B, T, C]                r_t * (decay accumulated from the chunk start to before t); of a mild chunk
+//                                         times 2^-m: the very operand Rt that the per-chunk backward kernel forms
+//                                         again, so that the large terms of the decay gradient cancel exactly
+//   dchunk  fp32 [B*H, nchunk, 64]        decay of each whole chunk per key channel, see ChunkDecay
 //   mild    u8   [B*H * nchunk]           1 = the chunk is mild (see decay_scan8), 0 = steep: which body of
 //                                         the per-chunk backward kernel the chunk needs
+// m = c/2 rounded to a whole number, c the log2-decay of the whole chunk: the reference point that a mild chunk is
+// factored around.  The states on either side of the chunk come with it, so that their products share accumulators
+// (and operands) with those inside the chunk; being whole, it changes no operand's rounding on the r side.
 struct CkptLayout {
     size_t sck, rhat, dchunk, mild, total;
 };
@@ -182,6 +198,19 @@ inline CkptLayout ckpt_layout(int B, int T, int H) {
     L.mild = L.dchunk + al(bh * n * 64 * 4);
     L.total = L.mild + al(bh * n);
     return L;
+}
+
+// An entry of dchunk: a mild chunk's c / 2 (<= 0), a steep chunk's -c (> 0).
+__device__ __forceinline__ float chunk_decay_entry(float c, bool mild) { return mild ? 0.5f * c : -c; }
+__device__ __forceinline__ float pow2i(float m) { return __int_as_float((127 + __float2int_rn(m)) << 23); }   // m whole, > -127
+struct ChunkDecay {
+    float d;              // decay of the whole chunk
+    float hs, hd, hsinv;  // scales of the states at its start and its end, 2^m and 2^{c-m}, and 2^-m (1 for a steep chunk)
+};
+__device__ __forceinline__ ChunkDecay chunk_decay(float entry) {
+    if (entry > 0.f) return {exp2f(-entry), 1.f, 1.f, 1.f};
+    const float e = exp2f(entry), m = rintf(entry);
+    return {e * e, pow2i(m), exp2f(2.f * entry - m), pow2i(-m)};
 }
 
 // Time groups (see the head of wkv56_chunked.cu): G groups of L consecutive chunks per chain.

@@ -77,6 +77,7 @@ __device__ __forceinline__ f2 add2(f2 a, f2 b) {
     asm("add.rn.ftz.f32x2 %0, %1, %2;" : "=l"(r) : "l"(bits(a)), "l"(bits(b)));
     return from_bits(r);
 }
+__device__ __forceinline__ f2 unpack2(uint32_t q) { return make_float2(__uint_as_float(q << 16), __uint_as_float(q & 0xFFFF0000u)); }
 __device__ __forceinline__ f2 both(float x) { return make_float2(x, x); }
 __device__ __forceinline__ f2 sub2(f2 a, f2 b) { return fma2(b, both(-1.f), a); }
 __device__ __forceinline__ f2 neg2(f2 a) { return make_float2(-a.x, -a.y); }
@@ -110,6 +111,15 @@ __device__ __forceinline__ void vfma(float *o, const float *a, const float *b, c
 #pragma unroll
     for (int i = 0; i < N; i += 2) {
         const f2 r = fma2(make_float2(a[i], a[i + 1]), make_float2(b[i], b[i + 1]), make_float2(c[i], c[i + 1]));
+        o[i] = r.x; o[i + 1] = r.y;
+    }
+}
+// o = a + s
+template <int N>
+__device__ __forceinline__ void vadds(float *o, const float *a, float s) {
+#pragma unroll
+    for (int i = 0; i < N; i += 2) {
+        const f2 r = add2(make_float2(a[i], a[i + 1]), both(s));
         o[i] = r.x; o[i + 1] = r.y;
     }
 }
