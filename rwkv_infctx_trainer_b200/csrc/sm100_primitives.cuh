@@ -211,6 +211,14 @@ __device__ __forceinline__ uint64_t desc_mnmajor(const void *tile, int row0, int
     return make_desc(smem_u32(tile) + (row0 + 16 * k16) * TILE_ROW_BYTES);
 }
 
+// One lane of a converged warp, always the same.  A tcgen05.mma that stands in a branch on this is known to have one thread
+// and takes its operands from uniform registers; in a branch on the lane number an issue costs about 160 cycles instead of 41.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t one;
+    asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.b32 %0, 1, 0, p;\n}" : "=r"(one));
+    return one != 0;
+}
+
 // D[tmem] (+)= A[smem] * B[smem]; issued by ONE thread.
 __device__ __forceinline__ void mma_ss(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc,
                                        bool accumulate) {

@@ -97,7 +97,8 @@ k_chunk_dscan(const __grid_constant__ CUtensorMap map_rh, const __grid_constant_
     // itself (not to an integer copy of its address), so the compiler still knows that everything
     // behind `s` is shared memory and uses shared-memory loads and stores for the tiles.
     DscanSmem &s = *reinterpret_cast<DscanSmem *>(smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u));
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, lane = tid & 31;
+    const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);   // tells the compiler it is uniform across the warp
     // one CTA per (chain, group); a summary pass leaves out group 0, which nothing needs
     const int skip = P.summary ? 1 : 0, bh = blockIdx.x / (P.G - skip), grp = blockIdx.x - bh * (P.G - skip) + skip;
     const int unit = bh * P.G + grp, b = bh / P.H, h = bh % P.H;
@@ -115,17 +116,19 @@ k_chunk_dscan(const __grid_constant__ CUtensorMap map_rh, const __grid_constant_
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tm = s.tmem_base;
+    const uint32_t tm = __shfl_sync(0xffffffffu, s.tmem_base, 0);
     auto load_parity = [&](int i) { return (uint32_t)((i / DS_STAGES) & 1); };
     auto prod_parity = [&](int i) { return (uint32_t)((i >> 1) & 1); };
     int fail = 0;
 
     if (warp == 4) {
-        if (lane == 0) {
-            int issued = -1, landed = -1, mma_issued = -1;
-            auto issue_load = [&](int i) {
-                if (i == P.skip_load) return;
-                const int st = i % DS_STAGES, j = j0 + n - 1 - i;      // global chunk of step i
+        // (the whole warp runs this, one elected lane issues)
+        auto wait = [&](uint64_t *bar, uint32_t parity, uint32_t limit) { return __all_sync(0xffffffffu, mbar_wait(bar, parity, limit)) != 0; };
+        int issued = -1, landed = -1, mma_issued = -1;
+        auto issue_load = [&](int i) {
+            if (i == P.skip_load) return;
+            const int st = i % DS_STAGES, j = j0 + n - 1 - i;      // global chunk of step i
+            if (elect_one()) {
                 mbar_expect_tx(&s.load_bar[st], (i < n ? 2 * TILE_BYTES + CH * 4 : 0) + (summary ? 0 : TILE_BYTES));
                 if (i < n) {
                     tma_load_3d(&s.in[st][0], &map_rh, &s.load_bar[st], h * 64, j * CH, b);
@@ -133,18 +136,20 @@ k_chunk_dscan(const __grid_constant__ CUtensorMap map_rh, const __grid_constant_
                     bulk_load_1d(s.dvec[st], P.dchunk + ((size_t)bh * N + j) * 64, CH * 4, &s.load_bar[st]);
                 }
                 if (!summary) tma_load_3d(&s.in[st][2], &map_s, &s.load_bar[st], 0, 0, bh * (N + 1) + j + 1);
-                issued = i;
-            };
-            for (int i = 0; i < DS_STAGES && i < nsteps; i++) issue_load(i);
-            const uint32_t id = make_idesc(64, 32, true, true);
-            for (int i = 0; i < nsteps && !fail; i++) {
-                if (!mbar_wait(&s.load_bar[i % DS_STAGES], load_parity(i), LIM)) { fail = 1; break; }
-                landed = i;
-                if (i < n) {
-                    // buffer i&1 held the product of step i-2
-                    if (i >= 2 && !mbar_wait(&s.prod_free[i & 1], prod_parity(i - 2), LIM)) { fail = 1; break; }
-                    tc_fence_after();
-                    Tile *in = s.in[i % DS_STAGES];
+            }
+            issued = i;
+        };
+        for (int i = 0; i < DS_STAGES && i < nsteps; i++) issue_load(i);
+        const uint32_t id = make_idesc(64, 32, true, true);
+        for (int i = 0; i < nsteps && !fail; i++) {
+            if (!wait(&s.load_bar[i % DS_STAGES], load_parity(i), LIM)) { fail = 1; break; }
+            landed = i;
+            if (i < n) {
+                // buffer i&1 held the product of step i-2
+                if (i >= 2 && !wait(&s.prod_free[i & 1], prod_parity(i - 2), LIM)) { fail = 1; break; }
+                tc_fence_after();
+                Tile *in = s.in[i % DS_STAGES];
+                if (elect_one()) {
                     // value columns 0..31 into lanes 0..15 of each quarter, 32..63 into lanes 16..31
 #pragma unroll
                     for (int hf = 0; hf < 2; hf++)
@@ -153,22 +158,22 @@ k_chunk_dscan(const __grid_constant__ CUtensorMap map_rh, const __grid_constant_
                             mma_ss(tm + (hf ? (16u << 16) : 0u) + 32u * (i & 1), desc_mnmajor(&in[0], 0, k),
                                    desc_mnmajor(&in[1], 0, k) + (hf ? 4 : 0), id, k > 0);
                     mma_commit(&s.mma_bar[i & 1]);
-                    mma_issued = i;
                 }
-                // the stage of step i-1 goes to step i-1+DS_STAGES as soon as the scan warps are done with it
-                if (i >= 1 && i + DS_STAGES - 1 < nsteps) {
-                    if (!mbar_wait(&s.stage_free[(i - 1) % DS_STAGES], load_parity(i - 1), LIM)) { fail = 1; break; }
-                    issue_load(i + DS_STAGES - 1);
-                }
+                mma_issued = i;
             }
-            if (fail) {
-                // let everything in flight land before the shared and tensor memory go away
-                for (int q = landed + 1; q <= issued; q++)
-                    if (q != P.skip_load) mbar_wait(&s.load_bar[q % DS_STAGES], load_parity(q), 200000u);
-                if (mma_issued >= 0) mbar_wait(&s.mma_bar[mma_issued & 1], prod_parity(mma_issued), 100000u);
-                if (mma_issued >= 1) mbar_wait(&s.mma_bar[(mma_issued - 1) & 1], prod_parity(mma_issued - 1), 100000u);
-                if (P.status) atomicOr(P.status, 2);
+            // the stage of step i-1 goes to step i-1+DS_STAGES as soon as the scan warps are done with it
+            if (i >= 1 && i + DS_STAGES - 1 < nsteps) {
+                if (!wait(&s.stage_free[(i - 1) % DS_STAGES], load_parity(i - 1), LIM)) { fail = 1; break; }
+                issue_load(i + DS_STAGES - 1);
             }
+        }
+        if (fail) {
+            // let everything in flight land before the shared and tensor memory go away
+            for (int q = landed + 1; q <= issued; q++)
+                if (q != P.skip_load) mbar_wait(&s.load_bar[q % DS_STAGES], load_parity(q), 200000u);
+            if (mma_issued >= 0) mbar_wait(&s.mma_bar[mma_issued & 1], prod_parity(mma_issued), 100000u);
+            if (mma_issued >= 1) mbar_wait(&s.mma_bar[(mma_issued - 1) & 1], prod_parity(mma_issued - 1), 100000u);
+            if (P.status && lane == 0) atomicOr(P.status, 2);
         }
         __syncwarp();
     } else {
@@ -985,7 +990,7 @@ bwd_steep(const CUtensorMap &map_gr, const CUtensorMap &map_gk, const CUtensorMa
 // 16 (warp >> 2) .. +15) walk over the group's chunks, and a feeder warp issues every load, a chunk ahead, and every
 // tcgen05.mma.  (One chunk per CTA, two CTAs on an SM: of 15.6 k cycles per chunk 8 k went to the start of the CTA, its
 // first loads and the drain of its stores.)
-// 4 rows of 4096 tokens x 64 heads: 505 us with one CTA per chunk and the 4 x 4 threads, 400 with this arithmetic, 290
+// 4 rows of 4096 tokens x 64 heads: 505 us with one CTA per chunk and the 4 x 4 threads, 400 with this arithmetic, 300
 // with both; what is left is spread over waits for products (2.3 k of 9.1 k cycles per chunk and group), issue (50 %)
 // and shared memory (46 % of its cycles).
 //
@@ -1026,10 +1031,11 @@ __device__ __forceinline__ bool
 mild_feed(const CUtensorMap &map_r, const CUtensorMap &map_k, const CUtensorMap &map_v, const CUtensorMap &map_w,
          const CUtensorMap &map_gy, const CUtensorMap &map_s, const CUtensorMap &map_d,
           const BwdParams &P, MildSmem &s, const uint32_t tm, const int first, const int stride) {
-    const int lane = threadIdx.x & 31, n = P.nchunk;
+    const int n = P.nchunk;
     const uint32_t LIM = P.wait_limit, tm_hi = tm + (16u << 16);
+    // (the whole warp runs this, one elected lane issues)
     auto wait = [&](uint64_t *bar, uint32_t ph) {
-        if (mbar_wait_or_abort(bar, ph, &s.abort_flag, LIM)) return true;
+        if (__all_sync(0xffffffffu, mbar_wait_or_abort(bar, ph, &s.abort_flag, LIM))) return true;
         *reinterpret_cast<volatile int *>(&s.abort_flag) = 1;
         return false;
     };
@@ -1060,26 +1066,26 @@ mild_feed(const CUtensorMap &map_r, const CUtensorMap &map_k, const CUtensorMap 
     // (a chunk whose loads are left out on the host's word: the wait-timeout test)
     auto skip = [&](int c) { return c - P.by_n.div(c) * n == P.skip_load; };
     bool loads = !skip(chunk);         // the current chunk's have been issued
-    if (lane == 0 && loads) {
+    if (loads) {
         const At x = at(chunk);
-        load0(x, 0); load1a(x); load1b(x);
+        if (elect_one()) { load0(x, 0); load1a(x); load1b(x); }
     }
     bool fine = true;
     for (uint32_t ph = 0; chunk >= 0 && fine; ph ^= 1) {
         const int next = walk.next();
         const bool more = next >= 0 && !skip(next);
-        if (lane == 0) {
-            const At x = at(next >= 0 ? next : chunk);
-            int stage = 0;       // barriers committed to
-            // operand descriptors: that of the structure's first tile plus an offset
-            const uint64_t d0 = make_desc(smem_u32(&s));
-            auto kmaj = [&](uint32_t off, int k16) { return d0 + ((off + 32 * k16) >> 4); };
-            auto mnmaj = [&](uint32_t off, int k16) { return d0 + ((off + 16 * TILE_ROW_BYTES * k16) >> 4); };
-            do {
-                if (!wait(&s.full[0], ph)) break;
-                tc_fence_after();
-                // X^T[k, t] = sum_t' X[t', k] I[t', t], 16 tokens at a time
-                const uint32_t id_turn = make_idesc(64, 16, true, false);
+        const At x = at(next >= 0 ? next : chunk);
+        int stage = 0;       // barriers committed to
+        // operand descriptors: that of the structure's first tile plus an offset
+        const uint64_t d0 = make_desc(smem_u32(&s));
+        auto kmaj = [&](uint32_t off, int k16) { return d0 + ((off + 32 * k16) >> 4); };
+        auto mnmaj = [&](uint32_t off, int k16) { return d0 + ((off + 16 * TILE_ROW_BYTES * k16) >> 4); };
+        do {
+            if (!wait(&s.full[0], ph)) break;
+            tc_fence_after();
+            // X^T[k, t] = sum_t' X[t', k] I[t', t], 16 tokens at a time
+            const uint32_t id_turn = make_idesc(64, 16, true, false);
+            if (elect_one()) {
                 if (PER_TOKEN) {
 #pragma unroll
                     for (int q = 0; q < 4; q++)
@@ -1092,10 +1098,12 @@ mild_feed(const CUtensorMap &map_r, const CUtensorMap &map_k, const CUtensorMap 
                 for (int q = 0; q < 4; q++)
                     mma_ss(tm + U_KV + 16 * q, mnmaj(offsetof(MildSmem, in) + T_K * TILE_BYTES, q), kmaj(offsetof(MildSmem, ident), 0), id_turn, false);
                 mma_commit(&s.turned);
-                stage = 1;
-                if (!wait(&s.full[1], ph)) break;
-                const uint32_t id_kk = make_idesc(64, 64, false, false), id_mm = make_idesc(64, 64, true, true),
-                               id_km = make_idesc(64, 64, false, true);
+            }
+            stage = 1;
+            if (!wait(&s.full[1], ph)) break;
+            const uint32_t id_kk = make_idesc(64, 64, false, false), id_mm = make_idesc(64, 64, true, true),
+                           id_km = make_idesc(64, 64, false, true);
+            if (elect_one()) {
                 // P[t,s] = sum_v gy[t,v] v[s,v]
 #pragma unroll
                 for (int q = 0; q < 4; q++)
@@ -1108,18 +1116,22 @@ mild_feed(const CUtensorMap &map_r, const CUtensorMap &map_k, const CUtensorMap 
                 for (int q = 0; q < 4; q++)
                     mma_ss(tm_hi + U_G, kmaj(offsetof(MildSmem, in) + T_D * TILE_BYTES, q), kmaj(offsetof(MildSmem, in) + T_V * TILE_BYTES, q), id_kk, q > 0);
                 mma_commit(&s.early);
-                stage = 2;
-                if (!wait(&s.ops, ph)) break;
-                tc_fence_after();
-                // A[t,s] = sum_k Rt[t,k] Kt[s,k]   (both tiles are [channel][token])
+            }
+            stage = 2;
+            if (!wait(&s.ops, ph)) break;
+            tc_fence_after();
+            // A[t,s] = sum_k Rt[t,k] Kt[s,k]   (both tiles are [channel][token])
+            if (elect_one()) {
 #pragma unroll
                 for (int q = 0; q < 4; q++)
                     mma_ss(tm + U_AP, mnmaj(offsetof(MildSmem, rt), q), mnmaj(offsetof(MildSmem, kt), q), id_mm, q > 0);
                 mma_commit(&s.score);
-                stage = 3;
                 if (more) load0(x, ph ^ 1);
-                if (!wait(&s.mask, ph)) break;
-                tc_fence_after();
+            }
+            stage = 3;
+            if (!wait(&s.mask, ph)) break;
+            tc_fence_after();
+            if (elect_one()) {
                 // Gr[k,t] += sum_s Kt[s,k] P~[t,s];  Gk[k,s] += sum_t Rt[t,k] P~[t,s]
 #pragma unroll
                 for (int q = 0; q < 4; q++)
@@ -1136,29 +1148,28 @@ mild_feed(const CUtensorMap &map_r, const CUtensorMap &map_k, const CUtensorMap 
                 for (int q = 0; q < 4; q++)
                     mma_ss(tm_hi + U_KV, mnmaj(offsetof(MildSmem, kt), q), mnmaj(offsetof(MildSmem, in) + T_D * TILE_BYTES, q), id_mm, true);
                 mma_commit(&s.gv);
-                stage = 4;
                 if (more) load1a(x);
-                if (!wait(&s.gv, ph)) break;
-                if (more) load1b(x);
-                if (!wait(&s.epi, ph)) break;
-                tc_fence_after();
-                stage = 5;
-            } while (false);
-            if (stage < 5) {
-                fine = false;
-                if (P.status) atomicOr(P.status, 4);
-                // let whatever is in flight finish before shared and tensor memory go away
-                if (loads) { mbar_wait(&s.full[0], ph, 200000u); mbar_wait(&s.full[1], ph, 200000u); }
-                uint64_t *last[5] = {nullptr, &s.turned, &s.early, &s.score, &s.gv};
-                for (int q = 1; q <= stage; q++) mbar_wait(last[q], ph, 200000u);
-                if (more && stage >= 3) {
-                    // (those of the next chunk; the second group may be short of two loads and never complete)
-                    mbar_wait(&s.full[0], ph ^ 1, 200000u);
-                    if (stage == 4) mbar_wait(&s.full[1], ph ^ 1, 20000u);
-                }
+            }
+            stage = 4;
+            if (!wait(&s.gv, ph)) break;
+            if (more && elect_one()) load1b(x);
+            if (!wait(&s.epi, ph)) break;
+            tc_fence_after();
+            stage = 5;
+        } while (false);
+        if (stage < 5) {
+            fine = false;
+            if (P.status && elect_one()) atomicOr(P.status, 4);
+            // let whatever is in flight finish before shared and tensor memory go away
+            if (loads) { mbar_wait(&s.full[0], ph, 200000u); mbar_wait(&s.full[1], ph, 200000u); }
+            uint64_t *last[5] = {nullptr, &s.turned, &s.early, &s.score, &s.gv};
+            for (int q = 1; q <= stage; q++) mbar_wait(last[q], ph, 200000u);
+            if (more && stage >= 3) {
+                // (those of the next chunk; the second group may be short of two loads and never complete)
+                mbar_wait(&s.full[0], ph ^ 1, 200000u);
+                if (stage == 4) mbar_wait(&s.full[1], ph ^ 1, 20000u);
             }
         }
-        fine = __shfl_sync(0xffffffffu, (int)fine, 0) != 0;
         loads = more;
         chunk = next;
     }
@@ -1534,7 +1545,7 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) k_chunk_bwd(BWD_MAPS, const Bw
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tm0 = *tmem_base, tm = tm0 + BWD_TMEM_COLS * grp;
+    const uint32_t tm0 = __shfl_sync(0xffffffffu, *tmem_base, 0), tm = tm0 + BWD_TMEM_COLS * grp;
     const int first = (int)blockIdx.x * BWD_GROUPS + grp, stride = (int)gridDim.x * BWD_GROUPS;
     const int bar = 1 + grp, bar_all = 1 + BWD_GROUPS + grp;     // named barriers: of the compute warps, of the whole group
     if (feeder) {
