@@ -153,8 +153,8 @@ k_chunk_fwd(const __grid_constant__ CUtensorMap map_r, const __grid_constant__ C
             auto issue_load = [&](int c) {
                 if (c == P.skip_load) return;
                 const int st = c & 1, t0 = (j0 + c) * CH;
-                mbar_expect_tx(&s.load_bar[st], (PER_TOKEN ? 4 : 3) * TILE_BYTES);
-                tma_load_3d(&s.in[st][0], &map_r, &s.load_bar[st], h * 64, t0, b);
+                mbar_expect_tx(&s.load_bar[st], ((PER_TOKEN ? 4 : 3) - (summary ? 1 : 0)) * TILE_BYTES);
+                if (!summary) tma_load_3d(&s.in[st][0], &map_r, &s.load_bar[st], h * 64, t0, b);
                 tma_load_3d(&s.in[st][1], &map_k, &s.load_bar[st], h * 64, t0, b);
                 tma_load_3d(&s.in[st][2], &map_v, &s.load_bar[st], h * 64, t0, b);
                 if (PER_TOKEN) tma_load_3d(&s.in[st][3], &map_w, &s.load_bar[st], h * 64, t0, b);
@@ -343,14 +343,17 @@ k_chunk_fwd(const __grid_constant__ CUtensorMap map_r, const __grid_constant__ C
             float other[4];          // 2^{total of the other block}
 #pragma unroll
             for (int ch = 0; ch < 4; ch++) other[ch] = exp2f(other_l2[ch]);
-            if (warp == 0 && lane < 16) {
+            // the chunk's decay and the scale of its states: a channel of each thread's four per warp
+            if (lane < 16) {
 #pragma unroll
                 for (int ch = 0; ch < 4; ch++) {
-                    const float d = exp2f(D.e[ch]) * other[ch];
-                    s.dvec[j & 1][ch0 + ch] = d;
-                    const float e = chunk_decay_entry(D.e[ch] + other_l2[ch], mild);
-                    s.hvec[j & 1][ch0 + ch] = chunk_decay(e).hs;
-                    if (P.dchunk) P.dchunk[((size_t)bh * P.nchunk + jg) * 64 + ch0 + ch] = e;
+                    if (warp != ch) continue;
+                    s.dvec[j & 1][ch0 + ch] = exp2f(D.e[ch]) * other[ch];
+                    if (!summary) {
+                        const float e = chunk_decay_entry(D.e[ch] + other_l2[ch], mild);
+                        s.hvec[j & 1][ch0 + ch] = chunk_decay(e).hs;
+                        if (P.dchunk) P.dchunk[((size_t)bh * P.nchunk + jg) * 64 + ch0 + ch] = e;
+                    }
                 }
             }
             if (mild) {
@@ -561,7 +564,7 @@ k_chunk_fwd(const __grid_constant__ CUtensorMap map_r, const __grid_constant__ C
                 if (summary) dprod *= d;
                 vaxpy<16>(S, d, S, uacc);
             }
-            publish_state(j + 1);
+            if (!summary) publish_state(j + 1);
             // (M) masked scores of chunk j+1: lo lanes own columns 0..31 of token row t, hi lanes 32..63;
             // this warp group 16 of them
             if (j + 1 < n && full) {
