@@ -980,7 +980,7 @@ bwd_steep(const CUtensorMap &map_gr, const CUtensorMap &map_gk, const CUtensorMa
 // What bounds a chunk's CUDA-core work is the number of instructions, so everything elementwise is done by threads
 // that own one channel and 16 consecutive tokens: the decay sums, the factors, the gradients and the token scan of the
 // decay gradient are then serial code on registers, with no shuffles, no table of sums and nothing to read again
-// by other threads (83 instructions per 32 elements, where threads of 4 x 4 elements and of one token took 129).
+// by other threads (77 instructions per 32 elements, where threads of 4 x 4 elements and of one token took 129).
 // Inputs come [token][channel]; the tensor core turns them: w, r, k times a 16 x 16 identity, exact in
 // fp32, and a thread reads its 16 values with one tcgen05.ld.  All accumulators are [channel][token] likewise, read
 // by the 16-lane load (tmem_ld16_split32), which covers an M = 64, N = 64 accumulator with all threads: no product
