@@ -26,6 +26,7 @@
 // Math reference: RWKV-v6/src/module/cuda/wkv6state_cuda_v1.cu:70-293 (what the
 // gradients are), RWKV-v6/src/module/rwkv_inner.py:48-113 (the chunked form).
 #include <algorithm>
+#include <cfloat>
 #include <cstddef>
 
 #include "wkv56_chunked.cuh"
@@ -982,7 +983,8 @@ bwd_steep(const CUtensorMap &map_gr, const CUtensorMap &map_gk, const CUtensorMa
 // decay gradient are then serial code on registers, with no shuffles, no table of sums and nothing to read again
 // by other threads (77 instructions per 32 elements, where threads of 4 x 4 elements and of one token took 129).
 // Inputs come [token][channel]; the tensor core turns them: w, r, k times a 16 x 16 identity, exact in
-// fp32, and a thread reads its 16 values with one tcgen05.ld.  All accumulators are [channel][token] likewise, read
+// fp32, and a thread reads its 16 values with one tcgen05.ld.  (An infinite one, times the identity's zeros, spoils the
+// other 15 of its run: those are then read from the tile, element by element.)  All accumulators are [channel][token] likewise, read
 // by the 16-lane load (tmem_ld16_split32), which covers an M = 64, N = 64 accumulator with all threads: no product
 // is cut into column halves.  gr, gk and gw go back to [token][channel] by 2-byte stores.
 //
@@ -1176,6 +1178,40 @@ mild_feed(const CUtensorMap &map_r, const CUtensorMap &map_k, const CUtensorMap 
     return fine;
 }
 
+// What the turned inputs should have been where an element of the chunk is infinite or NaN: it has met the identity's
+// zeros and made the other 15 of its run NaN.  The thread's r and k and, summed up, its log2-decays (of `nv` valid tokens)
+// go to their places in tensor memory (wr: w's), the decays' total to stot; returned: which decays are below the floor.
+// (Out of line: written into the loop, where it never ran, it made the backward pass of a 7B segment 421 us instead of 407.)
+template <bool PER_TOKEN>
+__device__ __noinline__ unsigned mild_inputs_again(MildSmem &s, uint32_t wr, int k, int t0, int nv) {
+    auto at = [&](const Tile &t, int i) {
+        return __bfloat162float(*reinterpret_cast<const __nv_bfloat16 *>(t.b + tile_off(t0 + i, k >> 3) + 2 * (k & 7)));
+    };
+    unsigned dead = 0;
+    float v[16];
+    if (PER_TOKEN) {
+        float sum = 0.f;
+#pragma unroll
+        for (int i = 0; i < 16; i++) {
+            bool live;
+            const float l2 = log2_decay(at(s.in[T_W], i), WKV_W_RAW, live);
+            if (!live) dead |= 1u << i;
+            if (t0 + i < nv) sum += l2;
+            v[i] = sum;
+        }
+        s.stot[t0 >> 4][k] = sum;
+        tmem_st16_split32(wr, v);
+    }
+#pragma unroll
+    for (int i = 0; i < 16; i++) v[i] = at(s.in[T_R], i);
+    tmem_st16_split32(wr + (16u << 16), v);
+#pragma unroll
+    for (int i = 0; i < 16; i++) v[i] = at(s.in[T_K], i);
+    tmem_st16_split32(wr + (U_KV - U_WR), v);
+    tmem_st_wait();
+    return dead;
+}
+
 // The compute warps of the same chunks; bar: their named barrier.
 template <bool PER_TOKEN>
 __device__ __forceinline__ bool
@@ -1225,6 +1261,7 @@ mild_compute(const CUtensorMap &map_gr, const CUtensorMap &map_gk, const CUtenso
         // first, while the inputs are being turned: the bonus term of the score diagonal, sum_k r_t u k_t, from the raw
         // tiles: a thread takes 16 channels of token k
         wait(&s.full[0], ph);
+        bool odd;                 // an infinite or NaN r or k among those that the thread has seen
         {
             f2 d2 = both(0.f);
 #pragma unroll
@@ -1242,6 +1279,7 @@ mild_compute(const CUtensorMap &map_gr, const CUtensorMap &map_gk, const CUtenso
                     d2 = fma2(mul2(make_float2(a[q], a[q + 1]), make_float2(uq[q], uq[q + 1])), make_float2(d[q], d[q + 1]), d2);
             }
             float diag = d2.x + d2.y;
+            odd = !(fabsf(diag) <= FLT_MAX);
             diag += __shfl_xor_sync(0xffffffffu, diag, 16);
             if (hh == 0) s.dpart[wg][k] = diag;
         }
@@ -1274,12 +1312,17 @@ mild_compute(const CUtensorMap &map_gr, const CUtensorMap &map_gk, const CUtenso
                 c[0] = -c[0];
 #pragma unroll
                 for (int i = 1; i < 16; i++) c[i] = c[i - 1] - c[i];
+                odd |= !(c[15] <= 0.f);
                 // the four runs of 16 tokens of a channel meet
                 s.stot[run4][k] = c[15];
             }
             // the outputs of the chunk before have left their tiles (read below by everyone's writes)
             if (tid == 0) tma_store_wait_read();
-            compute_sync(bar);
+            if (compute_sync_or(odd, bar)) {
+                dead = mild_inputs_again<PER_TOKEN>(s, tmem_addr(tm, lo_lanes, U_WR + tcol), k, t0, P.T - j * CH);
+                if (PER_TOKEN) { tmem_ld16_split32(tmem_addr(tm, lo_lanes, U_WR + tcol), c); tmem_ld_wait(); }
+                compute_sync(bar);
+            }
             tmem_ld16_split32(tmem_addr(tm, hi_lanes, U_WR + tcol), r);
             const float m = rintf(s.cst[ph][0][k]);
             if (PER_TOKEN) {

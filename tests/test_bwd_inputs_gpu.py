@@ -1,0 +1,79 @@
+"""Infinite inputs of the chunked v5/v6 kernels.
+
+The backward kernel reads w, r and k through a product with an identity matrix, in which an infinite element meets the
+zeros of its 15 neighbours."""
+import numpy as np
+import pytest
+import torch
+
+import wkv_testlib as TL
+import test_chunked_gpu as CG
+
+pytestmark = pytest.mark.gpu
+BF = torch.bfloat16
+NAMES = ("gr", "gk", "gv", "gw", "gu", "gstate_in")
+INF = float("inf")
+
+
+def both_paths(variant, x, r, k, v, gy, u, s, gs, w_kind=None):
+    """(y, state_out and gradients) on the chunked and on the token-serial kernels"""
+    W, wkv56 = CG._pkg()
+    w_kind = W.WKV_W_RAW if w_kind is None else w_kind
+    name, out = "wkv6" if variant == "v6" else "wkv5", []
+    for path in (W.WKV_PATH_CHUNKED, W.WKV_PATH_SCALAR):
+        kw = dict(w_kind=w_kind, layout=W.WKV_STATE_KV, path=path)
+        out.append(dict(zip(("y", "state_out"), wkv56.forward(name, r, k, v, x, u, s, **kw)))
+                   | dict(zip(NAMES, wkv56.backward(name, r, k, v, x, u, s, gy, gs, **kw))))
+    return out
+
+
+def normal(g, *shape, std=1.0, mean=0.0, dtype=BF):
+    return (torch.randn(shape, generator=g, device="cuda") * std + mean).to(dtype)
+
+
+# (row, token, channel): the first and last token of a run of 16, of a chunk and of a row, one channel twice
+PLACES = [(0, 0, 3), (0, 17, 3), (0, 31, 64), (0, 63, 5), (1, 64, 70), (1, 100, 70), (1, 108, 70), (1, 199, 127)]
+
+
+@pytest.mark.parametrize("encoding", ["raw", "negexp"])
+def test_infinite_decay_activations(encoding):
+    """x = -inf is a decay of exactly 1, x = +inf the floor; neither has a gradient, and no other token notices"""
+    W, wkv56 = CG._pkg()
+    q = TL.case56("v6", 2, 200, 2, BF, seed=93)
+    for i, at in enumerate(PLACES):
+        q["x"][at] = INF if i % 2 else -INF
+    with np.errstate(over="ignore", divide="ignore", invalid="ignore"):
+        want = CG.floored_oracle("v6", q)
+    d = {n: TL.to_dev(q[n], BF) for n in ("r", "k", "v", "gy", "u")}
+    x = TL.to_dev(q["x"], BF)
+    s, gs = TL.to_dev(q["state_in"], torch.float32), TL.to_dev(q["gstate_out"], torch.float32)
+    if encoding == "negexp":
+        x, kind = -torch.exp(x.float()), W.WKV_W_NEGEXP
+    else:
+        kind = W.WKV_W_RAW
+    got = both_paths("v6", x, d["r"], d["k"], d["v"], d["gy"], d["u"], s, gs, kind)[0]
+    for n in CG.EXTREME_CHECKED:
+        if n != "gw" or encoding == "raw":      # (the literal call's gw is with respect to ew)
+            TL.assert_close(f"v6.{n} {encoding}", got[n], want[n], 2e-2)
+        assert torch.isfinite(got[n].float()).all(), n
+
+
+@pytest.mark.parametrize("which", ["r", "k"])
+def test_an_infinite_element_stays_with_its_own_token(which):
+    """gr does not depend on r nor gk on k; gv depends on r at later tokens and on k at its own"""
+    T, t, g = 192, 83, torch.Generator(device="cuda").manual_seed(94)
+    r, k, v, gy = (normal(g, 1, T, 64) for _ in range(4))
+    x = normal(g, 1, T, 64, std=0.5, mean=-0.6)
+    u, s, gs = normal(g, 1, 64), normal(g, 1, 1, 64, 64, dtype=torch.float32), normal(g, 1, 1, 64, 64, dtype=torch.float32)
+    (r if which == "r" else k)[0, t, 9] = INF
+    got, want = both_paths("v6", x, r, k, v, gy, u, s, gs)
+    keep = torch.ones(T, dtype=torch.bool, device="cuda")
+    keep[t] = False
+    if which == "r":
+        keep[:t] = False          # (those gradients are infinite: the token's output is)
+    own = "gr" if which == "r" else "gk"
+    for n, a, b in ((own, got[own], want[own]), ("gv", got["gv"][:, keep], want["gv"][:, keep])):
+        if n == own:              # the bonus term of the other side's element
+            a, b = a[:, keep], b[:, keep]
+        assert torch.isfinite(b.float()).all(), n
+        TL.assert_close(n, a, TL.back(b), 2e-2)
