@@ -77,3 +77,18 @@ def test_an_infinite_element_stays_with_its_own_token(which):
             a, b = a[:, keep], b[:, keep]
         assert torch.isfinite(b.float()).all(), n
         TL.assert_close(n, a, TL.back(b), 2e-2)
+
+
+@pytest.mark.parametrize("bits", [2.1, 2.8, 3.7, 4.5])
+def test_gradient_of_a_strong_static_decay(bits):
+    """v5's decay gradient is what is left of a sum over all tokens in which large terms cancel; against the token-serial
+    fp32 kernels, the worst of six draws at the bar of every bf16 output"""
+    B, T, H, mean = 1, 330, 2, float(np.log(bits * np.log(2)))
+    for seed in range(6):
+        g = torch.Generator(device="cuda").manual_seed(seed)
+        r, k, v, gy = (normal(g, B, T, 64 * H) for _ in range(4))
+        x, u = normal(g, H, 64, std=0.02, mean=mean, dtype=torch.float32), normal(g, H, 64)
+        s, gs = (normal(g, B, H, 64, 64, dtype=torch.float32) for _ in range(2))
+        got, want = both_paths("v5", x, r, k, v, gy, u, s, gs)
+        for n in got:
+            TL.assert_close(f"v5.{n}", got[n], TL.back(want[n]), 2e-2, extra=f"(bits={bits}, seed={seed})")
