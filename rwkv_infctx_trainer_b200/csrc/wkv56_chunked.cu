@@ -65,7 +65,7 @@ struct FwdSmem {
     uint64_t y_bar;        // tensor core: y of a chunk
     uint32_t tmem_base;
     int abort_flag;        // set by any thread whose bounded wait ran out; ends every other wait
-    int mild_flag[2];      // compute warps -> feeder, by chunk parity: the chunk is mild (see decay_scan8)
+    int mild_flag[2];      // compute warps -> feeder, by chunk parity: the chunk is mild (see chunk_is_mild)
 };
 
 struct FwdParams {
@@ -289,7 +289,7 @@ k_chunk_fwd(const __grid_constant__ CUtensorMap map_r, const __grid_constant__ C
             bool live;
             lwc[ch] = PER_TOKEN ? 0.f : log2_decay(P.wvec[h * 64 + ch0 + ch], P.w_kind, live);
             wc[ch] = exp2f(lwc[ch]);
-            steep_static |= 8.f * lwc[ch] < MILD_L2_PER_8;
+            steep_static |= 64.f * lwc[ch] < MILD_L2;
         }
         // static decay: whether the head's chunks are mild is known once and for all
         const bool mild_static = PER_TOKEN ? false : !compute_sync_or(steep_static);
@@ -327,7 +327,8 @@ k_chunk_fwd(const __grid_constant__ CUtensorMap map_r, const __grid_constant__ C
                         for (int ch = 0; ch < 4; ch++) c[i][ch] = valid ? lwc[ch] : 0.f;
                     }
                 }
-                mild = decay_scan8(c, warp, lane, &s.wtot[0][0], D, other_l2, [](bool p) { return compute_sync_or(p); });
+                decay_scan8(c, warp, lane, &s.wtot[0][0], D, other_l2, [] { compute_sync(); });
+                mild = chunk_is_mild(D, other_l2);
             }
             if (tid == 0) s.mild_flag[j & 1] = mild;
             // The warp reconverges here before it touches the r and k tiles.  The barrier also keeps the

@@ -73,20 +73,12 @@ struct Decay {           // of a thread's 4 tokens x 4 channels
 //
 // In: l2[i][ch] per-token log2-decay.  Out: l2 holds the block-local inclusive sums c; D;
 // other_l2 = log2-decay total of the other block.  The totals of the eight warps go
-// through `wtot` ([8][CH] floats of shared memory); `sync(pred)` is the barrier of the 256 threads,
-// returning the OR of `pred` over them.
-//
-// Returns true when the chunk is "mild": no 8 consecutive tokens decay by more than 2^-28 in any
-// channel, so that the whole chunk can be factored around ONE reference point, half of the chunk's total log-decay
-// (every factor then stays within 2^+-113, which leaves operands 13 bits above the smallest normal number), and the
-// separate treatment of the pairs across the two blocks is not needed.
-constexpr float MILD_L2_PER_8 = -28.f;
+// through `wtot` ([8][CH] floats of shared memory); `sync()` is the barrier of the 256 threads.
 template <class Sync>
-__device__ __forceinline__ bool decay_scan8(float (&l2)[4][4], int warp, int lane, float *wtot, Decay &D,
+__device__ __forceinline__ void decay_scan8(float (&l2)[4][4], int warp, int lane, float *wtot, Decay &D,
                                             float (&other_l2)[4], Sync sync) {
     const int r = lane >> 4, ch0 = (lane & 15) * 4, blk = warp >> 2, wb = warp & 3;
     float tot[4], first[4], o[4];
-    bool steep = false;
 #pragma unroll
     for (int ch = 0; ch < 4; ch++) {
 #pragma unroll
@@ -98,10 +90,8 @@ __device__ __forceinline__ bool decay_scan8(float (&l2)[4][4], int warp, int lan
 #pragma unroll
     for (int ch = 0; ch < 4; ch++) o[ch] = __shfl_xor_sync(0xffffffffu, l2[3][ch], 16);
     vadd<4>(tot, l2[3], o);
-#pragma unroll
-    for (int ch = 0; ch < 4; ch++) steep |= tot[ch] < MILD_L2_PER_8;
     if (r) *reinterpret_cast<float4 *>(wtot + warp * CH + ch0) = make_float4(tot[0], tot[1], tot[2], tot[3]);
-    const bool mild = !sync(steep);
+    sync();
     const float *own = wtot + 4 * blk * CH + ch0, *oth = wtot + 4 * (blk ^ 1) * CH + ch0;
     // what lies in the block before the thread's tokens: its warp's other half and the earlier warps
     float base[4], m[4], e[4];
@@ -136,10 +126,24 @@ __device__ __forceinline__ bool decay_scan8(float (&l2)[4][4], int warp, int lan
         D.m[ch] = m[ch];
         D.e[ch] = e[ch];
     }
-    return mild;
 }
 
-// The same quantities for a static per-channel decay (v5) and a chunk with all 64 tokens in range:
+// Whether the chunk is "mild": no channel decays by more than 2^-128 over the whole of it, so that it can be
+// factored around ONE reference point, half of the chunk's total log-decay, and the separate treatment of the pairs across
+// the two blocks is not needed.  Every factor then stays within 2^+-64.  The line lies there because operands, states and gradients
+// among them, are scaled by these factors, and underflow below 2^-126: values down to 2^-62 (2e-19) keep their digits, those of
+// a mean loss over many tokens and products of two small ones included, and up to 2^63 nothing overflows.  (At 2^+-112 a
+// state of 1e-6 was lost at 3.3 bits of decay per token.)  All threads get the same answer: every warp has
+// summed the eight totals in the same order.
+constexpr float MILD_L2 = -128.f;
+__device__ __forceinline__ bool chunk_is_mild(const Decay &D, const float (&other_l2)[4]) {
+    bool steep = false;
+#pragma unroll
+    for (int ch = 0; ch < 4; ch++) steep |= D.e[ch] + other_l2[ch] < MILD_L2;
+    return !__any_sync(0xffffffffu, steep);
+}
+
+// What decay_scan8 gives, for a static per-channel decay (v5) and a chunk with all 64 tokens in range:
 // every token of channel ch decays by lw[ch] (log2), so nothing has to be scanned or exchanged.
 // w[ch] = 2^{lw[ch]}; tok0 = first of the thread's 4 tokens (0..63).
 __device__ __forceinline__ void decay_static(const float (&lw)[4], const float (&w)[4], int tok0, float (&l2)[4][4],
@@ -180,7 +184,7 @@ __device__ __forceinline__ void st_tile4(Tile &t, int row, int chunk, int half, 
 //                                         times 2^-m: the very operand Rt that the per-chunk backward kernel forms
 //                                         again, so that the large terms of the decay gradient cancel exactly
 //   dchunk  fp32 [B*H, nchunk, 64]        decay of each whole chunk per key channel, see ChunkDecay
-//   mild    u8   [B*H * nchunk]           1 = the chunk is mild (see decay_scan8), 0 = steep: which body of
+//   mild    u8   [B*H * nchunk]           1 = the chunk is mild (see chunk_is_mild), 0 = steep: which body of
 //                                         the per-chunk backward kernel the chunk needs
 // m = c/2 rounded to a whole number, c the log2-decay of the whole chunk: the reference point that a mild chunk is
 // factored around.  The states on either side of the chunk come with it, so that their products share accumulators

@@ -8,7 +8,7 @@
 //      (bf16), E_j = rowsum(S_j * D_j) and the state gradient D_0;
 //   3. k_chunk_bwd handles every (batch, head, chunk) independently from S_j and
 //      D_{j+1}: recomputes the masked scores A, P = gy v^T, and from them the gradients, with every product on
-//      tcgen05.mma.  It has two bodies.  A mild chunk (all chunks of ordinary data, see decay_scan8) is factored
+//      tcgen05.mma.  It has two bodies.  A mild chunk (all chunks of ordinary data, see chunk_is_mild) is factored
 //      around one reference point, see mild_compute.  A steep chunk takes
 //         gv = A^T gy + khat D
 //         gr = fr*(P~d Kt) + g*(P~x X) + e^{cp}*(gy S^T) + p_tt u k
@@ -513,7 +513,7 @@ bwd_steep(const CUtensorMap &map_gr, const CUtensorMap &map_gk, const CUtensorMa
                 }
             }
             // (the barrier inside: every w value has been read, so its slot may take the table)
-            decay_scan8(c, warp, lane, wtot, D, other_l2, [&](bool p) { return compute_sync_or(p, bar); });
+            decay_scan8(c, warp, lane, wtot, D, other_l2, [&] { compute_sync(bar); });
         }
         float before[4];      // log2-decay of the block before the thread's own
 #pragma unroll

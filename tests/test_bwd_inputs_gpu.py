@@ -1,7 +1,7 @@
-"""Infinite inputs of the chunked v5/v6 kernels.
+"""Infinite, small and large inputs of the chunked v5/v6 kernels.
 
 The backward kernel reads w, r and k through a product with an identity matrix, in which an infinite element meets the
-zeros of its 15 neighbours."""
+zeros of its 15 neighbours; states and gradients are scaled by powers of two taken from a mild chunk's decay."""
 import numpy as np
 import pytest
 import torch
@@ -92,3 +92,39 @@ def test_gradient_of_a_strong_static_decay(bits):
         got, want = both_paths("v5", x, r, k, v, gy, u, s, gs)
         for n in got:
             TL.assert_close(f"v5.{n}", got[n], TL.back(want[n]), 2e-2, extra=f"(bits={bits}, seed={seed})")
+
+
+@pytest.mark.parametrize("bits", [1.9, 2.1, 2.8, 3.4, 3.7])
+@pytest.mark.parametrize("kv,gs", [(1, 1e-4), (1, 1e-6), (1, 1e-8), (1e-3, 1), (1e-3, 1e-3), (1e-3, 1e-6), (1e-6, 1), (1, 1e6)])
+@pytest.mark.parametrize("variant", ["v6", "v5"])
+def test_small_and_large_values_at_strong_decay(variant, bits, kv, gs):
+    """`bits` of decay per token on average, k and v of size kv (states kv^2), gradients of size gs: each output against the
+    token-serial fp32 kernels, relative to its own maximum"""
+    B, T, H, g = 1, 330, 2, torch.Generator(device="cuda").manual_seed(95)
+    r, k, v, gy = normal(g, B, T, 64 * H), normal(g, B, T, 64 * H, std=kv), normal(g, B, T, 64 * H, std=kv), normal(g, B, T, 64 * H, std=gs)
+    mean = float(np.log(bits * np.log(2)))
+    x = normal(g, B, T, 64 * H, std=0.02, mean=mean) if variant == "v6" else normal(g, H, 64, std=0.02, mean=mean, dtype=torch.float32)
+    u = normal(g, H, 64)
+    s = normal(g, B, H, 64, 64, std=kv * kv, dtype=torch.float32)
+    gso = normal(g, B, H, 64, 64, std=gs, dtype=torch.float32)
+    got, want = both_paths(variant, x, r, k, v, gy, u, s, gso)
+    for n in got:
+        TL.assert_close(f"{variant}.{n}", got[n], TL.back(want[n]), 2e-2, extra=f"(bits={bits}, kv={kv}, gs={gs})")
+    # what a chunk's first token takes from the carried state
+    first = torch.arange(64, T, 64, device="cuda")
+    TL.assert_close("y at chunk starts", got["y"][:, first], TL.back(want["y"][:, first]), 2e-2)
+
+
+@pytest.mark.parametrize("tokens,kv,gs", [(n, *s) for n in (8, 15, 16, 17) for s in ((1, 1), (1e-3, 1e-6))] + [(24, 1, 1)])
+def test_bursts_of_strong_decay(tokens, kv, gs):
+    """`tokens` of a chunk decay by 5.8 bits each in a few channels, the others by 0.5: on either side of what one
+    reference point takes (128 bits a chunk), however the decay is spread"""
+    B, T, H, g = 1, 320, 2, torch.Generator(device="cuda").manual_seed(96 + tokens)
+    r, k, v, gy = normal(g, B, T, 64 * H), normal(g, B, T, 64 * H, std=kv), normal(g, B, T, 64 * H, std=kv), normal(g, B, T, 64 * H, std=gs)
+    x = normal(g, B, T, 64 * H, std=0.1, mean=-1.1)
+    for chunk, at in ((0, 0), (1, 20), (3, 64 - tokens), (4, 31)):
+        x[:, 64 * chunk + at:64 * chunk + at + tokens, 5::40] = 1.39
+    u, s = normal(g, H, 64), normal(g, B, H, 64, 64, std=kv * kv, dtype=torch.float32)
+    got, want = both_paths("v6", x, r, k, v, gy, u, s, normal(g, B, H, 64, 64, std=gs, dtype=torch.float32))
+    for n in got:
+        TL.assert_close(n, got[n], TL.back(want[n]), 2e-2, extra=f"(tokens={tokens}, kv={kv}, gs={gs})")
