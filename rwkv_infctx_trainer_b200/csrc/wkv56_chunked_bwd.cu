@@ -1593,7 +1593,8 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) k_chunk_bwd(BWD_MAPS, const Bw
     __syncthreads();
     tc_fence_after();
     const uint32_t tm0 = __shfl_sync(0xffffffffu, *tmem_base, 0), tm = tm0 + BWD_TMEM_COLS * grp;
-    const int first = (int)blockIdx.x * BWD_GROUPS + grp, stride = (int)gridDim.x * BWD_GROUPS;
+    // (the CTAs' first groups come first: a call of few chunks has an SM for each, and so has a last round of few)
+    const int first = grp * (int)gridDim.x + (int)blockIdx.x, stride = (int)gridDim.x * BWD_GROUPS;
     const int bar = 1 + grp, bar_all = 1 + BWD_GROUPS + grp;     // named barriers: of the compute warps, of the whole group
     if (feeder) {
         regs_give_up<32>();
@@ -1785,8 +1786,8 @@ int chunked_backward(const wkv_args_t *a0, bool per_token_w, const CallOpts &opt
         auto kern = per_token_w ? k_chunk_bwd<true> : k_chunk_bwd<false>;
         static unsigned char attr_done[2][64];
         if (!set_max_smem_once(kern, (int)smem, attr_done[per_token_w ? 1 : 0])) return WKV_ERR_LAUNCH;
-        if (launch_chained(kern, dim3(std::min((p.total + BWD_GROUPS - 1) / BWD_GROUPS, device_sm_count())), dim3(BWD_THREADS), smem, stream, mr, mk, mv, mw, mgy, ms, md, mgr, mgk, mgv,
-                           mgw, p) != WKV_OK)
+        if (launch_chained(kern, dim3(std::min(p.total, device_sm_count())), dim3(BWD_THREADS), smem, stream, mr, mk, mv, mw, mgy, ms, md, mgr,
+                           mgk, mgv, mgw, p) != WKV_OK)
             return WKV_ERR_LAUNCH;
     }
     // 4. fold the per-chunk partial sums: over the chunks and the batch, or over the chunks alone
