@@ -311,7 +311,6 @@ struct MildSmem {
     uint64_t grad;             // tensor core: gr, gk
     uint64_t gv;               // ... gv
     uint64_t epi;              // compute warps: gr, gk and the turned inputs have been read
-    uint32_t tmem_base;
     int abort_flag;            // set by any thread whose bounded wait ran out; ends every other wait
 };
 
@@ -1567,7 +1566,8 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) k_chunk_bwd(BWD_MAPS, const Bw
     const int grp = feeder ? warp_id & 1 : warp_id >> 3, warp = warp_id & 7;
     unsigned char *mem = smem_raw + grp * BWD_SMEM;
     MildSmem &s = *reinterpret_cast<MildSmem *>(mem);
-    uint32_t *tmem_base = &reinterpret_cast<MildSmem *>(smem_raw)->tmem_base;
+    // (behind both groups' memory, of which each makes another use once its mild chunks are done)
+    uint32_t *tmem_base = reinterpret_cast<uint32_t *>(smem_raw + BWD_GROUPS * BWD_SMEM);
 
     // the swizzled tiles need a 1024-byte aligned base; refuse to run otherwise
     if ((smem_u32(smem_raw) & 1023u) != 0) {
@@ -1782,7 +1782,7 @@ int chunked_backward(const wkv_args_t *a0, bool per_token_w, const CallOpts &opt
         p.wait_limit = opt.wait_limit;
         p.skip_load = opt.kernel == 2 ? opt.skip_load : -1;
         p.mildflag = (const unsigned char *)(fwd_ck + CL.mild);
-        const size_t smem = BWD_SMEM * BWD_GROUPS;
+        const size_t smem = BWD_SMEM * BWD_GROUPS + 16;     // (and the tensor memory's address)
         auto kern = per_token_w ? k_chunk_bwd<true> : k_chunk_bwd<false>;
         static unsigned char attr_done[2][64];
         if (!set_max_smem_once(kern, (int)smem, attr_done[per_token_w ? 1 : 0])) return WKV_ERR_LAUNCH;
