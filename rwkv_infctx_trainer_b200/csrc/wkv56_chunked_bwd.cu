@@ -966,6 +966,7 @@ bwd_steep(const CUtensorMap &map_gr, const CUtensorMap &map_gk, const CUtensorMa
     if (abort3 && tid == 0) {
         // every warp has arrived on every barrier: whatever was issued is done once they complete
         mbar_wait(&s.bar_early, ph); mbar_wait(&s.bar_score, ph); mbar_wait(&s.bar_grad, ph); mbar_wait(&s.bar_gv, ph);
+        if (j != P.skip_load) mbar_wait(&s.load_bar, ph, 200000u);
         if (P.status) atomicOr(P.status, 4);
     }
     return abort3 == 0;
@@ -1081,6 +1082,7 @@ mild_feed(const CUtensorMap &map_r, const CUtensorMap &map_k, const CUtensorMap 
         const bool more = next >= 0 && !skip(next);
         const At x = at(next >= 0 ? next : chunk);
         int stage = 0;       // barriers committed to
+        bool all = !more;    // the next chunk's loads have all been issued
         // operand descriptors: that of the structure's first tile plus an offset
         const uint64_t d0 = make_desc(smem_u32(&s));
         auto kmaj = [&](uint32_t off, int k16) { return d0 + ((off + 32 * k16) >> 4); };
@@ -1158,6 +1160,7 @@ mild_feed(const CUtensorMap &map_r, const CUtensorMap &map_k, const CUtensorMap 
             stage = 4;
             if (!wait(&s.gv, ph)) break;
             if (more && elect_one()) load1b(x);
+            all = true;
             if (!wait(&s.epi, ph)) break;
             tc_fence_after();
             stage = 5;
@@ -1170,9 +1173,11 @@ mild_feed(const CUtensorMap &map_r, const CUtensorMap &map_k, const CUtensorMap 
             uint64_t *last[5] = {nullptr, &s.turned, &s.early, &s.score, &s.gv};
             for (int q = 1; q <= stage; q++) mbar_wait(last[q], ph, 200000u);
             if (more && stage >= 3) {
-                // (those of the next chunk; the second group may be short of two loads and never complete)
+                // (those of the next chunk: the second group is short of two loads if the wait for gv ran out, and would
+                // never complete)
                 mbar_wait(&s.full[0], ph ^ 1, 200000u);
-                if (stage == 4) mbar_wait(&s.full[1], ph ^ 1, 20000u);
+                if (stage == 4 && !all && elect_one()) load1b(x);
+                if (stage == 4) mbar_wait(&s.full[1], ph ^ 1, 200000u);
             }
         }
         loads = more;
