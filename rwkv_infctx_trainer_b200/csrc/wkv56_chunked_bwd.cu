@@ -441,7 +441,8 @@ bwd_steep(const CUtensorMap &map_gr, const CUtensorMap &map_gk, const CUtensorMa
     // The products that need only the raw tiles go to the tensor core before the operand pass
     // (a tcgen05.mma is issued by one thread and costs it ~100 cycles of descriptor arithmetic:
     // the accumulators of a group go out from different warps at once).
-    if (lane == 0) {
+    __syncwarp();
+    if (elect_one()) {
         const uint32_t id64 = make_idesc(64, 64, false, false), id32 = make_idesc(64, 32, false, false);
         if (!fail) {
             if (warp == 0) {
@@ -585,7 +586,8 @@ bwd_steep(const CUtensorMap &map_gr, const CUtensorMap &map_gk, const CUtensorMa
     const int abort1 = compute_sync_or(fail, bar);
 
     // ------------------------------------------------- phase 1: the scores A1, A2
-    if (lane == 0) {
+    __syncwarp();
+    if (elect_one()) {
         if (!abort1) {
             tc_fence_after();
             if (warp == 0) {
@@ -693,7 +695,8 @@ bwd_steep(const CUtensorMap &map_gr, const CUtensorMap &map_gk, const CUtensorMa
     // every accumulator is [token, 32 channels]: channels 0..31 in the lo lanes, 32..63 in the hi lanes
     // gv is needed last: it goes to a barrier of its own, from the two warps that have no gradient
     // product to issue (so that no warp enters the epilogue later than the others).
-    if (lane == 0) {
+    __syncwarp();
+    if (elect_one()) {
         tc_fence_after();
         const uint32_t id_kn = make_idesc(64, 32, false, true), id_nn = make_idesc(64, 32, true, true);
         const int hf = warp & 1;
