@@ -8,24 +8,25 @@
 namespace wkv {
 namespace {
 
-// One CTA per (head, parameter): 64 groups of 16 threads (four channels each) take every 64th of the
+// One CTA per (head, parameter): GROUPS groups of 16 threads (four channels each) take every GROUPS-th of the
 // B*n rows, the groups meet in shared memory in a fixed order.  Latency-bound (a few hundred KB from
 // L2): the width is there to have all loads of a few thousand tokens in flight at once (4 rows of 64 chunks x 64 heads:
 // 7.5 us with 16 groups of one channel a thread and a division per row, 4.8 with this).
-__global__ void __launch_bounds__(1024)
+template <int GROUPS>
+__global__ void __launch_bounds__(16 * GROUPS)
 k_fold_heads(const float *__restrict__ gu_part, const float *__restrict__ gw_part, void *gu, int gu_dtype, void *gw,
              int gw_dtype, int B, int H, int n) {
     pdl_wait();
     pdl_trigger();
-    __shared__ __align__(16) float red[64][64];
+    __shared__ __align__(16) float red[GROUPS][64];
     __shared__ float red2[16][64];
     const int h = blockIdx.x, q = threadIdx.x & 15, g = threadIdx.x >> 4;
     const float *part = (blockIdx.y ? gw_part : gu_part) + (size_t)h * n * 64 + 4 * q;
     float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
     int b = g / n, j = g - b * n;
-    const int step_b = 64 / n, step_j = 64 - step_b * n;
+    const int step_b = GROUPS / n, step_j = GROUPS - step_b * n;
 #pragma unroll 4
-    for (int i = g; i < B * n; i += 64) {
+    for (int i = g; i < B * n; i += GROUPS) {
         const float4 v = *reinterpret_cast<const float4 *>(part + ((size_t)b * H * n + j) * 64);
         acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
         b += step_b;
@@ -35,22 +36,30 @@ k_fold_heads(const float *__restrict__ gu_part, const float *__restrict__ gw_par
     *reinterpret_cast<float4 *>(&red[g][4 * q]) = acc;
     __syncthreads();
     const int k = threadIdx.x & 63, p = threadIdx.x >> 6;
-    red2[p][k] = (red[4 * p][k] + red[4 * p + 1][k]) + (red[4 * p + 2][k] + red[4 * p + 3][k]);
-    __syncthreads();
+    if (GROUPS > 16) {
+        red2[p][k] = (red[4 * p][k] + red[4 * p + 1][k]) + (red[4 * p + 2][k] + red[4 * p + 3][k]);
+        __syncthreads();
+    }
     if (p == 0) {
-        float t = red2[0][k];
+        const float(*r)[64] = GROUPS > 16 ? red2 : red;
+        float t = r[0][k];
 #pragma unroll
-        for (int i = 1; i < 16; i++) t += red2[i][k];
+        for (int i = 1; i < 16; i++) t += r[i][k];
         if (blockIdx.y) store_as(gw, gw_dtype, h * 64 + k, t);
         else store_as(gu, gu_dtype, h * 64 + k, t);
     }
 }
 
+// Up to a row for each of 16 groups: those alone, which start sooner and meet in one step (2, 8 and 16 rows: 2.95 us, with 64
+// groups 3.26; 24 and 32 rows: 3.6 and 3.8, with 64 groups 3.5 and 3.6).
+constexpr int FOLD_FEW_ROWS = 16;
+
 }  // namespace
 
 int fold_param_grads(const float *gu_part, const float *gw_part, int B, int H, int n, const CallOpts &opt, cudaStream_t s) {
-    return launch_chained(k_fold_heads, dim3(H, gw_part ? 2 : 1), dim3(1024), 0, s, gu_part, gw_part, opt.gu_sum,
-                          opt.gu_dtype, opt.gw_sum, opt.gw_dtype, B, H, n);
+    const bool few = (size_t)B * n <= FOLD_FEW_ROWS;
+    return launch_chained(few ? k_fold_heads<16> : k_fold_heads<64>, dim3(H, gw_part ? 2 : 1), dim3(few ? 256 : 1024), 0, s, gu_part,
+                          gw_part, opt.gu_sum, opt.gu_dtype, opt.gw_sum, opt.gw_dtype, B, H, n);
 }
 
 }  // namespace wkv
