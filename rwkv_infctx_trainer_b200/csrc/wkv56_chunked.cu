@@ -283,16 +283,12 @@ k_chunk_fwd(const __grid_constant__ CUtensorMap map_r, const __grid_constant__ C
         }
         float dprod = 1.f;      // summary pass: decay of the whole group for key channel `row`
         float lwc[4], wc[4];
-        bool steep_static = false;
 #pragma unroll
         for (int ch = 0; ch < 4; ch++) {
             bool live;
             lwc[ch] = PER_TOKEN ? 0.f : log2_decay(P.wvec[h * 64 + ch0 + ch], P.w_kind, live);
             wc[ch] = exp2f(lwc[ch]);
-            steep_static |= 64.f * lwc[ch] < MILD_L2;
         }
-        // static decay: whether the head's chunks are mild is known once and for all
-        const bool mild_static = PER_TOKEN ? false : !compute_sync_or(steep_static);
 
         // Operand pass for chunk j: scaled r/k tiles in place in stage j&1, x, khat[j&1], the
         // score-diagonal partials and the chunk decay.  Contains one barrier of the compute warps.
@@ -303,11 +299,9 @@ k_chunk_fwd(const __grid_constant__ CUtensorMap map_r, const __grid_constant__ C
             float c[4][4];
             Decay D;
             float other_l2[4];
-            bool mild;
             if (!PER_TOKEN && (jg + 1) * CH <= P.T) {
                 // static decay, whole chunk in range: closed form, nothing to scan or exchange
                 decay_static(lwc, wc, tok0, c, D, other_l2);
-                mild = mild_static;
             } else {
 #pragma unroll
                 for (int i = 0; i < 4; i++) {
@@ -328,8 +322,8 @@ k_chunk_fwd(const __grid_constant__ CUtensorMap map_r, const __grid_constant__ C
                     }
                 }
                 decay_scan8(c, warp, lane, &s.wtot[0][0], D, other_l2, [] { compute_sync(); });
-                mild = chunk_is_mild(D, other_l2);
             }
+            const bool mild = chunk_is_mild(D, other_l2);
             if (tid == 0) s.mild_flag[j & 1] = mild;
             // The warp reconverges here before it touches the r and k tiles.  The barrier also keeps the
             // tile loads below the decay scan: hoisted above it they push the pass over the 96 registers
