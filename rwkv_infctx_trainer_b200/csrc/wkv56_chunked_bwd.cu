@@ -28,6 +28,7 @@
 #include <algorithm>
 #include <cfloat>
 #include <cstddef>
+#include <type_traits>
 
 #include "wkv56_chunked.cuh"
 
@@ -775,10 +776,10 @@ bwd_steep(const CUtensorMap &map_gr, const CUtensorMap &map_gk, const CUtensorMa
     // The decay gradient of token t is  glw_t = K_j + sum_{t'<=t} (a_t' + b_t') - b_t  with
     //   a_t = -(qrS_t + qrI_t)   (gr side),     b_t = qkD_t + qkI_t   (gk side),
     // qrS/qkD the state parts of r*gr and k*gk and qrI/qkI their intra-chunk parts (file header).
-    // One code for both sides (compiled for each, it needs more registers than there are): sg = 1 for gr, -1 for gk.
-    {
-        const bool GR = wg == 0;
-        const float sg = GR ? 1.f : -1.f;
+    // Compiled for each side.  (One code for both, with 8-byte accesses of the tiles: an all-steep 7B segment 865 us, this 822.)
+    auto side_pass = [&](auto side) {
+        constexpr bool GR = decltype(side)::value;
+        constexpr float sg = GR ? 1.f : -1.f;
         const bool has2 = GR == (w4 >= 2);                    // the cross-block accumulator covers this token
         const Tile &t_own = GR ? s.rt : s.kt;
         const Tile &t_raw = GR ? s.in[T_R] : s.in[T_K], &t_oth = GR ? s.in[T_K] : s.in[T_R];
@@ -787,68 +788,81 @@ bwd_steep(const CUtensorMap &map_gr, const CUtensorMap &map_gk, const CUtensorMa
         Tile &exch = GR ? s.in[T_S] : s.ptil;                 // what the other group needs from this one
         const int zrow = GR ? t - 1 : t;                      // gr factors use c_{t-1}, gk factors c_t
         const int mrow = t < HB ? 15 : 47;                    // row of the table that holds the reference point
-        // four channels at a time: 4 c4 .. +3
+        // four channels at a time: 4 c4 .. +3; the tiles 16 bytes at a time (8-byte accesses of a column of rows find half
+        // of the banks)
 #pragma unroll 1
-        for (int bt = 0; bt < 8; bt++) {
-            const int c4 = 8 * hh + bt, c8 = c4 >> 1, half = bt & 1;
-            float g1[4], gs[4], g2[4];
-            tmem_ld4(tmem_addr(tm, lane_base, cG1 + 4 * bt), g1);
-            tmem_ld4(tmem_addr(tm, lane_base, cGS + 4 * bt), gs);
-            if (has2) tmem_ld4(tmem_addr(tm, lane_base, cG2 + 4 * bt), g2);
-            auto get4 = [](float *v, const float4 &f) { v[0] = f.x; v[1] = f.y; v[2] = f.z; v[3] = f.w; };
-            float own[4], raw[4], oth[4], uu[4], z[4], f1[4], fS[4], out[4], ab[4];
-            get4(z, zrow >= 0 ? *ctab_ptr4(ct_lo, ct_hi, zrow, c4) : make_float4(0.f, 0.f, 0.f, 0.f));
-            get4(f1, *ctab_ptr4(ct_lo, ct_hi, mrow, c4));
-            get4(fS, *ctab_ptr4(ct_lo, ct_hi, 63, c4));
-            get4(uu, *reinterpret_cast<const float4 *>(s.uf + 4 * c4));
-            unpack4(ld_tile4(t_own, t, c8, half), own);
-            unpack4(ld_tile4(t_raw, t, c8, half), raw);
-            unpack4(ld_tile4(t_oth, t, c8, half), oth);
-            tmem_ld_wait();
+        for (int bt8 = 0; bt8 < 4; bt8++) {
+            const int c8 = 4 * hh + bt8;
+            const uint4 own8 = ld_tile(t_own, t, c8), raw8 = ld_tile(t_raw, t, c8), oth8 = ld_tile(t_oth, t, c8);
+            uint4 out8;
 #pragma unroll
-            for (int q = 0; q < 4; q++) {
-                f1[q] = exp2f(sg * (z[q] - f1[q]));
-                fS[q] = exp2f(GR ? z[q] : fS[q] - z[q]);
-            }
-            // (the r side's state part from r e^{cp} as the dS scan had it, rounded: E_j then cancels against it.  Unrounded,
-            // the sum over the tokens that is a static decay's gradient was 2 to 4 % off, with it 0.3)
-            vmul<4>(ab, raw, fS);
-            if (GR) unpack4(pack4(ab), ab);
-            vmul<4>(ab, ab, gs);
-            vmul<4>(fS, fS, gs);
-            vfma<4>(out, f1, g1, fS);
-            vfma<4>(ab, own, g1, ab);
-            vmul<4>(uu, uu, oth);
-            vaxpy<4>(out, ptt_t, uu, out);
-            if (has2) {
-                float xx[4], e0r[4];
-                unpack4(ld_tile4(s.x, t, c8, half), xx);
-                get4(e0r, *ctab_ptr4(ct_lo, ct_hi, 31, c4));
+            for (int half = 0; half < 2; half++) {
+                const int bt = 2 * bt8 + half, c4 = 8 * hh + bt;
+                auto of8 = [&](const uint4 &q) { return half ? make_uint2(q.z, q.w) : make_uint2(q.x, q.y); };
+                float g1[4], gs[4], g2[4];
+                tmem_ld4(tmem_addr(tm, lane_base, cG1 + 4 * bt), g1);
+                tmem_ld4(tmem_addr(tm, lane_base, cGS + 4 * bt), gs);
+                if (has2) tmem_ld4(tmem_addr(tm, lane_base, cG2 + 4 * bt), g2);
+                auto get4 = [](float *v, const float4 &f) { v[0] = f.x; v[1] = f.y; v[2] = f.z; v[3] = f.w; };
+                float own[4], raw[4], oth[4], uu[4], z[4], f1[4], fS[4], out[4], ab[4];
+                get4(z, zrow >= 0 ? *ctab_ptr4(ct_lo, ct_hi, zrow, c4) : make_float4(0.f, 0.f, 0.f, 0.f));
+                get4(f1, *ctab_ptr4(ct_lo, ct_hi, mrow, c4));
+                get4(fS, *ctab_ptr4(ct_lo, ct_hi, 63, c4));
+                get4(uu, *reinterpret_cast<const float4 *>(s.uf + 4 * c4));
+                unpack4(of8(own8), own);
+                unpack4(of8(raw8), raw);
+                unpack4(of8(oth8), oth);
+                tmem_ld_wait();
 #pragma unroll
                 for (int q = 0; q < 4; q++) {
-                    out[q] += exp2f(sg * (z[q] - e0r[q])) * g2[q];
-                    ab[q] += xx[q] * g2[q];
+                    f1[q] = exp2f(sg * (z[q] - f1[q]));
+                    fS[q] = exp2f(GR ? z[q] : fS[q] - z[q]);
+                }
+                // (the r side's state part from r e^{cp} as the dS scan had it, rounded: E_j then cancels against it.  Unrounded,
+                // the sum over the tokens that is a static decay's gradient was 2 to 4 % off, with it 0.5)
+                vmul<4>(ab, raw, fS);
+                if (GR) unpack4(pack4(ab), ab);
+                vmul<4>(ab, ab, gs);
+                vmul<4>(fS, fS, gs);
+                vfma<4>(out, f1, g1, fS);
+                vfma<4>(ab, own, g1, ab);
+                vmul<4>(uu, uu, oth);
+                vaxpy<4>(out, ptt_t, uu, out);
+                if (has2) {
+                    float xx[4], e0r[4];
+                    unpack4(ld_tile4(s.x, t, c8, half), xx);
+                    get4(e0r, *ctab_ptr4(ct_lo, ct_hi, 31, c4));
+#pragma unroll
+                    for (int q = 0; q < 4; q++) {
+                        out[q] += exp2f(sg * (z[q] - e0r[q])) * g2[q];
+                        ab[q] += xx[q] * g2[q];
+                    }
+                }
+                {
+                    const uint2 o = pack4(out);
+                    if (half) { out8.z = o.x; out8.w = o.y; } else { out8.x = o.x; out8.y = o.y; }
+                }
+#pragma unroll
+                for (int q = 0; q < 4; q++) ab[q] *= -sg;
+                if (GR == (bt < 4)) {       // kept, in columns that have just been read
+                    tmem_st4(tmem_addr(tm, lane_base, cGS + 4 * bt), ab);
+                } else {
+                    *reinterpret_cast<float4 *>(exch.b + tile_off(t, 4 * hh + (bt & 3))) = make_float4(ab[0], ab[1], ab[2], ab[3]);
+                }
+                if (!GR) {
+                    // gu: sum over this warp's 16 tokens of p_tt r k, by a halving exchange
+                    float gue[4];
+#pragma unroll
+                    for (int q = 0; q < 4; q++) gue[q] = ptt_t * raw[q] * oth[q];
+                    const float tot = halving_sum4(gue, l16);
+                    if ((l16 & 3) == 0) gup[w4 * CH + 4 * c4 + (l16 >> 2)] = tot;
                 }
             }
-            st_tile4(o_main, t, c8, half, pack4(out));
-#pragma unroll
-            for (int q = 0; q < 4; q++) ab[q] *= -sg;
-            if (GR == (bt < 4)) {       // kept, in columns that have just been read
-                tmem_st4(tmem_addr(tm, lane_base, cGS + 4 * bt), ab);
-            } else {
-                *reinterpret_cast<float4 *>(exch.b + tile_off(t, 4 * hh + (bt & 3))) = make_float4(ab[0], ab[1], ab[2], ab[3]);
-            }
-            if (!GR) {
-                // gu: sum over this warp's 16 tokens of p_tt r k, by a halving exchange
-                float gue[4];
-#pragma unroll
-                for (int q = 0; q < 4; q++) gue[q] = ptt_t * raw[q] * oth[q];
-                const float tot = halving_sum4(gue, l16);
-                if ((l16 & 3) == 0) gup[w4 * CH + 4 * c4 + (l16 >> 2)] = tot;
-            }
+            st_tile(o_main, t, c8, out8);
         }
         tmem_st_wait();
-    }
+    };
+    if (wg == 0) side_pass(std::true_type{}); else side_pass(std::false_type{});
     {
         // gv: accumulator [s, v]; each group takes half of the columns
         if (!abort2 && !mbar_wait(&s.bar_gv, ph, LIM)) fail = 1;
