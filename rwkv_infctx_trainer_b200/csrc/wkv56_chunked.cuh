@@ -181,8 +181,10 @@ __device__ __forceinline__ void st_tile4(Tile &t, int row, int chunk, int half, 
 //   sck     bf16 [B*H, nchunk+1, 64, 64]  state at the start of every chunk (key rows, value columns); of a mild
 //                                         chunk times 2^m per key row
 //   rhat    bf16 [B, T, C]                r_t * (decay accumulated from the chunk start to before t); of a mild chunk
-//                                         times 2^-m: the very operand Rt that the per-chunk backward kernel forms
-//                                         again, so that the large terms of the decay gradient cancel exactly
+//                                         times 2^-m: the operand Rt that the per-chunk backward kernel forms again, so
+//                                         that the large terms of the decay gradient cancel.  (Not bit by bit: the two sum
+//                                         the log-decays in another order, and about one element in 6000 is rounded to
+//                                         the other side.)
 //   dchunk  fp32 [B*H, nchunk, 64]        decay of each whole chunk per key channel, see ChunkDecay
 //   mild    u8   [B*H * nchunk]           1 = the chunk is mild (see chunk_is_mild), 0 = steep: which body of
 //                                         the per-chunk backward kernel the chunk needs

@@ -789,11 +789,11 @@ bwd_steep(const CUtensorMap &map_gr, const CUtensorMap &map_gk, const CUtensorMa
         const int zrow = GR ? t - 1 : t;                      // gr factors use c_{t-1}, gk factors c_t
         const int mrow = t < HB ? 15 : 47;                    // row of the table that holds the reference point
         // four channels at a time: 4 c4 .. +3; the tiles 16 bytes at a time (8-byte accesses of a column of rows find half
-        // of the banks)
+        // of the banks), but for one of the three: its registers would be spilled
 #pragma unroll 1
         for (int bt8 = 0; bt8 < 4; bt8++) {
             const int c8 = 4 * hh + bt8;
-            const uint4 own8 = ld_tile(t_own, t, c8), raw8 = ld_tile(t_raw, t, c8), oth8 = ld_tile(t_oth, t, c8);
+            const uint4 own8 = ld_tile(t_own, t, c8), raw8 = ld_tile(t_raw, t, c8);
             uint4 out8;
 #pragma unroll
             for (int half = 0; half < 2; half++) {
@@ -811,7 +811,7 @@ bwd_steep(const CUtensorMap &map_gr, const CUtensorMap &map_gk, const CUtensorMa
                 get4(uu, *reinterpret_cast<const float4 *>(s.uf + 4 * c4));
                 unpack4(of8(own8), own);
                 unpack4(of8(raw8), raw);
-                unpack4(of8(oth8), oth);
+                unpack4(ld_tile4(t_oth, t, c8, half), oth);
                 tmem_ld_wait();
 #pragma unroll
                 for (int q = 0; q < 4; q++) {
@@ -1004,16 +1004,16 @@ bwd_steep(const CUtensorMap &map_gr, const CUtensorMap &map_gk, const CUtensorMa
 // decay gradient are then serial code on registers, with no shuffles, no table of sums and nothing to read again
 // by other threads (77 instructions per 32 elements, where threads of 4 x 4 elements and of one token took 129).
 // Inputs come [token][channel]; the tensor core turns them: w, r, k times a 16 x 16 identity, exact in
-// fp32, and a thread reads its 16 values with one tcgen05.ld.  (An infinite one, times the identity's zeros, spoils the
-// other 15 of its run: those are then read from the tile, element by element.)  All accumulators are [channel][token] likewise, read
-// by the 16-lane load (tmem_ld16_split32), which covers an M = 64, N = 64 accumulator with all threads: no product
+// fp32, and a thread reads its 16 values with one tcgen05.ld.  (An infinite one, times the identity's zeros, spoils
+// the other 15 of its run: the chunk is then read from the tiles, see mild_inputs_again.)  All accumulators are
+// [channel][token] likewise, read by the 16-lane load (tmem_ld16_split32), which covers an M = 64, N = 64 accumulator with all threads: no product
 // is cut into column halves.  gr, gk and gw go back to [token][channel] by 2-byte stores.
 //
 // Eight compute warps (w4 = warp & 3: channels 16 w4 .. +15; lane & 15: the channel; tokens 32 (lane >> 4) +
 // 16 (warp >> 2) .. +15) walk over the group's chunks, and a feeder warp issues every load, a chunk ahead, and every
 // tcgen05.mma.  (One chunk per CTA, two CTAs on an SM: of 15.6 k cycles per chunk 8 k went to the start of the CTA, its
 // first loads and the drain of its stores.)
-// 4 rows of 4096 tokens x 64 heads: 505 us with one CTA per chunk and the 4 x 4 threads, 400 with this arithmetic, 300
+// 4 rows of 4096 tokens x 64 heads: 505 us with one CTA per chunk and the 4 x 4 threads, 400 with this arithmetic, 304
 // with both; what is left is spread over waits for products (2.3 k of 9.1 k cycles per chunk and group), issue (50 %)
 // and shared memory (46 % of its cycles).
 //
