@@ -1002,7 +1002,7 @@ bwd_steep(const CUtensorMap &map_gr, const CUtensorMap &map_gk, const CUtensorMa
 // What bounds a chunk's CUDA-core work is the number of instructions, so everything elementwise is done by threads
 // that own one channel and 16 consecutive tokens: the decay sums, the factors, the gradients and the token scan of the
 // decay gradient are then serial code on registers, with no shuffles, no table of sums and nothing to read again
-// by other threads (77 instructions per 32 elements, where threads of 4 x 4 elements and of one token took 129).
+// by other threads (78 instructions per 32 elements, where threads of 4 x 4 elements and of one token took 129).
 // Inputs come [token][channel]; the tensor core turns them: w, r, k times a 16 x 16 identity, exact in
 // fp32, and a thread reads its 16 values with one tcgen05.ld.  (An infinite one, times the identity's zeros, spoils
 // the other 15 of its run: the chunk is then read from the tiles, see mild_inputs_again.)  All accumulators are
