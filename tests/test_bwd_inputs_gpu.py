@@ -58,15 +58,30 @@ def test_infinite_decay_activations(encoding):
         assert torch.isfinite(got[n].float()).all(), n
 
 
+def test_a_nan_decay_activation_is_the_floor():
+    """as x = +inf is, in the forward and in the backward pass"""
+    g = torch.Generator(device="cuda").manual_seed(97)
+    r, k, v, gy = (normal(g, 1, 150, 64) for _ in range(4))
+    x, u = normal(g, 1, 150, 64, std=0.5, mean=-0.6), normal(g, 1, 64)
+    s, gs = normal(g, 1, 1, 64, 64, dtype=torch.float32), normal(g, 1, 1, 64, 64, dtype=torch.float32)
+    runs = []
+    for value in (float("nan"), INF):
+        x[0, 70, 11] = x[0, 149, 63] = value
+        runs.append(both_paths("v6", x, r, k, v, gy, u, s, gs)[0])
+    for n in runs[0]:
+        assert torch.isfinite(runs[0][n].float()).all() and torch.equal(runs[0][n], runs[1][n]), n
+
+
+@pytest.mark.parametrize("variant", ["v6", "v5"])
 @pytest.mark.parametrize("which", ["r", "k"])
-def test_an_infinite_element_stays_with_its_own_token(which):
+def test_an_infinite_element_stays_with_its_own_token(which, variant):
     """gr does not depend on r nor gk on k; gv depends on r at later tokens and on k at its own"""
     T, t, g = 192, 83, torch.Generator(device="cuda").manual_seed(94)
     r, k, v, gy = (normal(g, 1, T, 64) for _ in range(4))
-    x = normal(g, 1, T, 64, std=0.5, mean=-0.6)
+    x = normal(g, 1, T, 64, std=0.5, mean=-0.6) if variant == "v6" else normal(g, 1, 64, mean=-3, dtype=torch.float32)
     u, s, gs = normal(g, 1, 64), normal(g, 1, 1, 64, 64, dtype=torch.float32), normal(g, 1, 1, 64, 64, dtype=torch.float32)
     (r if which == "r" else k)[0, t, 9] = INF
-    got, want = both_paths("v6", x, r, k, v, gy, u, s, gs)
+    got, want = both_paths(variant, x, r, k, v, gy, u, s, gs)
     keep = torch.ones(T, dtype=torch.bool, device="cuda")
     keep[t] = False
     if which == "r":
